@@ -832,7 +832,7 @@ static int prepare_run(lgpu_handle *h, ObsSorted &os, int &launches) {
 }
 
 static int learned_run(lgpu_handle *h);
-static int eig_scratch(lgpu_handle *h, int units, EigSplit &sp, int &batch);
+static int eig_scratch(lgpu_handle *h, int units, EigArgs &ea, EigSplit &sp, int &batch);
 static UpdateArgs update_args(lgpu_handle *h);
 
 // FP32_RESOLVE: the run's list of units for the FP64 re-solve, counters
@@ -856,28 +856,30 @@ static void flag_args(lgpu_handle *h, EigArgs &ea) {
   ea.flag_cap = 2 * std::max(1, h->nunits);
 }
 
-// eigensolve scratch of the split pipeline for `units` units (at most 8 GB,
-// units in batches); batch = 0 when it cannot be had (the fused kernel runs)
-static int eig_scratch(lgpu_handle *h, int units, EigSplit &sp, int &batch) {
+// scratch of the transforms of `units` units: the reflectors of the units in
+// flight, and with FP32_RESOLVE the gap test (at most 8 GB, units in batches)
+static int eig_scratch(lgpu_handle *h, int units, EigArgs &ea, EigSplit &sp, int &batch) {
+  sp = EigSplit{};
+  batch = std::max(1, units);
   const int k = h->k;
-  const size_t per = eig_split_bytes_per_unit(k);
-  const size_t budget = (size_t)8 << 30;
-  batch = (int)std::min<size_t>((size_t)std::max(1, units), std::max<size_t>(1024, budget / per));
-  const size_t need = per * (size_t)batch + 5 * 256;
-  if (h->buf[B_EIGSCR].cap >= need || h->buf[B_EIGSCR].ensure(need) == cudaSuccess) {
-    unsigned char *base = h->buf[B_EIGSCR].as<unsigned char>();
-    size_t off = 0;
-    auto take = [&](size_t bytes) { unsigned char *p = base + off; off += (bytes + 255) & ~(size_t)255; return p; };
-    sp.Q = reinterpret_cast<float *>(take((size_t)batch * k * k * 4));
-    sp.DE = reinterpret_cast<float *>(take((size_t)batch * 2 * k * 4));
-    sp.log = reinterpret_cast<float2 *>(take((size_t)batch * eig_log_cap(k) * 8));
-    sp.logn = reinterpret_cast<int *>(take((size_t)batch * 4));
-    sp.lam = reinterpret_cast<float *>(take((size_t)batch * k * 4));
-    sp.cap = eig_log_cap(k);
-  } else {
-    cudaGetLastError();   // clear the failed allocation
-    batch = 0;
+  const bool resolve = h->prec == LGPU_PREC_FP32_RESOLVE;
+  const size_t vb = eig_scratch_bytes(k, std::max(1, units), h->prec != LGPU_PREC_FP64, h->prec != LGPU_PREC_FP32);
+  size_t need = vb + 256;
+  if (resolve) {
+    const size_t per = eig_split_bytes_per_unit(k);
+    const size_t budget = (size_t)8 << 30;
+    batch = (int)std::min<size_t>((size_t)batch, std::max<size_t>(1024, budget / per));
+    need += per * (size_t)batch + 3 * 256;
   }
+  CK(h->buf[B_EIGSCR].ensure(need), "alloc transform scratch");
+  unsigned char *base = h->buf[B_EIGSCR].as<unsigned char>();
+  size_t off = 0;
+  auto take = [&](size_t bytes) { unsigned char *p = base + off; off += (bytes + 255) & ~(size_t)255; return p; };
+  ea.scratch = take(vb);
+  if (!resolve) return LGPU_OK;
+  sp.DE = reinterpret_cast<float *>(take((size_t)batch * 2 * k * 4));
+  sp.lam = reinterpret_cast<float *>(take((size_t)batch * k * 4));
+  sp.bad = reinterpret_cast<int *>(take((size_t)batch * 4));
   return LGPU_OK;
 }
 
@@ -1241,14 +1243,15 @@ static int solver_run(lgpu_handle *h) {
   if ((rc = flag_prepare(h)) != LGPU_OK) return rc;
   flag_args(h, ea);
   const bool fp64 = h->prec == LGPU_PREC_FP64;
-  // eigensolve scratch: the split pipeline (at most 8 GB, units in batches);
-  // the fused one-warp kernel over all units if the scratch cannot be had
-  // (no FP64 re-solve then)
-  EigSplit sp;
+  // FP32 solutions that become training rows keep their own form
+  const bool rows = ea.wbar && h->prec == LGPU_PREC_FP32;
+  EigSplit sp{};
   int batch = 0;
-  if (!fp64) {
-    if ((rc = eig_scratch(h, h->nunits, sp, batch)) != LGPU_OK) return rc;
-    if (batch == 0) CK(launch_eig(st, ea, &launches), "eigen kernel");
+  if (rows) {
+    CK(h->buf[B_EIGSCR].ensure(eig_rows_bytes(k, h->nunits)), "alloc transform scratch");
+    ea.scratch = h->buf[B_EIGSCR].p;
+  } else if ((rc = eig_scratch(h, h->nunits, ea, sp, batch)) != LGPU_OK) {
+    return rc;
   }
   const int nch = bound ? kOutChunks : 1;
   float eig_ms = 0.0f, upd_ms = 0.0f, fp64_ms = 0.0f;
@@ -1262,14 +1265,16 @@ static int solver_run(lgpu_handle *h) {
     for (int j = c0; j < c1 && a0 < 0; j++) if (h->h_col2act[j] >= 0) a0 = h->h_col2act[j];
     for (int j = c1 - 1; j >= c0 && a1 < 0; j--) if (h->h_col2act[j] >= 0) a1 = h->h_col2act[j] + 1;
     CK(cudaEventRecord(h->ev_chunk[c][0], st), "event");
-    if (!fp64 && batch > 0 && a0 >= 0)
+    if (rows)
+      CK(launch_eig_rows(st, ea, &launches), "eigen kernels");   // never with a bound state: one chunk
+    else if (!fp64 && a0 >= 0)
       CK(launch_eig_split(st, ea, sp, batch, a0 * G, (a1 - a0) * G, &launches), "eigen kernels");
     CK(cudaEventRecord(h->ev_chunk[c][3], st), "event");
     if (fp64 && a0 >= 0) {
       EigArgs e64 = ea;
       e64.nunits = (a1 - a0) * G;
       CK(launch_eig64(st, e64, a0 * G, &launches), "FP64 eigen kernel");
-    } else if (batch > 0 && a0 >= 0 && ea.flag_list) {
+    } else if (a0 >= 0 && ea.flag_list) {
       CK(launch_eig64_flagged(st, ea, &launches), "FP64 re-solve");
     }
     CK(cudaEventRecord(h->ev_chunk[c][1], st), "event");
@@ -1333,7 +1338,7 @@ static int solver_run(lgpu_handle *h) {
   h->tim.mma_chunks = h->used_tc ? stat4[2] : 0;
   h->tim.mma_n = h->used_tc ? h->mma_n : 0;
   h->tim.precision = h->prec;
-  h->tim.fp64_units = fp64 ? h->nunits : std::min(nflag, ea.flag_cap);   // with a fused-kernel fallback: 0
+  h->tim.fp64_units = fp64 ? h->nunits : std::min(nflag, ea.flag_cap);
   h->tim.fp64_ms = fp64_ms;
   h->tim.span_ms = h->tim.total_ms;
   if (bound) {
@@ -1574,7 +1579,6 @@ int lgpu_debug_transform(lgpu_handle *h, int nunits, int k, const float *gram, f
   if (e != cudaSuccess) return cuda_fail(h, e, "debug_transform");
   if (status & 1) return fail(h, LGPU_ERR_EIG, "eigensolver did not converge for at least one unit");
   if (status & 2) return fail(h, LGPU_ERR_EIG, "non-positive eigenvalue in at least one unit");
-  if (status & 32) return fail(h, LGPU_ERR_CUDA, "internal: malformed eigensolver rotation log");
   return LGPU_OK;
 }
 
@@ -2137,20 +2141,16 @@ static int learned_exact(lgpu_handle *h, const ObsSorted &os, int n, int &launch
   ea.ulist = nullptr;
   ea.status = h->buf[B_STATUS].as<int>();
   flag_args(h, ea);
+  EigSplit sp;
+  int batch = 0;
+  int rc = eig_scratch(h, n, ea, sp, batch);
+  if (rc != LGPU_OK) return rc;
   if (h->prec == LGPU_PREC_FP64) {
     CK(launch_eig64(st, ea, 0, &launches), "FP64 eigen kernel");
     return LGPU_OK;
   }
-  EigSplit sp;
-  int batch = 0;
-  int rc = eig_scratch(h, n, sp, batch);
-  if (rc != LGPU_OK) return rc;
-  if (batch == 0) {
-    CK(launch_eig(st, ea, &launches), "eigen kernel");
-  } else {
-    CK(launch_eig_split(st, ea, sp, batch, 0, n, &launches), "eigen kernels");
-    if (ea.flag_list) CK(launch_eig64_flagged(st, ea, &launches), "FP64 re-solve");
-  }
+  CK(launch_eig_split(st, ea, sp, batch, 0, n, &launches), "eigen kernels");
+  if (ea.flag_list) CK(launch_eig64_flagged(st, ea, &launches), "FP64 re-solve");
   return LGPU_OK;
 }
 
@@ -2338,7 +2338,6 @@ static int learned_run(lgpu_handle *h) {
   if (status & 2) return fail(h, LGPU_ERR_EIG, "non-positive eigenvalue in at least one unit");
   if (status & 4) return fail(h, LGPU_ERR_NONFINITE, "non-finite analysis mean or spread");
   if (status & 16) return fail(h, LGPU_ERR_CUDA, "tensor-core pipeline wait timed out");
-  if (status & 32) return fail(h, LGPU_ERR_CUDA, "internal: malformed eigensolver rotation log");
   if (status & 64) return fail(h, LGPU_ERR_CUDA, "update stage copy wait timed out");
   return LGPU_OK;
 }

@@ -1,35 +1,137 @@
-// lgpu_eig.cu -- batched symmetric eigensolve and LETKF transform per
-// (column, group) unit: FP32 (the reference's ssyev precision), with an FP64
-// form for the units flagged by the eigenvalue-gap test or for every unit.
+// lgpu_eig.cu -- the LETKF transform of every (column, group) unit: FP32 (the
+// reference's ssyev precision), with an FP64 form for the units flagged by
+// the eigenvalue-gap test or for every unit.
 //
-// Replaces src/letkf_core.F90:100-141: with A = G + (k-1)/infl I (G from
-// the Gram stage, upper triangle as ssyev('V','U') reads it),
-//   Pa   = V diag(1/lambda) V^T
-//   W    = V diag(sqrt((k-1)/lambda)) V^T
-//   wbar = Pa b               (b = Yb^T R^-1 rho dep, computed in the Gram stage)
+// Replaces src/letkf_core.F90:100-141: with A = G + (k-1)/infl I (G from the
+// Gram stage, upper triangle as ssyev('V','U') reads it),
+//   W    = sqrt(k-1) A^(-1/2)
+//   wbar = A^(-1) b           (b = Yb^T R^-1 rho dep, computed in the Gram stage)
 //   T    = W + wbar 1^T
-// The eigendecomposition is Householder tridiagonalisation (Golub & Van Loan,
-// Matrix Computations, 4th ed., Alg. 8.3.1) followed by the implicit-shift
-// QL iteration with Wilkinson shifts on the tridiagonal matrix (the
-// tql2 scheme of Bowdler, Martin, Reinsch & Wilkinson, Numer. Math. 11,
-// 1968), accumulating the rotations into Z, and back-transformation
-// V = Q Z.  The split pipeline (used whenever its scratch fits) reduces in
-// registers (k_eig_tri_r: a warp per unit up to k = 48; k_eig_tri_t: a team
-// of ceil(k / 32) warps, one row per thread, above), runs the QL scalar
-// recurrence once per unit (k_eig_ql) and replays the logged rotations on Q's
-// rows in shared memory (k_eig_vec: one warp, two rows per lane, up to
-// k = 64; four warps, one row per thread, above).  The fused kernel (k_eig,
-// the fallback) works on the matrices in shared memory with the rows spread
-// over a warp's or team's threads (tt + TS q) and evaluates the QL recurrence
-// redundantly on every lane (shared memory broadcasts) with lane 0 as the
-// only writer.  The FP64 form (k_eig64) runs the fused phases in double on a
-// team of 2 or 4 warps.
+// The reference forms both through the eigendecomposition of A.  T is a
+// function of the matrix alone, so no eigenvectors are needed:
+//   1. Householder tridiagonalisation A = Q S Q^T (Golub & Van Loan, Matrix
+//      Computations, 4th ed., Alg. 8.3.1), the reflectors kept in the lower
+//      triangle; y = Q^T b along with it.
+//   2. S^(-1/2) by partial fractions, x^(-1/2) = sum_p w_p / (x + s_p) with
+//      s_p, w_p > 0: the elliptic-function rule of Hale, Higham & Trefethen,
+//      "Computing A^alpha, log(A), and related matrix functions by contour
+//      integrals" (SIAM J. Numer. Anal. 46(5), 2008, method 3), which is
+//      Zolotarev's best approximation on [l0, lmax].  The number of terms
+//      follows the condition (4 to 16 in FP32).  Every (S + s_p I)^(-1) comes
+//      from one backward pivot recurrence: with eta_j its pivots and
+//      rho_j = -e_j / eta_(j+1), the inverse has
+//        g_00 = 1/eta_0,  g_(i+1)(i+1) = 1/eta_(i+1) + rho_i^2 g_ii,
+//        g_i(j+1) = g_ij rho_j  (j >= i),
+//      all terms of the diagonal positive.  One lane runs one shift; a further
+//      lane solves S z = y (shift 0), and one checks that S - l0 I is
+//      positive definite.
+//   3. W = Q S^(-1/2) Q^T and wbar = Q z, the reflectors applied to both
+//      sides from the last to the first.
+// The three-kernel form before it (reduction, QL on one thread per unit with
+// the rotations logged, their replay on Q) spent two thirds of its time in
+// the QL's serial recurrence and the replay.
+//
+// The work matrix lives in registers over a grid of LA x LB lanes: lane
+// (a, b) holds rows a + LA r and columns b + LB i.  A reduction step costs
+// 3 m^2 multiply-adds for a trailing block of m and a back-transformation
+// step K m + K m + m^2; in one row per lane every multiply-add also read a
+// quarter of a 16-byte shared-memory vector, and the shared-memory return
+// path bounded the reduction.  The 2-D grid reads R + C values per R x C
+// multiply-adds.  The steps are unrolled in phases of LA rows so that the
+// blocks left of and above the trailing one are dropped at compile time.
 #include "lgpu_internal.cuh"
 #include <algorithm>
+#include <cmath>
 
 namespace lgpu {
 
 namespace {
+
+constexpr int kLevels = 16;   // condition levels 4^1 .. 4^16
+
+// Shifts and weights of the partial fractions on [1, 4^(level + 1)].
+template <class R, int NP>
+struct Poles {
+  int n[kLevels];
+  R s[kLevels][NP], w[kLevels][NP];
+};
+
+// sn, cn, dn of parameter m = 1 - m1 at u, by descending Landen transformation
+// (Abramowitz & Stegun 16.4: the arithmetic-geometric mean scale)
+void ellip_sncndn(double u, double m1, double &sn, double &cn, double &dn) {
+  double a[32], c[32];
+  double b = std::sqrt(m1);
+  a[0] = 1.0;
+  c[0] = std::sqrt(1.0 - m1);
+  int n = 0;
+  while (std::fabs(c[n]) > 1e-17 && n < 30) {
+    a[n + 1] = 0.5 * (a[n] + b);
+    c[n + 1] = 0.5 * (a[n] - b);
+    b = std::sqrt(a[n] * b);
+    n++;
+  }
+  double phi = std::ldexp(a[n] * u, n), prev = phi;
+  for (; n > 0; n--) {
+    prev = phi;
+    phi = 0.5 * (phi + std::asin(c[n] / a[n] * std::sin(phi)));
+  }
+  sn = std::sin(phi);
+  cn = std::cos(phi);
+  const double den = std::cos(prev - phi);
+  dn = std::fabs(den) < 0.1 ? std::sqrt(1.0 - (1.0 - m1) * sn * sn) : cn / den;
+}
+
+// complete elliptic integral K of parameter 1 - m1
+double ellip_k(double m1) {
+  double a = 1.0, b = std::sqrt(m1);
+  for (int i = 0; i < 40 && std::fabs(a - b) > 1e-16 * a; i++) {
+    const double t = 0.5 * (a + b);
+    b = std::sqrt(a * b);
+    a = t;
+  }
+  return 1.5707963267948966 / a;
+}
+
+// Smallest term counts whose error over [1, 4^(level + 1)] is below `tol`
+// (NP at most: the wide levels, whose condition leaves the working precision
+// no digits at the small end anyway, keep the error NP terms give).
+template <class R, int NP>
+Poles<R, NP> make_poles(double tol) {
+  Poles<R, NP> P{};
+  for (int l = 0; l < kLevels; l++) {
+    const double kappa = std::ldexp(1.0, 2 * (l + 1)), K = ellip_k(1.0 / kappa);
+    double s[NP], w[NP];
+    for (int n = 3; n <= NP; n++) {
+      for (int j = 0; j < n; j++) {
+        double sn, cn, dn;
+        ellip_sncndn((j + 0.5) * K / n, 1.0 / kappa, sn, cn, dn);
+        s[j] = sn / cn * (sn / cn);
+        w[j] = 2.0 * K / (3.14159265358979323846 * n) * dn / (cn * cn);
+      }
+      double err = 0.0;
+      for (int t = 0; t <= 400; t++) {
+        const double x = std::exp(std::log(kappa) * t / 400.0);
+        double f = 0.0;
+        for (int j = 0; j < n; j++) f += w[j] / (x + s[j]);
+        err = std::max(err, std::fabs(f * std::sqrt(x) - 1.0));
+      }
+      P.n[l] = n;
+      if (err <= tol) break;
+    }
+    for (int j = 0; j < P.n[l]; j++) { P.s[l][j] = (R)s[j]; P.w[l][j] = (R)w[j]; }
+  }
+  return P;
+}
+
+using PolesF = Poles<float, 16>;
+using PolesD = Poles<double, 32>;
+// a quarter of the working precision's unit roundoff (FP64: what 32 terms and
+// the evaluation in double reach)
+const PolesF &poles_f() { static const PolesF P = make_poles<float, 16>(1.5e-8); return P; }
+const PolesD &poles_d() { static const PolesD P = make_poles<double, 32>(2e-15); return P; }
+template <class R> struct PolesOf;
+template <> struct PolesOf<float> { using type = PolesF; static const PolesF &get() { return poles_f(); } };
+template <> struct PolesOf<double> { using type = PolesD; static const PolesD &get() { return poles_d(); } };
 
 __device__ __forceinline__ float fmar(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fmar(double a, double b, double c) { return __fma_rn(a, b, c); }
@@ -37,808 +139,730 @@ __device__ __forceinline__ float rcpr(float x) { return __frcp_rn(x); }
 __device__ __forceinline__ double rcpr(double x) { return __drcp_rn(x); }
 // unit roundoff and the smallest scale treated as zero, per precision
 template <class R> struct Lim;
+// (`zero`: a squared norm that no rounding of the diagonal, at least 1, can see)
 template <> struct Lim<float> {
-  static constexpr float eps = 1.1920929e-7f, tiny = 1e-30f;
+  static constexpr float eps = 1.1920929e-7f, tiny = 1e-30f, zero = 1e-34f;
 };
 template <> struct Lim<double> {
-  static constexpr double eps = 2.220446049250313e-16, tiny = 1e-300;
+  static constexpr double eps = 2.220446049250313e-16, tiny = 1e-300, zero = 1e-200;
 };
 
-template <class R>
-__device__ __forceinline__ R wsum(R v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+// four consecutive values, 16-byte aligned
+__device__ __forceinline__ void ld4(const float *p, float *v) {
+  const float4 t = *reinterpret_cast<const float4 *>(p);
+  v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
+__device__ __forceinline__ void ld4(const double *p, double *v) {
+  const double2 t = *reinterpret_cast<const double2 *>(p), u = *reinterpret_cast<const double2 *>(p + 2);
+  v[0] = t.x; v[1] = t.y; v[2] = u.x; v[3] = u.y;
+}
+
+__device__ __forceinline__ void st4(float *p, const float *v) {
+  *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void st4(double *p, const double *v) {
+  *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
+  *reinterpret_cast<double2 *>(p + 2) = make_double2(v[2], v[3]);
+}
+
+// sqrt and reciprocal of positive normal values, to an ulp or so: the
+// hardware's approximations and one Newton step, without the rounded forms'
+// range checks
+__device__ __forceinline__ float sqrt_pos(float x) {
+  const float r = rsqrtf(x), q = x * r;
+  return fmar(0.5f * r, fmar(-q, q, x), q);
+}
+__device__ __forceinline__ double sqrt_pos(double x) { return sqrt(x); }
+__device__ __forceinline__ float rcp_pos(float x) {
+  const float r = __fdividef(1.0f, x);
+  return fmar(r, fmar(-x, r, 1.0f), r);
+}
+__device__ __forceinline__ double rcp_pos(double x) { return rcpr(x); }
+
+// 16 bytes global -> shared, asynchronously
+__device__ __forceinline__ void copy16_async(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// The lane grid of one unit: RN rows and CN columns per lane; LA is a
+// multiple of LB, and LB <= 8 divides a warp, so the lanes of a row lie in one warp.
+template <class R_, int RN_, int CN_, int LA_, int LB_, int MB_>
+struct Grid {
+  using R = R_;
+  static constexpr int RN = RN_, CN = CN_, LA = LA_, LB = LB_;
+  static constexpr int MB = MB_;                            // blocks per SM the registers are bounded for
+  static constexpr int L = LA * LB;
+  static constexpr int KR = LA * RN, KC = LB * CN;          // covered rows, columns
+  static constexpr int CP = (CN + 3) / 4 * 4;               // values of one lane column, padded to 16-byte vectors
+  static constexpr int VB = LB * CP;                        // one column-ordered vector
+  static constexpr int NP = sizeof(R) == 4 ? 16 : 32;
+  static constexpr int KM = KR > KC ? KR : KC;
+  static constexpr int KN = (KM + 3) / 4 * 4;               // one naturally ordered vector
+  static constexpr int PS = 2 * KN + 8 + VB;                // one shift's arrays: rho (8 zeros of slack), g, LB-products
+  static constexpr int VEC = 4 * KN;                        // d, e, tau, z
+  static constexpr int STEP = 6 * VB;                       // reduction: x, v, w (double-buffered); back: w, ring of 4 v
+  static constexpr int CH = L >= 32 ? NP : L - 2;           // shifts of one pass: with the solve and the test, a lane each
+  static constexpr int POLE = (CH + 2) * PS;
+  static constexpr int TRANS = LA * VB;                     // one row group
+  static constexpr int WORK0 = STEP > POLE ? STEP : POLE;
+  static constexpr int UNIT = VEC + (WORK0 > TRANS ? WORK0 : TRANS);   // values of one unit
+  static constexpr int REFL = KC * VB;                      // the reflectors of one unit (global scratch)
+  static constexpr int UPW = L < 32 ? 32 / L : 1;           // units per warp
+  static constexpr int UPB = L <= 32 ? 4 * UPW : 1;         // units per block
+  static constexpr int THREADS = L <= 32 ? 128 : L;
+  static_assert(LA % LB == 0 && LB <= 8, "lane grid");
+  static_assert(KR / LB <= CP && (L > 32 || KR == KC), "every row has a place in a column-ordered vector");
+};
+
+template <class G>
+__device__ __forceinline__ void team_sync() {
+  if constexpr (G::L <= 32) __syncwarp();
+  else __syncthreads();
+}
+
+// sum over the lanes of a row (consecutive lanes)
+template <class G, class R>
+__device__ __forceinline__ R sum_b(R v) {
+#pragma unroll
+  for (int o = 1; o < G::LB; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
-__host__ __device__ __forceinline__ int eig_floats_per_warp(int k) {
-  const int ld = k + 1;
-  return k * ld + 8 * k + 8;
-}
+// position of row / column c in a column-ordered vector (lane column c % LB first)
+template <class G>
+__device__ __forceinline__ int vpos(int c) { return (c % G::LB) * G::CP + c / G::LB; }
 
-// A team of NW warps works on one unit: thread tt of TS = 32 NW owns rows /
-// columns tt + TS q of the work matrices.  NW = 1 is one warp per unit
-// (several units per CTA); NW > 1 is one unit per CTA, so the CTA barrier is
-// the team barrier.  Sums run over the warp's butterfly, then over the warps
-// in warp order (deterministic).
-template <int NW, class R = float>
-struct Team {
-  static constexpr int TS = 32 * NW;
-  int tt, lane, warp;
-  R *red;       // NW values in shared memory (NW > 1)
-  __device__ __forceinline__ void sync() const {
-    if constexpr (NW == 1) __syncwarp();
-    else __syncthreads();
-  }
-  __device__ __forceinline__ R sum(R v) const {
-    v = wsum<R>(v);
-    if constexpr (NW == 1) {
-      return v;
-    } else {
-      if (lane == 0) red[warp] = v;
-      __syncthreads();
-      R t = red[0];
+// the lane's columns i >= I0 of a column-ordered vector
+template <class G, int I0, class R>
+__device__ __forceinline__ void load_cols(const R *buf, int b, R *v) {
+  const R *p = buf + b * G::CP;
 #pragma unroll
-      for (int q = 1; q < NW; q++) t += red[q];
-      __syncthreads();
-      return t;
-    }
+  for (int q = I0 / 4; q < G::CP / 4; q++) {
+    R t[4];
+    ld4(p + 4 * q, t);
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (4 * q + j >= I0 && 4 * q + j < G::CN) v[4 * q + j] = t[j];
   }
-};
-
-// Work arrays of one unit in shared memory: A (k x ld, ld = k + 1) holds A,
-// then Q, then V; then d, e, tau, bv, p, w, fl, gl (k each).
-template <class R = float>
-struct EigWork {
-  R *A, *d, *e, *tau, *bv, *p, *w, *fl, *gl;
-  __device__ EigWork(R *base, int k) {
-    A = base;
-    d = A + k * (k + 1);
-    e = d + k; tau = e + k; bv = tau + k; p = bv + k; w = p + k; fl = w + k; gl = fl + k;
-  }
-};
-
-// A = G + (k-1)/infl I from the packed Gram block, b from its tail
-template <int NW, class R>
-__device__ __forceinline__ void eig_load(const EigArgs &a, int unit, EigWork<R> &W, const Team<NW, R> &T) {
-  const int k = a.k, ld = k + 1, tt = T.tt, TS = T.TS;
-  R *A = W.A, *bv = W.bv;
-  const float *Gin = a.G + (size_t)unit * packed_size(k);
-  // (k-1)/infl on the diagonal, src/letkf_core.F90:101-104
-  const R shift = (R)(k - 1) * R(1) / (R)a.infl;
-  for (int t = tt; t < k * k; t += TS) {
-    const int i = t / k, j = t % k;
-    R v = (i <= j) ? (R)Gin[tri_idx(i, j, k)] : (R)Gin[tri_idx(j, i, k)];
-    if (i == j) v += shift;
-    A[i * ld + j] = v;
-  }
-  for (int i = tt; i < k; i += TS) bv[i] = (R)Gin[k * (k + 1) / 2 + i];
-  T.sync();
-
 }
 
-template <int NQ, int NW, class R>
-__device__ __forceinline__ void eig_form_q(int k, EigWork<R> &W, const Team<NW, R> &T);
+// the lane's rows r >= R0 of a column-ordered vector: row a + LA r sits at
+// lane column a % LB, place a / LB + (LA / LB) r
+template <class G, int R0, class R>
+__device__ __forceinline__ void load_rows(const R *buf, int a, R *v) {
+  const R *p = buf + (a % G::LB) * G::CP + a / G::LB;
+#pragma unroll
+  for (int r = R0; r < G::RN; r++) v[r] = p[(G::LA / G::LB) * r];
+}
 
-// Householder tridiagonalisation (d, e, tau; reflector vectors in the
-// columns of A) and Q formed in place.  NQ: rows / columns per lane
-// (tt + TS q, q < NQ).
-template <int NQ, int NW, class R>
-__device__ __forceinline__ void eig_tridiag_q(int k, EigWork<R> &W, const Team<NW, R> &T) {
-  const int ld = k + 1, tt = T.tt, TS = T.TS;
-  R *A = W.A, *d = W.d, *e = W.e, *tau = W.tau, *p = W.p, *w = W.w;
-  R *vv = W.fl;   // the current reflector, contiguous (fl is free until the transform)
-  // ---- Householder tridiagonalisation: column j's reflector zeroes A[j+2:, j];
-  // its vector v_j = A[j+1:, j] stays in column j
-  for (int j = 0; j < k - 2; j++) {
-    const int m = k - j - 1;                 // length of x = A[j+1:, j]
-    R s = R(0);
-    for (int r = tt; r < m; r += TS) { R x = A[(j + 1 + r) * ld + j]; s += x * x; }
-    const R sig = T.sum(s);
-    const R x0 = A[(j + 1) * ld + j];
-    const R s1 = sig - x0 * x0;
-    if (!(s1 > Lim<R>::tiny * sig) || sig == R(0)) {
-      if (tt == 0) { tau[j] = R(0); e[j] = x0; d[j] = A[j * ld + j]; }
-      T.sync();
-      continue;
+template <class G, int R0, class R>
+__device__ __forceinline__ void store_rows(R *buf, int a, const R *v) {
+  R *p = buf + (a % G::LB) * G::CP + a / G::LB;
+#pragma unroll
+  for (int r = R0; r < G::RN; r++) p[(G::LA / G::LB) * r] = v[r];
+}
+
+// the lane's columns i >= I0 into a column-ordered vector (whole 16-byte groups)
+template <class G, int I0, class R>
+__device__ __forceinline__ void store_cols(R *buf, int b, const R *v) {
+  R *p = buf + b * G::CP;
+#pragma unroll
+  for (int q = I0 / 4; q < G::CP / 4; q++) {
+    R t[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) t[j] = 4 * q + j < G::CN ? v[4 * q + j] : R(0);
+    st4(p + 4 * q, t);
+  }
+}
+
+// the unit's shared-memory vectors
+template <class G>
+struct UnitMem {
+  using R = typename G::R;
+  R *d, *e, *tau, *z, *work;
+  __device__ explicit UnitMem(R *base) {
+    d = base;
+    e = d + G::KN; tau = e + G::KN; z = tau + G::KN;
+    work = z + G::KN;
+  }
+  __device__ R *w(int j) const { return work + (j & 1) * G::VB; }
+  __device__ R *x(int j) const { return work + (2 + (j & 1)) * G::VB; }     // reduction: raw row
+  __device__ R *v(int j) const { return work + (4 + (j & 1)) * G::VB; }     // reduction: reflector
+  __device__ R *ring(int j) const { return work + (2 + (j & 3)) * G::VB; }  // back-transformation: reflectors
+};
+
+// The right-hand side (then z) of a unit on one warp: one warp's lanes hold
+// elements l + S q, in registers; a team keeps them in shared memory.
+template <class G>
+struct Vec {
+  using R = typename G::R;
+  static constexpr int S = G::L < 32 ? G::L : 32, Q = (G::KM + S - 1) / S;
+  R z[Q];
+  __device__ __forceinline__ void load(const UnitMem<G> &U, int l) {
+    if constexpr (G::L <= 32) {
+#pragma unroll
+      for (int q = 0; q < Q; q++) z[q] = l + S * q < G::KN ? U.z[l + S * q] : R(0);
     }
-    const R alpha = -copysign(sqrt(sig), x0);
-    const R v0 = x0 - alpha;
-    const R t = R(2) / (v0 * v0 + s1);
-    T.sync();
-    if (tt == 0) { A[(j + 1) * ld + j] = v0; tau[j] = t; e[j] = alpha; d[j] = A[j * ld + j]; }
-    for (int r = tt; r < m; r += TS) vv[r] = r == 0 ? v0 : A[(j + 1 + r) * ld + j];
-    T.sync();
-    // p = t * A22 v
-    for (int r = tt; r < m; r += TS) {
-      const R *row = A + (j + 1 + r) * ld + (j + 1);
-      R acc = R(0);
-#pragma unroll 4
-      for (int c = 0; c < m; c++) acc = fmar(row[c], vv[c], acc);
-      p[r] = t * acc;
+  }
+  __device__ __forceinline__ void store(const UnitMem<G> &U, int l) {
+    if constexpr (G::L <= 32) {
+#pragma unroll
+      for (int q = 0; q < Q; q++)
+        if (l + S * q < G::KN) U.z[l + S * q] = z[q];
     }
-    T.sync();
+  }
+  // z -= t (v.z) v, v column-ordered and zero before C0; a team's warp `warp` does it
+  template <int C0>
+  __device__ __forceinline__ void reflect(const UnitMem<G> &U, int k, int l, int warp, R t, const R *vbuf) {
+    if constexpr (G::L > 32) {
+      if ((l >> 5) != warp) return;
+      l &= 31;
+    }
+    R v[Q], s = R(0);
+#pragma unroll
+    for (int q = C0 / S; q < Q; q++) {
+      const int c = l + S * q;
+      v[q] = (q > C0 / S || c >= C0) && (q < Q - 1 || c < G::KC) ? vbuf[vpos<G>(c)] : R(0);
+      if constexpr (G::L > 32) z[q] = c < k ? U.z[c] : R(0);
+      s = fmar(v[q], z[q], s);
+    }
+#pragma unroll
+    for (int o = 1; o < S; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    s *= t;
+#pragma unroll
+    for (int q = C0 / S; q < Q; q++) {
+      z[q] = fmar(-s, v[q], z[q]);
+      if constexpr (G::L > 32)
+        if (l + S * q < k) U.z[l + S * q] = z[q];
+    }
+  }
+};
+
+// The two-sided update M -= v w^T + w v^T with w = p - (t/2)(p.v) v, p = t M v.
+// vcol / vrow: the reflector at the lane's columns and rows, zero up to j
+// (columns below I0 and rows below R0 not set).  FULL (back-transformation):
+// every row and column; else (reduction) the trailing block, where w is zero
+// up to j.
+template <class G, int R0, int I0, bool FULL>
+__device__ __forceinline__ void two_sided(typename G::R (&A)[G::RN][G::CN], typename G::R *wb, int j, int a, int b, typename G::R t,
+                                          const typename G::R *vcol, const typename G::R *vrow) {
+  using R = typename G::R;
+  constexpr int W0 = FULL ? 0 : R0, C0 = FULL ? 0 : I0;
+  R w[G::RN];
+#pragma unroll
+  for (int r = W0; r < G::RN; r++) {
+    R acc = R(0);
+#pragma unroll
+    for (int i = I0; i < G::CN; i++) acc = fmar(A[r][i], vcol[i], acc);
+    w[r] = acc;
+  }
+#pragma unroll
+  for (int r = W0; r < G::RN; r++) w[r] = t * sum_b<G>(w[r]);
+  if constexpr (G::L <= 32) {
+    // one warp: p.v over the rows, then the finished w is published
     R pv = R(0);
-    for (int r = tt; r < m; r += TS) pv = fmar(p[r], vv[r], pv);
-    const R beta = R(0.5) * t * T.sum(pv);
-    for (int r = tt; r < m; r += TS) w[r] = p[r] - beta * vv[r];
-    T.sync();
-    // A22 -= v w^T + w v^T
-    for (int r = tt; r < m; r += TS) {
-      R *row = A + (j + 1 + r) * ld + (j + 1);
-      const R vr = vv[r], wr = w[r];
-#pragma unroll 4
-      for (int c = 0; c < m; c++) row[c] = row[c] - fmar(vr, w[c], wr * vv[c]);
-    }
-    T.sync();
-  }
-  if (tt == 0) {
-    if (k >= 2) {
-      d[k - 2] = A[(k - 2) * ld + (k - 2)];
-      e[k - 2] = A[(k - 1) * ld + (k - 2)];
-    }
-    d[k - 1] = A[(k - 1) * ld + (k - 1)];
-    e[k - 1] = R(0);
-  }
-  T.sync();
-  eig_form_q<NQ>(k, W, T);
-}
-
-// Q = H_0 H_1 ... H_{k-3} formed in place from the reflectors in the columns
-// of A below the diagonal (v_j in column j, tau[j]), last reflector first:
-// the trailing block [j+1:, j+1:] holds H_{j+1}..H_{k-3} (identity on row
-// and column j+1); v_j is still in column j, outside the block.  Each thread
-// owns columns tt + TS q.  The entries on and above the diagonal are not read
-// before they are written.
-template <int NQ, int NW, class R>
-__device__ __forceinline__ void eig_form_q(int k, EigWork<R> &W, const Team<NW, R> &T) {
-  const int ld = k + 1, tt = T.tt, TS = T.TS;
-  R *A = W.A, *tau = W.tau;
-  R *vv = W.fl;
-  {
-    for (int j = k - 2; j >= 0; j--) {
-      // identity on row and column j + 1 of the block
 #pragma unroll
-      for (int q = 0; q < NQ; q++) {
-        const int c = tt + TS * q;
-        if (c > j + 1 && c < k) { A[(j + 1) * ld + c] = R(0); A[c * ld + (j + 1)] = R(0); }
-      }
-      if (tt == 0) A[(j + 1) * ld + (j + 1)] = R(1);
-      T.sync();
-      if (j > k - 3) continue;                 // the last block (2 x 2) has no reflector
-      const R t = tau[j];
-      if (t == R(0)) continue;
-      const int m = k - j - 1;
-      for (int r = tt; r < m; r += TS) vv[r] = A[(j + 1 + r) * ld + j];
-      T.sync();
-      // w_c = t * sum_r v_r Q[r][c]; Q[r][c] -= v_r w_c  (rows, columns j+1..k-1)
-      R wc[NQ];
-      bool in[NQ];
+    for (int r = R0; r < G::RN; r++) pv = fmar(w[r], vrow[r], pv);
 #pragma unroll
-      for (int q = 0; q < NQ; q++) {
-        const int c = tt + TS * q;
-        wc[q] = R(0);
-        in[q] = c > j && c < k;
-      }
-      for (int r = 0; r < m; r++) {
-        const R v = vv[r];
+    for (int o = G::LB; o < G::L; o <<= 1) pv += __shfl_xor_sync(0xffffffffu, pv, o);
+    const R beta = R(0.5) * t * pv;
 #pragma unroll
-        for (int q = 0; q < NQ; q++)
-          if (in[q]) wc[q] = fmar(v, A[(j + 1 + r) * ld + tt + TS * q], wc[q]);
-      }
+    for (int r = R0; r < G::RN; r++) w[r] = fmar(-beta, vrow[r], w[r]);
+    if (!FULL) w[R0] = a + G::LA * R0 > j ? w[R0] : R(0);
+    if (b == 0) store_rows<G, W0>(wb, a, w);
+    team_sync<G>();
+    const R *wp = wb + b * G::CP;
 #pragma unroll
-      for (int q = 0; q < NQ; q++) wc[q] *= t;
-      for (int r = 0; r < m; r++) {
-        const R v = vv[r];
+    for (int q = C0 / 4; q < G::CP / 4; q++) {
+      R wc[4];
+      ld4(wp + 4 * q, wc);
 #pragma unroll
-        for (int q = 0; q < NQ; q++)
-          if (in[q]) A[(j + 1 + r) * ld + tt + TS * q] -= v * wc[q];
-      }
-      T.sync();
-    }
-    // row and column 0: Q e_0 = e_0
+      for (int jj = 0; jj < 4; jj++) {
+        const int i = 4 * q + jj;
+        if (i < C0 || i >= G::CN) continue;
 #pragma unroll
-    for (int q = 0; q < NQ; q++) {
-      const int c = tt + TS * q;
-      if (c > 0 && c < k) { A[c] = R(0); A[c * ld] = R(0); }
-    }
-    if (tt == 0) A[0] = R(1);
-    T.sync();
-  }
-
-}
-
-// spectral functions and T = U U^T + wbar 1^T (A holds V, d the eigenvalues)
-template <int NQ, int NW, class R>
-__device__ __forceinline__ void eig_transform(const EigArgs &a, int unit, EigWork<R> &W, const Team<NW, R> &TM,
-                                              int &bad) {
-  const int k = a.k, ld = k + 1, tt = TM.tt, TS = TM.TS;
-  R *A = W.A, *d = W.d, *bv = W.bv, *p = W.p, *w = W.w, *fl = W.fl, *gl = W.gl;
-  // ---- spectral functions: f = sqrt((k-1)/lambda), g = 1/lambda
-  //      (src/letkf_core.F90:111-113, :128-131); fl holds sqrt(f)
-  for (int l = tt; l < k; l += TS) {
-    const R lam = d[l];
-    if (!(lam > R(0))) bad |= 2;
-    fl[l] = sqrt(sqrt((R)(k - 1) / lam));
-    gl[l] = R(1) / lam;
-  }
-  TM.sync();
-  // s_l = g_l * (V^T b)_l
-  for (int l = tt; l < k; l += TS) {
-    R acc = R(0);
-    for (int q = 0; q < k; q++) acc = fmar(A[q * ld + l], bv[q], acc);
-    p[l] = gl[l] * acc;
-  }
-  TM.sync();
-  // wbar_i = sum_l V[i][l] s_l
-  for (int i = tt; i < k; i += TS) {
-    R acc = R(0);
-    for (int l = 0; l < k; l++) acc = fmar(A[i * ld + l], p[l], acc);
-    w[i] = acc;
-    if (a.wbar) a.wbar[(size_t)unit * k + i] = (float)acc;
-  }
-  TM.sync();
-  // U = V diag(sqrt f) in place: T = U U^T + wbar 1^T
-  for (int t = tt; t < k * k; t += TS) { const int i = t / k, l = t % k; A[i * ld + l] *= fl[l]; }
-  TM.sync();
-  // T_ij = sum_l U[i][l] U[j][l] + wbar_i ; thread owns columns tt + TS q
-  // (a column past k repeats the thread's first column and is not stored)
-  float *Tout = a.T + (size_t)unit * k * k;
-  // rows in blocks of TRB (a row past k repeats row 0 and is not stored);
-  // every sum runs over l in ascending order
-  if (tt < k) {
-    constexpr int TRB = 4;
-    const R *u[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; q++) u[q] = A + (tt + TS * q < k ? tt + TS * q : tt) * ld;
-    for (int i0 = 0; i0 < k; i0 += TRB) {
-      const R *ur[TRB];
-#pragma unroll
-      for (int b = 0; b < TRB; b++) ur[b] = A + (i0 + b < k ? i0 + b : 0) * ld;
-      R acc[TRB][NQ];
-#pragma unroll
-      for (int b = 0; b < TRB; b++)
-#pragma unroll
-        for (int q = 0; q < NQ; q++) acc[b][q] = R(0);
-      for (int l = 0; l < k; l++) {
-        R uq[NQ];
-#pragma unroll
-        for (int q = 0; q < NQ; q++) uq[q] = u[q][l];
-#pragma unroll
-        for (int b = 0; b < TRB; b++) {
-          const R y = ur[b][l];
-#pragma unroll
-          for (int q = 0; q < NQ; q++) acc[b][q] = fmar(y, uq[q], acc[b][q]);
+        for (int r = W0; r < G::RN; r++) {
+          R x = A[r][i];
+          if (i >= I0) x = fmar(-w[r], vcol[i], x);
+          if (r >= R0) x = fmar(-vrow[r], wc[jj], x);
+          A[r][i] = x;
         }
       }
-#pragma unroll
-      for (int b = 0; b < TRB; b++)
-#pragma unroll
-        for (int q = 0; q < NQ; q++)
-          if (i0 + b < k && tt + TS * q < k) Tout[(i0 + b) * k + tt + TS * q] = (R)(acc[b][q] + w[i0 + b]);
     }
+  } else {
+    // a team of warps: p is published, and p.v is summed over the columns,
+    // whose lanes share a warp
+    if (!FULL) w[R0] = a + G::LA * R0 > j ? w[R0] : R(0);
+    if (b == 0) store_rows<G, W0>(wb, a, w);
+    team_sync<G>();
+    R wc[G::CN];
+    load_cols<G, C0>(wb, b, wc);
+    R pv = R(0);
+#pragma unroll
+    for (int i = I0; i < G::CN; i++) pv = fmar(wc[i], vcol[i], pv);
+    const R beta = R(0.5) * t * sum_b<G>(pv);
+#pragma unroll
+    for (int i = I0; i < G::CN; i++) wc[i] = fmar(-beta, vcol[i], wc[i]);
+#pragma unroll
+    for (int r = R0; r < G::RN; r++) w[r] = fmar(-beta, vrow[r], w[r]);
+#pragma unroll
+    for (int r = W0; r < G::RN; r++)
+#pragma unroll
+      for (int i = C0; i < G::CN; i++) {
+        R x = A[r][i];
+        if (i >= I0) x = fmar(-w[r], vcol[i], x);
+        if (r >= R0) x = fmar(-vrow[r], wc[i], x);
+        A[r][i] = x;
+      }
   }
 }
 
-// Deflation test of the QL iteration: e_m is negligible when it is below
-// eps32 of its two diagonal neighbours (the local test of LAPACK's ssteqr /
-// EISPACK's tql2 family) or, from the kQlAbsIter-th iteration on the current
-// eigenvalue, below eps32 times the norm of the whole tridiagonal matrix
-// (tql2's absolute test).  The second test ends the iteration where rounding
-// at the eps32 ||T|| level keeps a strongly graded block from meeting the
-// local test.  Applied from the first iteration it also deflated, at the
-// ||T|| level, off-diagonals between near-equal small eigenvalues that the
-// local test resolves in a few more sweeps (a rank-one update with k = 100
-// and condition ~1e5: those eigenvalues off by ~eps32 ||T||); the delay
-// keeps them.
-constexpr int kQlAbsIter = 6;
-
-template <class R>
-__device__ __forceinline__ bool ql_negligible(R em, R dm, R dm1, R tabs) {
-  const R ae = fabs(em);
-  return ae <= Lim<R>::eps * (fabs(dm) + fabs(dm1)) || ae <= tabs;
-}
-
-// eps32 * max_i (|d_i| + |e_i|), elements at stride `st`
-template <class R>
-__device__ __forceinline__ R ql_abs_tol(int k, const R *d, const R *e, int st) {
-  R an = R(0);
-  for (int i = 0; i < k; i++) an = fmax(an, fabs(d[(size_t)i * st]) + fabs(e[(size_t)i * st]));
-  return Lim<R>::eps * an;
-}
-
-// implicit-shift QL on (d, e) with the rotations applied to the columns of
-// A (Q -> V), one warp
-template <int NQ, class R>
-__device__ __forceinline__ void eig_ql_warp(int k, EigWork<R> &W, int lane, int &bad) {
-  const int ld = k + 1;
-  R *A = W.A, *d = W.d, *e = W.e;
-  // ---- implicit-shift QL on (d, e), rotations applied at once to the
-  // columns (i, i+1) of Q (V = Q Z).  The scalar recurrence is evaluated
-  // redundantly by every lane: d[i+1] is carried in a register and only e[i],
-  // d[i] (not yet written in this sweep) are read, so lane 0 alone writes
-  // results, without barriers inside the sweep.  Each lane owns rows
-  // lane + 32 q of Q and carries the pending column i+1 of its rows.
-  {
-    bool own[NQ];
-    R *qr[NQ];
+// Reduction steps of rows [LA P, LA P + LA): d, e, tau, the reflectors to the
+// scratch gv (one column-ordered vector a step), y = Q^T b.
+template <class G, int P>
+__device__ __forceinline__ void reduce_phase(typename G::R (&A)[G::RN][G::CN], const UnitMem<G> &U, Vec<G> &z,
+                                             typename G::R *gv, int k, int l, int a, int b) {
+  using R = typename G::R;
+  constexpr int R0 = P, I0 = (P * G::LA + 1) / G::LB;
+  constexpr int CB = P * G::LA / G::LB;                       // column group of column LA P
+  constexpr int NB = G::LA / G::LB;                           // column groups of the phase's columns
+  const int jend = k < P * G::LA + G::LA ? k : P * G::LA + G::LA;
+  for (int j = P * G::LA; j < jend; j++) {
+    const bool own = a == j - P * G::LA;
+    R vcol[G::CN], vrow[G::RN], t = R(0);
+    if constexpr (G::L <= 32) {
+      // one warp: the row is published as it stands, and every lane forms the
+      // reflector from its own columns
+      R *xb = U.x(j), *vb = U.v(j);
+      if (own) store_cols<G, CB>(xb, b, A[R0]);
+      team_sync<G>();
+      const R x0 = j + 1 < G::KC ? xb[vpos<G>(j + 1)] : R(0);
+      if (j >= k - 2) {                        // the last 2 x 2 block
+        if (l == 0) { U.d[j] = xb[vpos<G>(j)]; U.e[j] = j < k - 1 ? x0 : R(0); }
+        continue;
+      }
+      load_cols<G, I0>(xb, b, vcol);
+      load_rows<G, R0>(xb, a, vrow);
+      R s4[4] = {R(0), R(0), R(0), R(0)};
 #pragma unroll
-    for (int q = 0; q < NQ; q++) {
-      own[q] = lane + 32 * q < k;
-      qr[q] = A + (own[q] ? lane + 32 * q : 0) * ld;
-    }
-    const R tabs = ql_abs_tol(k, d, e, 1);
-    for (int l = 0; l < k; l++) {
-      int iter = 0;
-      for (;;) {
-        // first m >= l with a negligible e[m] (m = k-1 if none): lanes test
-        // 32 consecutive candidates at a time
-        int m = k - 1;
-        for (int base = l; base < k - 1; base += 32) {
-          const int mm = base + lane;
-          bool small = false;
-          if (mm < k - 1) small = ql_negligible(e[mm], d[mm], d[mm + 1], iter >= kQlAbsIter ? tabs : R(0));
-          const unsigned bal = __ballot_sync(0xffffffffu, small);
-          if (bal) { m = base + __ffs(bal) - 1; break; }
+      for (int i = I0; i < G::CN; i++) {
+        if (i <= CB + NB) vcol[i] = b + G::LB * i > j + 1 ? vcol[i] : R(0);
+        s4[i & 3] = fmar(vcol[i], vcol[i], s4[i & 3]);
+      }
+      const R s1 = sum_b<G>((s4[0] + s4[1]) + (s4[2] + s4[3]));
+      const R sig = fmar(x0, x0, s1);
+      const bool live = s1 > Lim<R>::tiny * sig && sig > Lim<R>::zero;
+      R alpha = x0;
+      if (live) {
+        alpha = -copysign(sqrt_pos(sig), x0);
+        t = rcp_pos(fmar(-alpha, x0, sig));     // 2 / v^T v, v = x - alpha e_1
+      }
+      const R v0 = x0 - alpha;
+#pragma unroll
+      for (int i = I0; i < G::CN; i++)
+        if (i <= CB + NB) vcol[i] = b + G::LB * i == j + 1 ? v0 : vcol[i];
+#pragma unroll
+      for (int r = R0; r < G::RN; r++)
+        if (r <= R0 + 1) {
+          const int row = a + G::LA * r;
+          vrow[r] = row > j + 1 ? vrow[r] : (row == j + 1 ? v0 : R(0));
         }
-        if (m == l) break;
-        if (++iter > 60) { bad = 1; break; }
-        const R dl = d[l], el = e[l];
-        R g = (d[l + 1] - dl) / (R(2) * el);
-        R r = sqrt(g * g + R(1));
-        g = d[m] - dl + el / (g + copysign(r, g));
-        R s = R(1), c = R(1), pp = R(0);
-        R di1 = d[m];
-        R z[NQ];   // pending column i+1
+      if (own) {
+        if (I0 > CB) vcol[CB] = R(0);
+        store_cols<G, CB>(vb, b, vcol);
+        store_cols<G, CB>(gv + (size_t)j * G::VB, b, vcol);
+      }
+      if (l == 0) { U.tau[j] = t; U.e[j] = alpha; U.d[j] = xb[vpos<G>(j)]; }
+    } else {
+      // a team: the warp of the row forms the reflector and publishes it
+      R *vb = U.v(j);
+      if ((l >> 5) == (j - P * G::LA) * G::LB / 32) {
+        R s1 = R(0), x0 = R(0), dj = R(0), x[G::CN];
 #pragma unroll
-        for (int q = 0; q < NQ; q++) z[q] = own[q] ? qr[q][m] : R(0);
-        R ei = e[m - 1], di = d[m - 1];
-        int i = m - 1;
-        bool deflate = false;
-        for (; i >= l; i--) {
-          const int in = i > 0 ? i - 1 : 0;
-          const R ei_n = e[in], di_n = d[in];           // next step's operands
-          R av[NQ];
-#pragma unroll
-          for (int q = 0; q < NQ; q++) av[q] = own[q] ? qr[q][i] : R(0);
-          const R f = s * ei, b = c * ei;
-          r = sqrt(f * f + g * g);
-          if (lane == 0) e[i + 1] = r;
-          if (r == R(0)) {
-            if (lane == 0) { d[i + 1] = di1 - pp; e[m] = R(0); }
-            deflate = true;
-            break;
+        for (int i = CB; i < G::CN; i++) {
+          const int c = b + G::LB * i;
+          x[i] = A[R0][i];
+          if (i <= CB + NB) {
+            if (c == j + 1) x0 = x[i];
+            if (c == j) dj = x[i];
+            x[i] = c > j + 1 ? x[i] : R(0);
           }
-          const R ir = rcpr(r);
-          s = f * ir;
-          c = g * ir;
-          g = di1 - pp;
-          const R rr = (di - g) * s + R(2) * c * b;
-          pp = s * rr;
-          if (lane == 0) d[i + 1] = g + pp;
-          g = c * rr - b;
-          di1 = di;
-          // rotation (c, s) on columns (i, i+1) of the lane's rows
-#pragma unroll
-          for (int q = 0; q < NQ; q++)
-            if (own[q]) { qr[q][i + 1] = s * av[q] + c * z[q]; z[q] = c * av[q] - s * z[q]; }
-          ei = ei_n;
-          di = di_n;
+          s1 = fmar(x[i], x[i], s1);
         }
-        const int ilo = deflate ? i + 1 : l;
+        s1 = sum_b<G>(s1);
+        x0 = sum_b<G>(x0);
+        const R sig = fmar(x0, x0, s1);
+        R alpha = x0;
+        if (j < k - 2 && s1 > Lim<R>::tiny * sig && sig > Lim<R>::zero) {
+          alpha = -copysign(sqrt_pos(sig), x0);
+          t = rcp_pos(fmar(-alpha, x0, sig));
+        }
+        const R v0 = x0 - alpha;
+        if (own) {
 #pragma unroll
-        for (int q = 0; q < NQ; q++)
-          if (own[q]) qr[q][ilo] = z[q];
-        if (!deflate && lane == 0) { d[l] = d[l] - pp; e[l] = g; e[m] = R(0); }
-        __syncwarp();
+          for (int i = CB; i < G::CN; i++)
+            if (i <= CB + NB) x[i] = b + G::LB * i == j + 1 ? v0 : x[i];
+          store_cols<G, CB>(vb, b, x);
+          store_cols<G, CB>(gv + (size_t)j * G::VB, b, x);
+          if (b == 0) { U.tau[j] = t; U.e[j] = alpha; }
+          if (b == j % G::LB) U.d[j] = dj;
+        }
       }
-      if (bad) break;
+      if (j >= k - 2) continue;
+      team_sync<G>();
+      t = U.tau[j];
+      load_cols<G, I0>(vb, b, vcol);
+      load_rows<G, R0>(vb, a, vrow);
     }
+    two_sided<G, R0, I0, false>(A, U.w(j), j, a, b, t, vcol, vrow);
+    z.template reflect<P * G::LA>(U, k, l, ((j - P * G::LA) * G::LB / 32 + G::L / 64) % (G::L < 32 ? 1 : G::L / 32), t,
+                                  U.v(j));
   }
-  __syncwarp();
-
 }
 
-template <int NQ>
-__global__ void k_eig(EigArgs a, int wpb) {
-  extern __shared__ __align__(16) float sm[];
-  const int k = a.k;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int un = blockIdx.x * wpb + warp;
-  if (un >= a.nunits) return;             // whole warps exit; no block-level barriers below
-  const int unit = a.ulist ? a.ulist[un] : un;
-  if (a.nkept[unit] <= 0) return;         // no local observations: the update keeps the background
-  EigWork W(sm + (size_t)warp * eig_floats_per_warp(k), k);
-  const Team<1> T{lane, lane, warp, nullptr};
-  eig_load(a, unit, W, T);
-  eig_tridiag_q<NQ>(k, W, T);
-  int bad = 0;
-  eig_ql_warp<NQ>(k, W, lane, bad);
-  eig_transform<NQ>(a, unit, W, T, bad);
-  bad = __reduce_or_sync(0xffffffffu, bad);
-  if (bad && lane == 0) atomicOr(a.status, bad);
+// the reflector of step j into its ring slot
+template <class G>
+__device__ __forceinline__ void fetch_reflector(const UnitMem<G> &U, const typename G::R *gv, int j, int l) {
+  using R = typename G::R;
+  constexpr int E = 16 / (int)sizeof(R);
+  if (j >= 0)
+    for (int c = l; c < G::VB / E; c += G::L) copy16_async(U.ring(j) + c * E, gv + (size_t)j * G::VB + c * E);
+  copy_commit();
 }
 
-// ---------------------------------------------------------------------------
-// Split pipeline (the arithmetic of k_eig):
-//   k_eig_tri_r / k_eig_tri_t  the Householder reduction and Q with the work
-//              matrix in registers (a warp per unit up to k = 48, a team of
-//              ceil(k / 32) warps with one row per thread above); Q, d and e
-//              to global
-//   k_eig_ql   thread per unit: the QL recurrence on (d, e) alone, logging
-//              every sweep (start index, rotation count) and rotation (c, s)
-//   k_eig_vec  team per unit: the logged rotations applied to Q's columns
-//              (V = Q Z), then the spectral functions and T
-//   k_eig_flag (FP32_RESOLVE) warp per unit: units for the FP64 re-solve
-// The scalar recurrence, which the fused kernel evaluates redundantly on all
-// 32 lanes, runs once per unit.
+// Back-transformation steps of columns [LA P, LA P + LA), last first:
+// M <- H_j M H_j and z <- H_j z.
+template <class G, int P>
+__device__ __forceinline__ void back_phase(typename G::R (&A)[G::RN][G::CN], const UnitMem<G> &U, Vec<G> &z,
+                                           const typename G::R *gv, int k, int l, int a, int b) {
+  using R = typename G::R;
+  constexpr int R0 = P, I0 = (P * G::LA + 1) / G::LB;
+  const int jtop = k - 3 < P * G::LA + G::LA - 1 ? k - 3 : P * G::LA + G::LA - 1;
+  for (int j = jtop; j >= P * G::LA; j--) {
+    copy_wait<2>();
+    team_sync<G>();
+    fetch_reflector<G>(U, gv, j - 3, l);       // into the slot of step j + 1, which every lane has left
+    const R *vb = U.ring(j);
+    const R t = U.tau[j];
+    R vcol[G::CN], vrow[G::RN];
+    load_cols<G, I0>(vb, b, vcol);
+    load_rows<G, R0>(vb, a, vrow);
+    two_sided<G, R0, I0, true>(A, U.w(j), j, a, b, t, vcol, vrow);
+    z.template reflect<P * G::LA>(U, k, l, j % (G::L < 32 ? 1 : G::L / 32), t, vb);
+  }
+}
 
-// The first stage for k <= 48 with the work matrix in registers: one warp
-// per unit, lane l holds rows l and l + 32 of A (K = k rounded up to 8
-// columns, zero beyond k).  Step j of the Householder reduction: the lane
-// owning row j publishes x = A[j][j+1:] (= A[j+1:][j]) as the reflector
-// row VH[j] in shared memory (zeros outside j+1..k-1); p = t A v and the
-// rank-two update A -= v w^T + w v^T run on every lane's rows over the full
-// row width (columns and rows outside the trailing block meet zeros in v and
-// w and are left exactly unchanged), in column groups of four skipped while
-// they lie left of the block.  The dot products run over the columns in
-// ascending order as the shared-memory form does.  Q = H_0 ... H_{k-3} is
-// then formed with lane l holding columns l and l + 32 in the same registers
-// (reflectors applied from the last to the first).  Output: Q
-// row-major and (d, e) to the scratch.
-constexpr int RWPB = 4;   // warps (units) per block
+template <class G, int P>
+__device__ __forceinline__ void reduce_all(typename G::R (&A)[G::RN][G::CN], const UnitMem<G> &U, Vec<G> &z,
+                                           typename G::R *gv, int k, int l, int a, int b) {
+  if constexpr (P < G::RN) {
+    reduce_phase<G, P>(A, U, z, gv, k, l, a, b);
+    reduce_all<G, P + 1>(A, U, z, gv, k, l, a, b);
+  }
+}
 
-template <int K>
-__global__ void __launch_bounds__(32 * RWPB, 4) k_eig_tri_r(EigArgs a, EigSplit sp, int u0, int nb) {
-  constexpr int NQ = (K + 31) / 32;
-  constexpr int NR = K > 2 ? K - 2 : 1;   // reflector rows
-  constexpr int K4 = K / 4;
-  __shared__ __align__(16) float sv[RWPB][NR * K + 4 * K];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int ub = blockIdx.x * RWPB + warp;
-  if (ub >= nb) return;
-  const int unit = a.ulist ? a.ulist[u0 + ub] : u0 + ub;
-  if (a.nkept[unit] <= 0) return;
-  const int k = a.k;
-  float *VH = sv[warp];            // reflector j in row j
-  float *ww = VH + NR * K;         // w of the current step
-  float *dd = ww + K, *ee = dd + K, *tau = ee + K;
-  // A = G + (k-1)/infl I (src/letkf_core.F90:101-104), upper triangle packed
-  const float *Gin = a.G + (size_t)unit * packed_size(k);
-  const float shift = (float)(k - 1) * 1.0f / a.infl;
-  float A[NQ][K];
+template <class G, int P>
+__device__ __forceinline__ void back_all(typename G::R (&A)[G::RN][G::CN], const UnitMem<G> &U, Vec<G> &z,
+                                         const typename G::R *gv, int k, int l, int a, int b) {
+  if constexpr (P >= 0) {
+    back_phase<G, P>(A, U, z, gv, k, l, a, b);
+    back_all<G, P - 1>(A, U, z, gv, k, l, a, b);
+  }
+}
+
+// M's lower triangle from its upper one, one row group at a time through
+// shared memory
+template <class G, int P>
+__device__ __forceinline__ void mirror_all(typename G::R (&A)[G::RN][G::CN], typename G::R *buf, int a, int b) {
+  if constexpr (P < G::RN) {
+    constexpr int CB = P * G::LA / G::LB, NB = G::LA / G::LB;
+    team_sync<G>();
+    store_cols<G, CB>(buf + a * G::VB, b, A[P]);
+    team_sync<G>();
 #pragma unroll
-  for (int q = 0; q < NQ; q++) {
-    const int r = lane + 32 * q;
+    for (int i = CB; i < CB + NB && i < G::CN; i++) {
+      typename G::R s[G::RN];
+      load_rows<G, P>(buf + (b + G::LB * (i - CB)) * G::VB, a, s);
 #pragma unroll
-    for (int c = 0; c < K; c++) {
-      float v = 0.0f;
-      if (r < k && c < k) {
-        v = r <= c ? Gin[tri_idx(r, c, k)] : Gin[tri_idx(c, r, k)];
-        if (r == c) v += shift;
+      for (int r = P; r < G::RN; r++)
+        if (r > P || a + G::LA * r > b + G::LB * i) A[r][i] = s[r];
+    }
+    mirror_all<G, P + 1>(A, buf, a, b);
+  }
+}
+
+// any lane of the unit
+template <class G>
+__device__ __forceinline__ bool unit_any(bool x) {
+  if constexpr (G::L <= 32) {
+    const unsigned m = G::L == 32 ? 0xffffffffu : ((1u << (G::L & 31)) - 1u) << ((threadIdx.x & 31) / G::L * G::L);
+    return (__ballot_sync(0xffffffffu, x) & m) != 0;
+  } else {
+    return __syncthreads_or(x) != 0;
+  }
+}
+
+// One unit's transform from its packed Gram block (null: a lane slot without a
+// unit; it runs along on A = I).  Returns status bits (1: non-finite, 2: not
+// positive definite).
+template <class G>
+__device__ __forceinline__ int unit_transform(typename G::R *mem, const typename PolesOf<typename G::R>::type &tab,
+                                              typename G::R *gv, int k, float infl, const float *Gin, float *Tout,
+                                              float *wout, float *de, int l) {
+  using R = typename G::R;
+  const UnitMem<G> U(mem);
+  const int a = l / G::LB, b = l % G::LB;
+  // ---- A = G + (k-1)/infl I, src/letkf_core.F90:101-104
+  const R shift = (R)(k - 1) * R(1) / (R)infl;
+  R A[G::RN][G::CN];
+#pragma unroll
+  for (int r = 0; r < G::RN; r++) {
+    const int row = a + G::LA * r;
+#pragma unroll
+    for (int i = 0; i < G::CN; i++) {
+      const int col = b + G::LB * i;
+      R v = R(0);
+      if (row < k && col < k) {
+        const int lo = row < col ? row : col, hi = row < col ? col : row;
+        if (Gin) v = (R)Gin[tri_idx(lo, hi, k)];
+        if (row == col) v += shift;
       }
-      A[q][c] = v;
+      A[r][i] = v;
     }
   }
-  for (int j = 0; j < k - 2; j++) {
-    float *vj = VH + j * K;
-    __syncwarp();
-    // the owner of row j stores it whole (columns past k are zero in A);
-    // then d_j is taken and columns 0..j are cleared, one per lane
-    if (lane == (j & 31)) {
-      if (NQ == 1 || (j >> 5) == 0) {
+  for (int c = l; c < G::KN; c += G::L) {
+    U.z[c] = Gin && c < k ? (R)Gin[k * (k + 1) / 2 + c] : R(0);
+    U.d[c] = R(1);
+    U.e[c] = R(0);
+    U.tau[c] = R(0);
+  }
+  team_sync<G>();
+  Vec<G> z;
+  z.load(U, l);
+  reduce_all<G, 0>(A, U, z, gv, k, l, a, b);
+  z.store(U, l);
+  team_sync<G>();
+  if (de) {
+    for (int c = l; c < k; c += G::L) { de[c] = (float)U.d[c]; de[k + c] = (float)U.e[c]; }
+  }
+  // ---- S^(-1/2) by partial fractions
+  constexpr int S = G::L < 32 ? G::L : 32;
+  R lmax = R(0);
+  for (int c = l % S; c < k; c += S) {
+    const R g = U.d[c] + fabs(U.e[c]) + (c > 0 ? fabs(U.e[c - 1]) : R(0));
+    lmax = fabs(g) < R(3e38) ? fmax(lmax, g) : R(INFINITY);
+  }
 #pragma unroll
-        for (int c4 = 0; c4 < K4; c4++)
-          *reinterpret_cast<float4 *>(vj + 4 * c4) =
-              make_float4(A[0][4 * c4], A[0][4 * c4 + 1], A[0][4 * c4 + 2], A[0][4 * c4 + 3]);
-      } else {
+  for (int o = 1; o < S; o <<= 1) lmax = fmax(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
+  const bool nan = !(lmax < R(3e38));
+  // l0 bounds the spectrum from below unless the input is no Gram matrix or
+  // its condition is beyond the working precision: then lower bounds are
+  // tried, down to the last level
+  R l0 = R(0.9) * shift;
+  int level = 0, np = 0;
+  bool bad = false;
 #pragma unroll
-        for (int c4 = 0; c4 < K4; c4++)
-          *reinterpret_cast<float4 *>(vj + 4 * c4) = make_float4(A[NQ - 1][4 * c4], A[NQ - 1][4 * c4 + 1],
-                                                                 A[NQ - 1][4 * c4 + 2], A[NQ - 1][4 * c4 + 3]);
+  for (int r = 0; r < G::RN; r++)
+#pragma unroll
+    for (int i = G::LA * r / G::LB; i < G::CN; i++)
+      if (b + G::LB * i >= a + G::LA * r) A[r][i] = R(0);
+  for (int p0 = 0;;) {
+    if (p0 == 0) {
+      level = nan ? 0 : ilogb((double)fmax(lmax / l0, R(1))) >> 1;
+      level = level < kLevels - 1 ? level : kLevels - 1;
+      np = tab.n[level];
+    }
+    const int nc = np - p0 < G::CH ? np - p0 : G::CH;
+    // one lane a shift: the pivots from the last row up (u = 1, or the
+    // right-hand side of S z = y), then the diagonal of the inverse (or z)
+    // down, and the products of LB consecutive ratios.  Slot CH solves
+    // S z = y, slot CH + 1 tests S - 0.999 l0 I (both in the first pass).
+    bool fail = false, neg0 = false;
+    const int jobs = p0 == 0 ? nc + 2 : nc;
+    for (int q = l; q < jobs; q += G::L) {
+      const bool solve = q == nc, test = q == nc + 1;
+      const R s = solve ? R(0) : (test ? R(-0.999) * l0 : l0 * tab.s[level][p0 + (q < nc ? q : 0)]);
+      R *rho = U.work + (q < nc ? q : G::CH + q - nc) * G::PS, *g = rho + G::KN + 8, *lp = g + G::KN;
+#pragma unroll
+      for (int t = 0; t < 8; t++) rho[G::KM - 1 + t] = R(0);
+      R eta = U.d[G::KM - 1] + s, inv = rcp_pos(eta), u = solve ? U.z[G::KM - 1] : R(1);
+      bool neg = k == G::KM && !(eta > R(0));
+      g[G::KM - 1] = u * inv;
+      for (int j = G::KM - 2; j >= 0; j--) {
+        const R ej = U.e[j], rj = -ej * inv;
+        rho[j] = rj;
+        eta = fmar(ej, rj, U.d[j] + s);
+        neg |= j < k && !(eta > R(0));
+        inv = rcp_pos(eta);
+        u = solve ? fmar(rj, u, U.z[j]) : R(1);
+        g[j] = u * inv;
+      }
+      R gi = g[0];
+      R win[G::LB];
+#pragma unroll
+      for (int t = 0; t < G::LB; t++) win[t] = R(0);
+      lp[0] = R(0);
+      for (int j = 0; j < G::KM - 1; j++) {
+        const R rj = rho[j];
+        gi = fmar(solve ? rj : rj * rj, gi, g[j + 1]);
+        g[j + 1] = gi;
+#pragma unroll
+        for (int t = 0; t + 1 < G::LB; t++) win[t] = win[t + 1];
+        win[G::LB - 1] = rj;
+        R pr = win[0];
+#pragma unroll
+        for (int t = 1; t < G::LB; t++) pr *= win[t];
+        if (j + 1 < G::KC) lp[vpos<G>(j + 1)] = pr;
+      }
+      fail |= test && neg;
+      neg0 |= solve && neg;
+    }
+    if (p0 == 0) {
+      fail = unit_any<G>(fail) && level < kLevels - 1 && !nan;
+      bad = unit_any<G>(neg0);
+      // every lane of the warp (team) starts over together
+      if (G::L < 32 ? __any_sync(0xffffffffu, fail) : fail) {
+        if (fail) l0 *= R(1.0 / 16.0);
+        team_sync<G>();
+        continue;
       }
     }
-    __syncwarp();
+    team_sync<G>();
+    // the upper triangle of sqrt(k-1) S^(-1/2)
+    const R scale = sqrt(l0 * (R)(k - 1));
+    for (int q = 0; q < nc; q++) {
+      const R wp = scale * tab.w[level][p0 + q];
+      const R *rho = U.work + q * G::PS, *g = rho + G::KN + 8, *lp = g + G::KN;
+      R prod[G::CN];
+      load_cols<G, 0>(lp, b, prod);
 #pragma unroll
-    for (int q = 0; q < NQ; q++) {
-      const int c = lane + 32 * q;
-      if (c <= j) {
-        if (c == j) dd[j] = vj[j];
-        vj[c] = 0.0f;
+      for (int r = 0; r < G::RN; r++) {
+        const int row = a + G::LA * r;
+        // the lane's first column at or right of the diagonal lies `first` steps off it
+        const int first = (b - a + G::LA) & (G::LB - 1);
+        R f = wp * g[row];
+#pragma unroll
+        for (int t = 0; t + 1 < G::LB; t++) f = t < first ? f * rho[row + t] : f;
+        R cur = R(0);
+#pragma unroll
+        for (int i = G::LA * r / G::LB; i < G::CN; i++) {
+          if (i <= (G::LA * r + G::LA - 1) / G::LB + 1) {
+            const int off = b + G::LB * i - row;
+            cur = off < 0 ? R(0) : (off < G::LB ? f : cur * prod[i]);
+          } else {
+            cur *= prod[i];
+          }
+          A[r][i] += cur;
+        }
       }
     }
-    __syncwarp();
-    float s = 0.0f;
-#pragma unroll
-    for (int q = 0; q < NQ; q++) {
-      const int c = lane + 32 * q;
-      if (c < K) { const float x = vj[c]; s += x * x; }
+    if (p0 == 0) {
+      for (int c = l; c < k; c += G::L) U.z[c] = U.work[G::CH * G::PS + G::KN + 8 + c];
     }
-    const float sig = wsum<float>(s);
-    const float x0 = vj[j + 1];
-    const float s1 = sig - x0 * x0;
-    if (!(s1 > Lim<float>::tiny * sig) || sig == 0.0f) {
-      if (lane == 0) { tau[j] = 0.0f; ee[j] = x0; }
+    p0 += nc;
+    const bool more = p0 < np;
+    // a unit of the warp that is done repeats nothing (nc = 0)
+    if (G::L < 32 ? !__any_sync(0xffffffffu, more) : !more) break;
+    team_sync<G>();
+  }
+  // ---- W = Q S^(-1/2) Q^T, wbar = Q z
+  mirror_all<G, 0>(A, U.work, a, b);
+  team_sync<G>();   // the steps' buffers overlay the shifts' arrays
+  z.load(U, l);
+  fetch_reflector<G>(U, gv, k - 3, l);
+  fetch_reflector<G>(U, gv, k - 4, l);
+  fetch_reflector<G>(U, gv, k - 5, l);
+  back_all<G, G::RN - 1>(A, U, z, gv, k, l, a, b);
+  copy_wait<0>();
+  z.store(U, l);
+  team_sync<G>();
+  R zr[G::RN];
+#pragma unroll
+  for (int r = 0; r < G::RN; r++) zr[r] = U.z[a + G::LA * r];
+  if (Tout) {
+#pragma unroll
+    for (int r = 0; r < G::RN; r++) {
+      const int row = a + G::LA * r;
+#pragma unroll
+      for (int i = 0; i < G::CN; i++) {
+        const int col = b + G::LB * i;
+        if (row < k && col < k) Tout[row * k + col] = (float)(A[r][i] + zr[r]);
+      }
+    }
+    if (wout)
+      for (int c = l; c < k; c += G::L) wout[c] = (float)U.z[c];
+  }
+  return nan ? 1 : (bad ? 2 : 0);
+}
+
+template <class G>
+__global__ void __launch_bounds__(G::THREADS, G::MB) k_transform(EigArgs a, typename PolesOf<typename G::R>::type tab,
+                                                          EigSplit sp, typename G::R *vscr, int u0, int nb,
+                                                          const int *range) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  using R = typename G::R;
+  const int slot = threadIdx.x / G::L, l = threadIdx.x % G::L;
+  R *mem = reinterpret_cast<R *>(smem_raw) + (size_t)slot * G::UNIT;
+  R *gv = vscr + ((size_t)blockIdx.x * G::UPB + slot) * G::REFL;
+  // units u0 .. u0 + nb (through ulist), or the flagged entries not yet re-solved
+  int beg = 0, end = nb;
+  const int *list = a.ulist;
+  if (range) {
+    beg = range[1];
+    end = min(range[0], a.flag_cap);
+    list = a.flag_list;
+    u0 = 0;
+  }
+  for (int first = beg + blockIdx.x * G::UPB; first < end; first += gridDim.x * G::UPB) {
+    const int un = first + slot;
+    int unit = -1;
+    if (un < end) unit = list ? list[u0 + un] : u0 + un;
+    // no local observations: the update keeps the background
+    const bool on = unit >= 0 && a.nkept[unit] > 0;
+    if (G::L > 32) {
+      if (!on) continue;
+    } else if (!__any_sync(0xffffffffu, on)) {
       continue;
     }
-    const float alpha = -copysignf(sqrtf(sig), x0);
-    const float v0 = x0 - alpha;
-    const float t = 2.0f / (v0 * v0 + s1);
-    __syncwarp();
-    if (lane == 0) { vj[j + 1] = v0; tau[j] = t; ee[j] = alpha; }
-    __syncwarp();
-    // p = t A v
-    float p[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; q++) {
-      float acc = 0.0f;
-#pragma unroll
-      for (int c4 = 0; c4 < K4; c4++) {
-        if (4 * c4 + 3 <= j) continue;
-        const float4 v4 = *reinterpret_cast<const float4 *>(vj + 4 * c4);
-        acc = __fmaf_rn(A[q][4 * c4 + 0], v4.x, acc);
-        acc = __fmaf_rn(A[q][4 * c4 + 1], v4.y, acc);
-        acc = __fmaf_rn(A[q][4 * c4 + 2], v4.z, acc);
-        acc = __fmaf_rn(A[q][4 * c4 + 3], v4.w, acc);
-      }
-      p[q] = t * acc;
+    const int k = a.k;
+    float *de = on && sp.DE ? sp.DE + (size_t)un * 2 * k : nullptr;
+    const int bad = unit_transform<G>(mem, tab, gv, k, a.infl, on ? a.G + (size_t)unit * packed_size(k) : nullptr,
+                                      on ? a.T + (size_t)unit * k * k : nullptr,
+                                      on && a.wbar ? a.wbar + (size_t)unit * k : nullptr, de, l);
+    if (on && l == 0) {
+      // with flagging, the FP64 re-solve takes a failed unit
+      if (sp.DE) sp.bad[un] = bad;
+      else if (bad) atomicOr(a.status, bad);
     }
-    float pv = 0.0f;
-#pragma unroll
-    for (int q = 0; q < NQ; q++) {
-      const int r = lane + 32 * q;
-      if (r < K) pv = __fmaf_rn(p[q], vj[r], pv);
-    }
-    const float beta = 0.5f * t * wsum<float>(pv);
-    float w[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; q++) {
-      const int r = lane + 32 * q;
-      w[q] = (r > j && r < k) ? p[q] - beta * vj[r] : 0.0f;
-      if (r < K) ww[r] = w[q];
-    }
-    __syncwarp();
-    // A -= v w^T + w v^T
-#pragma unroll
-    for (int q = 0; q < NQ; q++) {
-      const int r = lane + 32 * q;
-      const float vr = r < K ? vj[r] : 0.0f, wr = w[q];
-#pragma unroll
-      for (int c4 = 0; c4 < K4; c4++) {
-        if (4 * c4 + 3 <= j) continue;
-        const float4 v4 = *reinterpret_cast<const float4 *>(vj + 4 * c4);
-        const float4 w4 = *reinterpret_cast<const float4 *>(ww + 4 * c4);
-        A[q][4 * c4 + 0] = A[q][4 * c4 + 0] - __fmaf_rn(vr, w4.x, wr * v4.x);
-        A[q][4 * c4 + 1] = A[q][4 * c4 + 1] - __fmaf_rn(vr, w4.y, wr * v4.y);
-        A[q][4 * c4 + 2] = A[q][4 * c4 + 2] - __fmaf_rn(vr, w4.z, wr * v4.z);
-        A[q][4 * c4 + 3] = A[q][4 * c4 + 3] - __fmaf_rn(vr, w4.w, wr * v4.w);
-      }
-    }
+    team_sync<G>();
   }
-  __syncwarp();
-  // the last 2 x 2 block: d[k-2], d[k-1], e[k-2]
-#pragma unroll
-  for (int q = 0; q < NQ; q++) {
-    const int r = lane + 32 * q;
-    if (r == k - 2 || r == k - 1) {
-#pragma unroll
-      for (int c = 0; c < K; c++) {
-        if (c == r) dd[r] = A[q][c];
-        if (r == k - 1 && c == k - 2) ee[k - 2] = A[q][c];
-      }
-    }
-  }
-  if (lane == 0) ee[k - 1] = 0.0f;
-  __syncwarp();
-  // Q = H_0 H_1 ... H_{k-3} I, reflectors from the last to the first; lane l
-  // holds columns l and l + 32
-#pragma unroll
-  for (int q = 0; q < NQ; q++) {
-    const int c = lane + 32 * q;
-#pragma unroll
-    for (int r = 0; r < K; r++) A[q][r] = (r == c && c < k) ? 1.0f : 0.0f;
-  }
-  for (int j = k - 3; j >= 0; j--) {
-    const float t = tau[j];
-    if (t == 0.0f) continue;
-    const float *vj = VH + j * K;
-#pragma unroll
-    for (int q = 0; q < NQ; q++) {
-      float s = 0.0f;
-#pragma unroll
-      for (int r4 = 0; r4 < K4; r4++) {
-        if (4 * r4 + 3 <= j) continue;
-        const float4 v4 = *reinterpret_cast<const float4 *>(vj + 4 * r4);
-        s = __fmaf_rn(v4.x, A[q][4 * r4 + 0], s);
-        s = __fmaf_rn(v4.y, A[q][4 * r4 + 1], s);
-        s = __fmaf_rn(v4.z, A[q][4 * r4 + 2], s);
-        s = __fmaf_rn(v4.w, A[q][4 * r4 + 3], s);
-      }
-      s *= t;
-#pragma unroll
-      for (int r4 = 0; r4 < K4; r4++) {
-        if (4 * r4 + 3 <= j) continue;
-        const float4 v4 = *reinterpret_cast<const float4 *>(vj + 4 * r4);
-        A[q][4 * r4 + 0] -= v4.x * s;
-        A[q][4 * r4 + 1] -= v4.y * s;
-        A[q][4 * r4 + 2] -= v4.z * s;
-        A[q][4 * r4 + 3] -= v4.w * s;
-      }
-    }
-  }
-  float *Q = sp.Q + (size_t)ub * k * k;
-#pragma unroll
-  for (int q = 0; q < NQ; q++) {
-    const int c = lane + 32 * q;
-    if (c < k) {
-#pragma unroll
-      for (int r = 0; r < K; r++)
-        if (r < k) Q[(size_t)r * k + c] = A[q][r];
-    }
-  }
-  float *de = sp.DE + (size_t)ub * 2 * k;
-  for (int i = lane; i < k; i += 32) { de[i] = dd[i]; de[k + i] = ee[i]; }
 }
 
-// k_eig_tri_t<K, NW>: k_eig_tri_r for 48 < k <= K <= 64 with a team of NW
-// warps per unit (one unit per CTA, 32 NW >= K): thread t holds row t of the
-// work matrix in registers; the reflector row VH[j] is written by thread j,
-// the sums over the rows run through the team in warp order, and Q is formed
-// with thread t holding column t.  Shared memory (dynamic): the reflectors
-// (K - 2) x K, then w, d, e, tau (K each).  Same arithmetic as k_eig_tri_r,
-// one row per thread instead of two per lane.
-template <int K, int NW>
-__global__ void __launch_bounds__(32 * NW) k_eig_tri_t(EigArgs a, EigSplit sp, int u0, int nb) {
-  constexpr int NR = K - 2;
-  constexpr int K4 = K / 4;
-  static_assert(32 * NW >= K, "one row per thread");
-  extern __shared__ __align__(16) float tsm[];
-  __shared__ float red[NW];
-  float *VH = tsm;                 // reflector j in row j
-  float *ww = VH + NR * K;         // w of the current step
-  float *dd = ww + K, *ee = dd + K, *tau = ee + K;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int ub = blockIdx.x;
-  if (ub >= nb) return;
-  const int unit = a.ulist ? a.ulist[u0 + ub] : u0 + ub;
-  if (a.nkept[unit] <= 0) return;
-  const int k = a.k;
-  // the team's sum (butterfly in each warp, then the warps in order)
-  auto tsum = [&](float v) -> float {
-    v = wsum<float>(v);
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    float r = red[0];
-#pragma unroll
-    for (int q = 1; q < NW; q++) r += red[q];
-    __syncthreads();
-    return r;
-  };
-  // A = G + (k-1)/infl I (src/letkf_core.F90:101-104), row t
-  const float *Gin = a.G + (size_t)unit * packed_size(k);
-  const float shift = (float)(k - 1) * 1.0f / a.infl;
-  float A[K];
-#pragma unroll
-  for (int c = 0; c < K; c++) {
-    float v = 0.0f;
-    if (t < k && c < k) {
-      v = t <= c ? Gin[tri_idx(t, c, k)] : Gin[tri_idx(c, t, k)];
-      if (t == c) v += shift;
-    }
-    A[c] = v;
-  }
-  for (int j = 0; j < k - 2; j++) {
-    float *vj = VH + j * K;
-    __syncthreads();
-    // thread j stores its row whole (columns past k are zero in A); then d_j
-    // is taken and columns 0..j are cleared, one per thread
-    if (t == j) {
-#pragma unroll
-      for (int c4 = 0; c4 < K4; c4++)
-        *reinterpret_cast<float4 *>(vj + 4 * c4) = make_float4(A[4 * c4], A[4 * c4 + 1], A[4 * c4 + 2], A[4 * c4 + 3]);
-    }
-    __syncthreads();
-    if (t <= j) {
-      if (t == j) dd[j] = vj[j];
-      vj[t] = 0.0f;
-    }
-    __syncthreads();
-    const float xt = t < K ? vj[t] : 0.0f;
-    const float sig = tsum(xt * xt);
-    const float x0 = vj[j + 1];
-    const float s1 = sig - x0 * x0;
-    if (!(s1 > Lim<float>::tiny * sig) || sig == 0.0f) {
-      if (t == 0) { tau[j] = 0.0f; ee[j] = x0; }
-      continue;
-    }
-    const float alpha = -copysignf(sqrtf(sig), x0);
-    const float v0 = x0 - alpha;
-    const float tt = 2.0f / (v0 * v0 + s1);
-    __syncthreads();
-    if (t == 0) { vj[j + 1] = v0; tau[j] = tt; ee[j] = alpha; }
-    __syncthreads();
-    // p = t A v
-    float acc = 0.0f;
-#pragma unroll
-    for (int c4 = 0; c4 < K4; c4++) {
-      if (4 * c4 + 3 <= j) continue;
-      const float4 v4 = *reinterpret_cast<const float4 *>(vj + 4 * c4);
-      acc = __fmaf_rn(A[4 * c4 + 0], v4.x, acc);
-      acc = __fmaf_rn(A[4 * c4 + 1], v4.y, acc);
-      acc = __fmaf_rn(A[4 * c4 + 2], v4.z, acc);
-      acc = __fmaf_rn(A[4 * c4 + 3], v4.w, acc);
-    }
-    const float p = tt * acc;
-    const float vt = t < K ? vj[t] : 0.0f;
-    const float beta = 0.5f * tt * tsum(t < K ? __fmaf_rn(p, vt, 0.0f) : 0.0f);
-    const float w = (t > j && t < k) ? p - beta * vt : 0.0f;
-    if (t < K) ww[t] = w;
-    __syncthreads();
-    // A -= v w^T + w v^T
-#pragma unroll
-    for (int c4 = 0; c4 < K4; c4++) {
-      if (4 * c4 + 3 <= j) continue;
-      const float4 v4 = *reinterpret_cast<const float4 *>(vj + 4 * c4);
-      const float4 w4 = *reinterpret_cast<const float4 *>(ww + 4 * c4);
-      A[4 * c4 + 0] = A[4 * c4 + 0] - __fmaf_rn(vt, w4.x, w * v4.x);
-      A[4 * c4 + 1] = A[4 * c4 + 1] - __fmaf_rn(vt, w4.y, w * v4.y);
-      A[4 * c4 + 2] = A[4 * c4 + 2] - __fmaf_rn(vt, w4.z, w * v4.z);
-      A[4 * c4 + 3] = A[4 * c4 + 3] - __fmaf_rn(vt, w4.w, w * v4.w);
-    }
-  }
-  __syncthreads();
-  // the last 2 x 2 block: d[k-2], d[k-1], e[k-2]
-  if (t == k - 2 || t == k - 1) {
-#pragma unroll
-    for (int c = 0; c < K; c++) {
-      if (c == t) dd[t] = A[c];
-      if (t == k - 1 && c == k - 2) ee[k - 2] = A[c];
-    }
-  }
-  if (t == 0) ee[k - 1] = 0.0f;
-  __syncthreads();
-  // Q = H_0 H_1 ... H_{k-3} I, reflectors from the last to the first; thread
-  // t holds column t
-#pragma unroll
-  for (int r = 0; r < K; r++) A[r] = (r == t && t < k) ? 1.0f : 0.0f;
-  for (int j = k - 3; j >= 0; j--) {
-    const float tj = tau[j];
-    if (tj == 0.0f) continue;
-    const float *vj = VH + j * K;
-    float s = 0.0f;
-#pragma unroll
-    for (int r4 = 0; r4 < K4; r4++) {
-      if (4 * r4 + 3 <= j) continue;
-      const float4 v4 = *reinterpret_cast<const float4 *>(vj + 4 * r4);
-      s = __fmaf_rn(v4.x, A[4 * r4 + 0], s);
-      s = __fmaf_rn(v4.y, A[4 * r4 + 1], s);
-      s = __fmaf_rn(v4.z, A[4 * r4 + 2], s);
-      s = __fmaf_rn(v4.w, A[4 * r4 + 3], s);
-    }
-    s *= tj;
-#pragma unroll
-    for (int r4 = 0; r4 < K4; r4++) {
-      if (4 * r4 + 3 <= j) continue;
-      const float4 v4 = *reinterpret_cast<const float4 *>(vj + 4 * r4);
-      A[4 * r4 + 0] -= v4.x * s;
-      A[4 * r4 + 1] -= v4.y * s;
-      A[4 * r4 + 2] -= v4.z * s;
-      A[4 * r4 + 3] -= v4.w * s;
-    }
-  }
-  float *Q = sp.Q + (size_t)ub * k * k;
-  if (t < k) {
-#pragma unroll
-    for (int r = 0; r < K; r++)
-      if (r < k) Q[(size_t)r * k + t] = A[r];
-  }
-  float *de = sp.DE + (size_t)ub * 2 * k;
-  for (int i = t; i < k; i += 32 * NW) { de[i] = dd[i]; de[k + i] = ee[i]; }
+// FP32_RESOLVE: the eigenvalues of every unit's tridiagonal matrix, for the
+// gap test (one thread per unit, implicit-shift QL with Wilkinson shifts
+// without vectors: the tql2 scheme of Bowdler, Martin, Reinsch & Wilkinson,
+// Numer. Math. 11, 1968).
+//
+// Deflation test: e_m is negligible when it is below eps32 of its two
+// diagonal neighbours (the local test of LAPACK's ssteqr / EISPACK's tql2
+// family) or, from the kQlAbsIter-th iteration on the current eigenvalue,
+// below eps32 times the norm of the whole tridiagonal matrix (tql2's absolute
+// test).  The second test ends the iteration where rounding at the eps32
+// ||T|| level keeps a strongly graded block from meeting the local test.
+// Applied from the first iteration it also deflated, at the ||T|| level,
+// off-diagonals between near-equal small eigenvalues that the local test
+// resolves in a few more sweeps; the delay keeps them.
+constexpr int kQlAbsIter = 6;
+constexpr int QLT = 64;   // threads (units) per block
+
+__device__ __forceinline__ bool ql_negligible(float em, float dm, float dm1, float tabs) {
+  const float ae = fabsf(em);
+  return ae <= Lim<float>::eps * (fabsf(dm) + fabsf(dm1)) || ae <= tabs;
 }
-
-template <int K, int NW>
-static size_t tri_t_smem() { return ((size_t)(K - 2) * K + 4 * K) * sizeof(float); }
-
-constexpr int QLT = 64;   // threads (units) per block of k_eig_ql
 
 __global__ void __launch_bounds__(QLT) k_eig_ql(EigArgs a, EigSplit sp, int u0, int nb) {
   extern __shared__ __align__(16) float qs[];   // d[k][QLT], e[k][QLT]
@@ -850,11 +874,16 @@ __global__ void __launch_bounds__(QLT) k_eig_ql(EigArgs a, EigSplit sp, int u0, 
   if (ub >= nb) return;
   const int unit = a.ulist ? a.ulist[u0 + ub] : u0 + ub;
   if (a.nkept[unit] <= 0) return;
+  if (sp.bad[ub]) return;
   const float *de = sp.DE + (size_t)ub * 2 * k;
-  for (int i = 0; i < k; i++) { D(i) = de[i]; E(i) = de[k + i]; }
-  const float tabs = ql_abs_tol(k, d, e, QLT);
-  float2 *lg = sp.log + (size_t)ub * sp.cap;
-  int pos = 0, bad = 0;
+  float an = 0.0f;
+  for (int i = 0; i < k; i++) {
+    D(i) = de[i];
+    E(i) = de[k + i];
+    an = fmaxf(an, fabsf(D(i)) + fabsf(E(i)));
+  }
+  const float tabs = Lim<float>::eps * an;
+  int bad = 0;
   for (int l = 0; l < k; l++) {
     int iter = 0;
     for (;;) {
@@ -862,15 +891,13 @@ __global__ void __launch_bounds__(QLT) k_eig_ql(EigArgs a, EigSplit sp, int u0, 
       const float tab = iter >= kQlAbsIter ? tabs : 0.0f;
       while (m < k - 1 && !ql_negligible(E(m), D(m), D(m + 1), tab)) m++;
       if (m == l) break;
-      if (++iter > 60) { bad |= 1; break; }
+      if (++iter > 60) { bad = 1; break; }
       const float dl = D(l), el = E(l);
       float g = (D(l + 1) - dl) / (2.0f * el);
       float r = sqrtf(g * g + 1.0f);
       g = D(m) - dl + el / (g + copysignf(r, g));
       float s = 1.0f, c = 1.0f, pp = 0.0f;
       float di1 = D(m);
-      const int hdr = pos++;
-      int cnt = 0;
       bool deflate = false;
       for (int i = m - 1; i >= l; i--) {
         const float ei = E(i), di = D(i);
@@ -892,129 +919,24 @@ __global__ void __launch_bounds__(QLT) k_eig_ql(EigArgs a, EigSplit sp, int u0, 
         D(i + 1) = g + pp;
         g = c * rr - b;
         di1 = di;
-        if (pos < sp.cap) lg[pos] = make_float2(c, s);
-        pos++;
-        cnt++;
       }
-      if (hdr < sp.cap) lg[hdr] = make_float2(__int_as_float(m), __int_as_float(cnt));
       if (!deflate) { D(l) = D(l) - pp; E(l) = g; E(m) = 0.0f; }
     }
     if (bad) break;
   }
 #undef D
 #undef E
-  // -1: no convergence (status bit 1); -2: log overflow (k_eig_vec reruns the QL)
-  sp.logn[ub] = bad ? -1 : (pos > sp.cap ? -2 : pos);
+  if (bad) sp.bad[ub] = bad;
   float *lam = sp.lam + (size_t)ub * k;
   for (int i = 0; i < k; i++) lam[i] = d[(size_t)i * QLT];
-  if (bad && !a.flag_list) atomicOr(a.status, bad);   // with flagging, the FP64 re-solve takes the unit
 }
 
-template <int NQ, int NW>
-__global__ void k_eig_vec(EigArgs a, EigSplit sp, int wpb, int u0, int nb) {
-  extern __shared__ __align__(16) float sm[];
-  __shared__ float tred[NW];
-  const int k = a.k, ld = k + 1;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int slot = NW == 1 ? warp : 0;
-  const int ub = blockIdx.x * wpb + slot;
-  if (ub >= nb) return;
-  const int unit = a.ulist ? a.ulist[u0 + ub] : u0 + ub;
-  if (a.nkept[unit] <= 0) return;
-  const int total = sp.logn[ub];
-  if (total == -1) return;                // no convergence: status set by k_eig_ql
-  EigWork W(sm + (size_t)slot * eig_floats_per_warp(k), k);
-  const Team<NW> T{NW == 1 ? lane : (int)threadIdx.x, lane, warp, tred};
-  const int tt = T.tt, TS = T.TS;
-  float *A = W.A;
-  const float *Q = sp.Q + (size_t)ub * k * k;
-  for (int t = tt; t < k * k; t += TS) A[(t / k) * ld + (t % k)] = Q[t];
-  const float *lam = sp.lam + (size_t)ub * k;
-  for (int t = tt; t < k; t += TS) W.d[t] = lam[t];
-  const float *G = a.G + (size_t)unit * packed_size(k);
-  T.sync();
-  int bad = 0;
-  if (total < 0) {
-    // the rotation log overflowed: the first warp runs the QL here from the
-    // tridiagonal form, on all rows
-    const float *de = sp.DE + (size_t)ub * 2 * k;
-    for (int t = tt; t < k; t += TS) { W.d[t] = de[t]; W.e[t] = de[k + t]; }
-    T.sync();
-    constexpr int NQW = 32 * NW * NQ <= 64 ? 2 : 4;
-    if (warp == 0 || NW == 1) eig_ql_warp<NQW>(k, W, lane, bad);
-  } else {
-    // replay the rotations on the thread's rows (tt + TS q).  The log passes
-    // through a window in the scratch vectors e .. gl (free until the
-    // transform; 8-byte aligned), refilled by the team at a sweep boundary
-    // whenever the next sweep (header + cnt <= k entries) would not fit, so
-    // that a sweep's rotations are read with one broadcast load each
-    const float2 *lg = sp.log + (size_t)ub * sp.cap;
-    const int wofs = (k * (k + 2)) & 1;   // e sits k (k + 2) floats into the unit's scratch
-    float2 *win = reinterpret_cast<float2 *>(W.e + wofs);
-    const int WN = (7 * k + 8 - wofs) / 2;   // e, tau, bv, p, w, fl, gl and the 8 spare floats
-    bool own[NQ];
-    float *qr[NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; q++) {
-      own[q] = tt + TS * q < k;
-      qr[q] = A + (own[q] ? tt + TS * q : 0) * ld;
-    }
-    int base = 0;
-    auto refill = [&](int from) {   // team-uniform
-      T.sync();
-      base = from;
-      const int n = total - from < WN ? total - from : WN;
-      for (int t = tt; t < n; t += TS) win[t] = lg[from + t];
-      T.sync();
-    };
-    refill(0);
-    int pidx = 0;
-    while (pidx < total) {
-      if (pidx >= base + WN) refill(pidx);
-      const float2 h = win[pidx - base];
-      const int m = __float_as_int(h.x), cnt = __float_as_int(h.y);
-      if (m < 1 || m >= k || cnt < 0 || cnt > m || pidx + 1 + cnt > total) { bad |= 32; break; }   // malformed log
-      if (pidx + 1 + cnt > base + WN) refill(pidx);
-      const float2 *rot = win + (pidx + 1 - base);
-      pidx += 1 + cnt;
-      float z[NQ];
-#pragma unroll
-      for (int q = 0; q < NQ; q++) z[q] = own[q] ? qr[q][m] : 0.0f;
-#pragma unroll 2
-      for (int r = 0; r < cnt; r++) {
-        const float2 cs = rot[r];
-        const float c = cs.x, s = cs.y;
-        const int i = m - 1 - r;
-#pragma unroll
-        for (int q = 0; q < NQ; q++) {
-          const float av = own[q] ? qr[q][i] : 0.0f;
-          if (own[q]) { qr[q][i + 1] = s * av + c * z[q]; z[q] = c * av - s * z[q]; }
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < NQ; q++)
-        if (own[q]) qr[q][m - cnt] = z[q];
-    }
-  }
-  // b after the replay: its slot is part of the log window
-  T.sync();
-  for (int i = tt; i < k; i += TS) W.bv[i] = G[k * (k + 1) / 2 + i];
-  T.sync();
-  eig_transform<NQ>(a, unit, W, T, bad);
-  bad = __reduce_or_sync(0xffffffffu, bad);
-  if (bad && a.flag_list) {
-    if (lane == 0) sp.logn[ub] = -1;   // k_eig_flag hands the unit to the FP64 re-solve
-  } else if (bad && lane == 0) {
-    atomicOr(a.status, bad);
-  }
-}
-
-// FP64 re-solve candidates of a batch (warp per unit, after k_eig_vec):
-// the FP32 solve failed, or two relevant eigenvalues lie within
-// gap_thresh * max l of each other.  The eigenvalues at the (k-1)/infl floor
-// (the null space of the Gram, k - n of them when n < k) are exactly
-// degenerate and harmless, since T is a function of the matrix and not of
-// the basis chosen in an eigenspace; they are left out of the test.
+// FP64 re-solve candidates of a batch (warp per unit, after k_eig_ql): the
+// FP32 solve failed, or two relevant eigenvalues lie within gap_thresh *
+// max l of each other.  The eigenvalues at the (k-1)/infl floor (the null
+// space of the Gram, k - n of them when n < k) are exactly degenerate and
+// harmless, since T is a function of the matrix and not of the basis chosen
+// in an eigenspace; they are left out of the test.
 __global__ void k_eig_flag(EigArgs a, EigSplit sp, int u0, int nb) {
   const int lane = threadIdx.x & 31;
   const int ub = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -1022,7 +944,7 @@ __global__ void k_eig_flag(EigArgs a, EigSplit sp, int u0, int nb) {
   const int unit = a.ulist ? a.ulist[u0 + ub] : u0 + ub;
   if (a.nkept[unit] <= 0) return;
   const int k = a.k;
-  bool flag = sp.logn[ub] == -1;
+  bool flag = sp.bad[ub] != 0;
   if (!flag) {
     const float *lam = sp.lam + (size_t)ub * k;
     float lmax = 0.0f;
@@ -1032,8 +954,10 @@ __global__ void k_eig_flag(EigArgs a, EigSplit sp, int u0, int nb) {
     const float floor_v = (float)(k - 1) / a.infl;
     const float tol = 4.0f * (float)k * 1.1920929e-7f * lmax;
     float gap = 3.0e38f;
+    bool neg = false;
     for (int i = lane; i < k; i += 32) {
       const float li = lam[i];
+      neg |= !(li > 0.0f);
       if (li - floor_v <= tol) continue;
       for (int j = 0; j < k; j++) {
         const float lj = lam[j];
@@ -1041,7 +965,7 @@ __global__ void k_eig_flag(EigArgs a, EigSplit sp, int u0, int nb) {
       }
     }
     for (int o = 16; o > 0; o >>= 1) gap = fminf(gap, __shfl_xor_sync(0xffffffffu, gap, o));
-    flag = gap <= a.gap_thresh * lmax;
+    flag = gap <= a.gap_thresh * lmax || __any_sync(0xffffffffu, neg);
   }
   if (flag && lane == 0) {
     const int pos = atomicAdd(a.flag_n, 1);
@@ -1050,305 +974,125 @@ __global__ void k_eig_flag(EigArgs a, EigSplit sp, int u0, int nb) {
   }
 }
 
-// Implicit-shift QL for a team of NW warps: per sweep, warp 0 evaluates the
-// scalar recurrence (as eig_ql_warp: redundantly on its lanes, lane 0
-// writing d, e and the rotations (c, s) of the sweep into cs_c / cs_s), then
-// every thread of the team applies the sweep's rotations to its own rows of
-// Q (rows tt + TS q) in the same order and arithmetic as eig_ql_warp.
-// ctl[0]: the sweep's m (-1: l converged, -2: no convergence), ctl[1]: the
-// lowest rotated column.
-template <int NQ, int NW, class R>
-__device__ __forceinline__ void eig_ql_team(int k, EigWork<R> &W, const Team<NW, R> &T, R *cs_c, R *cs_s,
-                                            int *ctl, int &bad) {
-  const int ld = k + 1, tt = T.tt, TS = T.TS, lane = T.lane;
-  R *A = W.A, *d = W.d, *e = W.e;
-  bool own[NQ];
-  R *qr[NQ];
-#pragma unroll
-  for (int q = 0; q < NQ; q++) {
-    own[q] = tt + TS * q < k;
-    qr[q] = A + (own[q] ? tt + TS * q : 0) * ld;
-  }
-  const R tabs = ql_abs_tol(k, d, e, 1);
-  for (int l = 0; l < k; l++) {
-    int iter = 0;
-    for (;;) {
-      if (T.warp == 0) {
-        int m = k - 1;
-        for (int base = l; base < k - 1; base += 32) {
-          const int mm = base + lane;
-          bool small = false;
-          if (mm < k - 1) small = ql_negligible(e[mm], d[mm], d[mm + 1], iter >= kQlAbsIter ? tabs : R(0));
-          const unsigned bal = __ballot_sync(0xffffffffu, small);
-          if (bal) { m = base + __ffs(bal) - 1; break; }
-        }
-        int c0 = m, c1 = l;
-        if (m == l) {
-          c0 = -1;
-        } else if (++iter > 60) {
-          c0 = -2;
-        } else {
-          const R dl = d[l], el = e[l];
-          R g = (d[l + 1] - dl) / (R(2) * el);
-          R r = sqrt(g * g + R(1));
-          g = d[m] - dl + el / (g + copysign(r, g));
-          R s = R(1), c = R(1), pp = R(0);
-          R di1 = d[m];
-          R ei = e[m - 1], di = d[m - 1];
-          int i = m - 1;
-          bool deflate = false;
-          for (; i >= l; i--) {
-            const int in = i > 0 ? i - 1 : 0;
-            const R ei_n = e[in], di_n = d[in];
-            const R f = s * ei, b = c * ei;
-            r = sqrt(f * f + g * g);
-            if (lane == 0) e[i + 1] = r;
-            if (r == R(0)) {
-              if (lane == 0) { d[i + 1] = di1 - pp; e[m] = R(0); }
-              deflate = true;
-              break;
-            }
-            const R ir = rcpr(r);
-            s = f * ir;
-            c = g * ir;
-            g = di1 - pp;
-            const R rr = (di - g) * s + R(2) * c * b;
-            pp = s * rr;
-            if (lane == 0) { d[i + 1] = g + pp; cs_c[i] = c; cs_s[i] = s; }
-            g = c * rr - b;
-            di1 = di;
-            ei = ei_n;
-            di = di_n;
-          }
-          c1 = deflate ? i + 1 : l;
-          if (!deflate && lane == 0) { d[l] = d[l] - pp; e[l] = g; e[m] = R(0); }
-        }
-        if (lane == 0) { ctl[0] = c0; ctl[1] = c1; }
-      }
-      T.sync();
-      const int m = ctl[0], ilo = ctl[1];
-      if (m < 0) {
-        if (m == -2) bad = 1;
-        T.sync();   // ctl is read by every thread before warp 0 writes it again
-        break;
-      }
-      R z[NQ];
-#pragma unroll
-      for (int q = 0; q < NQ; q++) z[q] = own[q] ? qr[q][m] : R(0);
-      for (int i = m - 1; i >= ilo; i--) {
-        const R c = cs_c[i], s = cs_s[i];
-#pragma unroll
-        for (int q = 0; q < NQ; q++)
-          if (own[q]) {
-            const R av = qr[q][i];
-            qr[q][i + 1] = s * av + c * z[q];
-            z[q] = c * av - s * z[q];
-          }
-      }
-#pragma unroll
-      for (int q = 0; q < NQ; q++)
-        if (own[q]) qr[q][ilo] = z[q];
-      T.sync();
-    }
-    if (bad) break;
-  }
-  T.sync();
+// resident blocks of the whole GPU: the register bound, or shared memory
+template <class G>
+constexpr int resident_blocks() {
+  const int bytes = G::UPB * G::UNIT * (int)sizeof(typename G::R) + 1024, fit = 227 * 1024 / bytes;
+  return 152 * (fit < G::MB ? fit : G::MB);
 }
 
-// FP64 eigensolve + transform, a team of NW warps per unit (one unit per
-// block at a time), grid-stride over the units: ulist / ubase + 0..nunits,
-// or (range != null) the flagged entries flag_list[range[1] ..
-// min(range[0], flag_cap)).  GB300 runs FP64 at 1/64 of the FP32 rate, so a
-// single unit's latency (the re-solve of a few flagged units) is spread over
-// the SM's four schedulers.
-template <int NW>
-__global__ void k_eig64(EigArgs a, int ubase, const int *range) {
-  extern __shared__ __align__(16) double smd[];
-  __shared__ double tred[NW];
-  __shared__ int ctl[2];
-  const int k = a.k;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int beg = 0, end = a.nunits;
-  const int *list = a.ulist;
-  if (range) {
-    beg = range[1];
-    end = min(range[0], a.flag_cap);
-    list = a.flag_list;
-  }
-  EigWork<double> W(smd, k);
-  const Team<NW, double> T{(int)threadIdx.x, lane, warp, tred};
-  for (int un = beg + blockIdx.x; un < end; un += gridDim.x) {
-    const int unit = list ? list[un] : ubase + un;
-    if (a.nkept[unit] <= 0) continue;
-    __syncthreads();   // the previous unit's transform has read the work arrays
-    eig_load(a, unit, W, T);
-    eig_tridiag_q<1>(k, W, T);
-    int bad = 0;
-    eig_ql_team<1>(k, W, T, W.p, W.w, ctl, bad);
-    eig_transform<1>(a, unit, W, T, bad);
-    bad = __reduce_or_sync(0xffffffffu, bad);
-    if (bad && lane == 0) atomicOr(a.status, bad);
-  }
-}
-
-}  // namespace
-
-namespace {
-// warps per unit of the FP64 kernel: every row of Q on its own thread
-int eig64_team(int k) { return k <= 64 ? 2 : 4; }
-
-template <int NW>
-cudaError_t eig64_go_t(cudaStream_t st, const EigArgs &a, int ubase, const int *range, int blocks, int *launches) {
-  const size_t smem = (size_t)eig_floats_per_warp(a.k) * sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(k_eig64<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// The grid is one wave, each block striding over the units: the reflectors'
+// scratch is one slot per resident unit and stays in L2.
+template <class G>
+cudaError_t launch_g(cudaStream_t st, const EigArgs &a, const EigSplit &sp, int u0, int nb, const int *range,
+                     int *launches) {
+  const size_t smem = (size_t)G::UPB * G::UNIT * sizeof(typename G::R);
+  cudaError_t e = cudaFuncSetAttribute(k_transform<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k_eig64<NW><<<blocks, 32 * NW, smem, st>>>(a, ubase, range);
+  const int grid = std::min(resident_blocks<G>(), (nb + G::UPB - 1) / G::UPB);
+  k_transform<G><<<grid, G::THREADS, smem, st>>>(a, PolesOf<typename G::R>::get(), sp,
+                                                 reinterpret_cast<typename G::R *>(a.scratch), u0, nb, range);
   (*launches)++;
   return cudaGetLastError();
 }
 
-cudaError_t eig64_go(cudaStream_t st, const EigArgs &a, int ubase, const int *range, int blocks, int *launches) {
-  return eig64_team(a.k) == 2 ? eig64_go_t<2>(st, a, ubase, range, blocks, launches)
-                              : eig64_go_t<4>(st, a, ubase, range, blocks, launches);
+// calls f with the lane grid of an ensemble size
+// FP32: one warp holds four units up to k = 24, two up to 40, one up to 64; a
+// team of two warps a unit up to 80, of four above.
+template <class F>
+auto with_grid_f32(int k, F f) {
+#define LGPU_GRID(RN, CN, LA, LB, MB) return f(Grid<float, RN, CN, LA, LB, MB>())
+  switch ((k + 7) / 8) {
+  case 1: LGPU_GRID(1, 8, 8, 1, 6);
+  case 2: LGPU_GRID(2, 16, 8, 1, 4);
+  case 3: LGPU_GRID(3, 24, 8, 1, 4);
+  case 4: LGPU_GRID(4, 16, 8, 2, 4);
+  case 5: LGPU_GRID(5, 20, 8, 2, 3);
+  case 6: LGPU_GRID(6, 12, 8, 4, 4);
+  case 7: LGPU_GRID(7, 14, 8, 4, 3);
+  case 8: LGPU_GRID(8, 16, 8, 4, 2);
+  case 9: LGPU_GRID(5, 18, 16, 4, 6);
+  case 10: LGPU_GRID(5, 20, 16, 4, 6);
+  case 11: LGPU_GRID(6, 11, 16, 8, 4);
+  case 12: LGPU_GRID(6, 12, 16, 8, 4);
+  case 13: LGPU_GRID(7, 13, 16, 8, 3);
+  case 14: LGPU_GRID(7, 14, 16, 8, 3);
+  case 15: LGPU_GRID(8, 15, 16, 8, 2);
+  default: LGPU_GRID(8, 16, 16, 8, 2);
+  }
+#undef LGPU_GRID
 }
 
-// resident units per SM (one per block), from the shared memory of one unit
-int eig64_per_sm(int k) {
-  const size_t per = (size_t)eig_floats_per_warp(k) * sizeof(double) + 1024;
-  return std::max(1, std::min(16, (int)((227 * 1024) / per)));
+// FP64: GB300 runs FP64 at 1/64 of the FP32 rate, so a unit is spread over two
+// warps up to k = 64 and eight above
+template <class F>
+auto with_grid_f64(int k, F f) {
+#define LGPU_GRID(RN, CN, LA, LB, MB) return f(Grid<double, RN, CN, LA, LB, MB>())
+  if (k <= 16) LGPU_GRID(2, 2, 8, 8, 8);
+  if (k <= 32) LGPU_GRID(4, 4, 8, 8, 8);
+  if (k <= 40) LGPU_GRID(5, 5, 8, 8, 6);
+  if (k <= 64) LGPU_GRID(8, 8, 8, 8, 4);
+  if (k <= 96) LGPU_GRID(3, 12, 32, 8, 1);
+  LGPU_GRID(4, 16, 32, 8, 1);
+#undef LGPU_GRID
 }
+
+cudaError_t launch_f32(cudaStream_t st, const EigArgs &a, const EigSplit &sp, int u0, int nb, int *launches) {
+  return with_grid_f32(a.k, [&](auto g) { return launch_g<decltype(g)>(st, a, sp, u0, nb, nullptr, launches); });
+}
+
+cudaError_t launch_f64(cudaStream_t st, const EigArgs &a, int u0, int nb, const int *range, int *launches) {
+  return with_grid_f64(a.k, [&](auto g) { return launch_g<decltype(g)>(st, a, EigSplit{}, u0, nb, range, launches); });
+}
+
+struct ScratchOf {
+  int units;
+  template <class G>
+  size_t operator()(G) const {
+    const size_t blocks = std::min<size_t>(resident_blocks<G>(), ((size_t)units + G::UPB - 1) / G::UPB);
+    return blocks * G::UPB * G::REFL * sizeof(typename G::R);
+  }
+};
+
 }  // namespace
+
+size_t eig_scratch_bytes(int k, int units, bool fp32, bool fp64) {
+  const ScratchOf f{std::max(1, units)};
+  return std::max(fp32 ? with_grid_f32(k, f) : 0, fp64 ? with_grid_f64(k, f) : 0);
+}
 
 cudaError_t launch_eig64(cudaStream_t st, const EigArgs &a, int ubase, int *launches) {
   if (a.nunits <= 0) return cudaSuccess;
-  return eig64_go(st, a, ubase, nullptr, std::min(a.nunits, 152 * eig64_per_sm(a.k)), launches);
+  return launch_f64(st, a, ubase, a.nunits, nullptr, launches);
 }
 
 cudaError_t launch_eig64_flagged(cudaStream_t st, const EigArgs &a, int *launches) {
   if (!a.flag_list || a.flag_cap <= 0) return cudaSuccess;
-  // one block per flagged unit up to the resident limit; the count stays on the device
-  cudaError_t e = eig64_go(st, a, 0, a.flag_n, std::min(a.flag_cap, 152 * eig64_per_sm(a.k)), launches);
+  // the count stays on the device: the wave of blocks strides over the list
+  cudaError_t e = launch_f64(st, a, 0, a.nunits, a.flag_n, launches);
   if (e != cudaSuccess) return e;
   return cudaMemcpyAsync(a.flag_n + 1, a.flag_n, sizeof(int), cudaMemcpyDeviceToDevice, st);
 }
 
-cudaError_t launch_eig(cudaStream_t st, const EigArgs &a, int *launches);
-
-static int eig_wpb_floats(int floats) {
-  // warps per block: the most resident warps per SM for this unit size
-  const size_t per = (size_t)floats * sizeof(float);
-  const size_t sm_bytes = 227 * 1024;
-  int wpb = 1, best = 0;
-  for (int c = 1; c <= 8; c++) {
-    if ((size_t)c * per > sm_bytes) break;
-    int blocks = (int)(sm_bytes / ((size_t)c * per + 1024));   // 1 KB reserved per block
-    if (blocks > 32) blocks = 32;
-    int warps = blocks * c;
-    if (warps > 64) warps = 64;
-    if (warps > best) { best = warps; wpb = c; }
-  }
-  return wpb;
-}
-
-static int eig_wpb(int k) { return eig_wpb_floats(eig_floats_per_warp(k)); }
-
-// warps per unit of k_eig_vec, measured on GB300: k <= 64 one warp (two
-// rows per lane; C2, k = 40: 26 ms against 33 with two warps), k > 64 four
-// warps (one row per thread; C4, k = 100: eigensolve 693 ms against 717 with
-// two warps of two rows per thread, whose 64-thread teams left 15% of the
-// warp slots filled)
-static int eig_team(int k) { return k <= 64 ? 1 : 4; }
-
-// The first stage, in registers with Q formed there: one warp up to k = 48
-// (k_eig_tri_r), above a team of ceil(k / 32) warps with one row per thread
-// (k_eig_tri_t).  Measured on GB300 (eigensolve ms): k = 40 shared-memory
-// full matrix 25.8, packed lower triangle 26.6, registers 23.7; k = 64 full
-// 57.2, packed 53.8, team registers 38.4; C4 (k = 100) full 1057, packed
-// (Q formed in k_eig_vec) 855, four-warp team registers 718.  The shared-memory
-// and packed forms are not built.
-
-// the register-resident first stage (k <= 48)
-static cudaError_t launch_tri_r(cudaStream_t st, const EigArgs &a, const EigSplit &sp, int u0, int nb) {
-  const int grid = (nb + RWPB - 1) / RWPB;
-  switch ((a.k + 7) & ~7) {
-  case 8: k_eig_tri_r<8><<<grid, 32 * RWPB, 0, st>>>(a, sp, u0, nb); break;
-  case 16: k_eig_tri_r<16><<<grid, 32 * RWPB, 0, st>>>(a, sp, u0, nb); break;
-  case 24: k_eig_tri_r<24><<<grid, 32 * RWPB, 0, st>>>(a, sp, u0, nb); break;
-  case 32: k_eig_tri_r<32><<<grid, 32 * RWPB, 0, st>>>(a, sp, u0, nb); break;
-  case 40: k_eig_tri_r<40><<<grid, 32 * RWPB, 0, st>>>(a, sp, u0, nb); break;
-  case 48: k_eig_tri_r<48><<<grid, 32 * RWPB, 0, st>>>(a, sp, u0, nb); break;
-  default: return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
-}
-
-// the register-resident first stage with a two-warp team per unit (48 < k <= 64)
-template <int K, int NW>
-static cudaError_t launch_tri_t_k(cudaStream_t st, const EigArgs &a, const EigSplit &sp, int u0, int nb) {
-  const size_t smem = tri_t_smem<K, NW>();
-  cudaError_t e = cudaFuncSetAttribute(k_eig_tri_t<K, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  k_eig_tri_t<K, NW><<<nb, 32 * NW, smem, st>>>(a, sp, u0, nb);
-  return cudaGetLastError();
-}
-
-static cudaError_t launch_tri_t(cudaStream_t st, const EigArgs &a, const EigSplit &sp, int u0, int nb) {
-  switch ((a.k + 7) & ~7) {
-  case 56: return launch_tri_t_k<56, 2>(st, a, sp, u0, nb);
-  case 64: return launch_tri_t_k<64, 2>(st, a, sp, u0, nb);
-  case 72: return launch_tri_t_k<72, 3>(st, a, sp, u0, nb);
-  case 80: return launch_tri_t_k<80, 3>(st, a, sp, u0, nb);
-  case 88: return launch_tri_t_k<88, 3>(st, a, sp, u0, nb);
-  case 96: return launch_tri_t_k<96, 3>(st, a, sp, u0, nb);
-  case 104: return launch_tri_t_k<104, 4>(st, a, sp, u0, nb);
-  case 112: return launch_tri_t_k<112, 4>(st, a, sp, u0, nb);
-  case 120: return launch_tri_t_k<120, 4>(st, a, sp, u0, nb);
-  case 128: return launch_tri_t_k<128, 4>(st, a, sp, u0, nb);
-  default: return cudaErrorInvalidValue;
-  }
-}
-
-template <int NQ, int NW>
-static cudaError_t launch_split_t(cudaStream_t st, const EigArgs &a, const EigSplit &sp, int batch, int ustart,
-                                  int ucount, int *launches) {
-  // k_eig_vec: its own warps per block from its shared memory
-  const int wpb = NW == 1 ? eig_wpb(a.k) : 1;
-  const size_t smem = (size_t)wpb * eig_floats_per_warp(a.k) * sizeof(float);
-  const int threads = NW == 1 ? 32 * wpb : 32 * NW;
-  cudaError_t e;
-  if ((e = cudaFuncSetAttribute(k_eig_vec<NQ, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-      cudaSuccess)
-    return e;
-  const size_t qsm = (size_t)2 * a.k * QLT * sizeof(float);
-  if ((e = cudaFuncSetAttribute(k_eig_ql, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qsm)) != cudaSuccess)
-    return e;
-  const int uend = ustart + ucount;
-  for (int u0 = ustart; u0 < uend; u0 += batch) {
-    const int nb = uend - u0 < batch ? uend - u0 : batch;
-    if ((e = a.k <= 48 ? launch_tri_r(st, a, sp, u0, nb) : launch_tri_t(st, a, sp, u0, nb)) != cudaSuccess) return e;
-    k_eig_ql<<<(nb + QLT - 1) / QLT, QLT, qsm, st>>>(a, sp, u0, nb);
-    k_eig_vec<NQ, NW><<<(nb + wpb - 1) / wpb, threads, smem, st>>>(a, sp, wpb, u0, nb);
-    (*launches) += 3;
-    if (a.flag_list) {
-      k_eig_flag<<<(nb + 7) / 8, 256, 0, st>>>(a, sp, u0, nb);
-      (*launches)++;
-    }
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  }
-  return cudaSuccess;
-}
-
-int eig_log_cap(int k) { return 2 * k * k + 4 * k + 64; }
-
-size_t eig_split_bytes_per_unit(int k) {
-  return (size_t)k * k * 4 + (size_t)2 * k * 4 + (size_t)eig_log_cap(k) * 8 + 4 + (size_t)k * 4;
-}
+size_t eig_split_bytes_per_unit(int k) { return (size_t)3 * k * 4 + 4; }
 
 cudaError_t launch_eig_split(cudaStream_t st, const EigArgs &a, const EigSplit &sp, int batch, int ustart, int ucount,
                              int *launches) {
   if (ucount <= 0) return cudaSuccess;
-  if (eig_team(a.k) == 1) return launch_split_t<2, 1>(st, a, sp, batch, ustart, ucount, launches);   // k <= 64
-  return launch_split_t<1, 4>(st, a, sp, batch, ustart, ucount, launches);                            // k <= 128
+  if (!a.flag_list) return launch_f32(st, a, EigSplit{}, ustart, ucount, launches);
+  const size_t qsm = (size_t)2 * a.k * QLT * sizeof(float);
+  cudaError_t e = cudaFuncSetAttribute(k_eig_ql, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qsm);
+  if (e != cudaSuccess) return e;
+  const int uend = ustart + ucount;
+  for (int u0 = ustart; u0 < uend; u0 += batch) {
+    const int nb = uend - u0 < batch ? uend - u0 : batch;
+    if ((e = launch_f32(st, a, sp, u0, nb, launches)) != cudaSuccess) return e;
+    k_eig_ql<<<(nb + QLT - 1) / QLT, QLT, qsm, st>>>(a, sp, u0, nb);
+    k_eig_flag<<<(nb + 7) / 8, 256, 0, st>>>(a, sp, u0, nb);
+    (*launches) += 2;
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 cudaError_t launch_eig_debug(cudaStream_t st, int nunits, int k, const float *G, const int *nkept, float *T,
@@ -1369,55 +1113,41 @@ cudaError_t launch_eig_debug(cudaStream_t st, int nunits, int k, const float *G,
   a.status = status;
   *nfp64 = 0;
   int l = 0;
+  // as lgpu_solver_run uses it
+  const size_t n = nunits > 0 ? nunits : 1;
+  const bool resolve = prec == LGPU_PREC_FP32_RESOLVE;
+  unsigned char *buf = nullptr;
+  const size_t vb = eig_scratch_bytes(k, (int)n, prec != LGPU_PREC_FP64, prec != LGPU_PREC_FP32);
+  // five arrays, each start rounded up to 256 bytes
+  cudaError_t e = cudaMalloc(&buf, vb + (resolve ? eig_split_bytes_per_unit(k) * n + 16 + 4 * n : 0) + 5 * 256);
+  if (e != cudaSuccess) return e;
+  size_t off = 0;
+  auto take = [&](size_t bytes) { unsigned char *p = buf + off; off += (bytes + 255) & ~(size_t)255; return p; };
+  a.scratch = take(vb);
   if (prec == LGPU_PREC_FP64) {
-    cudaError_t e = launch_eig64(st, a, 0, &l);
+    e = launch_eig64(st, a, 0, &l);
     cudaError_t e2 = cudaStreamSynchronize(st);
+    cudaFree(buf);
     *nfp64 = nunits;
     return e != cudaSuccess ? e : e2;
   }
-  // the split pipeline, as lgpu_solver_run uses it
-  const size_t per = eig_split_bytes_per_unit(k);
-  const size_t n = nunits > 0 ? nunits : 1;
-  unsigned char *buf = nullptr;
-  // six arrays, each start rounded up to 256 bytes (at most 5 * 255 bytes of padding)
-  cudaError_t e = cudaMalloc(&buf, per * n + 16 + 4 * n + 6 * 256);
-  if (e != cudaSuccess) return e;
-  EigSplit sp;
-  size_t off = 0;
-  auto take = [&](size_t bytes) { unsigned char *p = buf + off; off += (bytes + 255) & ~(size_t)255; return p; };
-  sp.Q = reinterpret_cast<float *>(take(n * k * k * 4));
-  sp.DE = reinterpret_cast<float *>(take(n * 2 * k * 4));
-  sp.log = reinterpret_cast<float2 *>(take(n * (size_t)eig_log_cap(k) * 8));
-  sp.logn = reinterpret_cast<int *>(take(n * 4));
-  sp.lam = reinterpret_cast<float *>(take(n * k * 4));
-  sp.cap = eig_log_cap(k);
-  if (prec == LGPU_PREC_FP32_RESOLVE) {
+  EigSplit sp{};
+  if (resolve) {
+    sp.DE = reinterpret_cast<float *>(take(n * 2 * k * 4));
+    sp.lam = reinterpret_cast<float *>(take(n * k * 4));
+    sp.bad = reinterpret_cast<int *>(take(n * 4));
     a.flag_n = reinterpret_cast<int *>(take(16 + 4 * n));
     a.flag_list = a.flag_n + 4;
     a.flag_cap = (int)n;
     e = cudaMemsetAsync(a.flag_n, 0, 16, st);
   }
-  if (e == cudaSuccess) e = launch_eig_split(st, a, sp, nunits, 0, nunits, &l);
+  if (e == cudaSuccess) e = launch_eig_split(st, a, sp, (int)n, 0, nunits, &l);
   if (e == cudaSuccess && a.flag_list) e = launch_eig64_flagged(st, a, &l);
   if (e == cudaSuccess && a.flag_n) e = cudaMemcpyAsync(nfp64, a.flag_n, 4, cudaMemcpyDeviceToHost, st);
   cudaError_t e2 = cudaStreamSynchronize(st);
   cudaFree(buf);
   if (*nfp64 > (int)n) *nfp64 = (int)n;
   return e != cudaSuccess ? e : e2;
-}
-
-cudaError_t launch_eig(cudaStream_t st, const EigArgs &a, int *launches) {
-  if (a.nunits <= 0) return cudaSuccess;
-  const int wpb = eig_wpb(a.k);
-  const size_t per = (size_t)eig_floats_per_warp(a.k) * sizeof(float);
-  const size_t smem = (size_t)wpb * per;
-  auto fused = a.k > 64 ? k_eig<4> : k_eig<2>;
-  cudaError_t e = cudaFuncSetAttribute(fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  const int grid = (a.nunits + wpb - 1) / wpb;
-  fused<<<grid, 32 * wpb, smem, st>>>(a, wpb);
-  (*launches)++;
-  return cudaGetLastError();
 }
 
 }  // namespace lgpu

@@ -522,8 +522,8 @@ struct EigArgs {
   float *wbar;            // [unit][k] mean weights, or null
   const int *ulist;       // units to solve (the i-th is ulist[i]), or null: units 0..nunits-1
   int *status;            // [1] accumulated error bits
-  // FP64 re-solve (split pipeline): a unit whose FP32 solve failed (no
-  // convergence, a non-positive or non-finite eigenvalue) or whose relevant
+  // FP64 re-solve: a unit whose FP32 solve failed (non-finite, or not
+  // positive definite) or whose relevant
   // FP32 eigenvalues (those above the (k-1)/infl floor by more than the
   // rounding level) have a relative gap min|l_i - l_j| / max l <= gap_thresh
   // is appended to flag_list (flag_n[0] = entries written, at most
@@ -531,26 +531,28 @@ struct EigArgs {
   int *flag_list, *flag_n;
   int flag_cap;
   float gap_thresh;
+  void *scratch;          // eig_scratch_bytes: the reflectors of the units in flight
 };
-// FP64 eigensolve + transform (a team of warps per unit): units ulist[0..nunits) or
+// the FP32 eigendecomposition form (lgpu_eig_rows.cu) of units 0..nunits, for
+// the solutions stored as training rows; scratch of eig_rows_bytes
+size_t eig_rows_bytes(int k, int units);
+cudaError_t launch_eig_rows(cudaStream_t st, const EigArgs &a, int *launches);
+// scratch of launches over at most `units` units at a time in the precisions named
+size_t eig_scratch_bytes(int k, int units, bool fp32, bool fp64);
+// FP64 transform (a team of warps per unit): units ulist[0..nunits) or
 // ubase + 0..nunits; T (and w-bar) written in FP32
 cudaError_t launch_eig64(cudaStream_t st, const EigArgs &a, int ubase, int *launches);
 // FP64 re-solve of the flagged units not yet re-solved (flag_list entries
 // flag_n[1] .. flag_n[0]); the count stays on the device
 cudaError_t launch_eig64_flagged(cudaStream_t st, const EigArgs &a, int *launches);
-cudaError_t launch_eig(cudaStream_t st, const EigArgs &a, int *launches);
-// scratch of the split eigensolve pipeline, for `batch` units
+// scratch of the gap test (FP32_RESOLVE) for `batch` units; null: no test
 struct EigSplit {
-  float *Q;        // [batch][k][k] Householder Q, row-major
-  float *DE;       // [batch][2k] diagonal, off-diagonal
-  float2 *log;     // [batch][cap] sweep headers (start, count) and rotations (c, s)
-  int *logn;       // [batch] log entries, -1 no convergence, -2 overflow
+  float *DE;       // [batch][2k] diagonal, off-diagonal of the tridiagonal form
   float *lam;      // [batch][k] eigenvalues
-  int cap;
+  int *bad;        // [batch] FP32 solve failed
 };
-int eig_log_cap(int k);
 size_t eig_split_bytes_per_unit(int k);
-// units [ustart, ustart + ucount), in batches of at most `batch`
+// units [ustart, ustart + ucount); with flagging in batches of at most `batch`
 cudaError_t launch_eig_split(cudaStream_t st, const EigArgs &a, const EigSplit &sp, int batch, int ustart, int ucount,
                              int *launches);
 
