@@ -869,7 +869,7 @@ static int eig_scratch(lgpu_handle *h, int units, EigArgs &ea, EigSplit &sp, int
     const size_t per = eig_split_bytes_per_unit(k);
     const size_t budget = (size_t)8 << 30;
     batch = (int)std::min<size_t>((size_t)batch, std::max<size_t>(1024, budget / per));
-    need += per * (size_t)batch + 3 * 256;
+    need += per * (size_t)batch + 2 * 256;
   }
   CK(h->buf[B_EIGSCR].ensure(need), "alloc transform scratch");
   unsigned char *base = h->buf[B_EIGSCR].as<unsigned char>();
@@ -878,7 +878,6 @@ static int eig_scratch(lgpu_handle *h, int units, EigArgs &ea, EigSplit &sp, int
   ea.scratch = take(vb);
   if (!resolve) return LGPU_OK;
   sp.DE = reinterpret_cast<float *>(take((size_t)batch * 2 * k * 4));
-  sp.lam = reinterpret_cast<float *>(take((size_t)batch * k * 4));
   sp.bad = reinterpret_cast<int *>(take((size_t)batch * 4));
   return LGPU_OK;
 }

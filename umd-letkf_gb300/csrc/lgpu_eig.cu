@@ -135,49 +135,91 @@ template <> struct PolesOf<double> { using type = PolesD; static const PolesD &g
 
 __device__ __forceinline__ float fmar(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fmar(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float rcpr(float x) { return __frcp_rn(x); }
-__device__ __forceinline__ double rcpr(double x) { return __drcp_rn(x); }
-// unit roundoff and the smallest scale treated as zero, per precision
+// the smallest scale treated as zero, per precision
 template <class R> struct Lim;
 // (`zero`: a squared norm that no rounding of the diagonal, at least 1, can see)
 template <> struct Lim<float> {
-  static constexpr float eps = 1.1920929e-7f, tiny = 1e-30f, zero = 1e-34f;
+  static constexpr float tiny = 1e-30f, zero = 1e-34f;
 };
 template <> struct Lim<double> {
-  static constexpr double eps = 2.220446049250313e-16, tiny = 1e-300, zero = 1e-200;
+  static constexpr double tiny = 1e-300, zero = 1e-200;
 };
 
-// four consecutive values, 16-byte aligned
-__device__ __forceinline__ void ld4(const float *p, float *v) {
-  const float4 t = *reinterpret_cast<const float4 *>(p);
-  v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+// Two values of neighbouring lane columns.  FP32: a register pair for the
+// packed multiply-add, which does both in one issue slot.
+template <class R> struct Pair;
+template <>
+struct Pair<float> {
+  unsigned long long u;
+  __device__ __forceinline__ Pair() {}
+  __device__ __forceinline__ Pair(float x, float y) { asm("mov.b64 %0, {%1, %2};" : "=l"(u) : "f"(x), "f"(y)); }
+  __device__ __forceinline__ float x() const { return __uint_as_float((unsigned)u); }
+  __device__ __forceinline__ float y() const { return __uint_as_float((unsigned)(u >> 32)); }
+};
+template <>
+struct Pair<double> {
+  double a, b;
+  __device__ __forceinline__ Pair() {}
+  __device__ __forceinline__ Pair(double x, double y) : a(x), b(y) {}
+  __device__ __forceinline__ double x() const { return a; }
+  __device__ __forceinline__ double y() const { return b; }
+};
+__device__ __forceinline__ Pair<float> pfma(Pair<float> a, Pair<float> b, Pair<float> c) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c.u) : "l"(a.u), "l"(b.u));
+  return c;
 }
-__device__ __forceinline__ void ld4(const double *p, double *v) {
-  const double2 t = *reinterpret_cast<const double2 *>(p), u = *reinterpret_cast<const double2 *>(p + 2);
-  v[0] = t.x; v[1] = t.y; v[2] = u.x; v[3] = u.y;
+__device__ __forceinline__ Pair<double> pfma(Pair<double> a, Pair<double> b, Pair<double> c) {
+  return Pair<double>(__fma_rn(a.a, b.a, c.a), __fma_rn(a.b, b.b, c.b));
+}
+__device__ __forceinline__ Pair<float> padd(Pair<float> a, Pair<float> b) {
+  asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a.u) : "l"(b.u));
+  return a;
+}
+__device__ __forceinline__ Pair<double> padd(Pair<double> a, Pair<double> b) { return Pair<double>(a.a + b.a, a.b + b.b); }
+
+// the element of lane column i (a constant after unrolling) of a row of pairs
+template <class R>
+__device__ __forceinline__ R get(const Pair<R> *p, int i) { return i & 1 ? p[i / 2].y() : p[i / 2].x(); }
+template <class R>
+__device__ __forceinline__ void set(Pair<R> *p, int i, R v) {
+  p[i / 2] = i & 1 ? Pair<R>(p[i / 2].x(), v) : Pair<R>(v, p[i / 2].y());
 }
 
-__device__ __forceinline__ void st4(float *p, const float *v) {
-  *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+// two pairs, 16-byte aligned in FP32
+__device__ __forceinline__ void ld2(const float *p, Pair<float> *v) {
+  const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(p);
+  v[0].u = t.x;
+  v[1].u = t.y;
 }
-__device__ __forceinline__ void st4(double *p, const double *v) {
-  *reinterpret_cast<double2 *>(p) = make_double2(v[0], v[1]);
-  *reinterpret_cast<double2 *>(p + 2) = make_double2(v[2], v[3]);
+__device__ __forceinline__ void ld2(const double *p, Pair<double> *v) {
+  const double2 t = *reinterpret_cast<const double2 *>(p), u = *reinterpret_cast<const double2 *>(p + 2);
+  v[0] = Pair<double>(t.x, t.y);
+  v[1] = Pair<double>(u.x, u.y);
+}
+__device__ __forceinline__ void st2(float *p, Pair<float> a, Pair<float> b) {
+  *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(a.u, b.u);
+}
+__device__ __forceinline__ void st2(double *p, Pair<double> a, Pair<double> b) {
+  *reinterpret_cast<double2 *>(p) = make_double2(a.a, a.b);
+  *reinterpret_cast<double2 *>(p + 2) = make_double2(b.a, b.b);
 }
 
 // sqrt and reciprocal of positive normal values, to an ulp or so: the
 // hardware's approximations and one Newton step, without the rounded forms'
 // range checks
 __device__ __forceinline__ float sqrt_pos(float x) {
-  const float r = rsqrtf(x), q = x * r;
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  const float q = x * r;
   return fmar(0.5f * r, fmar(-q, q, x), q);
 }
 __device__ __forceinline__ double sqrt_pos(double x) { return sqrt(x); }
 __device__ __forceinline__ float rcp_pos(float x) {
-  const float r = __fdividef(1.0f, x);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return fmar(r, fmar(-x, r, 1.0f), r);
 }
-__device__ __forceinline__ double rcp_pos(double x) { return rcpr(x); }
+__device__ __forceinline__ double rcp_pos(double x) { return __drcp_rn(x); }
 
 // 16 bytes global -> shared, asynchronously
 __device__ __forceinline__ void copy16_async(void *dst, const void *src) {
@@ -190,32 +232,44 @@ __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group 
 
 // The lane grid of one unit: RN rows and CN columns per lane; LA is a
 // multiple of LB, and LB <= 8 divides a warp, so the lanes of a row lie in one warp.
-template <class R_, int RN_, int CN_, int LA_, int LB_, int MB_>
+template <class R_, int RN_, int CN_, int LA_, int LB_, int MB_, bool KEEP_ = true>
 struct Grid {
   using R = R_;
   static constexpr int RN = RN_, CN = CN_, LA = LA_, LB = LB_;
+  static constexpr bool KEEP = KEEP_;                       // the reflector stays in registers between its two uses
   static constexpr int MB = MB_;                            // blocks per SM the registers are bounded for
   static constexpr int L = LA * LB;
+  static constexpr int CH2 = CN / 2;                        // column pairs per lane
+  using Row = Pair<R>[CN / 2];
   static constexpr int KR = LA * RN, KC = LB * CN;          // covered rows, columns
-  static constexpr int CP = (CN + 3) / 4 * 4;               // values of one lane column, padded to 16-byte vectors
+  // values of one lane column: whole 16-byte vectors, one more where the lane
+  // columns' vectors would start in the same banks
+  static constexpr int CP4 = (CN + 3) / 4 * 4;
+  static constexpr int CP = LB > 1 && CP4 % (64 / LB) == 0 ? CP4 + 4 : CP4;
   static constexpr int VB = LB * CP;                        // one column-ordered vector
   static constexpr int NP = sizeof(R) == 4 ? 16 : 32;
   static constexpr int KM = KR > KC ? KR : KC;
   static constexpr int KN = (KM + 3) / 4 * 4;               // one naturally ordered vector
-  static constexpr int PS = 2 * KN + 8 + VB;                // one shift's arrays: rho (8 zeros of slack), g, LB-products
+  // one shift's arrays: rho (8 zeros of slack), g, LB-products; the lanes'
+  // arrays start a 16-byte bank group apart
+  static constexpr int PS = (2 * KN + 8 + VB + 27) / 32 * 32 + 4;
   static constexpr int VEC = 4 * KN;                        // d, e, tau, z
   static constexpr int STEP = 6 * VB;                       // reduction: x, v, w (double-buffered); back: w, ring of 4 v
   static constexpr int CH = L >= 32 ? NP : L - 2;           // shifts of one pass: with the solve and the test, a lane each
   static constexpr int POLE = (CH + 2) * PS;
   static constexpr int TRANS = LA * VB;                     // one row group
-  static constexpr int WORK0 = STEP > POLE ? STEP : POLE;
-  static constexpr int UNIT = VEC + (WORK0 > TRANS ? WORK0 : TRANS);   // values of one unit
+  static constexpr int PACK = KC * (KC + 3) / 2;            // the packed Gram block
+  static constexpr int WORK0 = STEP > POLE ? STEP : POLE, WORK1 = WORK0 > TRANS ? WORK0 : TRANS;
+  static constexpr int UNIT0 = VEC + (WORK1 > PACK ? WORK1 : PACK);
+  // values of one unit: 8 past a multiple of 32, so that the units of a warp
+  // read different banks
+  static constexpr int UNIT = (UNIT0 + 23) / 32 * 32 + 8;
   static constexpr int REFL = KC * VB;                      // the reflectors of one unit (global scratch)
   static constexpr int UPW = L < 32 ? 32 / L : 1;           // units per warp
   static constexpr int UPB = L <= 32 ? 4 * UPW : 1;         // units per block
   static constexpr int THREADS = L <= 32 ? 128 : L;
-  static_assert(LA % LB == 0 && LB <= 8, "lane grid");
-  static_assert(KR / LB <= CP && (L > 32 || KR == KC), "every row has a place in a column-ordered vector");
+  static_assert(LA % LB == 0 && LB <= 8 && CN % 2 == 0, "lane grid");
+  static_assert(KR / LB <= CP && KR >= KC && (L > 32 || KR == KC), "every row has a place in a column-ordered vector");
 };
 
 template <class G>
@@ -236,17 +290,17 @@ __device__ __forceinline__ R sum_b(R v) {
 template <class G>
 __device__ __forceinline__ int vpos(int c) { return (c % G::LB) * G::CP + c / G::LB; }
 
-// the lane's columns i >= I0 of a column-ordered vector
-template <class G, int I0, class R>
-__device__ __forceinline__ void load_cols(const R *buf, int b, R *v) {
+// the lane's column pairs q >= Q0 of a column-ordered vector
+template <class G, int Q0, class R>
+__device__ __forceinline__ void load_cols(const R *buf, int b, Pair<R> *v) {
   const R *p = buf + b * G::CP;
 #pragma unroll
-  for (int q = I0 / 4; q < G::CP / 4; q++) {
-    R t[4];
-    ld4(p + 4 * q, t);
+  for (int q = Q0 / 2; q < G::CP / 4; q++) {
+    Pair<R> t[2];
+    ld2(p + 4 * q, t);
 #pragma unroll
-    for (int j = 0; j < 4; j++)
-      if (4 * q + j >= I0 && 4 * q + j < G::CN) v[4 * q + j] = t[j];
+    for (int j = 0; j < 2; j++)
+      if (2 * q + j >= Q0 && 2 * q + j < G::CH2) v[2 * q + j] = t[j];
   }
 }
 
@@ -266,17 +320,14 @@ __device__ __forceinline__ void store_rows(R *buf, int a, const R *v) {
   for (int r = R0; r < G::RN; r++) p[(G::LA / G::LB) * r] = v[r];
 }
 
-// the lane's columns i >= I0 into a column-ordered vector (whole 16-byte groups)
-template <class G, int I0, class R>
-__device__ __forceinline__ void store_cols(R *buf, int b, const R *v) {
+// the lane's column pairs into a column-ordered vector, from the 16-byte group
+// of pair Q0 on
+template <class G, int Q0, class R>
+__device__ __forceinline__ void store_cols(R *buf, int b, const Pair<R> *v) {
   R *p = buf + b * G::CP;
 #pragma unroll
-  for (int q = I0 / 4; q < G::CP / 4; q++) {
-    R t[4];
-#pragma unroll
-    for (int j = 0; j < 4; j++) t[j] = 4 * q + j < G::CN ? v[4 * q + j] : R(0);
-    st4(p + 4 * q, t);
-  }
+  for (int q = Q0 / 2; q < G::CP / 4; q++)
+    st2(p + 4 * q, v[2 * q], 2 * q + 1 < G::CH2 ? v[2 * q + 1] : Pair<R>(R(0), R(0)));
 }
 
 // the unit's shared-memory vectors
@@ -343,22 +394,23 @@ struct Vec {
 };
 
 // The two-sided update M -= v w^T + w v^T with w = p - (t/2)(p.v) v, p = t M v.
-// vcol / vrow: the reflector at the lane's columns and rows, zero up to j
-// (columns below I0 and rows below R0 not set).  FULL (back-transformation):
-// every row and column; else (reduction) the trailing block, where w is zero
-// up to j.
-template <class G, int R0, int I0, bool FULL>
-__device__ __forceinline__ void two_sided(typename G::R (&A)[G::RN][G::CN], typename G::R *wb, int j, int a, int b, typename G::R t,
-                                          const typename G::R *vcol, const typename G::R *vrow) {
+// vb, vcol / vrow: the reflector in shared memory and at the lane's column
+// pairs from Q0 and rows from R0, zero up to j.  FULL (back-transformation): every row and column; else
+// (reduction) the trailing block, where w is zero up to j.
+template <class G, int R0, int Q0, bool FULL>
+__device__ __forceinline__ void two_sided(typename G::Row (&A)[G::RN], typename G::R *wb, int j, int a, int b,
+                                          typename G::R t, const typename G::R *vb, const Pair<typename G::R> *vcol,
+                                          const typename G::R *vrow) {
   using R = typename G::R;
-  constexpr int W0 = FULL ? 0 : R0, C0 = FULL ? 0 : I0;
+  using P2 = Pair<R>;
+  constexpr int W0 = FULL ? 0 : R0, C0 = FULL ? 0 : Q0;
   R w[G::RN];
 #pragma unroll
   for (int r = W0; r < G::RN; r++) {
-    R acc = R(0);
+    P2 acc(R(0), R(0));
 #pragma unroll
-    for (int i = I0; i < G::CN; i++) acc = fmar(A[r][i], vcol[i], acc);
-    w[r] = acc;
+    for (int q = Q0; q < G::CH2; q++) acc = pfma(A[r][q], vcol[q], acc);
+    w[r] = acc.x() + acc.y();
   }
 #pragma unroll
   for (int r = W0; r < G::RN; r++) w[r] = t * sum_b<G>(w[r]);
@@ -375,20 +427,27 @@ __device__ __forceinline__ void two_sided(typename G::R (&A)[G::RN][G::CN], type
     if (!FULL) w[R0] = a + G::LA * R0 > j ? w[R0] : R(0);
     if (b == 0) store_rows<G, W0>(wb, a, w);
     team_sync<G>();
-    const R *wp = wb + b * G::CP;
+    P2 nw[G::RN], nv[G::RN];
 #pragma unroll
-    for (int q = C0 / 4; q < G::CP / 4; q++) {
-      R wc[4];
-      ld4(wp + 4 * q, wc);
+    for (int r = W0; r < G::RN; r++) {
+      nw[r] = P2(-w[r], -w[r]);
+      if (r >= R0) nv[r] = P2(-vrow[r], -vrow[r]);
+    }
+    const R *wp = wb + b * G::CP, *vp = vb + b * G::CP;
 #pragma unroll
-      for (int jj = 0; jj < 4; jj++) {
-        const int i = 4 * q + jj;
-        if (i < C0 || i >= G::CN) continue;
+    for (int q = C0 / 2; q < G::CP / 4; q++) {
+      P2 wc[2], vc[2];
+      ld2(wp + 4 * q, wc);
+      if (!G::KEEP && q >= Q0 / 2) ld2(vp + 4 * q, vc);
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int i = 2 * q + h;
+        if (i < C0 || i >= G::CH2) continue;
 #pragma unroll
         for (int r = W0; r < G::RN; r++) {
-          R x = A[r][i];
-          if (i >= I0) x = fmar(-w[r], vcol[i], x);
-          if (r >= R0) x = fmar(-vrow[r], wc[jj], x);
+          P2 x = A[r][i];
+          if (i >= Q0) x = pfma(nw[r], G::KEEP ? vcol[i] : vc[h], x);
+          if (r >= R0) x = pfma(nv[r], wc[h], x);
           A[r][i] = x;
         }
       }
@@ -399,72 +458,85 @@ __device__ __forceinline__ void two_sided(typename G::R (&A)[G::RN][G::CN], type
     if (!FULL) w[R0] = a + G::LA * R0 > j ? w[R0] : R(0);
     if (b == 0) store_rows<G, W0>(wb, a, w);
     team_sync<G>();
-    R wc[G::CN];
+    P2 wc[G::CH2], pv(R(0), R(0));
     load_cols<G, C0>(wb, b, wc);
-    R pv = R(0);
 #pragma unroll
-    for (int i = I0; i < G::CN; i++) pv = fmar(wc[i], vcol[i], pv);
-    const R beta = R(0.5) * t * sum_b<G>(pv);
+    for (int q = Q0; q < G::CH2; q++) pv = pfma(wc[q], vcol[q], pv);
+    const R beta = R(0.5) * t * sum_b<G>(pv.x() + pv.y());
+    const P2 nb(-beta, -beta);
 #pragma unroll
-    for (int i = I0; i < G::CN; i++) wc[i] = fmar(-beta, vcol[i], wc[i]);
+    for (int q = Q0; q < G::CH2; q++) wc[q] = pfma(nb, vcol[q], wc[q]);
 #pragma unroll
     for (int r = R0; r < G::RN; r++) w[r] = fmar(-beta, vrow[r], w[r]);
 #pragma unroll
-    for (int r = W0; r < G::RN; r++)
+    for (int r = W0; r < G::RN; r++) {
+      const P2 nw(-w[r], -w[r]), nv(r >= R0 ? -vrow[r] : R(0), r >= R0 ? -vrow[r] : R(0));
 #pragma unroll
-      for (int i = C0; i < G::CN; i++) {
-        R x = A[r][i];
-        if (i >= I0) x = fmar(-w[r], vcol[i], x);
-        if (r >= R0) x = fmar(-vrow[r], wc[i], x);
-        A[r][i] = x;
+      for (int q = C0; q < G::CH2; q++) {
+        P2 x = A[r][q];
+        if (q >= Q0) x = pfma(nw, vcol[q], x);
+        if (r >= R0) x = pfma(nv, wc[q], x);
+        A[r][q] = x;
       }
+    }
   }
+}
+
+// alpha = -sign(x0) |x| and t = 2 / v^T v of v = x - alpha e_1 (t = 0, alpha =
+// x0: x is e_1's multiple to the last bit)
+template <class R>
+__device__ __forceinline__ void reflector(bool on, R s1, R x0, R &alpha, R &t) {
+  const R sig = fmar(x0, x0, s1);
+  const bool live = on && s1 > Lim<R>::tiny * sig && sig > Lim<R>::zero;
+  const R root = -copysign(sqrt_pos(sig), x0);
+  const R rt = rcp_pos(fmar(-root, x0, sig));
+  alpha = live ? root : x0;
+  t = live ? rt : R(0);
 }
 
 // Reduction steps of rows [LA P, LA P + LA): d, e, tau, the reflectors to the
 // scratch gv (one column-ordered vector a step), y = Q^T b.
 template <class G, int P>
-__device__ __forceinline__ void reduce_phase(typename G::R (&A)[G::RN][G::CN], const UnitMem<G> &U, Vec<G> &z,
+__device__ __forceinline__ void reduce_phase(typename G::Row (&A)[G::RN], const UnitMem<G> &U, Vec<G> &z,
                                              typename G::R *gv, int k, int l, int a, int b) {
   using R = typename G::R;
-  constexpr int R0 = P, I0 = (P * G::LA + 1) / G::LB;
+  constexpr int R0 = P, I0 = (P * G::LA + 1) / G::LB, Q0 = I0 / 2;
   constexpr int CB = P * G::LA / G::LB;                       // column group of column LA P
   constexpr int NB = G::LA / G::LB;                           // column groups of the phase's columns
   const int jend = k < P * G::LA + G::LA ? k : P * G::LA + G::LA;
+  R tp = R(0);
+#pragma unroll 1
   for (int j = P * G::LA; j < jend; j++) {
     const bool own = a == j - P * G::LA;
-    R vcol[G::CN], vrow[G::RN], t = R(0);
+    Pair<R> vcol[G::CH2];
+    R vrow[G::RN], t = R(0);
     if constexpr (G::L <= 32) {
       // one warp: the row is published as it stands, and every lane forms the
-      // reflector from its own columns
+      // reflector from its own columns; the right-hand side takes the
+      // reflector of the step before meanwhile
       R *xb = U.x(j), *vb = U.v(j);
-      if (own) store_cols<G, CB>(xb, b, A[R0]);
+      if (own) store_cols<G, CB / 2>(xb, b, A[R0]);
       team_sync<G>();
       const R x0 = j + 1 < G::KC ? xb[vpos<G>(j + 1)] : R(0);
       if (j >= k - 2) {                        // the last 2 x 2 block
         if (l == 0) { U.d[j] = xb[vpos<G>(j)]; U.e[j] = j < k - 1 ? x0 : R(0); }
         continue;
       }
-      load_cols<G, I0>(xb, b, vcol);
+      load_cols<G, Q0>(xb, b, vcol);
       load_rows<G, R0>(xb, a, vrow);
-      R s4[4] = {R(0), R(0), R(0), R(0)};
+      if (j > P * G::LA) z.template reflect<P * G::LA>(U, k, l, 0, tp, U.v(j - 1));
 #pragma unroll
-      for (int i = I0; i < G::CN; i++) {
-        if (i <= CB + NB) vcol[i] = b + G::LB * i > j + 1 ? vcol[i] : R(0);
-        s4[i & 3] = fmar(vcol[i], vcol[i], s4[i & 3]);
-      }
-      const R s1 = sum_b<G>((s4[0] + s4[1]) + (s4[2] + s4[3]));
-      const R sig = fmar(x0, x0, s1);
-      const bool live = s1 > Lim<R>::tiny * sig && sig > Lim<R>::zero;
-      R alpha = x0;
-      if (live) {
-        alpha = -copysign(sqrt_pos(sig), x0);
-        t = rcp_pos(fmar(-alpha, x0, sig));     // 2 / v^T v, v = x - alpha e_1
-      }
+      for (int i = 2 * Q0; i < G::CN; i++)
+        if (i <= CB + NB) set(vcol, i, b + G::LB * i > j + 1 ? get(vcol, i) : R(0));
+      Pair<R> s2[2] = {Pair<R>(R(0), R(0)), Pair<R>(R(0), R(0))};
+#pragma unroll
+      for (int q = Q0; q < G::CH2; q++) s2[q & 1] = pfma(vcol[q], vcol[q], s2[q & 1]);
+      R alpha;
+      reflector(true, sum_b<G>((s2[0].x() + s2[0].y()) + (s2[1].x() + s2[1].y())), x0, alpha, t);
       const R v0 = x0 - alpha;
 #pragma unroll
-      for (int i = I0; i < G::CN; i++)
-        if (i <= CB + NB) vcol[i] = b + G::LB * i == j + 1 ? v0 : vcol[i];
+      for (int i = 2 * Q0; i < G::CN; i++)
+        if (i <= CB + NB) set(vcol, i, b + G::LB * i == j + 1 ? v0 : get(vcol, i));
 #pragma unroll
       for (int r = R0; r < G::RN; r++)
         if (r <= R0 + 1) {
@@ -472,42 +544,40 @@ __device__ __forceinline__ void reduce_phase(typename G::R (&A)[G::RN][G::CN], c
           vrow[r] = row > j + 1 ? vrow[r] : (row == j + 1 ? v0 : R(0));
         }
       if (own) {
-        if (I0 > CB) vcol[CB] = R(0);
-        store_cols<G, CB>(vb, b, vcol);
-        store_cols<G, CB>(gv + (size_t)j * G::VB, b, vcol);
+        if (Q0 > CB / 2) vcol[CB / 2] = Pair<R>(R(0), R(0));
+        store_cols<G, CB / 2>(vb, b, vcol);
+        store_cols<G, CB / 2>(gv + (size_t)j * G::VB, b, vcol);
       }
       if (l == 0) { U.tau[j] = t; U.e[j] = alpha; U.d[j] = xb[vpos<G>(j)]; }
     } else {
       // a team: the warp of the row forms the reflector and publishes it
       R *vb = U.v(j);
       if ((l >> 5) == (j - P * G::LA) * G::LB / 32) {
-        R s1 = R(0), x0 = R(0), dj = R(0), x[G::CN];
+        R x0 = R(0), dj = R(0);
+        Pair<R> x[G::CH2], s2(R(0), R(0));
 #pragma unroll
-        for (int i = CB; i < G::CN; i++) {
-          const int c = b + G::LB * i;
-          x[i] = A[R0][i];
+        for (int q = CB / 2; q < G::CH2; q++) x[q] = A[R0][q];
+#pragma unroll
+        for (int i = CB / 2 * 2; i < G::CN; i++)
           if (i <= CB + NB) {
-            if (c == j + 1) x0 = x[i];
-            if (c == j) dj = x[i];
-            x[i] = c > j + 1 ? x[i] : R(0);
+            const int c = b + G::LB * i;
+            const R xi = get(x, i);
+            if (c == j + 1) x0 = xi;
+            if (c == j) dj = xi;
+            set(x, i, c > j + 1 ? xi : R(0));
           }
-          s1 = fmar(x[i], x[i], s1);
-        }
-        s1 = sum_b<G>(s1);
+#pragma unroll
+        for (int q = CB / 2; q < G::CH2; q++) s2 = pfma(x[q], x[q], s2);
+        R alpha;
         x0 = sum_b<G>(x0);
-        const R sig = fmar(x0, x0, s1);
-        R alpha = x0;
-        if (j < k - 2 && s1 > Lim<R>::tiny * sig && sig > Lim<R>::zero) {
-          alpha = -copysign(sqrt_pos(sig), x0);
-          t = rcp_pos(fmar(-alpha, x0, sig));
-        }
+        reflector(j < k - 2, sum_b<G>(s2.x() + s2.y()), x0, alpha, t);
         const R v0 = x0 - alpha;
         if (own) {
 #pragma unroll
-          for (int i = CB; i < G::CN; i++)
-            if (i <= CB + NB) x[i] = b + G::LB * i == j + 1 ? v0 : x[i];
-          store_cols<G, CB>(vb, b, x);
-          store_cols<G, CB>(gv + (size_t)j * G::VB, b, x);
+          for (int i = CB / 2 * 2; i < G::CN; i++)
+            if (i <= CB + NB) set(x, i, b + G::LB * i == j + 1 ? v0 : get(x, i));
+          store_cols<G, CB / 2>(vb, b, x);
+          store_cols<G, CB / 2>(gv + (size_t)j * G::VB, b, x);
           if (b == 0) { U.tau[j] = t; U.e[j] = alpha; }
           if (b == j % G::LB) U.d[j] = dj;
         }
@@ -515,12 +585,18 @@ __device__ __forceinline__ void reduce_phase(typename G::R (&A)[G::RN][G::CN], c
       if (j >= k - 2) continue;
       team_sync<G>();
       t = U.tau[j];
-      load_cols<G, I0>(vb, b, vcol);
+      load_cols<G, Q0>(vb, b, vcol);
       load_rows<G, R0>(vb, a, vrow);
     }
-    two_sided<G, R0, I0, false>(A, U.w(j), j, a, b, t, vcol, vrow);
-    z.template reflect<P * G::LA>(U, k, l, ((j - P * G::LA) * G::LB / 32 + G::L / 64) % (G::L < 32 ? 1 : G::L / 32), t,
-                                  U.v(j));
+    two_sided<G, R0, Q0, false>(A, U.w(j), j, a, b, t, U.v(j), vcol, vrow);
+    if constexpr (G::L > 32)
+      z.template reflect<P * G::LA>(U, k, l, ((j - P * G::LA) * G::LB / 32 + G::L / 64) % (G::L / 32), t, U.v(j));
+    tp = t;
+  }
+  if constexpr (G::L <= 32) {
+    // the phase's last reflector
+    const int jl = jend - 1 < k - 3 ? jend - 1 : k - 3;
+    if (jl >= P * G::LA) z.template reflect<P * G::LA>(U, k, l, 0, tp, U.v(jl));
   }
 }
 
@@ -537,27 +613,30 @@ __device__ __forceinline__ void fetch_reflector(const UnitMem<G> &U, const typen
 // Back-transformation steps of columns [LA P, LA P + LA), last first:
 // M <- H_j M H_j and z <- H_j z.
 template <class G, int P>
-__device__ __forceinline__ void back_phase(typename G::R (&A)[G::RN][G::CN], const UnitMem<G> &U, Vec<G> &z,
+__device__ __forceinline__ void back_phase(typename G::Row (&A)[G::RN], const UnitMem<G> &U, Vec<G> &z,
                                            const typename G::R *gv, int k, int l, int a, int b) {
   using R = typename G::R;
-  constexpr int R0 = P, I0 = (P * G::LA + 1) / G::LB;
+  constexpr int R0 = P, Q0 = (P * G::LA + 1) / G::LB / 2;
   const int jtop = k - 3 < P * G::LA + G::LA - 1 ? k - 3 : P * G::LA + G::LA - 1;
+#pragma unroll 1
   for (int j = jtop; j >= P * G::LA; j--) {
     copy_wait<2>();
     team_sync<G>();
     fetch_reflector<G>(U, gv, j - 3, l);       // into the slot of step j + 1, which every lane has left
     const R *vb = U.ring(j);
     const R t = U.tau[j];
-    R vcol[G::CN], vrow[G::RN];
-    load_cols<G, I0>(vb, b, vcol);
+    Pair<R> vcol[G::CH2];
+    R vrow[G::RN];
+    load_cols<G, Q0>(vb, b, vcol);
     load_rows<G, R0>(vb, a, vrow);
-    two_sided<G, R0, I0, true>(A, U.w(j), j, a, b, t, vcol, vrow);
-    z.template reflect<P * G::LA>(U, k, l, j % (G::L < 32 ? 1 : G::L / 32), t, vb);
+    if constexpr (G::L <= 32) z.template reflect<P * G::LA>(U, k, l, 0, t, vb);
+    two_sided<G, R0, Q0, true>(A, U.w(j), j, a, b, t, vb, vcol, vrow);
+    if constexpr (G::L > 32) z.template reflect<P * G::LA>(U, k, l, j % (G::L / 32), t, vb);
   }
 }
 
 template <class G, int P>
-__device__ __forceinline__ void reduce_all(typename G::R (&A)[G::RN][G::CN], const UnitMem<G> &U, Vec<G> &z,
+__device__ __forceinline__ void reduce_all(typename G::Row (&A)[G::RN], const UnitMem<G> &U, Vec<G> &z,
                                            typename G::R *gv, int k, int l, int a, int b) {
   if constexpr (P < G::RN) {
     reduce_phase<G, P>(A, U, z, gv, k, l, a, b);
@@ -566,7 +645,7 @@ __device__ __forceinline__ void reduce_all(typename G::R (&A)[G::RN][G::CN], con
 }
 
 template <class G, int P>
-__device__ __forceinline__ void back_all(typename G::R (&A)[G::RN][G::CN], const UnitMem<G> &U, Vec<G> &z,
+__device__ __forceinline__ void back_all(typename G::Row (&A)[G::RN], const UnitMem<G> &U, Vec<G> &z,
                                          const typename G::R *gv, int k, int l, int a, int b) {
   if constexpr (P >= 0) {
     back_phase<G, P>(A, U, z, gv, k, l, a, b);
@@ -577,11 +656,11 @@ __device__ __forceinline__ void back_all(typename G::R (&A)[G::RN][G::CN], const
 // M's lower triangle from its upper one, one row group at a time through
 // shared memory
 template <class G, int P>
-__device__ __forceinline__ void mirror_all(typename G::R (&A)[G::RN][G::CN], typename G::R *buf, int a, int b) {
+__device__ __forceinline__ void mirror_all(typename G::Row (&A)[G::RN], typename G::R *buf, int a, int b) {
   if constexpr (P < G::RN) {
     constexpr int CB = P * G::LA / G::LB, NB = G::LA / G::LB;
     team_sync<G>();
-    store_cols<G, CB>(buf + a * G::VB, b, A[P]);
+    store_cols<G, CB / 2>(buf + a * G::VB, b, A[P]);
     team_sync<G>();
 #pragma unroll
     for (int i = CB; i < CB + NB && i < G::CN; i++) {
@@ -589,7 +668,7 @@ __device__ __forceinline__ void mirror_all(typename G::R (&A)[G::RN][G::CN], typ
       load_rows<G, P>(buf + (b + G::LB * (i - CB)) * G::VB, a, s);
 #pragma unroll
       for (int r = P; r < G::RN; r++)
-        if (r > P || a + G::LA * r > b + G::LB * i) A[r][i] = s[r];
+        set(A[r], i, r > P || a + G::LA * r > b + G::LB * i ? s[r] : get(A[r], i));
     }
     mirror_all<G, P + 1>(A, buf, a, b);
   }
@@ -618,24 +697,31 @@ __device__ __forceinline__ int unit_transform(typename G::R *mem, const typename
   const int a = l / G::LB, b = l % G::LB;
   // ---- A = G + (k-1)/infl I, src/letkf_core.F90:101-104
   const R shift = (R)(k - 1) * R(1) / (R)infl;
-  R A[G::RN][G::CN];
+  typename G::Row A[G::RN];
+  float *gs = reinterpret_cast<float *>(U.work);
+  if (Gin) {
+    // the packed block through shared memory, in order
+    const int nf = packed_size(k);
+#pragma unroll 8
+    for (int f = l; f < nf; f += G::L) gs[f] = Gin[f];
+  }
+  team_sync<G>();
 #pragma unroll
   for (int r = 0; r < G::RN; r++) {
-    const int row = a + G::LA * r;
+    const int row = a + G::LA * r, ro = tri_off(row, k) - row;
 #pragma unroll
     for (int i = 0; i < G::CN; i++) {
       const int col = b + G::LB * i;
       R v = R(0);
       if (row < k && col < k) {
-        const int lo = row < col ? row : col, hi = row < col ? col : row;
-        if (Gin) v = (R)Gin[tri_idx(lo, hi, k)];
+        if (Gin) v = (R)gs[row < col ? ro + col : tri_off(col, k) - col + row];
         if (row == col) v += shift;
       }
-      A[r][i] = v;
+      set(A[r], i, v);
     }
   }
   for (int c = l; c < G::KN; c += G::L) {
-    U.z[c] = Gin && c < k ? (R)Gin[k * (k + 1) / 2 + c] : R(0);
+    U.z[c] = Gin && c < k ? (R)gs[k * (k + 1) / 2 + c] : R(0);
     U.d[c] = R(1);
     U.e[c] = R(0);
     U.tau[c] = R(0);
@@ -669,7 +755,7 @@ __device__ __forceinline__ int unit_transform(typename G::R *mem, const typename
   for (int r = 0; r < G::RN; r++)
 #pragma unroll
     for (int i = G::LA * r / G::LB; i < G::CN; i++)
-      if (b + G::LB * i >= a + G::LA * r) A[r][i] = R(0);
+      set(A[r], i, b + G::LB * i >= a + G::LA * r ? R(0) : get(A[r], i));
   for (int p0 = 0;;) {
     if (p0 == 0) {
       level = nan ? 0 : ilogb((double)fmax(lmax / l0, R(1))) >> 1;
@@ -692,6 +778,7 @@ __device__ __forceinline__ int unit_transform(typename G::R *mem, const typename
       R eta = U.d[G::KM - 1] + s, inv = rcp_pos(eta), u = solve ? U.z[G::KM - 1] : R(1);
       bool neg = k == G::KM && !(eta > R(0));
       g[G::KM - 1] = u * inv;
+#pragma unroll 4
       for (int j = G::KM - 2; j >= 0; j--) {
         const R ej = U.e[j], rj = -ej * inv;
         rho[j] = rj;
@@ -706,6 +793,7 @@ __device__ __forceinline__ int unit_transform(typename G::R *mem, const typename
 #pragma unroll
       for (int t = 0; t < G::LB; t++) win[t] = R(0);
       lp[0] = R(0);
+#pragma unroll 4
       for (int j = 0; j < G::KM - 1; j++) {
         const R rj = rho[j];
         gi = fmar(solve ? rj : rj * rj, gi, g[j + 1]);
@@ -734,10 +822,11 @@ __device__ __forceinline__ int unit_transform(typename G::R *mem, const typename
     team_sync<G>();
     // the upper triangle of sqrt(k-1) S^(-1/2)
     const R scale = sqrt(l0 * (R)(k - 1));
+#pragma unroll 1
     for (int q = 0; q < nc; q++) {
       const R wp = scale * tab.w[level][p0 + q];
       const R *rho = U.work + q * G::PS, *g = rho + G::KN + 8, *lp = g + G::KN;
-      R prod[G::CN];
+      Pair<R> prod[G::CH2];
       load_cols<G, 0>(lp, b, prod);
 #pragma unroll
       for (int r = 0; r < G::RN; r++) {
@@ -747,16 +836,18 @@ __device__ __forceinline__ int unit_transform(typename G::R *mem, const typename
         R f = wp * g[row];
 #pragma unroll
         for (int t = 0; t + 1 < G::LB; t++) f = t < first ? f * rho[row + t] : f;
-        R cur = R(0);
+        R cur = R(0), even = R(0);
+        constexpr int X = G::LB;
 #pragma unroll
-        for (int i = G::LA * r / G::LB; i < G::CN; i++) {
-          if (i <= (G::LA * r + G::LA - 1) / G::LB + 1) {
-            const int off = b + G::LB * i - row;
-            cur = off < 0 ? R(0) : (off < G::LB ? f : cur * prod[i]);
+        for (int i = G::LA * r / X; i < G::CN; i++) {
+          if (i <= (G::LA * r + G::LA - 1) / X + 1) {
+            const int off = b + X * i - row;
+            cur = off < 0 ? R(0) : (off < X ? f : cur * get(prod, i));
           } else {
-            cur *= prod[i];
+            cur *= get(prod, i);
           }
-          A[r][i] += cur;
+          if (i & 1) A[r][i / 2] = padd(A[r][i / 2], Pair<R>(i > G::LA * r / X ? even : R(0), cur));
+          even = cur;
         }
       }
     }
@@ -790,7 +881,7 @@ __device__ __forceinline__ int unit_transform(typename G::R *mem, const typename
 #pragma unroll
       for (int i = 0; i < G::CN; i++) {
         const int col = b + G::LB * i;
-        if (row < k && col < k) Tout[row * k + col] = (float)(A[r][i] + zr[r]);
+        if (row < k && col < k) Tout[row * k + col] = (float)(get(A[r], i) + zr[r]);
       }
     }
     if (wout)
@@ -842,114 +933,68 @@ __global__ void __launch_bounds__(G::THREADS, G::MB) k_transform(EigArgs a, type
   }
 }
 
-// FP32_RESOLVE: the eigenvalues of every unit's tridiagonal matrix, for the
-// gap test (one thread per unit, implicit-shift QL with Wilkinson shifts
-// without vectors: the tql2 scheme of Bowdler, Martin, Reinsch & Wilkinson,
-// Numer. Math. 11, 1968).
+// FP32_RESOLVE: the units of a batch for the FP64 re-solve, a warp per unit on
+// the tridiagonal form k_transform left.  A unit is flagged when its FP32
+// solve failed, an eigenvalue is not positive, or two relevant eigenvalues lie
+// within gap_thresh * max l of each other.  The eigenvalues at the (k-1)/infl
+// floor (the null space of the Gram, k - n of them when n < k) are exactly
+// degenerate and harmless, since T is a function of the matrix and not of the
+// basis chosen in an eigenspace; they are left out of the test.
 //
-// Deflation test: e_m is negligible when it is below eps32 of its two
-// diagonal neighbours (the local test of LAPACK's ssteqr / EISPACK's tql2
-// family) or, from the kQlAbsIter-th iteration on the current eigenvalue,
-// below eps32 times the norm of the whole tridiagonal matrix (tql2's absolute
-// test).  The second test ends the iteration where rounding at the eps32
-// ||T|| level keeps a strongly graded block from meeting the local test.
-// Applied from the first iteration it also deflated, at the ||T|| level,
-// off-diagonals between near-equal small eigenvalues that the local test
-// resolves in a few more sweeps; the delay keeps them.
-constexpr int kQlAbsIter = 6;
-constexpr int QLT = 64;   // threads (units) per block
+// Each lane bisects eigenvalues lane, lane + 32, ... on the count of negative
+// pivots of T - x I (Sturm; Wilkinson & Reinsch, Handbook for Automatic
+// Computation II, 1971, contribution II/5): kBisect halvings of the Gershgorin
+// interval, past which FP32 resolves nothing of max l.  A QL iteration on one
+// thread per unit did the same arithmetic in one serial chain: 0.35 ms
+// whatever the number of units (k = 37), against 0.05.
+constexpr int kBisect = 26;
+constexpr int GAPW = 4;   // warps (units) per block
 
-__device__ __forceinline__ bool ql_negligible(float em, float dm, float dm1, float tabs) {
-  const float ae = fabsf(em);
-  return ae <= Lim<float>::eps * (fabsf(dm) + fabsf(dm1)) || ae <= tabs;
-}
-
-__global__ void __launch_bounds__(QLT) k_eig_ql(EigArgs a, EigSplit sp, int u0, int nb) {
-  extern __shared__ __align__(16) float qs[];   // d[k][QLT], e[k][QLT]
-  const int k = a.k, t = threadIdx.x;
-  const int ub = blockIdx.x * QLT + t;
-  float *d = qs + t, *e = qs + (size_t)k * QLT + t;   // element i at [i * QLT]
-#define D(i) d[(size_t)(i) * QLT]
-#define E(i) e[(size_t)(i) * QLT]
-  if (ub >= nb) return;
-  const int unit = a.ulist ? a.ulist[u0 + ub] : u0 + ub;
-  if (a.nkept[unit] <= 0) return;
-  if (sp.bad[ub]) return;
-  const float *de = sp.DE + (size_t)ub * 2 * k;
-  float an = 0.0f;
-  for (int i = 0; i < k; i++) {
-    D(i) = de[i];
-    E(i) = de[k + i];
-    an = fmaxf(an, fabsf(D(i)) + fabsf(E(i)));
-  }
-  const float tabs = Lim<float>::eps * an;
-  int bad = 0;
-  for (int l = 0; l < k; l++) {
-    int iter = 0;
-    for (;;) {
-      int m = l;
-      const float tab = iter >= kQlAbsIter ? tabs : 0.0f;
-      while (m < k - 1 && !ql_negligible(E(m), D(m), D(m + 1), tab)) m++;
-      if (m == l) break;
-      if (++iter > 60) { bad = 1; break; }
-      const float dl = D(l), el = E(l);
-      float g = (D(l + 1) - dl) / (2.0f * el);
-      float r = sqrtf(g * g + 1.0f);
-      g = D(m) - dl + el / (g + copysignf(r, g));
-      float s = 1.0f, c = 1.0f, pp = 0.0f;
-      float di1 = D(m);
-      bool deflate = false;
-      for (int i = m - 1; i >= l; i--) {
-        const float ei = E(i), di = D(i);
-        const float f = s * ei, b = c * ei;
-        r = sqrtf(f * f + g * g);
-        E(i + 1) = r;
-        if (r == 0.0f) {
-          D(i + 1) = di1 - pp;
-          E(m) = 0.0f;
-          deflate = true;
-          break;
-        }
-        const float ir = __frcp_rn(r);
-        s = f * ir;
-        c = g * ir;
-        g = di1 - pp;
-        const float rr = (di - g) * s + 2.0f * c * b;
-        pp = s * rr;
-        D(i + 1) = g + pp;
-        g = c * rr - b;
-        di1 = di;
-      }
-      if (!deflate) { D(l) = D(l) - pp; E(l) = g; E(m) = 0.0f; }
-    }
-    if (bad) break;
-  }
-#undef D
-#undef E
-  if (bad) sp.bad[ub] = bad;
-  float *lam = sp.lam + (size_t)ub * k;
-  for (int i = 0; i < k; i++) lam[i] = d[(size_t)i * QLT];
-}
-
-// FP64 re-solve candidates of a batch (warp per unit, after k_eig_ql): the
-// FP32 solve failed, or two relevant eigenvalues lie within gap_thresh *
-// max l of each other.  The eigenvalues at the (k-1)/infl floor (the null
-// space of the Gram, k - n of them when n < k) are exactly degenerate and
-// harmless, since T is a function of the matrix and not of the basis chosen
-// in an eigenspace; they are left out of the test.
-__global__ void k_eig_flag(EigArgs a, EigSplit sp, int u0, int nb) {
-  const int lane = threadIdx.x & 31;
-  const int ub = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+__global__ void __launch_bounds__(32 * GAPW) k_eig_gap(EigArgs a, EigSplit sp, int u0, int nb) {
+  __shared__ float sd[GAPW][kMaxK], se[GAPW][kMaxK], sl[GAPW][kMaxK];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ub = blockIdx.x * GAPW + warp;
   if (ub >= nb) return;
   const int unit = a.ulist ? a.ulist[u0 + ub] : u0 + ub;
   if (a.nkept[unit] <= 0) return;
   const int k = a.k;
   bool flag = sp.bad[ub] != 0;
   if (!flag) {
-    const float *lam = sp.lam + (size_t)ub * k;
-    float lmax = 0.0f;
-    for (int i = lane; i < k; i += 32) lmax = fmaxf(lmax, lam[i]);
-    for (int o = 16; o > 0; o >>= 1) lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
+    float *d = sd[warp], *e2 = se[warp], *lam = sl[warp];
+    const float *de = sp.DE + (size_t)ub * 2 * k;
+    float glo = 3.0e38f, ghi = -3.0e38f;
+    for (int i = lane; i < k; i += 32) {
+      const float di = de[i], el = i > 0 ? fabsf(de[k + i - 1]) : 0.0f, er = i < k - 1 ? fabsf(de[k + i]) : 0.0f;
+      d[i] = di;
+      e2[i] = el * el;
+      glo = fminf(glo, di - el - er);
+      ghi = fmaxf(ghi, di + el + er);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      glo = fminf(glo, __shfl_xor_sync(0xffffffffu, glo, o));
+      ghi = fmaxf(ghi, __shfl_xor_sync(0xffffffffu, ghi, o));
+    }
+    __syncwarp();
+    const float tiny = fmaxf(1e-30f, 1e-14f * fmaxf(fabsf(glo), fabsf(ghi)));
+    for (int i = lane; i < k; i += 32) {
+      float lo = glo, hi = ghi;
+      for (int it = 0; it < kBisect; it++) {
+        const float x = 0.5f * (lo + hi);
+        int below = 0;
+        float q = 1.0f;
+#pragma unroll 4
+        for (int j = 0; j < k; j++) {
+          q = (d[j] - x) - __fdividef(e2[j], q);
+          q = fabsf(q) < tiny ? -tiny : q;
+          below += q < 0.0f;
+        }
+        if (below > i) hi = x;
+        else lo = x;
+      }
+      lam[i] = 0.5f * (lo + hi);
+    }
+    __syncwarp();
+    const float lmax = lam[k - 1];
     // rounding level of the FP32 eigenvalues: a few k eps of the largest
     const float floor_v = (float)(k - 1) / a.infl;
     const float tol = 4.0f * (float)k * 1.1920929e-7f * lmax;
@@ -958,11 +1003,8 @@ __global__ void k_eig_flag(EigArgs a, EigSplit sp, int u0, int nb) {
     for (int i = lane; i < k; i += 32) {
       const float li = lam[i];
       neg |= !(li > 0.0f);
-      if (li - floor_v <= tol) continue;
-      for (int j = 0; j < k; j++) {
-        const float lj = lam[j];
-        if (j != i && lj - floor_v > tol) gap = fminf(gap, fabsf(li - lj));
-      }
+      // ascending: the nearest relevant neighbour is the next one
+      if (li - floor_v > tol && i + 1 < k) gap = fminf(gap, fabsf(lam[i + 1] - li));
     }
     for (int o = 16; o > 0; o >>= 1) gap = fminf(gap, __shfl_xor_sync(0xffffffffu, gap, o));
     flag = gap <= a.gap_thresh * lmax || __any_sync(0xffffffffu, neg);
@@ -1001,38 +1043,42 @@ cudaError_t launch_g(cudaStream_t st, const EigArgs &a, const EigSplit &sp, int 
 // team of two warps a unit up to 80, of four above.
 template <class F>
 auto with_grid_f32(int k, F f) {
-#define LGPU_GRID(RN, CN, LA, LB, MB) return f(Grid<float, RN, CN, LA, LB, MB>())
+#define LGPU_GRID(...) return f(Grid<float, __VA_ARGS__>())
   switch ((k + 7) / 8) {
   case 1: LGPU_GRID(1, 8, 8, 1, 6);
-  case 2: LGPU_GRID(2, 16, 8, 1, 4);
-  case 3: LGPU_GRID(3, 24, 8, 1, 4);
-  case 4: LGPU_GRID(4, 16, 8, 2, 4);
-  case 5: LGPU_GRID(5, 20, 8, 2, 3);
-  case 6: LGPU_GRID(6, 12, 8, 4, 4);
-  case 7: LGPU_GRID(7, 14, 8, 4, 3);
+  case 2: LGPU_GRID(2, 16, 8, 1, 5);
+  case 3: LGPU_GRID(3, 24, 8, 1, 3);
+  case 4: LGPU_GRID(4, 16, 8, 2, 3);
+  case 5: LGPU_GRID(5, 20, 8, 2, 2);
+  case 6: LGPU_GRID(6, 12, 8, 4, 3);
+  case 7: LGPU_GRID(7, 14, 8, 4, 2);
   case 8: LGPU_GRID(8, 16, 8, 4, 2);
-  case 9: LGPU_GRID(5, 18, 16, 4, 6);
+  case 9: LGPU_GRID(9, 18, 8, 4, 2);
   case 10: LGPU_GRID(5, 20, 16, 4, 6);
-  case 11: LGPU_GRID(6, 11, 16, 8, 4);
-  case 12: LGPU_GRID(6, 12, 16, 8, 4);
-  case 13: LGPU_GRID(7, 13, 16, 8, 3);
-  case 14: LGPU_GRID(7, 14, 16, 8, 3);
-  case 15: LGPU_GRID(8, 15, 16, 8, 2);
+  case 11: LGPU_GRID(6, 22, 16, 4, 4);
+  case 12: LGPU_GRID(6, 24, 16, 4, 4);
+  case 13: LGPU_GRID(7, 26, 16, 4, 4);
+  case 14: LGPU_GRID(7, 28, 16, 4, 4);
   default: LGPU_GRID(8, 16, 16, 8, 2);
   }
 #undef LGPU_GRID
 }
 
-// FP64: GB300 runs FP64 at 1/64 of the FP32 rate, so a unit is spread over two
-// warps up to k = 64 and eight above
+// FP64: GB300 runs FP64 at 1/64 of the FP32 rate, two multiply-adds a clock on
+// an SM, so the grids follow the size closely: one warp a unit up to k = 48
+// (the most a lane's registers hold), two up to 64, four up to 112, eight above
 template <class F>
 auto with_grid_f64(int k, F f) {
-#define LGPU_GRID(RN, CN, LA, LB, MB) return f(Grid<double, RN, CN, LA, LB, MB>())
-  if (k <= 16) LGPU_GRID(2, 2, 8, 8, 8);
-  if (k <= 32) LGPU_GRID(4, 4, 8, 8, 8);
-  if (k <= 40) LGPU_GRID(5, 5, 8, 8, 6);
+#define LGPU_GRID(...) return f(Grid<double, __VA_ARGS__>())
+  if (k <= 16) LGPU_GRID(2, 4, 8, 4, 4);
+  if (k <= 24) LGPU_GRID(3, 6, 8, 4, 4);
+  if (k <= 32) LGPU_GRID(4, 8, 8, 4, 2);
+  if (k <= 40) LGPU_GRID(5, 10, 8, 4, 2);
+  if (k <= 48) LGPU_GRID(6, 12, 8, 4, 1);
   if (k <= 64) LGPU_GRID(8, 8, 8, 8, 4);
-  if (k <= 96) LGPU_GRID(3, 12, 32, 8, 1);
+  if (k <= 80) LGPU_GRID(5, 10, 16, 8, 2);
+  if (k <= 96) LGPU_GRID(6, 12, 16, 8, 2);
+  if (k <= 112) LGPU_GRID(7, 14, 16, 8, 2);
   LGPU_GRID(4, 16, 32, 8, 1);
 #undef LGPU_GRID
 }
@@ -1074,22 +1120,19 @@ cudaError_t launch_eig64_flagged(cudaStream_t st, const EigArgs &a, int *launche
   return cudaMemcpyAsync(a.flag_n + 1, a.flag_n, sizeof(int), cudaMemcpyDeviceToDevice, st);
 }
 
-size_t eig_split_bytes_per_unit(int k) { return (size_t)3 * k * 4 + 4; }
+size_t eig_split_bytes_per_unit(int k) { return (size_t)2 * k * 4 + 4; }
 
 cudaError_t launch_eig_split(cudaStream_t st, const EigArgs &a, const EigSplit &sp, int batch, int ustart, int ucount,
                              int *launches) {
   if (ucount <= 0) return cudaSuccess;
   if (!a.flag_list) return launch_f32(st, a, EigSplit{}, ustart, ucount, launches);
-  const size_t qsm = (size_t)2 * a.k * QLT * sizeof(float);
-  cudaError_t e = cudaFuncSetAttribute(k_eig_ql, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)qsm);
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
   const int uend = ustart + ucount;
   for (int u0 = ustart; u0 < uend; u0 += batch) {
     const int nb = uend - u0 < batch ? uend - u0 : batch;
     if ((e = launch_f32(st, a, sp, u0, nb, launches)) != cudaSuccess) return e;
-    k_eig_ql<<<(nb + QLT - 1) / QLT, QLT, qsm, st>>>(a, sp, u0, nb);
-    k_eig_flag<<<(nb + 7) / 8, 256, 0, st>>>(a, sp, u0, nb);
-    (*launches) += 2;
+    k_eig_gap<<<(nb + GAPW - 1) / GAPW, 32 * GAPW, 0, st>>>(a, sp, u0, nb);
+    (*launches)++;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -1118,8 +1161,8 @@ cudaError_t launch_eig_debug(cudaStream_t st, int nunits, int k, const float *G,
   const bool resolve = prec == LGPU_PREC_FP32_RESOLVE;
   unsigned char *buf = nullptr;
   const size_t vb = eig_scratch_bytes(k, (int)n, prec != LGPU_PREC_FP64, prec != LGPU_PREC_FP32);
-  // five arrays, each start rounded up to 256 bytes
-  cudaError_t e = cudaMalloc(&buf, vb + (resolve ? eig_split_bytes_per_unit(k) * n + 16 + 4 * n : 0) + 5 * 256);
+  // four arrays, each start rounded up to 256 bytes
+  cudaError_t e = cudaMalloc(&buf, vb + (resolve ? eig_split_bytes_per_unit(k) * n + 16 + 4 * n : 0) + 4 * 256);
   if (e != cudaSuccess) return e;
   size_t off = 0;
   auto take = [&](size_t bytes) { unsigned char *p = buf + off; off += (bytes + 255) & ~(size_t)255; return p; };
@@ -1134,7 +1177,6 @@ cudaError_t launch_eig_debug(cudaStream_t st, int nunits, int k, const float *G,
   EigSplit sp{};
   if (resolve) {
     sp.DE = reinterpret_cast<float *>(take(n * 2 * k * 4));
-    sp.lam = reinterpret_cast<float *>(take(n * k * 4));
     sp.bad = reinterpret_cast<int *>(take(n * 4));
     a.flag_n = reinterpret_cast<int *>(take(16 + 4 * n));
     a.flag_list = a.flag_n + 4;

@@ -548,7 +548,6 @@ cudaError_t launch_eig64_flagged(cudaStream_t st, const EigArgs &a, int *launche
 // scratch of the gap test (FP32_RESOLVE) for `batch` units; null: no test
 struct EigSplit {
   float *DE;       // [batch][2k] diagonal, off-diagonal of the tridiagonal form
-  float *lam;      // [batch][k] eigenvalues
   int *bad;        // [batch] FP32 solve failed
 };
 size_t eig_split_bytes_per_unit(int k);
