@@ -149,12 +149,10 @@ template <> struct Lim<double> {
 // packed multiply-add, which does both in one issue slot.
 template <class R> struct Pair;
 template <>
-struct Pair<float> {
-  unsigned long long u;
+struct Pair<float> : F2 {
   __device__ __forceinline__ Pair() {}
-  __device__ __forceinline__ Pair(float x, float y) { asm("mov.b64 %0, {%1, %2};" : "=l"(u) : "f"(x), "f"(y)); }
-  __device__ __forceinline__ float x() const { return __uint_as_float((unsigned)u); }
-  __device__ __forceinline__ float y() const { return __uint_as_float((unsigned)(u >> 32)); }
+  __device__ __forceinline__ Pair(F2 v) : F2(v) {}
+  __device__ __forceinline__ Pair(float x, float y) : F2(x, y) {}
 };
 template <>
 struct Pair<double> {
@@ -164,17 +162,11 @@ struct Pair<double> {
   __device__ __forceinline__ double x() const { return a; }
   __device__ __forceinline__ double y() const { return b; }
 };
-__device__ __forceinline__ Pair<float> pfma(Pair<float> a, Pair<float> b, Pair<float> c) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c.u) : "l"(a.u), "l"(b.u));
-  return c;
-}
+__device__ __forceinline__ Pair<float> pfma(Pair<float> a, Pair<float> b, Pair<float> c) { return f2_fma(a, b, c); }
 __device__ __forceinline__ Pair<double> pfma(Pair<double> a, Pair<double> b, Pair<double> c) {
   return Pair<double>(__fma_rn(a.a, b.a, c.a), __fma_rn(a.b, b.b, c.b));
 }
-__device__ __forceinline__ Pair<float> padd(Pair<float> a, Pair<float> b) {
-  asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a.u) : "l"(b.u));
-  return a;
-}
+__device__ __forceinline__ Pair<float> padd(Pair<float> a, Pair<float> b) { return f2_add(a, b); }
 __device__ __forceinline__ Pair<double> padd(Pair<double> a, Pair<double> b) { return Pair<double>(a.a + b.a, a.b + b.b); }
 
 // the element of lane column i (a constant after unrolling) of a row of pairs
@@ -186,19 +178,13 @@ __device__ __forceinline__ void set(Pair<R> *p, int i, R v) {
 }
 
 // two pairs, 16-byte aligned in FP32
-__device__ __forceinline__ void ld2(const float *p, Pair<float> *v) {
-  const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(p);
-  v[0].u = t.x;
-  v[1].u = t.y;
-}
+__device__ __forceinline__ void ld2(const float *p, Pair<float> *v) { f2_load2(p, v[0], v[1]); }
 __device__ __forceinline__ void ld2(const double *p, Pair<double> *v) {
   const double2 t = *reinterpret_cast<const double2 *>(p), u = *reinterpret_cast<const double2 *>(p + 2);
   v[0] = Pair<double>(t.x, t.y);
   v[1] = Pair<double>(u.x, u.y);
 }
-__device__ __forceinline__ void st2(float *p, Pair<float> a, Pair<float> b) {
-  *reinterpret_cast<ulonglong2 *>(p) = make_ulonglong2(a.u, b.u);
-}
+__device__ __forceinline__ void st2(float *p, Pair<float> a, Pair<float> b) { f2_store2(p, a, b); }
 __device__ __forceinline__ void st2(double *p, Pair<double> a, Pair<double> b) {
   *reinterpret_cast<double2 *>(p) = make_double2(a.a, a.b);
   *reinterpret_cast<double2 *>(p + 2) = make_double2(b.a, b.b);
@@ -208,15 +194,12 @@ __device__ __forceinline__ void st2(double *p, Pair<double> a, Pair<double> b) {
 // hardware's approximations and one Newton step, without the rounded forms'
 // range checks
 __device__ __forceinline__ float sqrt_pos(float x) {
-  float r;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  const float q = x * r;
+  const float r = rsqrt_approx(x), q = x * r;
   return fmar(0.5f * r, fmar(-q, q, x), q);
 }
 __device__ __forceinline__ double sqrt_pos(double x) { return sqrt(x); }
 __device__ __forceinline__ float rcp_pos(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  const float r = rcp_approx(x);
   return fmar(r, fmar(-x, r, 1.0f), r);
 }
 __device__ __forceinline__ double rcp_pos(double x) { return __drcp_rn(x); }

@@ -373,12 +373,13 @@ __global__ void k_debug_weight(int n, const float *lat1, const float *lon1, cons
   if (i >= n) return;
   float3 a = unitvec_exact(lat1[i], lon1[i]), b = unitvec_exact(lat2[i], lon2[i]);
   const float de = dist_from_chord2(chord2_exact(a.x, a.y, a.z, b.x, b.y, b.z));
-  const float df = dist_fast(chord2_fast(a.x, a.y, a.z, b.x, b.y, b.z));
+  const F2 c2 = chord2_fast(f2_all(-a.x), f2_all(-a.y), f2_all(-a.z), f2_all(b.x), f2_all(b.y), f2_all(b.z));
+  const F2 df = dist_fast(c2, false);
   out[i] = de;
-  out[n + i] = df;
+  out[n + i] = df.x();
   out[2 * n + i] = gc_exact(de, L[i]);
-  out[3 * n + i] = gc_branchless(df * inv_c_of(L[i]));
-  out[4 * n + i] = dist_fast(chord2_fast(a.x, a.y, a.z, b.x, b.y, b.z), true);
+  out[3 * n + i] = gc_branchless(f2_mul(df, f2_all(inv_c_of(L[i]))), true).x();
+  out[4 * n + i] = dist_fast(c2, true).x();
 }
 
 }  // namespace

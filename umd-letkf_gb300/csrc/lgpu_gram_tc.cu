@@ -17,9 +17,9 @@
 // Candidate streams.  Before the GEMM, three small kernels turn each tile's
 // search window (latitude bands x longitude range of its cap) into a record
 // stream: every observation inside the tile's cap, in window order, packed
-// per chunk of 16 as [16 x (ux,uy,uz,1/err)] [16 x (dep,time,zdim,surf)]
-// [member-major y: (k+1 rounded to 4) rows x 16] -- one contiguous block per
-// chunk, read once per (group, pass) CTA with one bulk async copy.
+// per chunk of 16 as ux[16] uy[16] uz[16] 1/err[16] dep[16] time[16] zdim[16]
+// surf[16] and member-major y: (k+1 rounded to 4) rows x 16 -- one contiguous
+// block per chunk, read once per (group, pass) CTA with one bulk async copy.
 //
 // GEMM CTA roles (17 warps):
 //   warps 0-15  producers; thread t owns column t % 128 for observations
@@ -69,7 +69,6 @@ constexpr uint32_t SBO = (KC / 4) * CMB;      // bytes per 8-row group (all K of
 constexpr uint32_t WB = (TM / 8) * SBO;       // bytes per W operand copy
 constexpr size_t kSmemBudget = 227 * 1024 - 4096;   // dynamic shared memory (static part below 4 KB)
 constexpr int WT = 256;        // threads of the stream kernels
-constexpr int WCB = 2 * WB;   // bytes of one chunk's cached weight operand block (hi | lo)
 constexpr int YS = 20;         // floats per member row of a chunk record (16 observations + 4: conflict-free rows)
 __device__ __forceinline__ uint32_t kmaj(int row, int kk) {
   return (uint32_t)(row >> 3) * SBO + (uint32_t)(kk >> 2) * CMB + (uint32_t)(row & 7) * 16u + (uint32_t)(kk & 3) * 4u;
@@ -228,8 +227,9 @@ __device__ __forceinline__ void put_record(unsigned char *rec0, int cb, int k, i
                                            const float4 &B, const float *hx) {
   unsigned char *r = rec0 + (size_t)(q >> 4) * cb;
   const int e = q & 15;
-  reinterpret_cast<float4 *>(r)[e] = A;
-  reinterpret_cast<float4 *>(r + 256)[e] = B;
+  float *r0 = reinterpret_cast<float *>(r);
+  r0[e] = A.x; r0[16 + e] = A.y; r0[32 + e] = A.z; r0[48 + e] = A.w;
+  r0[64 + e] = B.x; r0[80 + e] = B.y; r0[96 + e] = B.z; r0[112 + e] = B.w;
   float *yT = reinterpret_cast<float *>(r + 512);
   if (hx) {
     // the member row through the read-only path, four 16-byte loads in
@@ -323,9 +323,19 @@ __global__ void __launch_bounds__(WT) k_tile_fill(int ntiles, const TilePar *tps
   }
   if (tid < pend) write(base + tid, qpos[tid]);
   base += pend;
-  const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int q = base + tid; q < cap; q += WT) put_record(rec0, cb, k, kp, kr, q, z, z, nullptr);
+  // padding: a point out of every column's reach, weight 0
+  const float4 z = make_float4(0.f, 0.f, 0.f, 0.f), far = make_float4(4.f, 0.f, 0.f, 0.f);
+  for (int q = base + tid; q < cap; q += WT) put_record(rec0, cb, k, kp, kr, q, far, z, nullptr);
   if (tid == 0 && (base > cap || cap - base >= KC)) atomicOr(status, 16);   // count and fill disagree
+}
+
+// fp32 pair -> TF32 hi + lo (tc::split_tf32 on both halves)
+__device__ __forceinline__ void split2(F2 v, F2 &hi, F2 &lo) {
+  uint32_t h0, h1;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h0) : "f"(v.x()));
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h1) : "f"(v.y()));
+  hi = F2(__uint_as_float(h0), __uint_as_float(h1));
+  lo = f2_fma(hi, f2_all(-1.0f), v);   // exact
 }
 
 struct TcSmem {
@@ -348,19 +358,33 @@ struct LocK {
   float ictp, icts;           // ocean: their 1/c
 };
 
-// fast localisation weight (no branches); LOC selects the localizer class
+// a producer thread's column, both halves of the pairs alike
+struct ColFast {
+  F2 nx, ny, nz;              // negated unit vector
+  float ic1, ic2;             // 1/c of the length scales
+  float c2in, c2max;          // squared chord of the search radius; with its margin
+  float cscale;               // |c2 - c2in| * cscale <= kGuardFast: within the chord band
+};
+
+// fast localisation weights of observations e, e + 1 (no branches) at the
+// distances d; LOC selects the localizer class.  Beyond the search radius the
+// single-factor class may return anything.
 template <int LOC>
-__device__ __forceinline__ float loc_fast(const LocK &lk, const ColPar &cp, int g, float d, const float4 &B) {
+__device__ __forceinline__ F2 loc_fast(const LocK &lk, const ColFast &cf, int g, F2 d, const float *rec, int e) {
   if (LOC == LOC_VTGC) {
-    return gc_branchless(d * cp.ic1) * gc_branchless(fabsf(B.z - lk.levg) * lk.icv);
+    const float z0 = fabsf(rec[96 + e] - lk.levg), z1 = fabsf(rec[97 + e] - lk.levg);
+    return f2_mul(gc_branchless(f2_mul(d, f2_all(cf.ic1)), true), gc_branchless(F2(z0 * lk.icv, z1 * lk.icv), true));
   } else if (LOC == LOC_OCEAN) {
-    const bool sat = B.w != 0.0f;
-    const float rh = gc_branchless(d * (sat ? cp.ic2 : cp.ic1));
-    const float tl = sat ? lk.tsat : lk.tprof;
-    const float rt = tl > 0.0f ? gc_branchless(fabsf(B.y) * (sat ? lk.icts : lk.ictp)) : 1.0f;
-    return (sat && g == 1) ? 0.0f : rh * rt;
+    float w[2];
+    const bool s0 = rec[112 + e] != 0.0f, s1 = rec[113 + e] != 0.0f;
+    const F2 rh = gc_branchless(f2_mul(d, F2(s0 ? cf.ic2 : cf.ic1, s1 ? cf.ic2 : cf.ic1)), true);
+    const F2 rt = gc_branchless(F2(fabsf(rec[80 + e]) * (s0 ? lk.icts : lk.ictp),
+                                   fabsf(rec[81 + e]) * (s1 ? lk.icts : lk.ictp)), true);
+    w[0] = rh.x() * ((s0 ? lk.tsat : lk.tprof) > 0.0f ? rt.x() : 1.0f);
+    w[1] = rh.y() * ((s1 ? lk.tsat : lk.tprof) > 0.0f ? rt.y() : 1.0f);
+    return F2(s0 && g == 1 ? 0.0f : w[0], s1 && g == 1 ? 0.0f : w[1]);
   } else {
-    return gc_branchless(d * cp.ic1);
+    return gc_branchless(f2_mul(d, f2_all(cf.ic1)), false);
   }
 }
 
@@ -368,25 +392,21 @@ __device__ __forceinline__ void bar_arrive(unsigned long long *b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(b)) : "memory");
 }
 
-// WMODE: 0 = weights computed; 1 = weights computed and written to the
-// weight cache as the stage's TF32 hi/lo operand block, with the chunk's
-// MMA flag (first feature pass of a tile); 2 = the operand block is
-// bulk-copied from the cache into the stage (later passes: the producers
-// form only the feature products).  CULL (WMODE 0, 1): a warp whose 32
-// columns have none of its four records within their search chords skips
-// the distance and localizer evaluation (their weights are zero either way;
-// results are bit-identical); pays where search radii are small next to the
-// tile caps, costs registers where they are not
-template <int LOC, int NS, int NR, int WMODE, bool CULL>
+// CULL: a warp whose 32 columns have none of its four records within their
+// search chords skips the distance and localizer evaluation (their weights are
+// zero either way; results are bit-identical); pays where search radii are
+// small next to the tile caps, costs registers where they are not
+template <int LOC, int NS, int NR, bool CULL>
 __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
   static_assert(NS <= NSMAX && NR <= NRMAX, "operand stages / record slots beyond the barrier arrays");
   extern __shared__ __align__(1024) unsigned char dsm[];
   __shared__ __align__(16) TcSmem S;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  // block = (work item, group, pass of this launch), pass fastest
-  const int pass = a.pass0 + blockIdx.x % a.npl;
-  const int g = (blockIdx.x / a.npl) % a.groups;
-  const TcWork wk = a.work[blockIdx.x / (a.npl * a.groups)];
+  // block = (work item, group, pass), pass fastest: the passes of a work item
+  // run side by side and share its records in L2
+  const int pass = blockIdx.x % a.npass;
+  const int g = (blockIdx.x / a.npass) % a.groups;
+  const TcWork wk = a.work[blockIdx.x / (a.npass * a.groups)];
   const int tile = wk.tile;
   const int k = a.k, NP = a.np, nf = a.nf, cb = a.cb;
   const int slotb = cb;   // ring slot: one chunk record
@@ -398,17 +418,14 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
   const int t0 = a.tile_off[tile], tn = a.tile_off[tile + 1] - t0;
   const int cs = min(tn, wk.cs), ce = min(tn, wk.ce);
   const int c0 = t0 + cs;
-  float *wcache = WMODE != 0 ? a.wcache + (size_t)g * a.nchunk_total * (WCB / 4) : nullptr;
-  int *wflag = WMODE != 0 ? a.wflag + (size_t)g * a.nchunk_total : nullptr;
   const int nchunks = ce - cs;
-  const int ntile = a.tile_n[tile] - cs * KC;   // candidates from the segment's first chunk on
   const uint32_t tmem_cols = a.tmem_cols;
 
   // ---- setup: TMEM, barriers, feature table
   if (wid == 0) tc::tmem_alloc(&S.tmem, tmem_cols);
   if (tid == 0) {
     for (int s = 0; s < NS; s++) {
-      tc::mbar_init(reinterpret_cast<uint64_t *>(&S.full[s]), WMODE == 2 ? NPW + 1 : NPW);
+      tc::mbar_init(reinterpret_cast<uint64_t *>(&S.full[s]), NPW);
       tc::mbar_init(reinterpret_cast<uint64_t *>(&S.empty[s]), 1);
       S.anyk[s] = 0;
     }
@@ -483,17 +500,28 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
   if (wid < NPW) {
     const int col = a.tile_cols[(size_t)tile * TM + wc];
     const bool colv = col >= 0;
-    ColPar cp;
-    if (colv) cp = a.cp[col];
-    else { cp.ux = cp.uy = cp.uz = 0.0f; cp.rmax = -1.0f; cp.L1 = cp.L2 = 1.0f; cp.ic1 = cp.ic2 = 1.0f; }
-    float c2max = -1.0f;
-    if (colv) {
-      const float hq = fminf(cp.rmax / 12742000.0f, 1.5707963f);
-      const float sh = sinf(hq);
-      c2max = 4.0f * sh * sh * 1.0001f + 1e-12f;
+    ColFast cf;
+    {
+      // no column: a point out of reach of every record
+      float ux = -4.0f, uy = 0.0f, uz = 0.0f, rmax = 0.0f;
+      cf.ic1 = cf.ic2 = 1.0f;
+      if (colv) {
+        const ColPar &cp = a.cp[col];
+        ux = cp.ux; uy = cp.uy; uz = cp.uz; rmax = cp.rmax;
+        cf.ic1 = cp.ic1;
+        cf.ic2 = cp.ic2;
+      }
+      cf.nx = f2_all(-ux);
+      cf.ny = f2_all(-uy);
+      cf.nz = f2_all(-uz);
+      const float sh = sinf(fminf(rmax / 12742000.0f, 1.5707963f));
+      cf.c2in = colv ? 4.0f * sh * sh : 0.0f;
+      cf.c2max = colv ? cf.c2in * 1.0001f + 1e-12f : -1.0f;
+      // (a radius within rounding of zero is all band)
+      cf.cscale = colv ? kGuardFast / (kFastChordBand * cf.c2in + 1e-14f) : 1.0f;
     }
-    const float rlo = cp.rmax * (1.0f - kFastDistBand), rhi = cp.rmax * (1.0f + kFastDistBand);
-    const bool short_asin = a.tp[tile].hmax <= 0.25f;   // CTA-uniform
+    const float hmax = a.tp[tile].hmax;   // CTA-uniform
+    const bool short_asin = hmax <= 0.25f, far = hmax > 0.5f;
     LocK lk;
     lk.icv = LOC == LOC_VTGC ? inv_c_of(a.loc.vloc) : 1.0f;
     lk.levg = LOC == LOC_VTGC ? a.loc.lev_depth[g] : 0.0f;
@@ -504,8 +532,8 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
     const int f = tid;
     const bool fin = f < NP;
     const int fi = fin ? S.fi[f] : 255, fj = fin ? S.fj[f] : 255;
-    const bool fv = fi != 255;
-    const int rowi = (fv ? fi : 0) * YS, rowj = (fv ? fj : 0) * YS;
+    // a feature past the last one multiplies row 0; its accumulator is not read
+    const int rowi = (fi != 255 ? fi : 0) * YS, rowj = (fi != 255 ? fj : 0) * YS;
 
     for (int ch = 0; ch < nchunks; ch++) {
       const int s = ch % NS, r = ch % NR;
@@ -519,112 +547,98 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
         break;
       }
       const unsigned char *rec = ring + (size_t)r * slotb;
-      const float4 *RA = reinterpret_cast<const float4 *>(rec);
+      const float *R = reinterpret_cast<const float *>(rec);
       unsigned char *Whi = stage_ptr(s), *Wlo = Whi + WB, *Phi = Whi + 2 * WB, *Plo = Phi + PB;
+      const int e0 = wq * 4;
       bool anyk = false;
-      if (WMODE == 2) {
-        // ---- the chunk's weight operand block (hi | lo) from the cache into
-        // the stage, counted on the stage's full barrier (the stage is free:
-        // its empty barrier was waited on above)
-        if (tid == 0) {
-          uint64_t *fb = reinterpret_cast<uint64_t *>(&S.full[s]);
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::smem_u32(fb)),
-                       "r"((uint32_t)WCB) : "memory");
-          tc::bulk_copy_g2s(Whi, wcache + (size_t)(c0 + ch) * (WCB / 4), (uint32_t)WCB, fb);
-        }
-      } else {
       // ---- weights: four observations, fast path without branches
       float w[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      unsigned unsure = 0, inr = 0;
-      unsigned candm = 0xfu;
-      if constexpr (CULL) {
-        candm = 0;
+      unsigned inr = 0;
+      F2 ox[2], oy[2], oz[2], c2[2];
+      f2_load2(R + e0, ox[0], ox[1]);
+      f2_load2(R + 16 + e0, oy[0], oy[1]);
+      f2_load2(R + 32 + e0, oz[0], oz[1]);
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int e = wq * 4 + u;
-          const float4 A = RA[e];
-          const float c2f = chord2_fast(cp.ux, cp.uy, cp.uz, A.x, A.y, A.z);
-          candm |= ((ch * KC + e < ntile) && (c2f <= c2max) ? 1u : 0u) << u;
+      for (int h = 0; h < 2; h++) c2[h] = chord2_fast(cf.nx, cf.ny, cf.nz, ox[h], oy[h], oz[h]);
+      bool go = true;
+      if constexpr (CULL)
+        go = __any_sync(0xffffffffu, fminf(fminf(c2[0].x(), c2[0].y()), fminf(c2[1].x(), c2[1].y())) <= cf.c2max);
+      if (go) {
+        float near = 1.0f;   // the smallest distance of a decision from its threshold, in units of kGuardFast's scale
+        float c[4] = {c2[0].x(), c2[0].y(), c2[1].x(), c2[1].y()}, rl[4];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const F2 r2 = loc_fast<LOC>(lk, cf, g, dist_fast(c2[h], short_asin), R, e0 + 2 * h);
+          rl[2 * h] = r2.x();
+          rl[2 * h + 1] = r2.y();
         }
-      }
-      if (!CULL || __any_sync(0xffffffffu, candm != 0)) {
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-          const int e = wq * 4 + u;
-          const float4 A = RA[e];
-          const float4 B = RA[16 + e];
-          const float c2f = chord2_fast(cp.ux, cp.uy, cp.uz, A.x, A.y, A.z);
-          const bool cand = (ch * KC + e < ntile) && (c2f <= c2max);
-          const float hf = 0.5f * c2f * rsqrtf(fmaxf(c2f, 1e-30f));
-          const float d = 12742000.0f * asin_fast(fminf(hf, 0.5f), short_asin);
-          const float rl = loc_fast<LOC>(lk, cp, g, d, B);
-          const bool in = cand && d <= cp.rmax;
-          const bool uns = cand && (hf > 0.5f || (d >= rlo && d <= rhi) || (in && fabsf(rl - kKeep) <= kGuardFast));
-          const bool kept = in && rl > kKeep;
-          w[u] = kept ? rl : 0.0f;
-          unsure |= (uns ? 1u : 0u) << u;
-          inr |= (in ? 1u : 0u) << u;
+          const bool in = c[u] <= cf.c2in;
+          near = fminf(near, fminf(fabsf(c[u] - cf.c2in) * cf.cscale, fabsf(rl[u] - kKeep)));
+          w[u] = in && rl[u] > kKeep ? rl[u] : 0.0f;
+          inr += in;
         }
-      }
-      // ---- rare: exact metric and the per-column localizer
-      if (__any_sync(0xffffffffu, unsure != 0)) {
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          if (!((unsure >> u) & 1u)) continue;
-          const int e = wq * 4 + u;
-          const float4 A = RA[e];
-          const float4 B = RA[16 + e];
-          const float de = dist_from_chord2(chord2_exact(cp.ux, cp.uy, cp.uz, A.x, A.y, A.z));
-          const bool in = de <= cp.rmax;
-          // the class's exact localizer with the column's parameters from
-          // global memory (keeps them out of the producers' registers)
-          float rl = in ? localize_cls<LOC>(a.loc, a.cp[col], g, de, B.y, B.z, B.w) : 0.0f;
-          w[u] = (in && rl > kKeep) ? rl : 0.0f;
-          inr = (inr & ~(1u << u)) | ((in ? 1u : 0u) << u);
+        // beyond a chord of 1 the fast distance does not hold
+        if (far) near = fmaxf(fmaxf(c[0], c[1]), fmaxf(c[2], c[3])) > 1.0f ? 0.0f : near;
+        // ---- rare: exact metric and the per-column localizer
+        if (__any_sync(0xffffffffu, near <= kGuardFast) && near <= kGuardFast) {
+          inr = 0;
+#pragma unroll 1
+          for (int u = 0; u < 4; u++) {
+            const float cu = u == 0 ? c[0] : u == 1 ? c[1] : u == 2 ? c[2] : c[3];
+            float wu = u == 0 ? w[0] : u == 1 ? w[1] : u == 2 ? w[2] : w[3];
+            const float ru = u == 0 ? rl[0] : u == 1 ? rl[1] : u == 2 ? rl[2] : rl[3];
+            bool in = cu <= cf.c2in;
+            const bool unsure = cu <= cf.c2max && (cu > 1.0f || fabsf(cu - cf.c2in) * cf.cscale <= kGuardFast ||
+                                                   (in && fabsf(ru - kKeep) <= kGuardFast));
+            if (unsure) {
+              const int e = e0 + u;
+              // the column's parameters from global memory (keeps them out of
+              // the producers' registers)
+              const ColPar &cp = a.cp[col];
+              const float de = dist_from_chord2(chord2_exact(cp.ux, cp.uy, cp.uz, R[e], R[16 + e], R[32 + e]));
+              in = de <= cp.rmax;
+              const float re = in ? localize_cls<LOC>(a.loc, cp, g, de, R[80 + e], R[96 + e], R[112 + e]) : 0.0f;
+              wu = re > kKeep ? re : 0.0f;
+            }
+            inr += in;
+            w[0] = u == 0 ? wu : w[0];
+            w[1] = u == 1 ? wu : w[1];
+            w[2] = u == 2 ? wu : w[2];
+            w[3] = u == 3 ? wu : w[3];
+          }
         }
       }
       {
-        float h4[4], l4[4];
+        ncand += inr;
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-          const float rl = w[u];
-          ncand += (inr >> u) & 1u;
-          float wv = 0.0f;
-          if (rl > 0.0f) {
-            nkeep++;
-            rsum += rl;
-            anyk = true;
-            wv = rl * RA[wq * 4 + u].w;   // the record holds 1/err
-          }
-          tc::split_tf32(wv, h4[u], l4[u]);
+          nkeep += w[u] > 0.0f;
+          rsum += w[u];
         }
-        const uint32_t off = kmaj(wc, wq * 4);
-        *reinterpret_cast<float4 *>(Whi + off) = make_float4(h4[0], h4[1], h4[2], h4[3]);
-        *reinterpret_cast<float4 *>(Wlo + off) = make_float4(l4[0], l4[1], l4[2], l4[3]);
-        if (WMODE == 1) {
-          float *blk = wcache + (size_t)(c0 + ch) * (WCB / 4);
-          *reinterpret_cast<float4 *>(reinterpret_cast<unsigned char *>(blk) + off) =
-              make_float4(h4[0], h4[1], h4[2], h4[3]);
-          *reinterpret_cast<float4 *>(reinterpret_cast<unsigned char *>(blk) + WB + off) =
-              make_float4(l4[0], l4[1], l4[2], l4[3]);
-        }
-      }
+        anyk = fmaxf(fmaxf(w[0], w[1]), fmaxf(w[2], w[3])) > 0.0f;
+        F2 ri[2], hi[2], lo[2];
+        f2_load2(R + 48 + e0, ri[0], ri[1]);   // 1/err
+#pragma unroll
+        for (int h = 0; h < 2; h++) split2(f2_mul(F2(w[2 * h], w[2 * h + 1]), ri[h]), hi[h], lo[h]);
+        const uint32_t off = kmaj(wc, e0);
+        f2_store2(reinterpret_cast<float *>(Whi + off), hi[0], hi[1]);
+        f2_store2(reinterpret_cast<float *>(Wlo + off), lo[0], lo[1]);
       }
       // ---- feature products: feature f over the 16 observations
       if (fin) {
-        const float *yT = reinterpret_cast<const float *>(rec + 512);
-        const float4 *yi = reinterpret_cast<const float4 *>(yT + rowi);
-        const float4 *yj = reinterpret_cast<const float4 *>(yT + rowj);
+        const float *yi = R + 128 + rowi, *yj = R + 128 + rowj;
 #pragma unroll
         for (int grp = 0; grp < 4; grp++) {
-          const float4 a4 = yi[grp], b4 = yj[grp];
-          const float v[4] = {a4.x * b4.x, a4.y * b4.y, a4.z * b4.z, a4.w * b4.w};
-          float h4[4], l4[4];
+          F2 ai[2], bj[2], hi[2], lo[2];
+          f2_load2(yi + 4 * grp, ai[0], ai[1]);
+          f2_load2(yj + 4 * grp, bj[0], bj[1]);
 #pragma unroll
-          for (int u = 0; u < 4; u++) tc::split_tf32(fv ? v[u] : 0.0f, h4[u], l4[u]);
+          for (int h = 0; h < 2; h++) split2(f2_mul(ai[h], bj[h]), hi[h], lo[h]);
           const uint32_t off = kmaj(f, grp * 4);
-          *reinterpret_cast<float4 *>(Phi + off) = make_float4(h4[0], h4[1], h4[2], h4[3]);
-          *reinterpret_cast<float4 *>(Plo + off) = make_float4(l4[0], l4[1], l4[2], l4[3]);
+          f2_store2(reinterpret_cast<float *>(Phi + off), hi[0], hi[1]);
+          f2_store2(reinterpret_cast<float *>(Plo + off), lo[0], lo[1]);
         }
       }
       if (__any_sync(0xffffffffu, anyk) && lane == 0) S.anyk[s] = ch + 1;
@@ -648,11 +662,6 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
       const uint32_t id0 = tc::idesc_tf32(TM, nb0), id1 = nb1 > 0 ? tc::idesc_tf32(TM, nb1) : 0u;
       bool issued = false;   // since the last drain
       int nmma = 0, fj = 0;
-      // later passes: the chunks' MMA flags from pass 0, loaded two chunks
-      // ahead into alternating registers (each is read two iterations after
-      // its load is issued)
-      auto flag_at = [&](int c) { return (WMODE == 2 && c < nchunks) ? wflag[c0 + c] : 0; };
-      int flag_even = flag_at(0), flag_odd = flag_at(1);
       for (int ch = 0; ch < nchunks; ch++) {
         const int s = ch % NS;
         if (ch > 0 && ch % a.drain == 0) {
@@ -666,17 +675,10 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
           fj++;
           issued = false;
         }
-        int cached_flag = 0;
-        if (WMODE == 2) {
-          if (ch & 1) { cached_flag = flag_odd; flag_odd = flag_at(ch + 2); }
-          else { cached_flag = flag_even; flag_even = flag_at(ch + 2); }
-        }
         if (!tc::mbar_wait(reinterpret_cast<uint64_t *>(&S.full[s]), (ch / NS) & 1)) { S.fault = 1; break; }
         // every producer is done with the records of chunk ch: refill the slot
         if (n_loaded < nchunks) load(n_loaded++);
-        const bool mma = WMODE == 2 ? cached_flag != 0 : S.anyk[s] == ch + 1;
-        if (WMODE == 1) wflag[c0 + ch] = mma ? 1 : 0;
-        if (mma) {
+        if (S.anyk[s] == ch + 1) {
           tc::fence_after();
           const uint32_t whi = tc::smem_u32(stage_ptr(s)), wlo = whi + WB, phi = whi + 2 * WB, plo = phi + PB;
 #pragma unroll
@@ -907,49 +909,27 @@ cudaError_t launch_tile_fill(cudaStream_t st, int ntiles, const TilePar *tp, con
   return cudaGetLastError();
 }
 
-template <int LOC, int NS, int NR, int WMODE, bool CULL>
+template <int LOC, bool CULL>
 static cudaError_t launch_gram_tc_c(cudaStream_t st, const TcArgs &a, size_t smem, long long grid) {
-  cudaError_t e = cudaFuncSetAttribute(k_gram_tc<LOC, NS, NR, WMODE, CULL>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(k_gram_tc<LOC, 2, 6, CULL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)smem);
   if (e != cudaSuccess) return e;
-  k_gram_tc<LOC, NS, NR, WMODE, CULL><<<(int)grid, NT, smem, st>>>(a);
+  k_gram_tc<LOC, 2, 6, CULL><<<(int)grid, NT, smem, st>>>(a);
   return cudaGetLastError();
 }
 
-template <int LOC, int NS, int NR, int WMODE>
-static cudaError_t launch_gram_tc_t(cudaStream_t st, const TcArgs &a, size_t smem, long long grid) {
-  if (WMODE != 2 && a.cull) return launch_gram_tc_c<LOC, NS, NR, WMODE, WMODE != 2>(st, a, smem, grid);
-  return launch_gram_tc_c<LOC, NS, NR, WMODE, false>(st, a, smem, grid);
-}
-
 template <int LOC>
-static cudaError_t launch_gram_tc_loc(cudaStream_t st, TcArgs a, int *launches) {
+static cudaError_t launch_gram_tc_loc(cudaStream_t st, const TcArgs &a, int *launches) {
   int ns, nr;
   size_t smem;
   gram_tc_config(a.k, a.np, &ns, &nr, &smem);   // two stages, six record slots
   (void)ns;
   (void)nr;
   if (smem > kSmemBudget) return cudaErrorInvalidValue;   // k <= 128 fits
-  const long long per_pass = (long long)a.nwork * a.groups;
-  if (per_pass * a.npass > 0x7fffffffLL) return cudaErrorInvalidValue;
-  cudaError_t e;
-  if (a.npass >= 2 && a.wcache) {
-    // first pass computes the weights and caches them; later passes read them
-    a.pass0 = 0;
-    a.npl = 1;
-    e = launch_gram_tc_t<LOC, 2, 6, 1>(st, a, smem, per_pass);
-    if (e != cudaSuccess) return e;
-    a.pass0 = 1;
-    a.npl = a.npass - 1;
-    e = launch_gram_tc_t<LOC, 2, 6, 2>(st, a, smem, per_pass * a.npl);
-    (*launches) += 2;
-    return e;
-  }
-  a.pass0 = 0;
-  a.npl = a.npass;
-  e = launch_gram_tc_t<LOC, 2, 6, 0>(st, a, smem, per_pass * a.npass);
+  const long long grid = (long long)a.nwork * a.groups * a.npass;
+  if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
   (*launches)++;
-  return e;
+  return a.cull ? launch_gram_tc_c<LOC, true>(st, a, smem, grid) : launch_gram_tc_c<LOC, false>(st, a, smem, grid);
 }
 
 cudaError_t launch_gram_tc(cudaStream_t st, const TcArgs &a_in, int *launches) {
@@ -1053,20 +1033,13 @@ cudaError_t launch_gram_segsum(cudaStream_t st, const TcArgs &a, const int *acti
   return cudaGetLastError();
 }
 
-size_t gram_tc_wcache_bytes(int groups, int nchunk_total) {
-  return (size_t)groups * nchunk_total * (WCB + sizeof(int));   // operand blocks, then the MMA flags
-}
-
 template <int LOC>
 static cudaError_t preload_gram_tc_loc() {
   cudaFuncAttributes fa;
   cudaError_t e = cudaSuccess;
   auto get = [&](const void *f) { if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, f); };
-  get((const void *)k_gram_tc<LOC, 2, 6, 0, false>);
-  get((const void *)k_gram_tc<LOC, 2, 6, 0, true>);
-  get((const void *)k_gram_tc<LOC, 2, 6, 1, false>);
-  get((const void *)k_gram_tc<LOC, 2, 6, 1, true>);
-  get((const void *)k_gram_tc<LOC, 2, 6, 2, false>);
+  get((const void *)k_gram_tc<LOC, 2, 6, false>);
+  get((const void *)k_gram_tc<LOC, 2, 6, true>);
   get((const void *)k_tile_prep);
   get((const void *)k_tile_count);
   get((const void *)k_tile_scan);

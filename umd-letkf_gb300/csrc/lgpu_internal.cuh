@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "letkf_gpu.h"
+#include "lgpu_f32x2.cuh"
 
 namespace lgpu {
 
@@ -186,72 +187,75 @@ constexpr float kGuard2 = 3.0e-6f;        // two-factor products
 constexpr float kStdev2Max = 3.65148377f; // SQRT(40.0/3.0) in REAL, src/letkf_solver.F90:47
 
 // ---------------------------------------------- fast weight path -----
-// The batched Gram evaluates distance and Gaspari-Cohn in float with fused
-// multiply-adds and approximate reciprocals, and falls back to the exact
-// metric and the per-column localizer for a pair whose fast distance lies
-// within kFastDistBand (relative) of the search radius or whose fast weight
-// lies within kGuardFast of the keep threshold.  Against the exact path the
-// fast distance is within 1e-6 relative and the fast weight within 2e-8
-// absolute near the keep threshold (tests/test_gpu_parity.py); the bands
-// hold a 5x margin over those bounds.
-constexpr float kFastDistBand = 5.0e-6f;
+// The batched Gram evaluates distance and Gaspari-Cohn in float for two
+// observations at a time (packed multiply-adds, approximate reciprocals and
+// roots), and falls back to the exact metric and the per-column localizer for
+// a pair whose squared chord lies within kFastChordBand (relative) of the
+// search radius' or whose fast weight lies within kGuardFast of the keep
+// threshold.  Against the exact path the fast distance is within 1e-6
+// relative and the fast weight within 2e-8 absolute near the keep threshold
+// (tests/test_gpu_parity.py); the bands hold a 5x margin over those bounds (a
+// chord's square moves by at most twice the distance's relative change).
+constexpr float kFastChordBand = 1.0e-5f;
 constexpr float kGuardFast = 1.0e-7f;
 
-// squared chord between unit vectors, fused multiply-adds
-__device__ __forceinline__ float chord2_fast(float ax, float ay, float az, float bx, float by, float bz) {
-  const float dx = __fsub_rn(ax, bx), dy = __fsub_rn(ay, by), dz = __fsub_rn(az, bz);
-  return __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
+// squared chords between a column (its negated unit vector, both halves) and
+// two observations; the 1e-30 keeps the root below finite
+__device__ __forceinline__ F2 chord2_fast(F2 nx, F2 ny, F2 nz, F2 ox, F2 oy, F2 oz) {
+  const F2 dx = f2_add(ox, nx), dy = f2_add(oy, ny), dz = f2_add(oz, nz);
+  return f2_fma(dx, dx, f2_fma(dy, dy, f2_fma(dz, dz, f2_all(1e-30f))));
 }
 
-// asin(x), 0 <= x <= 0.5: Taylor series of asin in Horner form with fused
-// multiply-adds (a few ulp).  x <= 0.25: terms to x^13 (truncation below
-// 2e-11 relative); otherwise to x^21.
-__device__ __forceinline__ float asin_fast(float x, bool short_series = false) {
-  const float x2 = x * x;
-  float p;
+// great-circle distances (m) from squared chords up to 1: 2 R asin(h), h half
+// the chord, by asin's Taylor series in h^2 = c2 / 4 (a few ulp).  Half-chords
+// up to 0.25: terms to h^13 (truncation below 2e-11 relative); else to h^21.
+__device__ __forceinline__ F2 dist_fast(F2 c2, bool short_series) {
+  constexpr float q = 0.25f;
+  F2 p;
   if (short_series) {
-    p = 0.017352763563394547f;
+    p = f2_all(0.017352763563394547f * q * q * q * q * q * q);
   } else {
-    p = 0.008390335366129875f;
-    p = __fmaf_rn(p, x2, 0.009761609137058258f);
-    p = __fmaf_rn(p, x2, 0.01155180111527443f);
-    p = __fmaf_rn(p, x2, 0.013964843936264515f);
-    p = __fmaf_rn(p, x2, 0.017352763563394547f);
+    p = f2_all(0.008390335366129875f * q * q * q * q * q * q * q * q * q * q);
+    p = f2_fma(p, c2, f2_all(0.009761609137058258f * q * q * q * q * q * q * q * q * q));
+    p = f2_fma(p, c2, f2_all(0.01155180111527443f * q * q * q * q * q * q * q * q));
+    p = f2_fma(p, c2, f2_all(0.013964843936264515f * q * q * q * q * q * q * q));
+    p = f2_fma(p, c2, f2_all(0.017352763563394547f * q * q * q * q * q * q));
   }
-  p = __fmaf_rn(p, x2, 0.022372158244252205f);
-  p = __fmaf_rn(p, x2, 0.0303819440305233f);
-  p = __fmaf_rn(p, x2, 0.0446428582072258f);
-  p = __fmaf_rn(p, x2, 0.07500000298023224f);
-  p = __fmaf_rn(p, x2, 0.1666666716337204f);
-  return __fmaf_rn(x * x2, p, x);
+  p = f2_fma(p, c2, f2_all(0.022372158244252205f * q * q * q * q * q));
+  p = f2_fma(p, c2, f2_all(0.0303819440305233f * q * q * q * q));
+  p = f2_fma(p, c2, f2_all(0.0446428582072258f * q * q * q));
+  p = f2_fma(p, c2, f2_all(0.07500000298023224f * q * q));
+  p = f2_fma(p, c2, f2_all(0.1666666716337204f * q));
+  const F2 h = f2_mul(f2_mul(c2, F2(rsqrt_approx(c2.x()), rsqrt_approx(c2.y()))), f2_all(6371000.0f));
+  return f2_fma(h, f2_mul(c2, p), h);
 }
 
 // Gaspari-Cohn of zc = |z| / c without branches: the same two polynomials as
-// gc_fast (outer one in the shifted variable t = 2 - zc, divided by zc with
-// the approximate divide); within 1e-6 of gc_exact.
-__device__ __forceinline__ float gc_branchless(float zc) {
-  const float t = 2.0f - zc;
-  float q = 0.08333f;
-  q = __fmaf_rn(q, t, -0.49996f);
-  q = __fmaf_rn(q, t, 0.6248f);
-  q = __fmaf_rn(q, t, 0.0005299999999996974f);
-  q = __fmaf_rn(q, t, -0.0007799999999991147f);
-  q = __fmaf_rn(q, t, 0.0005999999999986017f);
-  q = __fmaf_rn(q, t, -0.0001899999999991353f);
-  const float qo = __fdividef(q, zc);
-  float p = -0.25f;
-  p = __fmaf_rn(p, zc, 0.5f);
-  p = __fmaf_rn(p, zc, 0.625f);
-  p = __fmaf_rn(p, zc, -1.66667f);
-  const float pi = __fmaf_rn(p, zc * zc, 1.0f);
-  return zc >= 2.0f ? 0.0f : (zc > 1.0f ? qo : pi);
-}
-
-// great-circle distance (m) from the squared chord, fast path (chord <= 1;
-// short_series for half-chords up to 0.25)
-__device__ __forceinline__ float dist_fast(float c2f, bool short_series = false) {
-  const float hf = 0.5f * c2f * rsqrtf(fmaxf(c2f, 1e-30f));
-  return 12742000.0f * asin_fast(fminf(hf, 0.5f), short_series);
+// gc_fast (outer one in the shifted variable t = 2 - zc, divided by zc);
+// within 1e-6 of gc_exact up to zc = 2.  Beyond (outside the search radius,
+// where the caller drops the pair) it returns the outer polynomial unless
+// `cut`, then 0.
+__device__ __forceinline__ F2 gc_branchless(F2 zc, bool cut) {
+  const F2 t = f2_fma(zc, f2_all(-1.0f), f2_all(2.0f));
+  F2 q = f2_all(0.08333f);
+  q = f2_fma(q, t, f2_all(-0.49996f));
+  q = f2_fma(q, t, f2_all(0.6248f));
+  q = f2_fma(q, t, f2_all(0.0005299999999996974f));
+  q = f2_fma(q, t, f2_all(-0.0007799999999991147f));
+  q = f2_fma(q, t, f2_all(0.0005999999999986017f));
+  q = f2_fma(q, t, f2_all(-0.0001899999999991353f));
+  q = f2_mul(q, F2(rcp_approx(zc.x()), rcp_approx(zc.y())));
+  F2 p = f2_all(-0.25f);
+  p = f2_fma(p, zc, f2_all(0.5f));
+  p = f2_fma(p, zc, f2_all(0.625f));
+  p = f2_fma(p, zc, f2_all(-1.66667f));
+  p = f2_fma(p, f2_mul(zc, zc), f2_all(1.0f));
+  float x = zc.x() > 1.0f ? q.x() : p.x(), y = zc.y() > 1.0f ? q.y() : p.y();
+  if (cut) {
+    x = zc.x() >= 2.0f ? 0.0f : x;
+    y = zc.y() >= 2.0f ? 0.0f : y;
+  }
+  return F2(x, y);
 }
 
 // Packed Gram layout of one unit: the upper triangle of G (i <= j, row-major)
@@ -469,10 +473,6 @@ struct TcArgs {
   const int *tile_n;         // [ntiles] candidates of each tile
   int cb;                    // bytes per chunk record (set by the launcher)
   uint32_t tmem_cols;        // TMEM columns per CTA (set by the launcher)
-  float *wcache;             // weight cache [groups][chunks] TF32 hi | lo operand blocks, or null
-  int *wflag;                // [groups][chunks]: the chunk has a kept pair (MMA issued)
-  int nchunk_total;          // chunks over all tiles (weight cache indexing)
-  int pass0, npl;            // feature passes of one launch: [pass0, pass0 + npl) (set by the launcher)
   // accumulation segments and drains: each tile's chunk stream is split into
   // segments (one CTA each), and each CTA moves its tensor-core accumulator
   // out every `drain` chunks (the FP32 accumulation error of the tensor core
@@ -510,7 +510,6 @@ cudaError_t launch_gram_tc(cudaStream_t st, const TcArgs &a, int *launches);
 // (for one localizer class) Gram kernels ahead of a timed trial
 cudaError_t preload_gram(void);
 cudaError_t preload_gram_tc(int loc_cls);
-size_t gram_tc_wcache_bytes(int groups, int nchunk_total);
 void gram_tc_passes(int k, int *npass, int *np);
 
 struct EigArgs {
