@@ -2067,18 +2067,14 @@ int lgpu_learn_train(lgpu_handle *h, int epochs, int batch, float lr, float *los
                       L->H1.as<unsigned char>(), L->H2.as<unsigned char>(), Ycal, S.dout, h->buf[B_STATUS].as<int>(),
                       &launches),
        "network forward");
-    std::vector<float> y((size_t)ncal * S.dout);
-    CK(cudaMemcpyAsync(y.data(), Ycal, 4 * y.size(), cudaMemcpyDeviceToHost, st), "D2H");
+    // (the batch order is spent: its buffer takes the scores)
+    CK(mlp_row_rms(st, Ycal, ncal, S.dout, L->bidx.as<float>()), "network output RMS");
+    std::vector<float> sc(ncal);
+    CK(cudaMemcpyAsync(sc.data(), L->bidx.p, 4 * sc.size(), cudaMemcpyDeviceToHost, st), "D2H");
     int stat = 0;
     CK(cudaMemcpyAsync(&stat, h->buf[B_STATUS].p, 4, cudaMemcpyDeviceToHost, st), "D2H");
     CK(cudaStreamSynchronize(st), "calibration");
     if (stat & 16) return fail(h, LGPU_ERR_CUDA, "network forward: tensor-core pipeline wait timed out");
-    std::vector<float> sc(ncal);
-    for (int r = 0; r < ncal; r++) {
-      double q = 0.0;
-      for (int e = 0; e < S.dout; e++) q += (double)y[(size_t)r * S.dout + e] * y[(size_t)r * S.dout + e];
-      sc[r] = (float)std::sqrt(q / S.dout);
-    }
     std::sort(sc.begin(), sc.end());
     const double qf = 1.0 - (double)L->cfg.gate_frac;
     L->tau = L->cfg.gate_frac <= 0.0f ? 3.0e38f : sc[(size_t)std::min<double>(ncal - 1, std::floor(qf * (ncal - 1)))];

@@ -335,7 +335,7 @@ __device__ __forceinline__ void split2(F2 v, F2 &hi, F2 &lo) {
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h0) : "f"(v.x()));
   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h1) : "f"(v.y()));
   hi = F2(__uint_as_float(h0), __uint_as_float(h1));
-  lo = f2_fma(hi, f2_all(-1.0f), v);   // exact
+  lo = f2_fma(hi, F2(kFC.minus_one), v);   // exact
 }
 
 struct TcSmem {

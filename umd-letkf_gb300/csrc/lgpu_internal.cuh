@@ -199,34 +199,52 @@ constexpr float kStdev2Max = 3.65148377f; // SQRT(40.0/3.0) in REAL, src/letkf_s
 constexpr float kFastChordBand = 1.0e-5f;
 constexpr float kGuardFast = 1.0e-7f;
 
+// The constants of the packed weight path, both halves alike, in constant
+// memory: an instruction reads them from there, where a literal pair costs two
+// moves into registers each time it is used.
+struct FastConst {
+  unsigned long long asin_short, asin_c[10];   // asin's series in c2 = 4 h^2, highest power first
+  unsigned long long gq[7], gp[4], one, two, minus_one, tiny, radius;
+};
+constexpr unsigned long long f2_bits(float v) {
+  const unsigned long long b = __builtin_bit_cast(unsigned, v);
+  return b | b << 32;
+}
+constexpr float kQ = 0.25f, kQ2 = kQ * kQ, kQ4 = kQ2 * kQ2, kQ8 = kQ4 * kQ4;
+static __constant__ FastConst kFC = {
+    f2_bits(0.017352763563394547f * kQ4 * kQ2),
+    {f2_bits(0.008390335366129875f * kQ8 * kQ2), f2_bits(0.009761609137058258f * kQ8 * kQ),
+     f2_bits(0.01155180111527443f * kQ8), f2_bits(0.013964843936264515f * kQ4 * kQ2 * kQ),
+     f2_bits(0.017352763563394547f * kQ4 * kQ2), f2_bits(0.022372158244252205f * kQ4 * kQ),
+     f2_bits(0.0303819440305233f * kQ4), f2_bits(0.0446428582072258f * kQ2 * kQ), f2_bits(0.07500000298023224f * kQ2),
+     f2_bits(0.1666666716337204f * kQ)},
+    {f2_bits(0.08333f), f2_bits(-0.49996f), f2_bits(0.6248f), f2_bits(0.0005299999999996974f),
+     f2_bits(-0.0007799999999991147f), f2_bits(0.0005999999999986017f), f2_bits(-0.0001899999999991353f)},
+    {f2_bits(-0.25f), f2_bits(0.5f), f2_bits(0.625f), f2_bits(-1.66667f)},
+    f2_bits(1.0f), f2_bits(2.0f), f2_bits(-1.0f), f2_bits(1e-30f), f2_bits(6371000.0f)};
+
 // squared chords between a column (its negated unit vector, both halves) and
 // two observations; the 1e-30 keeps the root below finite
 __device__ __forceinline__ F2 chord2_fast(F2 nx, F2 ny, F2 nz, F2 ox, F2 oy, F2 oz) {
   const F2 dx = f2_add(ox, nx), dy = f2_add(oy, ny), dz = f2_add(oz, nz);
-  return f2_fma(dx, dx, f2_fma(dy, dy, f2_fma(dz, dz, f2_all(1e-30f))));
+  return f2_fma(dx, dx, f2_fma(dy, dy, f2_fma(dz, dz, F2(kFC.tiny))));
 }
 
 // great-circle distances (m) from squared chords up to 1: 2 R asin(h), h half
 // the chord, by asin's Taylor series in h^2 = c2 / 4 (a few ulp).  Half-chords
 // up to 0.25: terms to h^13 (truncation below 2e-11 relative); else to h^21.
 __device__ __forceinline__ F2 dist_fast(F2 c2, bool short_series) {
-  constexpr float q = 0.25f;
   F2 p;
   if (short_series) {
-    p = f2_all(0.017352763563394547f * q * q * q * q * q * q);
+    p = F2(kFC.asin_short);
   } else {
-    p = f2_all(0.008390335366129875f * q * q * q * q * q * q * q * q * q * q);
-    p = f2_fma(p, c2, f2_all(0.009761609137058258f * q * q * q * q * q * q * q * q * q));
-    p = f2_fma(p, c2, f2_all(0.01155180111527443f * q * q * q * q * q * q * q * q));
-    p = f2_fma(p, c2, f2_all(0.013964843936264515f * q * q * q * q * q * q * q));
-    p = f2_fma(p, c2, f2_all(0.017352763563394547f * q * q * q * q * q * q));
+    p = F2(kFC.asin_c[0]);
+#pragma unroll
+    for (int i = 1; i < 5; i++) p = f2_fma(p, c2, F2(kFC.asin_c[i]));
   }
-  p = f2_fma(p, c2, f2_all(0.022372158244252205f * q * q * q * q * q));
-  p = f2_fma(p, c2, f2_all(0.0303819440305233f * q * q * q * q));
-  p = f2_fma(p, c2, f2_all(0.0446428582072258f * q * q * q));
-  p = f2_fma(p, c2, f2_all(0.07500000298023224f * q * q));
-  p = f2_fma(p, c2, f2_all(0.1666666716337204f * q));
-  const F2 h = f2_mul(f2_mul(c2, F2(rsqrt_approx(c2.x()), rsqrt_approx(c2.y()))), f2_all(6371000.0f));
+#pragma unroll
+  for (int i = 5; i < 10; i++) p = f2_fma(p, c2, F2(kFC.asin_c[i]));
+  const F2 h = f2_mul(f2_mul(c2, F2(rsqrt_approx(c2.x()), rsqrt_approx(c2.y()))), F2(kFC.radius));
   return f2_fma(h, f2_mul(c2, p), h);
 }
 
@@ -236,20 +254,17 @@ __device__ __forceinline__ F2 dist_fast(F2 c2, bool short_series) {
 // where the caller drops the pair) it returns the outer polynomial unless
 // `cut`, then 0.
 __device__ __forceinline__ F2 gc_branchless(F2 zc, bool cut) {
-  const F2 t = f2_fma(zc, f2_all(-1.0f), f2_all(2.0f));
-  F2 q = f2_all(0.08333f);
-  q = f2_fma(q, t, f2_all(-0.49996f));
-  q = f2_fma(q, t, f2_all(0.6248f));
-  q = f2_fma(q, t, f2_all(0.0005299999999996974f));
-  q = f2_fma(q, t, f2_all(-0.0007799999999991147f));
-  q = f2_fma(q, t, f2_all(0.0005999999999986017f));
-  q = f2_fma(q, t, f2_all(-0.0001899999999991353f));
+  const F2 t = f2_fma(zc, F2(kFC.minus_one), F2(kFC.two));
+  F2 q = F2(kFC.gq[0]);
+#pragma unroll
+  for (int i = 1; i < 7; i++) q = f2_fma(q, t, F2(kFC.gq[i]));
   q = f2_mul(q, F2(rcp_approx(zc.x()), rcp_approx(zc.y())));
-  F2 p = f2_all(-0.25f);
-  p = f2_fma(p, zc, f2_all(0.5f));
-  p = f2_fma(p, zc, f2_all(0.625f));
-  p = f2_fma(p, zc, f2_all(-1.66667f));
-  p = f2_fma(p, f2_mul(zc, zc), f2_all(1.0f));
+  // 1 + zc^2 (-1.66667 + zc (0.625 + zc (0.5 - 0.25 zc)))
+  const F2 z2 = f2_mul(zc, zc);
+  F2 p = F2(kFC.gp[0]);
+#pragma unroll
+  for (int i = 1; i < 4; i++) p = f2_fma(p, zc, F2(kFC.gp[i]));
+  p = f2_fma(p, z2, F2(kFC.one));
   float x = zc.x() > 1.0f ? q.x() : p.x(), y = zc.y() > 1.0f ? q.y() : p.y();
   if (cut) {
     x = zc.x() >= 2.0f ? 0.0f : x;
@@ -600,6 +615,7 @@ cudaError_t mlp_grad(cudaStream_t st, const MlpShape &s, const float *wq, const 
 cudaError_t mlp_adam(cudaStream_t st, long long n, float *w, float *wq, const float *g, float *m, float *v, float lr,
                      int step);
 cudaError_t mlp_round(cudaStream_t st, long long n, const float *w, float *wq);
+cudaError_t mlp_row_rms(cudaStream_t st, const float *y, int rows, int n, float *out);   // RMS of each row
 
 // ---- learned analysis form (lgpu_learn.cu) ----
 struct LrnInterpArgs {

@@ -213,8 +213,20 @@ __global__ void __launch_bounds__(TC_THREADS) k_mlp_tc(MlpTcArgs a) {
 
 // ---------------------------------------------------------------------------
 // CUDA-core GEMM for training: C(m, n) = sum_k A(m, k) B(k, n) with
-// A(m, k) = A[m sam + k sak], B(k, n) = B[k sbk + n sbn]; 64 x 64 tiles, 16-wide
-// K slices, 256 threads, 4 x 4 outputs per thread, FP32 accumulation in k order.
+// A(m, k) = A[m sam + k sak], B(k, n) = B[k sbk + n sbn], one stride of each
+// operand being 1.  FP32 accumulation in k order, one multiply-add at a time
+// per output, so that the result does not depend on the tiling.
+//
+// A training batch's products are small (512 x 512 to 512 x 1072): with 64 x 64
+// tiles and one slice of operands in flight, 64 blocks waited on global memory
+// (130 us for 512 x 512 x 1072).  32 x 64 tiles give 128 to 272 blocks, three
+// slices of GK are on their way (asynchronous copies), and a thread's 4 x 4
+// outputs take two 16-byte reads a step (packed multiply-adds would need their
+// broadcast operand duplicated and run at the same rate).
+constexpr int GM = 32, GN = 64, GK = 32, GS = 4;   // tile, slice, slices resident
+constexpr int GT = 128;                            // threads
+constexpr int GAP = GM + 4, GBP = GN + 4;          // row pitches (16-byte rows, shifted banks)
+constexpr int GSTAGE = GK * (GAP + GBP);
 struct GemmArgs {
   const float *A, *B;
   long long sam, sak, sbk, sbn;
@@ -228,46 +240,80 @@ struct GemmArgs {
 
 // EPI 0: C = acc; 1: C = acc + bias (pre-activation), H = bf16(gelu(C));
 // 2: C = acc * gelu'(Zp); 3: C = acc + bias
+// one operand's slice (GK x W elements, element (kk, x) at dst[kk * pitch + x])
+// of a matrix with strides sx (along the tile) and sk; zero outside X x K.
+// 16 bytes at a time where the tile's direction is contiguous and aligned.
+template <int W, int PITCH>
+__device__ __forceinline__ void gemm_fetch(float *dst, const float *src, long long sx, long long sk, int x0, int k0,
+                                           int X, int K) {
+  if (sx == 1 && (sk & 3) == 0 && (X & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+#pragma unroll
+    for (int t = threadIdx.x; t < GK * W / 4; t += GT) {
+      const int kk = t / (W / 4), xx = t % (W / 4) * 4, x = x0 + xx, k = k0 + kk;
+      const bool in = x < X && k < K;
+      const float *p = in ? src + x + (long long)k * sk : src;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(tc::smem_u32(dst + kk * PITCH + xx)), "l"(p),
+                   "r"(in ? 16 : 0) : "memory");
+    }
+  } else {
+    // 8 k by 4 x per warp and step: 32-byte runs of the source where k is the
+    // contiguous direction, and 32 different banks
+    const int lane = threadIdx.x & 31, kk = 8 * (threadIdx.x >> 5) + (lane & 7), k = k0 + kk;
+    const float *p = src + (long long)(x0 + (lane >> 3)) * sx + (long long)k * sk;
+    uint32_t d = tc::smem_u32(dst + kk * PITCH + (lane >> 3));
+#pragma unroll 4
+    for (int xx = lane >> 3; xx < W; xx += 4) {
+      const bool in = x0 + xx < X && k < K;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(in ? p : src), "r"(in ? 4 : 0)
+                   : "memory");
+      p += 4 * sx;
+      d += 16;
+    }
+  }
+}
+static_assert(GT == 128 && GK == 32, "a slice's k over the warps");
+
 template <int EPI>
-__global__ void __launch_bounds__(256) k_mlp_gemm(GemmArgs g) {
-  __shared__ float As[16][64 + 1];
-  __shared__ float Bs[16][64 + 1];
+__global__ void __launch_bounds__(GT) k_mlp_gemm(GemmArgs g) {
+  extern __shared__ __align__(16) float gsm[];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
+  const int m0 = blockIdx.y * GM, n0 = blockIdx.x * GN;
+  const int nk = (g.K + GK - 1) / GK;
+  auto fetch = [&](int q) {
+    if (q < nk) {
+      float *st = gsm + (q % GS) * GSTAGE;
+      gemm_fetch<GM, GAP>(st, g.A, g.sam, g.sak, m0, q * GK, g.M, g.K);
+      gemm_fetch<GN, GBP>(st + GK * GAP, g.B, g.sbn, g.sbk, n0, q * GK, g.N, g.K);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
   float acc[4][4];
 #pragma unroll
   for (int i = 0; i < 4; i++)
 #pragma unroll
     for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
-  for (int k0 = 0; k0 < g.K; k0 += 16) {
-    for (int t = threadIdx.x; t < 64 * 16; t += 256) {
-      const int mm = t / 16, kk = t % 16;
-      const int m = m0 + mm, k = k0 + kk;
-      As[kk][mm] = (m < g.M && k < g.K) ? g.A[(long long)m * g.sam + (long long)k * g.sak] : 0.0f;
-      const int nn = t % 64, kb = t / 64;
-      const int n = n0 + nn, k2 = k0 + kb;
-      Bs[kb][nn] = (n < g.N && k2 < g.K) ? g.B[(long long)k2 * g.sbk + (long long)n * g.sbn] : 0.0f;
-    }
+  for (int q = 0; q < GS - 1; q++) fetch(q);
+  for (int q = 0; q < nk; q++) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(GS - 2) : "memory");
     __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < 16; kk++) {
-      float av[4], bv[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) av[i] = As[kk][ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; j++) bv[j] = Bs[kk][tx + 16 * j];
+    fetch(q + GS - 1);   // into the slot of slice q - 1, which every thread has left
+    const float *As = gsm + (q % GS) * GSTAGE + 4 * ty, *Bs = gsm + (q % GS) * GSTAGE + GK * GAP + 4 * tx;
+#pragma unroll 16
+    for (int kk = 0; kk < GK; kk++) {
+      const float4 av = *reinterpret_cast<const float4 *>(As + kk * GAP);
+      const float4 bv = *reinterpret_cast<const float4 *>(Bs + kk * GBP);
+      const float a4[4] = {av.x, av.y, av.z, av.w}, b4[4] = {bv.x, bv.y, bv.z, bv.w};
 #pragma unroll
       for (int i = 0; i < 4; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = __fmaf_rn(av[i], bv[j], acc[i][j]);
+        for (int j = 0; j < 4; j++) acc[i][j] = __fmaf_rn(a4[i], b4[j], acc[i][j]);
     }
-    __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < 4; i++)
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      const int m = m0 + ty + 16 * i, n = n0 + tx + 16 * j;
+      const int m = m0 + 4 * ty + i, n = n0 + 4 * tx + j;
       if (m >= g.M || n >= g.N) continue;
       const size_t o = (size_t)m * g.ldc + n;
       float v = acc[i][j];
@@ -308,13 +354,43 @@ __global__ void k_mlp_loss(const float *Y, const float *T, float *dY, int rows, 
   if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
 }
 
-// column sums of a [rows][n] matrix (bias gradients), row order fixed
-__global__ void k_mlp_colsum(const float *D, int rows, int n, float *out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
+// column sums of a [rows][n] matrix (bias gradients), row order fixed: a block
+// stages CSR rows of 32 columns at a time and one warp adds them in order
+// (with one thread a column straight from global memory the 512 rows' loads
+// took 33 us)
+constexpr int CSR = 128;
+__global__ void __launch_bounds__(256) k_mlp_colsum(const float *D, int rows, int n, float *out) {
+  __shared__ float st[CSR][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
   float s = 0.0f;
-  for (int r = 0; r < rows; r++) s += D[(size_t)r * n + c];
-  out[c] = s;
+  for (int r0 = 0; r0 < rows; r0 += CSR) {
+#pragma unroll
+    for (int q = 0; q < CSR / 8; q++) {
+      const int r = r0 + wid + 8 * q;
+      st[wid + 8 * q][lane] = c < n && r < rows ? D[(size_t)r * n + c] : 0.0f;
+    }
+    __syncthreads();
+    if (wid == 0) {
+      const int m = rows - r0 < CSR ? rows - r0 : CSR;
+#pragma unroll 16
+      for (int q = 0; q < m; q++) s += st[q][lane];
+    }
+    __syncthreads();
+  }
+  if (wid == 0 && c < n) out[c] = s;
+}
+
+// RMS of each row of a [rows][n] matrix, summed in FP64 (a warp per row)
+__global__ void k_mlp_rowrms(const float *Y, int rows, int n, float *out) {
+  const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= rows) return;
+  double q = 0.0;
+  for (int c = lane; c < n; c += 32) {
+    const double v = Y[(size_t)r * n + c];
+    q = __fma_rn(v, v, q);
+  }
+  for (int o = 16; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+  if (lane == 0) out[r] = (float)sqrt(q / n);
 }
 
 // Adam on FP32 masters, then the BF16-rounded copy used by the forward
@@ -448,8 +524,11 @@ cudaError_t mlp_forward_tc(cudaStream_t st, const MlpShape &s, const unsigned ch
 
 template <int EPI>
 static cudaError_t gemm(cudaStream_t st, const GemmArgs &g) {
-  dim3 grid((g.N + 63) / 64, (g.M + 63) / 64);
-  k_mlp_gemm<EPI><<<grid, 256, 0, st>>>(g);
+  dim3 grid((g.N + GN - 1) / GN, (g.M + GM - 1) / GM);
+  const size_t smem = (size_t)GS * GSTAGE * sizeof(float);
+  cudaError_t e = cudaFuncSetAttribute(k_mlp_gemm<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  k_mlp_gemm<EPI><<<grid, GT, smem, st>>>(g);
   return cudaGetLastError();
 }
 
@@ -510,20 +589,20 @@ cudaError_t mlp_grad(cudaStream_t st, const MlpShape &s, const float *wq, const 
   *nparts = nb;
   // layer 3: dW3 = dY^T H2, db3 = colsum dY, dZ2 = (dY W3) * gelu'(Z2)
   if ((e = gemm<0>(st, gargs(dY, 1, s.dout, H2, s.H, 1, s.dout, s.H, rows, grad + off[4], s.H))) != cudaSuccess) return e;
-  k_mlp_colsum<<<(s.dout + 255) / 256, 256, 0, st>>>(dY, rows, s.dout, grad + off[5]);
+  k_mlp_colsum<<<(s.dout + 31) / 32, 256, 0, st>>>(dY, rows, s.dout, grad + off[5]);
   GemmArgs g = gargs(dY, s.dout, 1, wq + off[4], s.H, 1, rows, s.H, s.dout, dZ2, s.H);
   g.Zp = Z2;
   if ((e = gemm<2>(st, g)) != cudaSuccess) return e;
   // layer 2
   if ((e = gemm<0>(st, gargs(dZ2, 1, s.H, H1, s.H, 1, s.H, s.H, rows, grad + off[2], s.H))) != cudaSuccess) return e;
-  k_mlp_colsum<<<(s.H + 255) / 256, 256, 0, st>>>(dZ2, rows, s.H, grad + off[3]);
+  k_mlp_colsum<<<(s.H + 31) / 32, 256, 0, st>>>(dZ2, rows, s.H, grad + off[3]);
   g = gargs(dZ2, s.H, 1, wq + off[2], s.H, 1, rows, s.H, s.H, dZ1, s.H);
   g.Zp = Z1;
   if ((e = gemm<2>(st, g)) != cudaSuccess) return e;
   // layer 1
   if ((e = gemm<0>(st, gargs(dZ1, 1, s.H, x, s.din, 1, s.H, s.din, rows, grad + off[0], s.din))) != cudaSuccess)
     return e;
-  k_mlp_colsum<<<(s.H + 255) / 256, 256, 0, st>>>(dZ1, rows, s.H, grad + off[1]);
+  k_mlp_colsum<<<(s.H + 31) / 32, 256, 0, st>>>(dZ1, rows, s.H, grad + off[1]);
   return cudaGetLastError();
 }
 
@@ -536,6 +615,11 @@ cudaError_t mlp_adam(cudaStream_t st, long long n, float *w, float *wq, const fl
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.0f - powf(b1, (float)step), c2 = 1.0f - powf(b2, (float)step);
   k_mlp_adam<<<grid_for(n), 256, 0, st>>>(w, wq, g, m, v, n, lr, b1, b2, 1e-8f, c1, c2);
+  return cudaGetLastError();
+}
+
+cudaError_t mlp_row_rms(cudaStream_t st, const float *y, int rows, int n, float *out) {
+  if (rows > 0) k_mlp_rowrms<<<(rows + 7) / 8, 256, 0, st>>>(y, rows, n, out);
   return cudaGetLastError();
 }
 
