@@ -79,3 +79,35 @@ def test_refusals(k, mode):
                 with pytest.raises(LgpuError) as e:
                     s.debug_transform(np.stack(batch))
                 assert e.value.code == 9
+
+
+@pytest.mark.parametrize("k,copies", [(k, 7) for k in (2, 8, 16, 17, 32, 33, 37, 48, 49, 64, 65, 100, 128)]
+                         + [(k, 120) for k in (16, 37, 64)])   # lists below and above one wave of units
+def test_resolve_of_flagged_units(k, copies):
+    """FP32_RESOLVE with a gap threshold just below 1 flags every unit that
+    has two relevant eigenvalues; these get the FP64 form's accuracy, in any
+    batch, and the others keep FP32's."""
+    from letkf_gb300 import Solver
+    rng = np.random.default_rng(500 + k)
+    cs = cases(k, rng)
+    packed = np.stack([pack(G, b) for G, b in cs] * copies)   # several blocks of the gap test, the last one part filled
+    with Solver(0) as s:
+        s.set_precision("fp32")
+        T32 = s.debug_transform(packed)
+        s.set_precision("fp32_resolve", 0.999)
+        T = s.debug_transform(packed)
+        again = s.debug_transform(packed[::-1])[::-1]
+    assert np.array_equal(T, again)
+    flagged = expected = 0
+    for p, t, t32 in zip(packed, T, T32):
+        G, b = _unpack(p, k)
+        lam = np.linalg.eigvalsh(G + (k - 1) * np.eye(k))
+        # a relevant eigenvalue (clear of the floor) with a neighbour within the threshold
+        expected += bool(np.any((lam[:-1] > k - 1 + 1e-2 * lam[-1]) & (np.diff(lam) < 0.99 * lam[-1])))
+        if np.array_equal(t, t32):
+            continue
+        flagged += 1
+        ref = transform64(G, b)
+        tol = 1e-6 + 4 * 2.3e-16 * lam[-1] / lam[0]
+        assert np.abs(t - ref).max() / max(1.0, np.abs(ref).max()) < tol
+    assert flagged > 0 or expected == 0

@@ -39,6 +39,7 @@
 // path bounded the reduction.  The 2-D grid reads R + C values per R x C
 // multiply-adds.  The steps are unrolled in phases of LA rows so that the
 // blocks left of and above the trailing one are dropped at compile time.
+#include <type_traits>
 #include "lgpu_internal.cuh"
 #include <algorithm>
 #include <cmath>
@@ -876,18 +877,20 @@ __device__ __forceinline__ int unit_transform(typename G::R *mem, const typename
 template <class G>
 __global__ void __launch_bounds__(G::THREADS, G::MB) k_transform(EigArgs a, typename PolesOf<typename G::R>::type tab,
                                                           EigSplit sp, typename G::R *vscr, int u0, int nb,
-                                                          const int *range) {
+                                                          const int *range, int above, int upto) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   using R = typename G::R;
   const int slot = threadIdx.x / G::L, l = threadIdx.x % G::L;
   R *mem = reinterpret_cast<R *>(smem_raw) + (size_t)slot * G::UNIT;
   R *gv = vscr + ((size_t)blockIdx.x * G::UPB + slot) * G::REFL;
-  // units u0 .. u0 + nb (through ulist), or the flagged entries not yet re-solved
+  // units u0 .. u0 + nb (through ulist), or the flagged entries not yet
+  // re-solved, if there are more than `above` and at most `upto`
   int beg = 0, end = nb;
   const int *list = a.ulist;
   if (range) {
     beg = range[1];
     end = min(range[0], a.flag_cap);
+    if (end - beg <= above || end - beg > upto) return;
     list = a.flag_list;
     u0 = 0;
   }
@@ -916,83 +919,89 @@ __global__ void __launch_bounds__(G::THREADS, G::MB) k_transform(EigArgs a, type
   }
 }
 
-// FP32_RESOLVE: the units of a batch for the FP64 re-solve, a warp per unit on
-// the tridiagonal form k_transform left.  A unit is flagged when its FP32
-// solve failed, an eigenvalue is not positive, or two relevant eigenvalues lie
-// within gap_thresh * max l of each other.  The eigenvalues at the (k-1)/infl
-// floor (the null space of the Gram, k - n of them when n < k) are exactly
-// degenerate and harmless, since T is a function of the matrix and not of the
-// basis chosen in an eigenspace; they are left out of the test.
+// FP32_RESOLVE: the units of a batch for the FP64 re-solve, on the tridiagonal
+// form k_transform left.  A unit is flagged when its FP32 solve failed, an
+// eigenvalue is not positive, or two relevant eigenvalues lie within
+// gap_thresh * max l of each other.  The eigenvalues at the (k-1)/infl floor
+// (the null space of the Gram, k - n of them when n < k) are exactly degenerate
+// and harmless, since T is a function of the matrix and not of the basis chosen
+// in an eigenspace; they are left out of the test.
 //
-// Each lane bisects eigenvalues lane, lane + 32, ... on the count of negative
+// Each thread bisects one eigenvalue of one unit on the count of negative
 // pivots of T - x I (Sturm; Wilkinson & Reinsch, Handbook for Automatic
 // Computation II, 1971, contribution II/5): kBisect halvings of the Gershgorin
-// interval, past which FP32 resolves nothing of max l.  A QL iteration on one
-// thread per unit did the same arithmetic in one serial chain: 0.35 ms
-// whatever the number of units (k = 37), against 0.05.
+// interval, past which FP32 resolves nothing of max l.  A block's threads run
+// over the eigenvalues of as many units as fill it: with a warp per unit,
+// k = 37 took two rounds, the second on five lanes (4,248 units: 129 us, now
+// 80).
 constexpr int kBisect = 26;
-constexpr int GAPW = 4;   // warps (units) per block
+constexpr int GAPT = 256;                 // most threads per block; at least two units of kMaxK
+constexpr int GAPU = 8;                   // most units per block
+inline int gap_units(int k) { return std::min(GAPU, GAPT / k); }
+static_assert(GAPT >= kMaxK, "a unit's eigenvalues fit a block");
 
-__global__ void __launch_bounds__(32 * GAPW) k_eig_gap(EigArgs a, EigSplit sp, int u0, int nb) {
-  __shared__ float sd[GAPW][kMaxK], se[GAPW][kMaxK], sl[GAPW][kMaxK];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int ub = blockIdx.x * GAPW + warp;
-  if (ub >= nb) return;
-  const int unit = a.ulist ? a.ulist[u0 + ub] : u0 + ub;
-  if (a.nkept[unit] <= 0) return;
-  const int k = a.k;
-  bool flag = sp.bad[ub] != 0;
-  if (!flag) {
-    float *d = sd[warp], *e2 = se[warp], *lam = sl[warp];
+__global__ void __launch_bounds__(GAPT) k_eig_gap(EigArgs a, EigSplit sp, int u0, int nb, int upb) {
+  // rows of k values, one apart from a multiple of the banks
+  __shared__ float sd[GAPT + GAPU], se[GAPT + GAPU], sl[GAPT + GAPU];
+  __shared__ int sflag[GAPU];
+  const int k = a.k, pitch = k + (k % 32 == 0);
+  const int u = threadIdx.x / k, i = threadIdx.x - u * k;
+  const int ub = blockIdx.x * upb + u;
+  int unit = -1;
+  if (u < upb && ub < nb) {
+    unit = a.ulist ? a.ulist[u0 + ub] : u0 + ub;
+    if (a.nkept[unit] <= 0) unit = -1;
+  }
+  const bool failed = unit >= 0 && sp.bad[ub] != 0, test = unit >= 0 && !failed;
+  float *d = sd + u * pitch, *e2 = se + u * pitch, *lam = sl + u * pitch;
+  if (unit >= 0 && i == 0) sflag[u] = failed;
+  if (test) {
     const float *de = sp.DE + (size_t)ub * 2 * k;
-    float glo = 3.0e38f, ghi = -3.0e38f;
-    for (int i = lane; i < k; i += 32) {
-      const float di = de[i], el = i > 0 ? fabsf(de[k + i - 1]) : 0.0f, er = i < k - 1 ? fabsf(de[k + i]) : 0.0f;
-      d[i] = di;
-      e2[i] = el * el;
-      glo = fminf(glo, di - el - er);
-      ghi = fmaxf(ghi, di + el + er);
+    d[i] = de[i];
+    e2[i] = fabsf(i > 0 ? de[k + i - 1] : 0.0f);   // |e| first, for the interval
+    lam[i] = i < k - 1 ? fabsf(de[k + i]) : 0.0f;
+  }
+  __syncthreads();
+  float lo = 3.0e38f, hi = -3.0e38f, el = 0.0f;
+  if (test) {
+    for (int j = 0; j < k; j++) {
+      lo = fminf(lo, d[j] - e2[j] - lam[j]);
+      hi = fmaxf(hi, d[j] + e2[j] + lam[j]);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      glo = fminf(glo, __shfl_xor_sync(0xffffffffu, glo, o));
-      ghi = fmaxf(ghi, __shfl_xor_sync(0xffffffffu, ghi, o));
-    }
-    __syncwarp();
-    const float tiny = fmaxf(1e-30f, 1e-14f * fmaxf(fabsf(glo), fabsf(ghi)));
-    for (int i = lane; i < k; i += 32) {
-      float lo = glo, hi = ghi;
-      for (int it = 0; it < kBisect; it++) {
-        const float x = 0.5f * (lo + hi);
-        int below = 0;
-        float q = 1.0f;
+    el = e2[i];
+  }
+  __syncthreads();
+  if (test) e2[i] = el * el;
+  __syncthreads();
+  if (test) {
+    const float tiny = fmaxf(1e-30f, 1e-14f * fmaxf(fabsf(lo), fabsf(hi)));
+    for (int it = 0; it < kBisect; it++) {
+      const float x = 0.5f * (lo + hi);
+      int below = 0;
+      float q = 1.0f;
 #pragma unroll 4
-        for (int j = 0; j < k; j++) {
-          q = (d[j] - x) - __fdividef(e2[j], q);
-          q = fabsf(q) < tiny ? -tiny : q;
-          below += q < 0.0f;
-        }
-        if (below > i) hi = x;
-        else lo = x;
+      for (int j = 0; j < k; j++) {
+        q = (d[j] - x) - __fdividef(e2[j], q);
+        q = fabsf(q) < tiny ? -tiny : q;
+        below += q < 0.0f;
       }
-      lam[i] = 0.5f * (lo + hi);
+      if (below > i) hi = x;
+      else lo = x;
     }
-    __syncwarp();
-    const float lmax = lam[k - 1];
+    lam[i] = 0.5f * (lo + hi);
+  }
+  __syncthreads();
+  if (test) {
+    const float li = lam[i], lmax = lam[k - 1], bound = a.gap_thresh * lmax;
     // rounding level of the FP32 eigenvalues: a few k eps of the largest
     const float floor_v = (float)(k - 1) / a.infl;
     const float tol = 4.0f * (float)k * 1.1920929e-7f * lmax;
-    float gap = 3.0e38f;
-    bool neg = false;
-    for (int i = lane; i < k; i += 32) {
-      const float li = lam[i];
-      neg |= !(li > 0.0f);
-      // ascending: the nearest relevant neighbour is the next one
-      if (li - floor_v > tol && i + 1 < k) gap = fminf(gap, fabsf(lam[i + 1] - li));
-    }
-    for (int o = 16; o > 0; o >>= 1) gap = fminf(gap, __shfl_xor_sync(0xffffffffu, gap, o));
-    flag = gap <= a.gap_thresh * lmax || __any_sync(0xffffffffu, neg);
+    // ascending: the nearest relevant neighbour is the next one
+    const bool near = li - floor_v > tol && i + 1 < k && fabsf(lam[i + 1 < k ? i + 1 : i] - li) <= bound;
+    if (near || !(li > 0.0f) || 3.0e38f <= bound) sflag[u] = 1;
   }
-  if (flag && lane == 0) {
+  __syncthreads();
+  if (unit >= 0 && i == 0 && sflag[u]) {
     const int pos = atomicAdd(a.flag_n, 1);
     if (pos < a.flag_cap) a.flag_list[pos] = unit;
     else atomicOr(a.status, 128);   // list full: the unit keeps its FP32 solve
@@ -1010,13 +1019,14 @@ constexpr int resident_blocks() {
 // scratch is one slot per resident unit and stays in L2.
 template <class G>
 cudaError_t launch_g(cudaStream_t st, const EigArgs &a, const EigSplit &sp, int u0, int nb, const int *range,
-                     int *launches) {
+                     int above, int upto, int *launches) {
   const size_t smem = (size_t)G::UPB * G::UNIT * sizeof(typename G::R);
   cudaError_t e = cudaFuncSetAttribute(k_transform<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int grid = std::min(resident_blocks<G>(), (nb + G::UPB - 1) / G::UPB);
   k_transform<G><<<grid, G::THREADS, smem, st>>>(a, PolesOf<typename G::R>::get(), sp,
-                                                 reinterpret_cast<typename G::R *>(a.scratch), u0, nb, range);
+                                                 reinterpret_cast<typename G::R *>(a.scratch), u0, nb, range,
+                                                 above, upto);
   (*launches)++;
   return cudaGetLastError();
 }
@@ -1066,12 +1076,50 @@ auto with_grid_f64(int k, F f) {
 #undef LGPU_GRID
 }
 
-cudaError_t launch_f32(cudaStream_t st, const EigArgs &a, const EigSplit &sp, int u0, int nb, int *launches) {
-  return with_grid_f32(a.k, [&](auto g) { return launch_g<decltype(g)>(st, a, sp, u0, nb, nullptr, launches); });
+// FP64 grids for a list of few flagged units: four warps or more a unit.  A
+// warp issues FP64 to its own quarter of the SM, one multiply-add in two
+// clocks, so one warp a unit runs a lone unit at a quarter of the SM's rate
+// (k = 37, 5 units: 442 us, now 324).  With many units the lists' larger
+// padding and barriers cost more than they gain (k = 37, 4,248 units: 6.5 ms
+// against 3.0), so a list beyond one wave of these blocks takes the other
+// grids.  The list's length stays on the device: both kernels are launched, and
+// the one whose range it is not in returns at once.
+template <class F>
+auto with_grid_f64_few(int k, F f) {
+#define LGPU_GRID(...) return f(Grid<double, __VA_ARGS__>())
+  if (k <= 16) LGPU_GRID(1, 2, 16, 8, 2);
+  if (k <= 32) LGPU_GRID(2, 4, 16, 8, 2);
+  if (k <= 48) LGPU_GRID(3, 6, 16, 8, 2);
+  if (k <= 64) LGPU_GRID(4, 8, 16, 8, 2);
+#undef LGPU_GRID
+  return with_grid_f64(k, f);
 }
 
-cudaError_t launch_f64(cudaStream_t st, const EigArgs &a, int u0, int nb, const int *range, int *launches) {
-  return with_grid_f64(a.k, [&](auto g) { return launch_g<decltype(g)>(st, a, EigSplit{}, u0, nb, range, launches); });
+cudaError_t launch_f32(cudaStream_t st, const EigArgs &a, const EigSplit &sp, int u0, int nb, int *launches) {
+  return with_grid_f32(a.k, [&](auto g) { return launch_g<decltype(g)>(st, a, sp, u0, nb, nullptr, 0, 0, launches); });
+}
+
+cudaError_t launch_f64(cudaStream_t st, const EigArgs &a, int u0, int nb, int *launches) {
+  return with_grid_f64(
+      a.k, [&](auto g) { return launch_g<decltype(g)>(st, a, EigSplit{}, u0, nb, nullptr, 0, 0, launches); });
+}
+
+constexpr int kAll = 0x7fffffff;
+
+// the entries [range[1], range[0]) of the flagged list (as many blocks as
+// nunits units have scratch for; the list itself may be longer)
+cudaError_t launch_f64_list(cudaStream_t st, const EigArgs &a, const int *range, int *launches) {
+  int few = kAll;   // lists up to here on the first grid
+  cudaError_t e = with_grid_f64_few(a.k, [&](auto g) {
+    using G = decltype(g);
+    with_grid_f64(a.k, [&](auto h) {
+      if (!std::is_same<G, decltype(h)>::value) few = resident_blocks<G>();
+    });
+    return launch_g<G>(st, a, EigSplit{}, 0, a.nunits, range, 0, few, launches);
+  });
+  if (e != cudaSuccess || few == kAll || a.flag_cap <= few) return e;
+  return with_grid_f64(
+      a.k, [&](auto g) { return launch_g<decltype(g)>(st, a, EigSplit{}, 0, a.nunits, range, few, kAll, launches); });
 }
 
 struct ScratchOf {
@@ -1087,18 +1135,19 @@ struct ScratchOf {
 
 size_t eig_scratch_bytes(int k, int units, bool fp32, bool fp64) {
   const ScratchOf f{std::max(1, units)};
-  return std::max(fp32 ? with_grid_f32(k, f) : 0, fp64 ? with_grid_f64(k, f) : 0);
+  return std::max(fp32 ? with_grid_f32(k, f) : 0,
+                  fp64 ? std::max(with_grid_f64(k, f), with_grid_f64_few(k, f)) : 0);
 }
 
 cudaError_t launch_eig64(cudaStream_t st, const EigArgs &a, int ubase, int *launches) {
   if (a.nunits <= 0) return cudaSuccess;
-  return launch_f64(st, a, ubase, a.nunits, nullptr, launches);
+  return launch_f64(st, a, ubase, a.nunits, launches);
 }
 
 cudaError_t launch_eig64_flagged(cudaStream_t st, const EigArgs &a, int *launches) {
   if (!a.flag_list || a.flag_cap <= 0) return cudaSuccess;
   // the count stays on the device: the wave of blocks strides over the list
-  cudaError_t e = launch_f64(st, a, 0, a.nunits, a.flag_n, launches);
+  cudaError_t e = launch_f64_list(st, a, a.flag_n, launches);
   if (e != cudaSuccess) return e;
   return cudaMemcpyAsync(a.flag_n + 1, a.flag_n, sizeof(int), cudaMemcpyDeviceToDevice, st);
 }
@@ -1114,7 +1163,8 @@ cudaError_t launch_eig_split(cudaStream_t st, const EigArgs &a, const EigSplit &
   for (int u0 = ustart; u0 < uend; u0 += batch) {
     const int nb = uend - u0 < batch ? uend - u0 : batch;
     if ((e = launch_f32(st, a, sp, u0, nb, launches)) != cudaSuccess) return e;
-    k_eig_gap<<<(nb + GAPW - 1) / GAPW, 32 * GAPW, 0, st>>>(a, sp, u0, nb);
+    const int upb = gap_units(a.k);
+    k_eig_gap<<<(nb + upb - 1) / upb, (upb * a.k + 31) / 32 * 32, 0, st>>>(a, sp, u0, nb, upb);
     (*launches)++;
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
