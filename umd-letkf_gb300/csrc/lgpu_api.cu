@@ -62,7 +62,7 @@ enum {
   B_LAT, B_LON, B_MASK, B_COL2ACT, B_ACTIVE,
   B_BKG, B_MEANB, B_SPRDB, B_ANA, B_MEANA, B_SPRDA, B_SLABVAR, B_SLABLEV, B_VARINC, B_VARLB, B_VARUB,
   B_OLAT, B_OLON, B_OZ, B_OTIME, B_OVAL, B_OERR, B_OOBSID, B_OPLATID, B_HX, B_HXM, B_SATOBS, B_SATPLATS,
-  B_GEOM, B_CELL, B_COUNT, B_FILL, B_POSTMP, B_ORDER, B_ATMP, B_BTMP, B_SA, B_SB, B_SHX, B_SIDX, B_CSTART,
+  B_GEOM, B_CELL, B_COUNT, B_SLOT, B_POSTMP, B_ATMP, B_BTMP, B_SA, B_SB, B_SHX, B_SIDX, B_CSTART,
   B_CP, B_G, B_T, B_NKEPT, B_DMAXHZ, B_DOBSC, B_DLGC, B_DLGL, B_STATUS, B_LEVDEPTH,
   B_LIST_IDX, B_LIST_R, B_LIST_CNT, B_FLUSH, B_TILECOLS, B_TILEPAR, B_TILEN, B_TILEOFF, B_TILEREC, B_EIGSCR,
   B_RAW0, B_RAW1, B_RAW2, B_RAW3, B_RAW4, B_RAW5, B_RAW6, B_RAW7, B_RAWQC, B_RAWHX, B_RAWHXM, B_FLAG, B_POS,
@@ -734,8 +734,13 @@ int lgpu_get_obs_prepared(lgpu_handle *h, float *hx, float *hx_mean, float *lat,
 
 // First part of a run: checks, buffers, the observation index and the
 // per-column parameters (events ev[0..2]); shared by the exact and the
-// learned forms.
-static int prepare_run(lgpu_handle *h, ObsSorted &os, int &launches) {
+// learned forms.  `tiles`: the tile set whose caps are wanted, or null.
+struct TileSet {
+  int ntiles;
+  DevBuf *cols, *par, *n, *off;
+};
+
+static int prepare_run(lgpu_handle *h, ObsSorted &os, int &launches, const TileSet *tiles) {
   if (!h) return LGPU_ERR_ARG;
   if (!h->solver_ok) return fail(h, LGPU_ERR_ORDER, "solver_run before solver_init");
   if (!h->loc_ok) return fail(h, LGPU_ERR_ORDER, "solver_run before loc_init");
@@ -769,9 +774,8 @@ static int prepare_run(lgpu_handle *h, ObsSorted &os, int &launches) {
     CK(cudaMemcpyAsync(h->buf[B_SATPLATS].p, h->sat_plats.data(), 4 * h->sat_plats.size(), cudaMemcpyHostToDevice, h->st), "H2D");
   CK(h->buf[B_CELL].ensure(4 * nobs), "alloc");
   CK(h->buf[B_COUNT].ensure(4 * (size_t)h->ncell), "alloc");
-  CK(h->buf[B_FILL].ensure(4 * (size_t)h->ncell), "alloc");
+  CK(h->buf[B_SLOT].ensure(4 * nobs), "alloc");
   CK(h->buf[B_POSTMP].ensure(4 * nobs), "alloc");
-  CK(h->buf[B_ORDER].ensure(4 * nobs), "alloc");
   CK(h->buf[B_ATMP].ensure(16 * nobs), "alloc");
   CK(h->buf[B_BTMP].ensure(16 * nobs), "alloc");
   CK(h->buf[B_SA].ensure(16 * nobs), "alloc");
@@ -806,27 +810,58 @@ static int prepare_run(lgpu_handle *h, ObsSorted &os, int &launches) {
     CK(cudaMemcpyAsync(h->buf[B_SPRDB].p, h->bound_sprd, nm * 4, cudaMemcpyHostToDevice, h->cst), "H2D sprd");
     CK(cudaEventRecord(h->ev_in[0], h->cst), "event");
   }
-  // ---- observation index (kd_init counterpart) ----
-  CK(launch_obs_index(st, h->nobs, k, kp, h->buf[B_OLAT].as<float>(), h->buf[B_OLON].as<float>(),
-                      h->buf[B_OZ].as<float>(), h->buf[B_OTIME].as<float>(), h->buf[B_OVAL].as<float>(),
-                      h->buf[B_OERR].as<float>(), h->buf[B_OOBSID].as<int>(), h->buf[B_OPLATID].as<int>(),
-                      h->buf[B_HX].as<float>(), h->buf[B_HXM].as<float>(), h->buf[B_SATOBS].as<int>(),
-                      (int)h->sat_obs.size(), h->buf[B_SATPLATS].as<int>(), (int)h->sat_plats.size(),
-                      h->buf[B_GEOM].as<IndexGeom>(), h->ncell, h->buf[B_CELL].as<int>(), h->buf[B_COUNT].as<int>(),
-                      h->buf[B_FILL].as<int>(), h->buf[B_POSTMP].as<int>(), h->buf[B_ORDER].as<int>(),
-                      h->buf[B_ATMP].as<float4>(), h->buf[B_BTMP].as<float4>(), os, &launches),
+  // ---- observation index (kd_init counterpart) and per-column parameters ----
+  ObsPrepArgs oa;
+  oa.nobs = h->nobs;
+  oa.lat = h->buf[B_OLAT].as<float>();
+  oa.lon = h->buf[B_OLON].as<float>();
+  oa.zdim = h->buf[B_OZ].as<float>();
+  oa.time = h->buf[B_OTIME].as<float>();
+  oa.val = h->buf[B_OVAL].as<float>();
+  oa.err = h->buf[B_OERR].as<float>();
+  oa.obsid = h->buf[B_OOBSID].as<int>();
+  oa.platid = h->buf[B_OPLATID].as<int>();
+  oa.hx_mean = h->buf[B_HXM].as<float>();
+  oa.sat_obs = h->buf[B_SATOBS].as<int>();
+  oa.n_sat_obs = (int)h->sat_obs.size();
+  oa.sat_plats = h->buf[B_SATPLATS].as<int>();
+  oa.n_sat_plats = (int)h->sat_plats.size();
+  oa.geom = h->buf[B_GEOM].as<IndexGeom>();
+  oa.cell = h->buf[B_CELL].as<int>();
+  oa.slot = h->buf[B_SLOT].as<int>();
+  oa.count = h->buf[B_COUNT].as<int>();
+  oa.A = h->buf[B_ATMP].as<float4>();
+  oa.B = h->buf[B_BTMP].as<float4>();
+  ColPrepArgs ca;
+  ca.ncol = h->ncol;
+  ca.ns = ns;
+  ca.lat = h->buf[B_LAT].as<float>();
+  ca.lon = h->buf[B_LON].as<float>();
+  ca.mask = h->buf[B_MASK].as<int>();
+  ca.mean_b = h->buf[B_MEANB].as<float>();
+  ca.loc = h->loc;
+  ca.cp = h->buf[B_CP].as<ColPar>();
+  ca.diag_maxhz = h->buf[B_DMAXHZ].as<float>();
+  ca.diag_obscount = h->buf[B_DOBSC].as<float>();
+  ca.diag_lg_obscount = h->buf[B_DLGC].as<float>();
+  ca.diag_lg_obsloc = h->buf[B_DLGL].as<float>();
+  ca.status = h->buf[B_STATUS].as<int>();
+  // a bound state's background mean is still on its way: the ocean localizer's
+  // columns, which read it, are prepared once it is here
+  const bool late = bound && h->loc.cls == LOC_OCEAN && h->loc.vtloc_surf == 1;
+  const int nt = tiles ? tiles->ntiles : 0;
+  const int *tc = nt > 0 ? tiles->cols->as<int>() : nullptr;
+  TilePar *tp = nt > 0 ? tiles->par->as<TilePar>() : nullptr;
+  CK(launch_prep(st, &oa, h->ncell, late ? nullptr : &ca, &launches), "observation and column prep");
+  CK(launch_obs_index(st, oa, k, kp, h->buf[B_HX].as<float>(), h->ncell, h->buf[B_POSTMP].as<int>(), os,
+                      late ? 0 : nt, tc, ca.cp, tp, &launches),
      "observation index");
   CK(cudaEventRecord(h->ev[1], st), "event");
-  // ---- per-column parameters (the ocean localizer reads the background mean) ----
   if (bound) CK(cudaStreamWaitEvent(st, h->ev_in[0], 0), "stream wait");
-  CK(launch_col_prep(st, h->ncol, h->buf[B_LAT].as<float>(), h->buf[B_LON].as<float>(), h->buf[B_MASK].as<int>(),
-                     h->buf[B_MEANB].as<float>(), ns, h->loc, h->buf[B_CP].as<ColPar>(),
-                     h->buf[B_DMAXHZ].as<float>(), &launches),
-     "column prep");
-  CK(cudaMemsetAsync(h->buf[B_DOBSC].p, 0, 4 * (size_t)h->ncol, st), "memset");
-  CK(cudaMemsetAsync(h->buf[B_DLGC].p, 0, 4 * (size_t)h->ncol * G, st), "memset");
-  CK(cudaMemsetAsync(h->buf[B_DLGL].p, 0, 4 * (size_t)h->ncol * G, st), "memset");
-  CK(cudaMemsetAsync(h->buf[B_STATUS].p, 0, 16, st), "memset");
+  if (late) {
+    CK(launch_prep(st, nullptr, 0, &ca, &launches), "column prep");
+    CK(launch_tile_prep(st, nt, tc, ca.cp, tp, &launches), "tile prep");
+  }
   CK(cudaEventRecord(h->ev[2], st), "event");
   return LGPU_OK;
 }
@@ -918,11 +953,6 @@ static UpdateArgs update_args(lgpu_handle *h) {
 // The batched tensor-core Gram over a tile set (tiles of 128 columns; the
 // records and the weight cache are the handle's scratch): G, nkept and the
 // diagnostics of the tiles' units.  Events ev[6] after the tile streams.
-struct TileSet {
-  int ntiles;
-  DevBuf *cols, *par, *n, *off;
-};
-
 static int upload_members(lgpu_handle *h, cudaEvent_t after);
 
 // start_upload: a bound state's members start uploading once the tile fill is
@@ -931,8 +961,6 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
                              bool start_upload) {
   cudaStream_t st = h->st;
   const int k = h->k, kp = h->kp, G = h->loc.groups;
-  CK(launch_tile_prep(st, ts.ntiles, (*ts.cols).as<int>(), h->buf[B_CP].as<ColPar>(),
-                      (*ts.par).as<TilePar>(), &launches), "tile prep");
   // tile candidate streams: count, size the record buffer, fill
   CK(launch_tile_count(st, ts.ntiles, (*ts.par).as<TilePar>(), h->buf[B_GEOM].as<IndexGeom>(), os,
                        (*ts.n).as<int>(), (*ts.off).as<int>(), &launches),
@@ -1138,14 +1166,14 @@ int lgpu_solver_run(lgpu_handle *h) {
 static int solver_run(lgpu_handle *h) {
   ObsSorted os;
   int launches = 0;
-  int rc0 = prepare_run(h, os, launches);
+  const TileSet grid_tiles{h->ntiles, &h->buf[B_TILECOLS], &h->buf[B_TILEPAR], &h->buf[B_TILEN], &h->buf[B_TILEOFF]};
+  int rc0 = prepare_run(h, os, launches, &grid_tiles);
   if (rc0 != LGPU_OK) return rc0;
   const int k = h->k, kp = h->kp, ns = h->ns, G = h->loc.groups;
   cudaStream_t st = h->st;
   const bool bound = h->bound_state != nullptr;
   // ---- search + localize + Gram ----
   // ---- Gram: the batched tensor-core form or the plain per-column form ----
-  const TileSet grid_tiles{h->ntiles, &h->buf[B_TILECOLS], &h->buf[B_TILEPAR], &h->buf[B_TILEN], &h->buf[B_TILEOFF]};
   bool uploading = false;   // a bound state's members are on their way
   auto run_batched = [&](bool start_upload) -> int {
     uploading = start_upload && bound;
@@ -1441,7 +1469,7 @@ int lgpu_solver_final(lgpu_handle *h) {
   if (!h) return LGPU_ERR_ARG;
   cudaSetDevice(h->device);
   cudaStreamSynchronize(h->st);
-  int work[] = {B_CELL, B_COUNT, B_FILL, B_POSTMP, B_ORDER, B_ATMP, B_BTMP, B_G, B_T};
+  int work[] = {B_CELL, B_COUNT, B_SLOT, B_POSTMP, B_ATMP, B_BTMP, B_G, B_T};
   for (int b : work) h->buf[b].release();
   return LGPU_OK;
 }
@@ -2139,7 +2167,7 @@ static int learned_run(lgpu_handle *h) {
   if (h->bound_state) return fail(h, LGPU_ERR_UNSUPPORTED, "the LEARNED variant with a bound state");
   ObsSorted os;
   int launches = 0;
-  int rc = prepare_run(h, os, launches);
+  int rc = prepare_run(h, os, launches, nullptr);
   if (rc != LGPU_OK) return rc;
   if ((rc = flag_prepare(h)) != LGPU_OK) return rc;
   cudaStream_t st = h->st;

@@ -787,73 +787,6 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
   if (wid == 0) tc::tmem_dealloc(tmem, tmem_cols);
 }
 
-// Tile caps: centre = normalised mean of the tile's unit vectors, angular
-// radius = max over columns of (angle to centre + search radius / R), then
-// the same conservative band / longitude window as a single column.
-__global__ void k_tile_prep(int ntiles, const int *tile_cols, const ColPar *cp, TilePar *tp) {
-  const int tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (tile >= ntiles) return;
-  double sx = 0, sy = 0, sz = 0;
-  for (int c = lane; c < TM; c += 32) {
-    const int col = tile_cols[(size_t)tile * TM + c];
-    if (col < 0) continue;
-    sx += cp[col].ux; sy += cp[col].uy; sz += cp[col].uz;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    sx += __shfl_xor_sync(0xffffffffu, sx, o);
-    sy += __shfl_xor_sync(0xffffffffu, sy, o);
-    sz += __shfl_xor_sync(0xffffffffu, sz, o);
-  }
-  const double nrm = sqrt(sx * sx + sy * sy + sz * sz);
-  const double cx = nrm > 0 ? sx / nrm : 1.0, cy = nrm > 0 ? sy / nrm : 0.0, cz = nrm > 0 ? sz / nrm : 0.0;
-  double amax = 0.0;
-  for (int c = lane; c < TM; c += 32) {
-    const int col = tile_cols[(size_t)tile * TM + c];
-    if (col < 0) continue;
-    const double dot = fmin(1.0, fmax(-1.0, cx * cp[col].ux + cy * cp[col].uy + cz * cp[col].uz));
-    const double ang = acos(dot) + (double)cp[col].rmax / 6371000.0;
-    amax = fmax(amax, ang);
-  }
-  for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-  // largest half-chord sqrt(c2max)/2 of a candidate pair (the weight producers' c2max)
-  float hm = 0.0f;
-  for (int c = lane; c < TM; c += 32) {
-    const int col = tile_cols[(size_t)tile * TM + c];
-    if (col < 0) continue;
-    const float hq = fminf(cp[col].rmax / 12742000.0f, 1.5707963f);
-    const float sh = sinf(hq);
-    hm = fmaxf(hm, sqrtf(4.0f * sh * sh * 1.0001f + 1e-12f) * 0.5f);
-  }
-  for (int o = 16; o > 0; o >>= 1) hm = fmaxf(hm, __shfl_xor_sync(0xffffffffu, hm, o));
-  if (lane == 0) {
-    TilePar t;
-    const double lat = asin(fmax(-1.0, fmin(1.0, cz))) * 57.29577951308232;
-    double lon = atan2(cy, cx) * 57.29577951308232;
-    if (lon < 0) lon += 360.0;
-    if (lon >= 360.0) lon -= 360.0;
-    const double alpha = amax * 1.0001 + 1e-6;
-    const double adeg = alpha * 57.29577951308232 + 0.05;
-    const bool full = (lat + adeg >= 90.0) || (lat - adeg <= -90.0) || alpha >= 1.5;
-    double dl = 180.0;
-    if (!full) {
-      const double sr = sin(alpha) / cos(lat * 0.017453292519943295);
-      dl = sr >= 1.0 ? 180.0 : asin(sr) * 57.29577951308232 * 1.0001 + 0.05;
-    }
-    t.lonn = (float)lon;
-    t.dlon = (float)dl;
-    t.cx = (float)cx;
-    t.cy = (float)cy;
-    t.cz = (float)cz;
-    const double ch = 2.0 * sin(0.5 * fmin(alpha, 3.14159265358979));
-    t.c2cap = (float)(ch * ch * 1.00001 + 1e-9);
-    t.hmax = hm * 1.0001f;
-    t.b0 = band_of((float)(lat - adeg));
-    t.b1 = band_of((float)(lat + adeg));
-    tp[tile] = t;
-  }
-}
-
 // Stage / ring depths: two operand stages and six record slots (k <= 128:
 // 2 x 70 KB + 6 x 10.8 KB).  At k = 40 they made the Gram 1.8 ms faster than
 // three stages with three slots (the producers waited on the record copies);
@@ -880,14 +813,6 @@ void gram_tc_passes(int k, int *npass, int *np) {
   while (n > NPMAX) { p++; n = ((nf + p - 1) / p + 15) & ~15; }
   *npass = p;
   *np = n;
-}
-
-cudaError_t launch_tile_prep(cudaStream_t st, int ntiles, const int *tile_cols, const ColPar *cp, TilePar *tp,
-                             int *launches) {
-  if (ntiles <= 0) return cudaSuccess;
-  k_tile_prep<<<(ntiles + 3) / 4, 128, 0, st>>>(ntiles, tile_cols, cp, tp);
-  (*launches)++;
-  return cudaGetLastError();
 }
 
 cudaError_t launch_tile_count(cudaStream_t st, int ntiles, const TilePar *tp, const IndexGeom *geom,
@@ -1040,7 +965,6 @@ static cudaError_t preload_gram_tc_loc() {
   auto get = [&](const void *f) { if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, f); };
   get((const void *)k_gram_tc<LOC, 2, 6, false>);
   get((const void *)k_gram_tc<LOC, 2, 6, true>);
-  get((const void *)k_tile_prep);
   get((const void *)k_tile_count);
   get((const void *)k_tile_scan);
   get((const void *)k_tile_fill);

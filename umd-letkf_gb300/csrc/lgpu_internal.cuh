@@ -424,17 +424,37 @@ __device__ __forceinline__ void list_search(int gid, const ColPar &cp, const Dev
   }
 }
 
-cudaError_t launch_obs_index(cudaStream_t st, int nobs, int k, int kp, const float *lat, const float *lon,
-                             const float *zdim, const float *time, const float *val, const float *err,
-                             const int *obsid, const int *platid, const float *hx, const float *hx_mean,
-                             const int *sat_obs, int n_sat_obs, const int *sat_plats, int n_sat_plats,
-                             const IndexGeom *geom_d, int ncell, int *d_cell, int *d_count, int *d_fill,
-                             int *d_pos_tmp, int *d_order, float4 *Atmp, float4 *Btmp, ObsSorted out,
-                             int *launches);
-
-cudaError_t launch_col_prep(cudaStream_t st, int ncol, const float *lat, const float *lon, const int *mask,
-                            const float *mean_b, int ns, const DevLoc &loc, ColPar *cp, float *diag_maxhz,
-                            int *launches);
+struct ObsPrepArgs {
+  int nobs;
+  const float *lat, *lon, *zdim, *time, *val, *err;
+  const int *obsid, *platid;
+  const float *hx_mean;
+  const int *sat_obs;
+  int n_sat_obs;
+  const int *sat_plats;
+  int n_sat_plats;
+  const IndexGeom *geom;   // device copy
+  int *cell, *slot;        // [nobs] cell, place among the cell's observations in arrival order
+  int *count;              // [ncell] observations per cell
+  float4 *A, *B;           // records in the given order
+};
+struct ColPrepArgs {
+  int ncol, ns;
+  const float *lat, *lon;
+  const int *mask;
+  const float *mean_b;     // read by loc_ocean's mixed-layer split only
+  DevLoc loc;
+  ColPar *cp;
+  float *diag_maxhz, *diag_obscount, *diag_lg_obscount, *diag_lg_obsloc;
+  int *status;             // [4]
+};
+// observations' cells and records and / or columns' parameters (null: not in this launch)
+cudaError_t launch_prep(cudaStream_t st, const ObsPrepArgs *o, int ncell, const ColPrepArgs *c, int *launches);
+// the sorted table from the prepared observations and, beside its scan, the caps of ntiles tiles
+struct TilePar;
+cudaError_t launch_obs_index(cudaStream_t st, const ObsPrepArgs &a, int k, int kp, const float *hx, int ncell,
+                             int *pos_tmp, ObsSorted out, int ntiles, const int *tile_cols, const ColPar *cp,
+                             TilePar *tp, int *launches);
 
 struct GramArgs {
   int nunits, groups, k, kp;
