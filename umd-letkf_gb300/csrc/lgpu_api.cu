@@ -64,7 +64,7 @@ enum {
   B_OLAT, B_OLON, B_OZ, B_OTIME, B_OVAL, B_OERR, B_OOBSID, B_OPLATID, B_HX, B_HXM, B_SATOBS, B_SATPLATS,
   B_GEOM, B_CELL, B_COUNT, B_SLOT, B_POSTMP, B_ATMP, B_BTMP, B_SA, B_SB, B_SHX, B_SIDX, B_CSTART,
   B_CP, B_G, B_T, B_NKEPT, B_DMAXHZ, B_DOBSC, B_DLGC, B_DLGL, B_STATUS, B_LEVDEPTH,
-  B_LIST_IDX, B_LIST_R, B_LIST_CNT, B_FLUSH, B_TILECOLS, B_TILEPAR, B_TILEN, B_TILEOFF, B_TILEREC, B_EIGSCR,
+  B_LIST_IDX, B_LIST_R, B_LIST_CNT, B_FLUSH, B_TILECOLS, B_TILEPAR, B_TILEN, B_TILEOFF, B_TILELIST, B_TILEREC, B_EIGSCR,
   B_RAW0, B_RAW1, B_RAW2, B_RAW3, B_RAW4, B_RAW5, B_RAW6, B_RAW7, B_RAWQC, B_RAWHX, B_RAWHXM, B_FLAG, B_POS,
   B_PTRS, B_TOTAL, B_GPART, B_GCNT, B_FLAGLIST, B_TCWORK, B_TCSEG,
   B_COUNT_ALL
@@ -467,7 +467,7 @@ int lgpu_set_grid(lgpu_handle *h, int nij, const float *lat, const float *lon, c
   const std::vector<int> tiles = build_tiles(act, lat, lon);
   CK(h->buf[B_TILECOLS].ensure(sizeof(int) * std::max<size_t>(1, tiles.size())), "alloc tiles");
   CK(h->buf[B_TILEPAR].ensure(sizeof(TilePar) * std::max<size_t>(1, tiles.size() / 128)), "alloc tiles");
-  CK(h->buf[B_TILEN].ensure(sizeof(int) * std::max<size_t>(1, tiles.size() / 128)), "alloc tiles");
+  CK(h->buf[B_TILEN].ensure(sizeof(int) * std::max<size_t>(1, tile_count_ints((int)(tiles.size() / 128)))), "alloc tiles");
   CK(h->buf[B_TILEOFF].ensure(sizeof(int) * (tiles.size() / 128 + 1)), "alloc tiles");
   if (!tiles.empty())
     CK(cudaMemcpyAsync(h->buf[B_TILECOLS].p, tiles.data(), sizeof(int) * tiles.size(), cudaMemcpyHostToDevice, h->st),
@@ -963,7 +963,7 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   const int k = h->k, kp = h->kp, G = h->loc.groups;
   // tile candidate streams: count, size the record buffer, fill
   CK(launch_tile_count(st, ts.ntiles, (*ts.par).as<TilePar>(), h->buf[B_GEOM].as<IndexGeom>(), os,
-                       (*ts.n).as<int>(), (*ts.off).as<int>(), &launches),
+                       (*ts.n).as<int>(), (*ts.n).as<int>() + ts.ntiles, (*ts.off).as<int>(), &launches),
      "tile count");
   // the stream offsets size the record buffer and split each tile's stream
   // into accumulation segments
@@ -981,8 +981,10 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   h->h_tile_off.assign(h->pin_off, h->pin_off + ts.ntiles + 1);
   const int nchunk_total = h->h_tile_off[ts.ntiles];
   CK(h->buf[B_TILEREC].ensure(std::max<size_t>(16, (size_t)nchunk_total * record_bytes(k))), "alloc tile streams");
-  CK(launch_tile_fill(st, ts.ntiles, (*ts.par).as<TilePar>(), h->buf[B_GEOM].as<IndexGeom>(), os, k, kp,
-                      (*ts.off).as<int>(), h->buf[B_TILEREC].as<unsigned char>(),
+  CK(h->buf[B_TILELIST].ensure(std::max<size_t>(16, (size_t)nchunk_total * 16 * sizeof(int))), "alloc tile streams");
+  CK(launch_tile_fill(st, ts.ntiles, nchunk_total, (*ts.par).as<TilePar>(), h->buf[B_GEOM].as<IndexGeom>(), os, k, kp,
+                      (*ts.n).as<int>(), (*ts.n).as<int>() + ts.ntiles, (*ts.off).as<int>(),
+                      h->buf[B_TILELIST].as<int>(), h->buf[B_TILEREC].as<unsigned char>(),
                       h->buf[B_STATUS].as<int>(), &launches),
      "tile fill");
   CK(cudaEventRecord(h->ev[6], st), "event");

@@ -14,7 +14,7 @@
 // most 432 so the accumulator fits TMEM), K = candidate observations in
 // chunks of 16.
 //
-// Candidate streams.  Before the GEMM, three small kernels turn each tile's
+// Candidate streams.  Before the GEMM, four small kernels turn each tile's
 // search window (latitude bands x longitude range of its cap) into a record
 // stream: every observation inside the tile's cap, in window order, packed
 // per chunk of 16 as ux[16] uy[16] uz[16] 1/err[16] dep[16] time[16] zdim[16]
@@ -165,19 +165,32 @@ __device__ __forceinline__ int window_pos(const Window &W, int j) {
   return W.seg_start[lo] + (j - W.seg_pref[lo]);
 }
 
-// candidates per tile: observations of the window inside the tile's cap
+// the window's candidates of warp w of WT / 32, whole groups of 32
+__device__ __forceinline__ void warp_range(const Window &W, int w, int &j0, int &j1) {
+  const int per = ((W.total + WT - 1) / WT) * 32;
+  j0 = min(W.total, w * per);
+  j1 = min(W.total, j0 + per);
+}
+
+// candidates per tile: observations of the window inside the tile's cap, per
+// warp range (tile_wn) and in all
 __global__ void __launch_bounds__(WT) k_tile_count(int ntiles, const TilePar *tps, const IndexGeom *geom,
-                                                   const float4 *obsA, const int *cell_start, int *tile_n) {
+                                                   const float4 *obsA, const int *cell_start, int *tile_n,
+                                                   int *tile_wn) {
   __shared__ Window W;
   __shared__ int red[WT / 32];
-  const int tile = blockIdx.x;
+  const int tile = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const TilePar tp = tps[tile];
   build_window(W, tp, geom, cell_start);
-  int cnt = 0;
+  int cnt = 0, j0, j1;
+  warp_range(W, wid, j0, j1);
 #pragma unroll 4
-  for (int j = threadIdx.x; j < W.total; j += WT) cnt += in_cap(tp, __ldg(obsA + window_pos(W, j)));
-  for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = cnt;
+  for (int j = j0 + lane; j < j1; j += 32) cnt += in_cap(tp, __ldg(obsA + window_pos(W, j)));
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  if (lane == 0) {
+    red[wid] = cnt;
+    tile_wn[(size_t)tile * (WT / 32) + wid] = cnt;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     int t = 0;
@@ -222,112 +235,91 @@ __global__ void k_tile_scan(int ntiles, const int *tile_n, int *tile_off) {
   if (threadIdx.x == 0) tile_off[ntiles] = carry;
 }
 
-// one record entry: slot e of chunk c of the tile stream
-__device__ __forceinline__ void put_record(unsigned char *rec0, int cb, int k, int kp, int kr, int q, const float4 &A,
-                                           const float4 &B, const float *hx) {
-  unsigned char *r = rec0 + (size_t)(q >> 4) * cb;
-  const int e = q & 15;
-  float *r0 = reinterpret_cast<float *>(r);
-  r0[e] = A.x; r0[16 + e] = A.y; r0[32 + e] = A.z; r0[48 + e] = A.w;
-  r0[64 + e] = B.x; r0[80 + e] = B.y; r0[96 + e] = B.z; r0[112 + e] = B.w;
-  float *yT = reinterpret_cast<float *>(r + 512);
-  if (hx) {
-    // the member row through the read-only path, four 16-byte loads in
-    // flight before their stores
-    const float4 *h4 = reinterpret_cast<const float4 *>(hx);
-    const int n4 = kp >> 2;
-    for (int q0 = 0; q0 < n4; q0 += 4) {
-      float4 v[4];
+// The tile streams, in two steps: the positions of the cap's members in window
+// order (order preserving; a warp writes its range of the window behind the
+// ranges before it), then the records.  In one kernel with a block per tile,
+// whose threads each copied an observation's whole row between the block's
+// barriers, the step had a few hundred blocks of long serial work (clustered
+// 240 x 120, k = 64: counts and streams 281 us, now 108).
+__global__ void __launch_bounds__(WT) k_tile_list(const TilePar *tps, const IndexGeom *geom, const float4 *obsA,
+                                                  const int *cell_start, const int *tile_n, const int *tile_wn,
+                                                  const int *tile_off, int *list, int *status) {
+  __shared__ Window W;
+  const int tile = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const TilePar tp = tps[tile];
+  build_window(W, tp, geom, cell_start);
+  const int c0 = tile_off[tile], cap = (tile_off[tile + 1] - c0) * KC, n = tile_n[tile];
+  int *out = list + (size_t)c0 * KC;
+  int q = 0;
+  for (int w = 0; w < wid; w++) q += tile_wn[(size_t)tile * (WT / 32) + w];
+  const int qend = q + tile_wn[(size_t)tile * (WT / 32) + wid];
+  int j0, j1;
+  warp_range(W, wid, j0, j1);
+  for (int jb = j0; jb < j1; jb += 128) {
+    int p[4];
+    bool ok[4];
 #pragma unroll
-      for (int u = 0; u < 4; u++) v[u] = q0 + u < n4 ? __ldg(h4 + q0 + u) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const int i = 4 * (q0 + u);
-        if (i + 0 < k) yT[(i + 0) * YS + e] = v[u].x;
-        if (i + 1 < k) yT[(i + 1) * YS + e] = v[u].y;
-        if (i + 2 < k) yT[(i + 2) * YS + e] = v[u].z;
-        if (i + 3 < k) yT[(i + 3) * YS + e] = v[u].w;
-      }
+    for (int u = 0; u < 4; u++) {
+      const int j = jb + 32 * u + lane;
+      p[u] = j < j1 ? window_pos(W, j) : -1;
     }
-    yT[k * YS + e] = B.x;
-  } else {
-    for (int i = 0; i <= k; i++) yT[i * YS + e] = 0.0f;
+#pragma unroll
+    for (int u = 0; u < 4; u++) ok[u] = p[u] >= 0 && in_cap(tp, __ldg(obsA + p[u]));
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const unsigned m = __ballot_sync(0xffffffffu, ok[u]);
+      const int at = q + __popc(m & ((1u << lane) - 1u));
+      if (ok[u] && at < cap) out[at] = p[u];
+      q += __popc(m);
+    }
   }
-  for (int i = k + 1; i < kr; i++) yT[i * YS + e] = 0.0f;
-  if (e < YS - 16)
-    for (int i = 0; i < kr; i++) yT[i * YS + 16 + e] = 0.0f;
+  for (int t = n + (int)threadIdx.x; t < cap; t += WT) out[t] = -1;
+  if (lane == 0 && (q != qend || n > cap || cap - n >= KC)) atomicOr(status, 16);   // the two scans disagree
 }
 
-// tile streams: the window scanned again in order, cap members compacted
-// (order preserving) into the tile's chunk records; the last chunk padded
-// with zero entries
-__global__ void __launch_bounds__(WT) k_tile_fill(int ntiles, const TilePar *tps, const IndexGeom *geom, ObsSorted obs,
-                                                  int k, int kp, int kr, int cb, const int *tile_off,
-                                                  unsigned char *rec, int *status) {
-  __shared__ Window W;
-  __shared__ int wsc[WT / 32];
-  __shared__ int qpos[2 * WT];   // in-cap window positions not yet written, in window order
-  const int tile = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const TilePar tp = tps[tile];
-  build_window(W, tp, geom, obs.cell_start);
-  const int c0 = tile_off[tile];
-  const int cap = (tile_off[tile + 1] - c0) * KC;
-  unsigned char *rec0 = rec + (size_t)c0 * cb;
-  // the in-cap observations are queued in window order and written WT at a
-  // time by the whole block (about a third of a window is in the cap)
-  auto write = [&](int q, int p) {
-    if (q < cap) {
-      const float4 A = obs.A[p];
-      put_record(rec0, cb, k, kp, kr, q, make_float4(A.x, A.y, A.z, __frcp_rn(A.w)), obs.B[p],
-                 obs.hx + (size_t)p * kp);
-    } else {
-      atomicOr(status, 16);
+// the records, a warp per chunk: lane e (and e + 16) owns entry e, the two
+// halves take the member row's 16-byte groups in turn.  A missing entry (the
+// last chunk's padding) is a point out of every column's reach with weight 0.
+constexpr int RW = 8;   // chunks per block
+__global__ void __launch_bounds__(32 * RW) k_tile_rec(int nchunks, ObsSorted obs, int k, int kp, int kr, int cb,
+                                                      const int *list, unsigned char *rec) {
+  const int c = blockIdx.x * RW + (threadIdx.x >> 5), lane = threadIdx.x & 31, e = lane & 15, h = lane >> 4;
+  if (c >= nchunks) return;
+  const int p = list[(size_t)c * KC + e];
+  const bool in = p >= 0;
+  float *r0 = reinterpret_cast<float *>(rec + (size_t)c * cb), *yT = r0 + 128;
+  const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 B = in ? __ldg(obs.B + p) : z;
+  if (h == 0) {
+    float4 A = make_float4(4.f, 0.f, 0.f, 0.f);
+    if (in) {
+      A = __ldg(obs.A + p);
+      A.w = __frcp_rn(A.w);
     }
-  };
-  int base = 0, pend = 0;
-  // the thread's next window candidate (position and record) is loaded one
-  // iteration ahead, so that its latency overlaps the current compaction
-  int p_nx = 0;
-  float4 a_nx = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (tid < W.total) {
-    p_nx = window_pos(W, tid);
-    a_nx = __ldg(obs.A + p_nx);
+    r0[e] = A.x; r0[16 + e] = A.y; r0[32 + e] = A.z; r0[48 + e] = A.w;
+  } else {
+    r0[64 + e] = B.x; r0[80 + e] = B.y; r0[96 + e] = B.z; r0[112 + e] = B.w;
   }
-  for (int jb = 0; jb < W.total; jb += WT) {
-    const int j = jb + tid;
-    const int p = p_nx;
-    const bool ok = j < W.total && in_cap(tp, a_nx);
-    if (j + WT < W.total) {
-      p_nx = window_pos(W, j + WT);
-      a_nx = __ldg(obs.A + p_nx);
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, ok);
-    if (lane == 0) wsc[wid] = __popc(m);
-    __syncthreads();
-    int before = 0, cnt = 0;
-    for (int w = 0; w < WT / 32; w++) {
-      before += w < wid ? wsc[w] : 0;
-      cnt += wsc[w];
-    }
-    if (ok) qpos[pend + before + __popc(m & ((1u << lane) - 1u))] = p;
-    pend += cnt;
-    __syncthreads();
-    if (pend >= WT) {
-      write(base + tid, qpos[tid]);
-      base += WT;
-      pend -= WT;
-      __syncthreads();
-      if (tid < pend) qpos[tid] = qpos[WT + tid];
-      __syncthreads();
+  const float4 *h4 = reinterpret_cast<const float4 *>(obs.hx + (size_t)(in ? p : 0) * kp);
+  const int n4 = in ? kp >> 2 : 0;
+  for (int q0 = h; q0 < kr >> 2; q0 += 8) {
+    float4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = q0 + 2 * u < n4 ? __ldg(h4 + q0 + 2 * u) : z;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int i = 4 * (q0 + 2 * u);
+      if (i < kr) {
+        yT[(i + 0) * YS + e] = i + 0 < k ? v[u].x : (i + 0 == k ? B.x : 0.0f);
+        yT[(i + 1) * YS + e] = i + 1 < k ? v[u].y : (i + 1 == k ? B.x : 0.0f);
+        yT[(i + 2) * YS + e] = i + 2 < k ? v[u].z : (i + 2 == k ? B.x : 0.0f);
+        yT[(i + 3) * YS + e] = i + 3 < k ? v[u].w : (i + 3 == k ? B.x : 0.0f);
+      }
     }
   }
-  if (tid < pend) write(base + tid, qpos[tid]);
-  base += pend;
-  // padding: a point out of every column's reach, weight 0
-  const float4 z = make_float4(0.f, 0.f, 0.f, 0.f), far = make_float4(4.f, 0.f, 0.f, 0.f);
-  for (int q = base + tid; q < cap; q += WT) put_record(rec0, cb, k, kp, kr, q, far, z, nullptr);
-  if (tid == 0 && (base > cap || cap - base >= KC)) atomicOr(status, 16);   // count and fill disagree
+  for (int t = lane; t < kr * (YS - 16); t += 32) yT[(t >> 2) * YS + 16 + (t & 3)] = 0.0f;
 }
+static_assert(YS - 16 == 4, "pad columns of a member row");
 
 // fp32 pair -> TF32 hi + lo (tc::split_tf32 on both halves)
 __device__ __forceinline__ void split2(F2 v, F2 &hi, F2 &lo) {
@@ -803,6 +795,8 @@ void gram_tc_config(int k, int np, int *ns, int *nr, size_t *smem) {
 
 }  // namespace
 
+size_t tile_count_ints(int ntiles) { return (size_t)ntiles * (1 + WT / 32); }
+
 size_t record_bytes(int k) { return 512 + (size_t)(((k + 4) & ~3) * YS) * sizeof(float); }
 
 void gram_tc_passes(int k, int *npass, int *np) {
@@ -816,21 +810,22 @@ void gram_tc_passes(int k, int *npass, int *np) {
 }
 
 cudaError_t launch_tile_count(cudaStream_t st, int ntiles, const TilePar *tp, const IndexGeom *geom,
-                              const ObsSorted &obs, int *tile_n, int *tile_off, int *launches) {
+                              const ObsSorted &obs, int *tile_n, int *tile_wn, int *tile_off, int *launches) {
   if (ntiles <= 0) return cudaMemsetAsync(tile_off, 0, sizeof(int), st);
-  k_tile_count<<<ntiles, WT, 0, st>>>(ntiles, tp, geom, obs.A, obs.cell_start, tile_n);
+  k_tile_count<<<ntiles, WT, 0, st>>>(ntiles, tp, geom, obs.A, obs.cell_start, tile_n, tile_wn);
   k_tile_scan<<<1, 1024, 0, st>>>(ntiles, tile_n, tile_off);
   (*launches) += 2;
   return cudaGetLastError();
 }
 
-cudaError_t launch_tile_fill(cudaStream_t st, int ntiles, const TilePar *tp, const IndexGeom *geom,
-                             const ObsSorted &obs, int k, int kp, const int *tile_off, unsigned char *rec,
-                             int *status, int *launches) {
-  if (ntiles <= 0) return cudaSuccess;
+cudaError_t launch_tile_fill(cudaStream_t st, int ntiles, int nchunks, const TilePar *tp, const IndexGeom *geom,
+                             const ObsSorted &obs, int k, int kp, const int *tile_n, const int *tile_wn,
+                             const int *tile_off, int *list, unsigned char *rec, int *status, int *launches) {
+  if (ntiles <= 0 || nchunks <= 0) return cudaSuccess;
   const int kr = (k + 4) & ~3;
-  k_tile_fill<<<ntiles, WT, 0, st>>>(ntiles, tp, geom, obs, k, kp, kr, (int)record_bytes(k), tile_off, rec, status);
-  (*launches)++;
+  k_tile_list<<<ntiles, WT, 0, st>>>(tp, geom, obs.A, obs.cell_start, tile_n, tile_wn, tile_off, list, status);
+  k_tile_rec<<<(nchunks + RW - 1) / RW, 32 * RW, 0, st>>>(nchunks, obs, k, kp, kr, (int)record_bytes(k), list, rec);
+  (*launches) += 2;
   return cudaGetLastError();
 }
 
@@ -967,7 +962,8 @@ static cudaError_t preload_gram_tc_loc() {
   get((const void *)k_gram_tc<LOC, 2, 6, true>);
   get((const void *)k_tile_count);
   get((const void *)k_tile_scan);
-  get((const void *)k_tile_fill);
+  get((const void *)k_tile_list);
+  get((const void *)k_tile_rec);
   get((const void *)k_gram_segsum);
   return e;
 }

@@ -532,14 +532,17 @@ struct TcArgs {
 cudaError_t launch_gram_segsum(cudaStream_t st, const TcArgs &a, const int *active, int *launches);
 cudaError_t launch_tile_prep(cudaStream_t st, int ntiles, const int *tile_cols, const ColPar *cp, TilePar *tp,
                              int *launches);
-// tile candidate streams: counts + chunk offsets (tile_off[ntiles] = total
-// chunks), then the records (record_bytes(k) per chunk of 16)
+// tile candidate streams: counts (in all, and per warp's part of the window) +
+// chunk offsets (tile_off[ntiles] = total chunks), then the list of the
+// streams' observations (16 per chunk) and the records (record_bytes(k) per
+// chunk of 16)
 size_t record_bytes(int k);
+size_t tile_count_ints(int ntiles);   // tile_n and, behind its ntiles ints, tile_wn
 cudaError_t launch_tile_count(cudaStream_t st, int ntiles, const TilePar *tp, const IndexGeom *geom,
-                              const ObsSorted &obs, int *tile_n, int *tile_off, int *launches);
-cudaError_t launch_tile_fill(cudaStream_t st, int ntiles, const TilePar *tp, const IndexGeom *geom,
-                             const ObsSorted &obs, int k, int kp, const int *tile_off, unsigned char *rec,
-                             int *status, int *launches);
+                              const ObsSorted &obs, int *tile_n, int *tile_wn, int *tile_off, int *launches);
+cudaError_t launch_tile_fill(cudaStream_t st, int ntiles, int nchunks, const TilePar *tp, const IndexGeom *geom,
+                             const ObsSorted &obs, int k, int kp, const int *tile_n, const int *tile_wn,
+                             const int *tile_off, int *list, unsigned char *rec, int *status, int *launches);
 cudaError_t launch_gram_tc(cudaStream_t st, const TcArgs &a, int *launches);
 // CUDA loads a kernel at its first use: these load the plain and the batched
 // (for one localizer class) Gram kernels ahead of a timed trial
