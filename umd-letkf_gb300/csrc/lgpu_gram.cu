@@ -293,9 +293,10 @@ __global__ void __launch_bounds__(GT) k_gram(GramArgs a) {
       }
     }
 
-    // ---- 3. reduce the K-split partial tiles and write G | b
+    // ---- 3. reduce the K-split partial tiles and write G | b (a unit without
+    // observations has no transform, and its G is never read)
     float *red = As;   // ntiles*16 floats (fits in the A/B staging area)
-    for (int s = 0; s < nslice; s++) {
+    for (int s = 0; s < (nkept > 0 ? nslice : 0); s++) {
       if (gram_thread && slice == s) {
 #pragma unroll
         for (int r2 = 0; r2 < 4; r2++)
@@ -317,7 +318,7 @@ __global__ void __launch_bounds__(GT) k_gram(GramArgs a) {
     }
     __syncthreads();
     float *G = a.G + (size_t)unit * packed_size(k);
-    for (int t = tid; t < packed_size(k); t += GT) {
+    for (int t = tid; t < (nkept > 0 ? packed_size(k) : 0); t += GT) {
       int i, jj;
       packed_ij(t, k, i, jj);
       const int tl = (i >> 2) * ntn + (jj >> 2);

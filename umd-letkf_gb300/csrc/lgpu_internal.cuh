@@ -282,7 +282,11 @@ __host__ __device__ __forceinline__ int packed_size(int k) { return k * (k + 3) 
 __host__ __device__ __forceinline__ void packed_ij(int f, int k, int &i, int &j) {
   const int nt = k * (k + 1) / 2;
   if (f >= nt) { i = f - nt; j = k; return; }
-  int r = 0;
+  // the row from the root of tri_off(r) = f, then exactly
+  const float b = (float)(2 * k + 1);
+  int r = (int)(0.5f * (b - sqrtf(b * b - 8.0f * (float)f)));
+  r = r < 0 ? 0 : r;
+  while (tri_off(r, k) > f) r--;
   while (tri_off(r + 1, k) <= f) r++;
   i = r;
   j = f - tri_off(r, k) + r;
@@ -463,7 +467,7 @@ struct GramArgs {
   DevLoc loc;
   ObsSorted obs;
   const IndexGeom *geom;  // device copy
-  float *G;               // [unit][packed_size(k)]  (upper triangle of G, then b)
+  float *G;               // [unit][packed_size(k)]  (upper triangle of G, then b); not written where nkept is 0
   int *nkept;             // [unit]
   float *diag_obscount;   // [ncol]
   float *diag_lg_obscount;// [group][ncol]
