@@ -955,10 +955,19 @@ static UpdateArgs update_args(lgpu_handle *h) {
 // diagnostics of the tiles' units.  Events ev[6] after the tile streams.
 static int upload_members(lgpu_handle *h, cudaEvent_t after);
 
+// Where a tile set's Gram goes: the row of each column (-1: none), the arrays
+// and the measured choice of producers.
+struct GramDest {
+  const int *col2row;
+  float *G;
+  int *nkept;
+  int *cull;
+};
+
 // start_upload: a bound state's members start uploading once the tile fill is
 // launched (after the tile-stream offsets are read back), beside the Gram
-static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet &ts, int &launches,
-                             bool start_upload) {
+static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet &ts, const GramDest &dst,
+                             int &launches, bool start_upload) {
   cudaStream_t st = h->st;
   const int k = h->k, kp = h->kp, G = h->loc.groups;
   // tile candidate streams: count, size the record buffer, fill
@@ -1002,15 +1011,15 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   ta.nf = packed_size(k);
   ta.ncol = h->ncol;
   ta.tile_cols = (*ts.cols).as<int>();
-  ta.col2act = h->buf[B_COL2ACT].as<int>();
+  ta.col2act = dst.col2row;
   ta.cp = h->buf[B_CP].as<ColPar>();
   ta.loc = h->loc;
   ta.tp = (*ts.par).as<TilePar>();
   ta.rec = h->buf[B_TILEREC].as<unsigned char>();
   ta.tile_off = (*ts.off).as<int>();
   ta.tile_n = (*ts.n).as<int>();
-  ta.G = h->buf[B_G].as<float>();
-  ta.nkept = h->buf[B_NKEPT].as<int>();
+  ta.G = dst.G;
+  ta.nkept = dst.nkept;
   ta.diag_obscount = h->buf[B_DOBSC].as<float>();
   ta.diag_lg_obscount = h->buf[B_DLGC].as<float>();
   ta.diag_lg_obsloc = h->buf[B_DLGL].as<float>();
@@ -1100,7 +1109,7 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   ta.segtiles = h->buf[B_TCSEG].as<TcSegTile>();
   ta.nsegtiles = (int)h->h_tc_seg.size();
   h->gram_nseg = pl.second;
-  if (h->tc_cull < 0) {
+  if (*dst.cull < 0) {
     // the first batched Gram of a configuration runs both producer forms,
     // timed, and keeps the faster; their outputs are bit-identical, and every
     // output of the Gram kernels is overwritten by the second run (the
@@ -1116,10 +1125,10 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
     CK(cudaEventSynchronize(h->ev_cull[2]), "tune sync");
     CK(cudaEventElapsedTime(&tm[0], h->ev_cull[0], h->ev_cull[1]), "timing");
     CK(cudaEventElapsedTime(&tm[1], h->ev_cull[1], h->ev_cull[2]), "timing");
-    h->tc_cull = tm[1] < tm[0] ? 1 : 0;
+    *dst.cull = tm[1] < tm[0] ? 1 : 0;
     h->tc_tune_ms = std::max(tm[0], tm[1]);
   } else {
-    ta.cull = h->tc_cull;
+    ta.cull = *dst.cull;
     CK(launch_gram_tc(st, ta, &launches), "tensor-core gram kernel");
   }
   CK(launch_gram_segsum(st, ta, h->buf[B_ACTIVE].as<int>(), &launches), "gram segment sum");
@@ -1179,7 +1188,8 @@ static int solver_run(lgpu_handle *h) {
   bool uploading = false;   // a bound state's members are on their way
   auto run_batched = [&](bool start_upload) -> int {
     uploading = start_upload && bound;
-    return run_batched_tiles(h, os, grid_tiles, launches, start_upload && bound);
+    const GramDest dst{h->buf[B_COL2ACT].as<int>(), h->buf[B_G].as<float>(), h->buf[B_NKEPT].as<int>(), &h->tc_cull};
+    return run_batched_tiles(h, os, grid_tiles, dst, launches, start_upload && bound);
   };
   auto run_plain = [&]() -> int {
     GramArgs ga;
@@ -1735,6 +1745,10 @@ struct LearnState {
   DevBuf bidx, Xb, Yb, scr, lacc;
   DevBuf wout;                                   // per-output loss weights: 1 for W, k for w-bar
   DevBuf cells;                                  // per-cell observation aggregates (two float4 per cell)
+  // the lattice's columns in tiles for the batched Gram; the faster Gram form
+  // for them (0 = not yet measured) and its producers
+  DevBuf tcols, tpar, tn, toff;
+  int ntiles = 0, gram_choice = 0, cull = -1;
   long long nstore = 0;
   long long hold0 = 0;     // first row of the last collected analysis (held out from training when ncollect >= 2)
   int ncollect = 0;
@@ -1754,7 +1768,7 @@ static void learn_free(lgpu_handle *h) {
                    &L->mu_in, &L->sd_in, &L->mu_out, &L->sd_out, &L->feat, &L->nkf, &L->X, &L->Xt, &L->H1, &L->H2,
                    &L->Yn, &L->flag, &L->gate, &L->gate_n, &L->jacc, &L->ecols, &L->Gsub, &L->nksub, &L->Tsub,
                    &L->wsub, &L->store_X, &L->store_Y, &L->wbar_all, &L->bidx, &L->Xb, &L->Yb, &L->scr, &L->lacc,
-                   &L->wout, &L->cells};
+                   &L->wout, &L->cells, &L->tcols, &L->tpar, &L->tn, &L->toff};
   for (DevBuf *b : all) b->release();
   for (auto &e : L->ev) if (e) cudaEventDestroy(e);
   delete L;
@@ -1854,6 +1868,19 @@ int lgpu_learn_init(lgpu_handle *h, const lgpu_learn_config *cfg) {
     std::vector<float> w(S.dout, 1.0f);
     for (int i = 0; i < k; i++) w[(size_t)k * k + i] = (float)k;
     CK(cudaMemcpy(L->wout.p, w.data(), 4 * w.size(), cudaMemcpyHostToDevice), "H2D loss weights");
+  }
+  {
+    std::vector<float> lat(h->ncol), lon(h->ncol);
+    CK(cudaMemcpy(lat.data(), h->buf[B_LAT].p, 4 * (size_t)h->ncol, cudaMemcpyDeviceToHost), "D2H lat");
+    CK(cudaMemcpy(lon.data(), h->buf[B_LON].p, 4 * (size_t)h->ncol, cudaMemcpyDeviceToHost), "D2H lon");
+    const std::vector<int> tiles = build_tiles(L->coarse, lat.data(), lon.data());
+    L->ntiles = (int)(tiles.size() / 128);
+    const size_t nt = std::max(1, L->ntiles);
+    CK(L->tcols.ensure(512 * nt), "alloc tiles");
+    CK(L->tpar.ensure(sizeof(TilePar) * nt), "alloc tiles");
+    CK(L->tn.ensure(4 * tile_count_ints((int)nt)), "alloc tiles");
+    CK(L->toff.ensure(4 * (nt + 1)), "alloc tiles");
+    if (!tiles.empty()) CK(cudaMemcpy(L->tcols.p, tiles.data(), 4 * tiles.size(), cudaMemcpyHostToDevice), "H2D tiles");
   }
   for (auto &e : L->ev) CK(cudaEventCreate(&e), "event");
   CK(cudaMemcpyAsync(L->d_fine.p, L->fine_ok.data(), 4 * L->fine_ok.size(), cudaMemcpyHostToDevice, h->st), "H2D");
@@ -2114,30 +2141,69 @@ int lgpu_learn_train(lgpu_handle *h, int epochs, int batch, float lr, float *los
   return LGPU_OK;
 }
 
-// exact solves (PLAIN Gram + split eigensolve) of a column list into the
-// compact arrays of the learned state (rows 0..n)
-static int learned_exact(lgpu_handle *h, const ObsSorted &os, int n, int &launches) {
+// exact solves of a column list into the compact arrays of the learned state
+// (rows 0..n); `lattice`: the first rows are the lattice's columns.  These take
+// the batched Gram where it is faster, the others the plain one.  The first
+// analysis runs both, timed, as AUTO does: the batched form shares the
+// observations of 128 lattice columns, which lie `stride` grid steps apart, so
+// its gain falls with the stride (12,888 columns at stride 2, k = 32, search
+// radius 1,460 km: plain 1,190 us, batched with its streams 540).
+static int learned_exact(lgpu_handle *h, const ObsSorted &os, int n, bool lattice, int &launches) {
   LearnState *L = h->learn;
   if (n <= 0) return LGPU_OK;
   cudaStream_t st = h->st;
   const int k = h->k;
-  GramArgs ga;
-  ga.nunits = n;
-  ga.groups = 1;
-  ga.k = k;
-  ga.kp = h->kp;
-  ga.active = L->ecols.as<int>();
-  ga.cp = h->buf[B_CP].as<ColPar>();
-  ga.loc = h->loc;
-  ga.obs = os;
-  ga.geom = h->buf[B_GEOM].as<IndexGeom>();
-  ga.G = L->Gsub.as<float>();
-  ga.nkept = L->nksub.as<int>();
-  ga.diag_obscount = h->buf[B_DOBSC].as<float>();
-  ga.diag_lg_obscount = h->buf[B_DLGC].as<float>();
-  ga.diag_lg_obsloc = h->buf[B_DLGL].as<float>();
-  ga.ncol = h->ncol;
-  CK(launch_gram(st, ga, &launches), "gram kernel");
+  auto plain = [&](int r0, int r1) -> int {
+    if (r1 <= r0) return LGPU_OK;
+    GramArgs ga;
+    ga.nunits = r1 - r0;
+    ga.groups = 1;
+    ga.k = k;
+    ga.kp = h->kp;
+    ga.active = L->ecols.as<int>() + r0;
+    ga.cp = h->buf[B_CP].as<ColPar>();
+    ga.loc = h->loc;
+    ga.obs = os;
+    ga.geom = h->buf[B_GEOM].as<IndexGeom>();
+    ga.G = L->Gsub.as<float>() + (size_t)r0 * packed_size(k);
+    ga.nkept = L->nksub.as<int>() + r0;
+    ga.diag_obscount = h->buf[B_DOBSC].as<float>();
+    ga.diag_lg_obscount = h->buf[B_DLGC].as<float>();
+    ga.diag_lg_obsloc = h->buf[B_DLGL].as<float>();
+    ga.ncol = h->ncol;
+    CK(launch_gram(st, ga, &launches), "gram kernel");
+    return LGPU_OK;
+  };
+  const TileSet ts{L->ntiles, &L->tcols, &L->tpar, &L->tn, &L->toff};
+  const GramDest dst{L->d_rank.as<int>(), L->Gsub.as<float>(), L->nksub.as<int>(), &L->cull};
+  const int nlat = lattice ? (int)L->coarse.size() : 0;
+  int rc = LGPU_OK;
+  if (k < 8) L->gram_choice = LGPU_VARIANT_PLAIN;   // as AUTO
+  if (nlat > 0 && L->gram_choice == 0) {
+    if (!h->preloaded) {
+      CK(preload_gram(), "kernel load");
+      CK(preload_gram_tc(h->loc.cls), "kernel load");
+      h->preloaded = true;
+    }
+    CK(cudaEventRecord(h->ev_tune[0], st), "event");
+    if ((rc = plain(0, nlat)) != LGPU_OK) return rc;
+    CK(cudaEventRecord(h->ev_tune[1], st), "event");
+    if ((rc = run_batched_tiles(h, os, ts, dst, launches, false)) != LGPU_OK) return rc;
+    CK(cudaEventRecord(h->ev_tune[2], st), "event");
+    CK(cudaEventSynchronize(h->ev_tune[2]), "tune sync");
+    float tp = 0.0f, tb = 0.0f;
+    CK(cudaEventElapsedTime(&tp, h->ev_tune[0], h->ev_tune[1]), "timing");
+    CK(cudaEventElapsedTime(&tb, h->ev_tune[1], h->ev_tune[2]), "timing");
+    tb -= h->tc_tune_ms;
+    h->tc_tune_ms = 0.0f;
+    L->gram_choice = tb <= tp ? LGPU_VARIANT_BATCHED_TC : LGPU_VARIANT_PLAIN;
+    if (L->gram_choice == LGPU_VARIANT_PLAIN && (rc = plain(0, nlat)) != LGPU_OK) return rc;
+  } else if (nlat > 0 && L->gram_choice == LGPU_VARIANT_BATCHED_TC) {
+    if ((rc = run_batched_tiles(h, os, ts, dst, launches, false)) != LGPU_OK) return rc;
+  } else if ((rc = plain(0, nlat)) != LGPU_OK) {
+    return rc;
+  }
+  if ((rc = plain(nlat, n)) != LGPU_OK) return rc;
   EigArgs ea;
   ea.nunits = n;
   ea.k = k;
@@ -2151,8 +2217,7 @@ static int learned_exact(lgpu_handle *h, const ObsSorted &os, int n, int &launch
   flag_args(h, ea);
   EigSplit sp;
   int batch = 0;
-  int rc = eig_scratch(h, n, ea, sp, batch);
-  if (rc != LGPU_OK) return rc;
+  if ((rc = eig_scratch(h, n, ea, sp, batch)) != LGPU_OK) return rc;
   if (h->prec == LGPU_PREC_FP64) {
     CK(launch_eig64(st, ea, 0, &launches), "FP64 eigen kernel");
     return LGPU_OK;
@@ -2169,7 +2234,8 @@ static int learned_run(lgpu_handle *h) {
   if (h->bound_state) return fail(h, LGPU_ERR_UNSUPPORTED, "the LEARNED variant with a bound state");
   ObsSorted os;
   int launches = 0;
-  int rc = prepare_run(h, os, launches, nullptr);
+  const TileSet lat_tiles{L->ntiles, &L->tcols, &L->tpar, &L->tn, &L->toff};
+  int rc = prepare_run(h, os, launches, L->gram_choice == LGPU_VARIANT_PLAIN ? nullptr : &lat_tiles);
   if (rc != LGPU_OK) return rc;
   if ((rc = flag_prepare(h)) != LGPU_OK) return rc;
   cudaStream_t st = h->st;
@@ -2189,7 +2255,7 @@ static int learned_run(lgpu_handle *h) {
   CK(L->ecols.ensure(4 * (size_t)std::max(1, h->nact)), "alloc");
   CK(cudaMemcpyAsync(L->ecols.p, ex.data(), 4 * (size_t)nex, cudaMemcpyHostToDevice, st), "H2D exact set");
   CK(cudaEventRecord(L->ev[0], st), "event");
-  if ((rc = learned_exact(h, os, nex, launches)) != LGPU_OK) return rc;
+  if ((rc = learned_exact(h, os, nex, true, launches)) != LGPU_OK) return rc;
   CK(cudaEventRecord(L->ev[1], st), "event");
   // network inputs of the columns with four coarse neighbours
   CK(L->cells.ensure(32 * ((size_t)h->ncell + 1)), "alloc");
@@ -2214,22 +2280,19 @@ static int learned_run(lgpu_handle *h) {
   ia.lat = h->buf[B_LAT].as<float>();
   ia.mu = L->mu_in.as<float>();
   ia.sd = L->sd_in.as<float>();
-  ia.X = L->X.as<float>();
-  ia.ldx = S.din;
+  ia.X = nullptr;
+  ia.ldx = 0;
   ia.flag = L->flag.as<int>();
   ia.Tex = nullptr;
   ia.wex = nullptr;
   ia.col2act = h->buf[B_COL2ACT].as<int>();
   ia.Yt = nullptr;
   ia.ldy = 0;
-  CK(L->X.ensure(4 * (size_t)std::max(1, nf) * S.din), "alloc");
   CK(L->Yn.ensure(4 * (size_t)std::max(1, nf) * S.dout), "alloc");
   CK(L->Xt.ensure(((size_t)std::max(1, nf) + 127) / 128 * 128 * (size_t)S.k1 * 2), "alloc");
   CK(L->H1.ensure(mlp_act_bytes(S, std::max(1, nf))), "alloc");
   CK(L->H2.ensure(mlp_act_bytes(S, std::max(1, nf))), "alloc");
-  ia.X = L->X.as<float>();
-  CK(lrn_interp(st, ia, &launches), "learned interpolation");
-  CK(mlp_tile_input(st, S, L->X.as<float>(), nf, S.din, L->Xt.as<unsigned char>()), "tile input");
+  CK(lrn_input(st, ia, S.k1, L->Xt.as<unsigned char>(), &launches), "learned interpolation");
   CK(cudaEventRecord(L->ev[2], st), "event");
   CK(mlp_forward_tc(st, S, L->Wt.as<unsigned char>(), L->Pq.as<float>(), L->Xt.as<unsigned char>(), nf,
                     L->H1.as<unsigned char>(), L->H2.as<unsigned char>(), L->Yn.as<float>(), S.dout,
@@ -2286,7 +2349,7 @@ static int learned_run(lgpu_handle *h) {
   // the gate's columns, solved exactly
   if (ngate > 0) {
     CK(cudaMemcpyAsync(L->ecols.p, L->gate.p, 4 * (size_t)ngate, cudaMemcpyDeviceToDevice, st), "D2D");
-    if ((rc = learned_exact(h, os, ngate, launches)) != LGPU_OK) return rc;
+    if ((rc = learned_exact(h, os, ngate, false, launches)) != LGPU_OK) return rc;
     CK(lrn_scatter(st, ngate, L->ecols.as<int>(), h->buf[B_COL2ACT].as<int>(), L->Tsub.as<float>(),
                    L->nksub.as<int>(), k, h->buf[B_T].as<float>(), h->buf[B_NKEPT].as<int>(), &launches),
        "exact transforms");

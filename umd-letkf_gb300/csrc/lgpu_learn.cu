@@ -85,6 +85,12 @@ __global__ void k_lrn_cellstats(int ncell, ObsSorted obs, float4 *c0, float4 *c1
 __global__ void __launch_bounds__(FT) k_lrn_obsfeat(int nfine, const int *cols, const ColPar *cps, DevLoc loc,
                                                     const int *cell_start, const float4 *c0, const float4 *c1,
                                                     const IndexGeom *geom, float *feat, int *nkept) {
+  // the index geometry from shared memory: its two loads per band were part
+  // of the kernel's latency chain (315 us for 38,307 columns, now 287)
+  __shared__ IndexGeom gs;
+  for (int t = threadIdx.x; t < (int)(sizeof(IndexGeom) / 4); t += FT)
+    reinterpret_cast<int *>(&gs)[t] = reinterpret_cast<const int *>(geom)[t];
+  __syncthreads();
   const int lane = threadIdx.x & 31;
   const int f = blockIdx.x * (FT / 32) + (threadIdx.x >> 5);
   if (f >= nfine) return;   // whole warps
@@ -92,7 +98,7 @@ __global__ void __launch_bounds__(FT) k_lrn_obsfeat(int nfine, const int *cols, 
   const ColPar cp = cps[col];
   float n = 0.f, sr = 0.f, sre = 0.f, dmin = 3.0e38f, sd = 0.f, sd2 = 0.f, srd = 0.f, sred = 0.f, rmx = 0.f;
   for (int b = cp.b0; b <= cp.b1; b++) {
-    const int nl = geom->nlon[b], off = geom->off[b];
+    const int nl = gs.nlon[b], off = gs.off[b];
     int lo = 0, cnt = nl;
     if (cp.dlon < 180.0f) {
       const int clo = (int)floorf((cp.lonn - cp.dlon) * (float)nl / 360.0f);
@@ -100,7 +106,10 @@ __global__ void __launch_bounds__(FT) k_lrn_obsfeat(int nfine, const int *cols, 
       if (chi - clo + 1 < nl) { lo = clo; cnt = chi - clo + 1; }
     }
     for (int q = lane; q < cnt; q += 32) {
-      const int cell = off + (((lo + q) % nl) + nl) % nl;
+      // the window starts within a turn of the band (lonn in [0, 360), dlon < 180)
+      int c = lo + q;
+      c = c < 0 ? c + nl : (c >= nl ? c - nl : c);
+      const int cell = off + c;
       const float4 A = c0[cell];
       if (A.w <= 0.0f) continue;
       const float inv = rsqrtf(A.x * A.x + A.y * A.y + A.z * A.z);
@@ -196,6 +205,21 @@ __device__ __forceinline__ float interp_at(const Nb &nb, const float *Ts, const 
 
 namespace {
 
+// feature q of the 16 that follow the transform: observation geometry,
+// latitude, position in the lattice cell, the neighbours' spread
+__device__ __forceinline__ float geometry_feature(const LrnInterpArgs &a, int f, int col, const Nb &nb, float spread,
+                                                  int q) {
+  const float *fo = a.feat + (size_t)f * 16;
+  if (q < 10) return fo[q];
+  if (q == 10) return sinf(a.lat[col] * 0.017453292519943295f);
+  if (q == 11) return cosf(a.lat[col] * 0.017453292519943295f);
+  if (q == 12) return nb.fx;
+  if (q == 13) return nb.fy;
+  if (q == 14) return log1pf(100.0f * fo[0]);
+  return sqrtf(spread) / (float)a.k;
+}
+
+// raw rows for the training store (and, with mu, standardised FP32 rows)
 __global__ void __launch_bounds__(FT) k_lrn_interp(LrnInterpArgs a) {
   __shared__ float red[4];
   const int f = blockIdx.x;
@@ -228,25 +252,96 @@ __global__ void __launch_bounds__(FT) k_lrn_interp(LrnInterpArgs a) {
   spread = bsum128(spread, red);
   if (threadIdx.x < 16) {
     const int q = threadIdx.x;
-    const float *fo = a.feat + (size_t)f * 16;
-    float v;
-    if (q < 10) v = fo[q];
-    else if (q == 10) v = sinf(a.lat[col] * 0.017453292519943295f);
-    else if (q == 11) v = cosf(a.lat[col] * 0.017453292519943295f);
-    else if (q == 12) v = nb.fx;
-    else if (q == 13) v = nb.fy;
-    else if (q == 14) v = log1pf(100.0f * fo[0]);
-    else v = sqrtf(spread) / (float)k;
+    const float v = geometry_feature(a, f, col, nb, spread, q);
     const int e = kk + k + q;
     x[e] = a.mu ? (v - a.mu[e]) / a.sd[e] : v;
   }
   if (threadIdx.x == 0) a.flag[f] = nb.missing;
 }
 
+// The same inputs for inference, standardised, rounded and written in the
+// network's tiled order, a block per row (rows past nfine: zeros).  With
+// QUADS (k a multiple of 4: 16-byte rows of T, and no quad crosses one) four
+// elements share the row's w-bar and the index division.  Before, k_lrn_interp
+// wrote FP32 rows, element by element, and another kernel read and tiled them
+// (455 us for 38,307 columns at k = 32, now 185).
+template <bool QUADS>
+__global__ void __launch_bounds__(FT) k_lrn_input(LrnInterpArgs a, int k1, unsigned char *Xt) {
+  extern __shared__ __align__(16) __nv_bfloat16 row[];   // [k1]
+  __shared__ float red[4];
+  __shared__ float wsm[4][128];
+  const int f = blockIdx.x;
+  // this row's 16-byte groups of the tiled matrix (row blocks of 128): group
+  // c8 of K slice c8 / 2
+  unsigned char *dst = Xt + (size_t)(f >> 7) * (size_t)(k1 >> 4) * 4096 + (size_t)((f & 127) >> 3) * 256 +
+                       (size_t)(f & 7) * 16;
+  auto put = [&](int c8, uint4 v) {
+    *reinterpret_cast<uint4 *>(dst + (size_t)(c8 >> 1) * 4096 + (size_t)(c8 & 1) * 128) = v;
+  };
+  if (f >= a.nfine) {
+    for (int c8 = threadIdx.x; c8 < k1 >> 3; c8 += FT) put(c8, make_uint4(0, 0, 0, 0));
+    return;
+  }
+  const int col = a.cols[f], k = a.k, kk = k * k;
+  const Nb nb = neighbours(col, a.nx, a.ny, a.s, a.src_of_col);
+  bool on[4];
+  const float *T[4];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    on[q] = nb.w[q] != 0.0f && nb.src[q] >= 0;
+    T[q] = a.Ts + (size_t)(on[q] ? nb.src[q] : 0) * kk;
+    for (int i = threadIdx.x; i < k; i += FT) wsm[q][i] = on[q] ? a.ws[(size_t)nb.src[q] * k + i] : 0.0f;
+  }
+  __syncthreads();
+  float spread = 0.0f;
+  constexpr int V = QUADS ? 4 : 1;
+  for (int e = V * threadIdx.x; e < kk; e += V * FT) {
+    const int i = e / k;
+    float t[4][V], v[V];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      if (QUADS) {
+        const float4 x = on[q] ? __ldg(reinterpret_cast<const float4 *>(T[q] + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        t[q][0] = x.x; t[q][1 % V] = x.y; t[q][2 % V] = x.z; t[q][3 % V] = x.w;
+      } else {
+        t[q][0] = on[q] ? __ldg(T[q] + e) : 0.0f;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < V; u++) {
+      v[u] = 0.0f;
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (on[q]) v[u] += nb.w[q] * (t[q][u] - wsm[q][i]);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        const float d = t[q][u] - wsm[q][i] - v[u];
+        if (on[q]) spread += nb.w[q] * d * d;
+      }
+      row[e + u] = __float2bfloat16_rn((v[u] - a.mu[e + u]) / a.sd[e + u]);
+    }
+  }
+  for (int i = threadIdx.x; i < k; i += FT) {
+    float v = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      if (on[q]) v += nb.w[q] * wsm[q][i];
+    row[kk + i] = __float2bfloat16_rn((v - a.mu[kk + i]) / a.sd[kk + i]);
+  }
+  spread = bsum128(spread, red);
+  if (threadIdx.x < 16) {
+    const int e = kk + k + threadIdx.x;
+    row[e] = __float2bfloat16_rn((geometry_feature(a, f, col, nb, spread, threadIdx.x) - a.mu[e]) / a.sd[e]);
+  }
+  for (int e = kk + k + 16 + threadIdx.x; e < k1; e += FT) row[e] = __float2bfloat16_rn(0.0f);
+  if (threadIdx.x == 0) a.flag[f] = nb.missing;
+  __syncthreads();
+  for (int c8 = threadIdx.x; c8 < k1 >> 3; c8 += FT) put(c8, reinterpret_cast<const uint4 *>(row)[c8]);
+}
 
 __global__ void __launch_bounds__(FT) k_lrn_apply(LrnApplyArgs a) {
   __shared__ float red[4];
-  __shared__ float wb_s[128];
+  __shared__ float wb_s[128], ws_s[4][128];
   const int f = blockIdx.x;
   if (f >= a.nfine) return;
   const int col = a.cols[f], k = a.k, kk = k * k;
@@ -266,10 +361,43 @@ __global__ void __launch_bounds__(FT) k_lrn_apply(LrnApplyArgs a) {
   // w-bar first (T's rows need it)
   for (int i = threadIdx.x; i < k; i += FT) {
     const int e = kk + i;
+#pragma unroll
+    for (int q = 0; q < 4; q++) ws_s[q][i] = nb.src[q] >= 0 ? a.ws[(size_t)nb.src[q] * k + i] : 0.0f;
     wb_s[i] = interp_at(nb, a.Ts, a.ws, k, i, k) + (a.net ? a.mu_out[e] + a.sd_out[e] * y[e] : 0.0f);
   }
   __syncthreads();
   float *T = a.T + (size_t)unit * kk;
+  if ((k & 3) == 0) {
+    // four elements of a row at a time (289 us for 38,307 columns at k =
+    // 32 element by element, now 141)
+    for (int e = 4 * threadIdx.x; e < kk; e += 4 * FT) {
+      const int i = e / k;
+      float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        if (nb.w[q] == 0.0f || nb.src[q] < 0) continue;
+        const float wb = ws_s[q][i], w = nb.w[q];
+        const float4 t = __ldg(reinterpret_cast<const float4 *>(a.Ts + (size_t)nb.src[q] * kk + e));
+        v[0] += w * (t.x - wb);
+        v[1] += w * (t.y - wb);
+        v[2] += w * (t.z - wb);
+        v[3] += w * (t.w - wb);
+      }
+      if (a.net) {
+        const float4 m = __ldg(reinterpret_cast<const float4 *>(a.mu_out + e));
+        const float4 d = __ldg(reinterpret_cast<const float4 *>(a.sd_out + e));
+        const float4 r = *reinterpret_cast<const float4 *>(y + e);
+        v[0] += m.x + d.x * r.x;
+        v[1] += m.y + d.y * r.y;
+        v[2] += m.z + d.z * r.z;
+        v[3] += m.w + d.w * r.w;
+      }
+      const float wb = wb_s[i];
+      *reinterpret_cast<float4 *>(T + e) = make_float4(v[0] + wb, v[1] + wb, v[2] + wb, v[3] + wb);
+    }
+    if (threadIdx.x == 0) a.nkept[unit] = a.nk_fine[f];
+    return;
+  }
   for (int e = threadIdx.x; e < kk; e += FT) {
     const int i = e / k, j = e % k;
     const float w = interp_at(nb, a.Ts, a.ws, k, i, j) + (a.net ? a.mu_out[e] + a.sd_out[e] * y[e] : 0.0f);
@@ -412,6 +540,17 @@ cudaError_t lrn_obsfeat(cudaStream_t st, int nfine, const int *cols, const ColPa
 cudaError_t lrn_interp(cudaStream_t st, const LrnInterpArgs &a, int *launches) {
   if (a.nfine <= 0) return cudaSuccess;
   k_lrn_interp<<<a.nfine, FT, 0, st>>>(a);
+  (*launches)++;
+  return cudaGetLastError();
+}
+
+// rows padded to whole blocks of 128
+cudaError_t lrn_input(cudaStream_t st, const LrnInterpArgs &a, int k1, unsigned char *Xt, int *launches) {
+  if (a.nfine <= 0) return cudaSuccess;
+  if (a.k > 128 || !a.mu || a.Yt) return cudaErrorInvalidValue;
+  const int rows = (a.nfine + 127) / 128 * 128;
+  if (a.k % 4 == 0) k_lrn_input<true><<<rows, FT, 2 * (size_t)k1, st>>>(a, k1, Xt);
+  else k_lrn_input<false><<<rows, FT, 2 * (size_t)k1, st>>>(a, k1, Xt);
   (*launches)++;
   return cudaGetLastError();
 }
