@@ -27,7 +27,7 @@ int noalloc_max_list();
 cudaError_t launch_obslist_noalloc(cudaStream_t st, int gid, const ColPar *cp_col, const DevLoc &loc, ObsSorted obs,
                                    const IndexGeom *geom, int nobs, int *scratch);
 cudaError_t launch_hx_stats(cudaStream_t st, int nobs, int k, float *hx, float *hx_mean, const int *qc, int *flag,
-                            int *pos, int *total);
+                            int *pos);
 cudaError_t launch_compact(cudaStream_t st, int nobs, int k, const int *flag, const int *pos, const float *const *src_f,
                            float *const *dst_f, int nf, const int *const *src_i, int *const *dst_i, int ni,
                            const float *hx, float *hx_out, const float *hxm, float *hxm_out);
@@ -66,7 +66,7 @@ enum {
   B_CP, B_G, B_T, B_NKEPT, B_DMAXHZ, B_DOBSC, B_DLGC, B_DLGL, B_STATUS, B_LEVDEPTH,
   B_LIST_IDX, B_LIST_R, B_LIST_CNT, B_FLUSH, B_TILECOLS, B_TILEPAR, B_TILEN, B_TILEOFF, B_TILELIST, B_TILEREC, B_EIGSCR,
   B_RAW0, B_RAW1, B_RAW2, B_RAW3, B_RAW4, B_RAW5, B_RAW6, B_RAW7, B_RAWQC, B_RAWHX, B_RAWHXM, B_FLAG, B_POS,
-  B_PTRS, B_TOTAL, B_GPART, B_GCNT, B_FLAGLIST, B_TCWORK, B_TCSEG,
+  B_PTRS, B_GPART, B_GCNT, B_FLAGLIST, B_TCWORK, B_TCSEG,
   B_COUNT_ALL
 };
 
@@ -546,8 +546,10 @@ int prepare_state(lgpu_handle *h, int k, int ns, const float *state, const float
 
 }  // namespace
 
-int lgpu_set_state(lgpu_handle *h, int k, int ns, const float *state, const float *mean, const float *sprd, int nvars,
-                   const lgpu_statevar *vars) {
+// `state` is the perturbations with their mean and spread, or (members) the
+// full members, whose statistics the device forms
+static int put_state(lgpu_handle *h, int k, int ns, const float *state, const float *mean, const float *sprd, int nvars,
+                     const lgpu_statevar *vars, bool members) {
   if (!h) return LGPU_ERR_ARG;
   h->state_ok = false;
   h->ran = false;
@@ -559,11 +561,22 @@ int lgpu_set_state(lgpu_handle *h, int k, int ns, const float *state, const floa
   if (rc != LGPU_OK) return rc;
   const size_t nx = (size_t)h->ncol * ns * k, nm = (size_t)h->ncol * ns;
   CK(cudaMemcpyAsync(h->buf[B_BKG].p, state, nx * 4, cudaMemcpyHostToDevice, h->st), "H2D state");
-  CK(cudaMemcpyAsync(h->buf[B_MEANB].p, mean, nm * 4, cudaMemcpyHostToDevice, h->st), "H2D mean");
-  CK(cudaMemcpyAsync(h->buf[B_SPRDB].p, sprd, nm * 4, cudaMemcpyHostToDevice, h->st), "H2D sprd");
+  if (members) {
+    CK(launch_state_stats(h->st, (long long)nm, k, h->buf[B_BKG].as<float>(), h->buf[B_MEANB].as<float>(),
+                          h->buf[B_SPRDB].as<float>()),
+       "background statistics");
+  } else {
+    CK(cudaMemcpyAsync(h->buf[B_MEANB].p, mean, nm * 4, cudaMemcpyHostToDevice, h->st), "H2D mean");
+    CK(cudaMemcpyAsync(h->buf[B_SPRDB].p, sprd, nm * 4, cudaMemcpyHostToDevice, h->st), "H2D sprd");
+  }
   CK(cudaStreamSynchronize(h->st), "set_state sync");
   h->state_ok = true;
   return LGPU_OK;
+}
+
+int lgpu_set_state(lgpu_handle *h, int k, int ns, const float *state, const float *mean, const float *sprd, int nvars,
+                   const lgpu_statevar *vars) {
+  return put_state(h, k, ns, state, mean, sprd, nvars, vars, false);
 }
 
 // In-place state, the reference's semantics: letkf_solver_run reads the
@@ -650,16 +663,14 @@ int lgpu_set_obs_raw(lgpu_handle *h, int nobs, const lgpu_obs *o, const int *qc,
   CK(h->buf[B_HXM].ensure(n * 4), "alloc hx_mean");
   CK(h->buf[B_RAWQC].ensure(n * 4), "alloc");
   CK(h->buf[B_FLAG].ensure(n * 4), "alloc");
-  CK(h->buf[B_POS].ensure(n * 4), "alloc");
-  CK(h->buf[B_TOTAL].ensure(16), "alloc");
+  CK(h->buf[B_POS].ensure((n + 1) * 4), "alloc");
   CK(h->buf[B_PTRS].ensure(32 * sizeof(void *)), "alloc");
   if (nobs > 0) {
     CK(cudaMemcpyAsync(h->buf[B_RAWHX].p, hx_members, (size_t)nobs * k * 4, cudaMemcpyHostToDevice, h->st), "H2D hx");
     if (qc) CK(cudaMemcpyAsync(h->buf[B_RAWQC].p, qc, (size_t)nobs * 4, cudaMemcpyHostToDevice, h->st), "H2D qc");
   }
   CK(launch_hx_stats(h->st, nobs, (int)k, h->buf[B_RAWHX].as<float>(), h->buf[B_RAWHXM].as<float>(),
-                     qc ? h->buf[B_RAWQC].as<int>() : nullptr, h->buf[B_FLAG].as<int>(), h->buf[B_POS].as<int>(),
-                     h->buf[B_TOTAL].as<int>()),
+                     qc ? h->buf[B_RAWQC].as<int>() : nullptr, h->buf[B_FLAG].as<int>(), h->buf[B_POS].as<int>()),
      "hx statistics");
   void *ptrs[32];
   for (int q = 0; q < 6; q++) { ptrs[q] = h->buf[raw[q]].p; ptrs[8 + q] = h->buf[dst[q]].p; }
@@ -673,7 +684,7 @@ int lgpu_set_obs_raw(lgpu_handle *h, int nobs, const lgpu_obs *o, const int *qc,
                     h->buf[B_HXM].as<float>()),
      "observation compaction");
   int kept = 0;
-  CK(cudaMemcpyAsync(&kept, h->buf[B_TOTAL].p, 4, cudaMemcpyDeviceToHost, h->st), "D2H total");
+  CK(cudaMemcpyAsync(&kept, h->buf[B_POS].as<int>() + nobs, 4, cudaMemcpyDeviceToHost, h->st), "D2H total");
   CK(cudaStreamSynchronize(h->st), "set_obs_raw");
   h->nobs = kept;
   if (nobs_kept) *nobs_kept = kept;
@@ -686,21 +697,8 @@ int lgpu_set_obs_raw(lgpu_handle *h, int nobs, const lgpu_obs *o, const int *qc,
 int lgpu_set_state_members(lgpu_handle *h, int k, int ns, const float *members, int nvars, const lgpu_statevar *vars) {
   if (!h) return LGPU_ERR_ARG;
   if (!members) return fail(h, LGPU_ERR_ARG, "set_state_members: bad arguments");
-  // validate and upload exactly as lgpu_set_state, with the members in place of the perturbations
-  const size_t nm = (size_t)h->ncol * (ns > 0 ? ns : 1);
-  int rc = LGPU_OK;
-  {
-    // lgpu_set_state copies mean/sprd from the host; give it placeholders and
-    // overwrite them with the device statistics below
-    std::vector<float> tmp(nm, 0.0f);
-    rc = lgpu_set_state(h, k, ns, members, tmp.data(), tmp.data(), nvars, vars);
-  }
-  if (rc != LGPU_OK) return rc;
-  CK(launch_state_stats(h->st, (long long)h->ncol * ns, k, h->buf[B_BKG].as<float>(), h->buf[B_MEANB].as<float>(),
-                        h->buf[B_SPRDB].as<float>()),
-     "background statistics");
-  CK(cudaStreamSynchronize(h->st), "set_state_members");
-  return LGPU_OK;
+  // validated as lgpu_set_state does (the members stand in for its mean and spread, which are not read)
+  return put_state(h, k, ns, members, members, members, nvars, vars, true);
 }
 
 int lgpu_get_background(lgpu_handle *h, float *state, float *mean, float *sprd) {

@@ -354,6 +354,11 @@ cudaError_t launch_obs_index(cudaStream_t st, const ObsPrepArgs &a, int k, int k
   return cudaGetLastError();
 }
 
+cudaError_t launch_scan(cudaStream_t st, int n, const int *count, int *start) {
+  k_scan_tiles<<<1, ST, 0, st>>>(n, count, start, nullptr, nullptr, nullptr);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_tile_prep(cudaStream_t st, int ntiles, const int *tile_cols, const ColPar *cp, TilePar *tp,
                              int *launches) {
   if (ntiles <= 0) return cudaSuccess;

@@ -460,6 +460,9 @@ cudaError_t launch_obs_index(cudaStream_t st, const ObsPrepArgs &a, int k, int k
                              int *pos_tmp, ObsSorted out, int ntiles, const int *tile_cols, const ColPar *cp,
                              TilePar *tp, int *launches);
 
+// start[0 .. n]: the exclusive scan of count[0 .. n) (one block; both 16-byte aligned)
+cudaError_t launch_scan(cudaStream_t st, int n, const int *count, int *start);
+
 struct GramArgs {
   int nunits, groups, k, kp;
   const int *active;      // active (unmasked) columns

@@ -12,52 +12,42 @@ namespace lgpu {
 
 namespace {
 
-// per observation: member mean and perturbations in place; keep flag
-__global__ void k_hx_stats(int nobs, int k, float *hx, float *hx_mean, const int *qc, int *flag) {
-  const int o = blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= nobs) return;
-  float *h = hx + (size_t)o * k;
-  float sum = 0.0f;
-  for (int m = 0; m < k; m++) sum = __fadd_rn(sum, h[m]);
-  const float mean = __fdiv_rn(sum, (float)k);
-  for (int m = 0; m < k; m++) h[m] = __fsub_rn(h[m], mean);
-  hx_mean[o] = mean;
-  flag[o] = qc ? (qc[o] > 0 ? 0 : 1) : 1;   // obs_def(i)%qc > 0 is dropped
+// A block's rows of k members pass through shared memory, RS rows at a time:
+// read and written whole, in order, while each thread runs along its own row
+// (a pitch of an odd number of words: no bank conflicts).  Straight from
+// global memory the rows' strides cost a 32-byte sector per value (members of
+// 144 x 72 columns x 21 slabs, k = 40: 59 us, now 22).
+constexpr int RS = 128;   // rows (threads) per block
+__device__ __forceinline__ void rows_in(float *sm, const float *x, long long r0, int n, int k, int pitch) {
+  const float *src = x + r0 * k;
+#pragma unroll 4
+  for (int t = threadIdx.x; t < n * k; t += RS) sm[(t / k) * pitch + t % k] = src[t];
+}
+__device__ __forceinline__ void rows_out(const float *sm, float *x, long long r0, int n, int k, int pitch) {
+  float *dst = x + r0 * k;
+#pragma unroll 4
+  for (int t = threadIdx.x; t < n * k; t += RS) dst[t] = sm[(t / k) * pitch + t % k];
 }
 
-// exclusive scan of the keep flags, one block (order preserving)
-__global__ void k_flag_scan(int n, const int *flag, int *pos, int *total) {
-  __shared__ int wsum[32];
-  __shared__ int carry;
-  if (threadIdx.x == 0) carry = 0;
+// per observation: member mean and perturbations in place; keep flag
+__global__ void __launch_bounds__(RS) k_hx_stats(int nobs, int k, float *hx, float *hx_mean, const int *qc, int *flag) {
+  extern __shared__ float rows[];
+  const long long r0 = (long long)blockIdx.x * RS;
+  const int n = (int)min((long long)RS, nobs - r0), pitch = k | 1;
+  rows_in(rows, hx, r0, n, k, pitch);
   __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int base = 0; base < n; base += blockDim.x) {
-    const int i = base + threadIdx.x;
-    const int v = i < n ? flag[i] : 0;
-    int x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) wsum[w] = x;
-    __syncthreads();
-    if (w == 0) {
-      int s = lane < nw ? wsum[lane] : 0;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, s, o);
-        if (lane >= o) s += y;
-      }
-      if (lane < nw) wsum[lane] = s;
-    }
-    __syncthreads();
-    const int excl = carry + (w > 0 ? wsum[w - 1] : 0) + x - v;
-    if (i < n) pos[i] = excl;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry = excl + v;
-    __syncthreads();
+  if ((int)threadIdx.x < n) {
+    float *h = rows + threadIdx.x * pitch;
+    const long long o = r0 + threadIdx.x;
+    float sum = 0.0f;
+    for (int m = 0; m < k; m++) sum = __fadd_rn(sum, h[m]);
+    const float mean = __fdiv_rn(sum, (float)k);
+    for (int m = 0; m < k; m++) h[m] = __fsub_rn(h[m], mean);
+    hx_mean[o] = mean;
+    flag[o] = qc ? (qc[o] > 0 ? 0 : 1) : 1;   // obs_def(i)%qc > 0 is dropped
   }
-  if (threadIdx.x == 0) *total = carry;
+  __syncthreads();
+  rows_out(rows, hx, r0, n, k, pitch);
 }
 
 // compaction: i -> pos[i] for kept observations (pos[i] <= i, so the
@@ -80,31 +70,43 @@ __global__ void k_compact(int nobs, int k, const int *flag, const int *pos, cons
 }
 
 // per (column, slab): background mean, perturbations in place, spread
-__global__ void k_state_stats(long long ncs, int k, float *x, float *mean, float *sprd) {
-  const long long cs = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (cs >= ncs) return;
-  float *v = x + cs * k;
-  float sum = 0.0f;
-  for (int m = 0; m < k; m++) sum = __fadd_rn(sum, v[m]);
-  const float mu = __fdiv_rn(sum, (float)k);
-  float dot = 0.0f;
-  for (int m = 0; m < k; m++) {
-    const float p = __fsub_rn(v[m], mu);
-    v[m] = p;
-    dot = __fadd_rn(dot, __fmul_rn(p, p));
+__global__ void __launch_bounds__(RS) k_state_stats(long long ncs, int k, float *x, float *mean, float *sprd) {
+  extern __shared__ float rows[];
+  const long long r0 = (long long)blockIdx.x * RS;
+  const int n = (int)min((long long)RS, ncs - r0), pitch = k | 1;
+  rows_in(rows, x, r0, n, k, pitch);
+  __syncthreads();
+  if ((int)threadIdx.x < n) {
+    float *v = rows + threadIdx.x * pitch;
+    float sum = 0.0f;
+    for (int m = 0; m < k; m++) sum = __fadd_rn(sum, v[m]);
+    const float mu = __fdiv_rn(sum, (float)k);
+    float dot = 0.0f;
+    for (int m = 0; m < k; m++) {
+      const float p = __fsub_rn(v[m], mu);
+      v[m] = p;
+      dot = __fadd_rn(dot, __fmul_rn(p, p));
+    }
+    mean[r0 + threadIdx.x] = mu;
+    sprd[r0 + threadIdx.x] = __fsqrt_rn(__fdiv_rn(dot, (float)(k - 1)));
   }
-  mean[cs] = mu;
-  sprd[cs] = __fsqrt_rn(__fdiv_rn(dot, (float)(k - 1)));
+  __syncthreads();
+  rows_out(rows, x, r0, n, k, pitch);
 }
+
+constexpr size_t rows_bytes(int k) { return (size_t)RS * (k | 1) * sizeof(float); }   // 66 KB at k = 128
 
 }  // namespace
 
+// the exclusive scan of the keep flags into pos[0 .. nobs]
 cudaError_t launch_hx_stats(cudaStream_t st, int nobs, int k, float *hx, float *hx_mean, const int *qc, int *flag,
-                            int *pos, int *total) {
-  if (nobs <= 0) return cudaMemsetAsync(total, 0, sizeof(int), st);
-  k_hx_stats<<<(nobs + 255) / 256, 256, 0, st>>>(nobs, k, hx, hx_mean, qc, flag);
-  k_flag_scan<<<1, 1024, 0, st>>>(nobs, flag, pos, total);
-  return cudaGetLastError();
+                            int *pos) {
+  if (nobs <= 0) return cudaMemsetAsync(pos, 0, sizeof(int), st);
+  const cudaError_t e =
+      cudaFuncSetAttribute(k_hx_stats, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_bytes(kMaxK));
+  if (e != cudaSuccess) return e;
+  k_hx_stats<<<(nobs + RS - 1) / RS, RS, rows_bytes(k), st>>>(nobs, k, hx, hx_mean, qc, flag);
+  return launch_scan(st, nobs, flag, pos);
 }
 
 cudaError_t launch_compact(cudaStream_t st, int nobs, int k, const int *flag, const int *pos, const float *const *src_f,
@@ -119,7 +121,10 @@ cudaError_t launch_compact(cudaStream_t st, int nobs, int k, const int *flag, co
 
 cudaError_t launch_state_stats(cudaStream_t st, long long ncs, int k, float *x, float *mean, float *sprd) {
   if (ncs <= 0) return cudaSuccess;
-  k_state_stats<<<(int)((ncs + 255) / 256), 256, 0, st>>>(ncs, k, x, mean, sprd);
+  const cudaError_t e =
+      cudaFuncSetAttribute(k_state_stats, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_bytes(kMaxK));
+  if (e != cudaSuccess) return e;
+  k_state_stats<<<(int)((ncs + RS - 1) / RS), RS, rows_bytes(k), st>>>(ncs, k, x, mean, sprd);
   return cudaGetLastError();
 }
 
