@@ -134,3 +134,38 @@ def test_learned_form_cycling():
     assert np.all(np.isfinite(le64[0])) and np.all(np.isfinite(le64[1]))
     err_64 = float(np.sqrt(np.mean((le64[1][act] - ex[1][act]) ** 2))) / spread
     assert err_64 <= 0.02
+
+
+@pytest.mark.parametrize("k", [9, 10, 12])   # member rows of 16 bytes and not
+def test_inference_inputs_and_transforms(k):
+    """Evaluated on the analysis it was trained on, the network has to bring
+    the inferred transforms nearer to the exact ones than the interpolation
+    alone; inputs out of place would take them further away."""
+    from letkf_gb300 import Solver, synth
+    p = synth.generate("c3", nx=72, ny=36, nz=2, n_obs=2000, k=k)
+    loc = {"class": "loc_novrt", "hzloc": {"type": "linearinterp_lat", "value": [{"lat": 0.0, "radius": 1000.0e3}]}}
+    with Solver(0) as s:
+        s.solver_init({})
+        s.loc_init(loc, p.vars)
+        s.set_variant("plain")
+        s.set_problem(p)
+        s.learn_init(p.nx, p.ny, stride=2, hidden=64, judge_frac=0.0, gate_frac=0.0, sample_frac=1.0,
+                     train_cap=10000, seed=5)
+        s.learn_collect()
+        ex = s.get_state()
+        s.learn_train(epochs=150, batch=256, lr=1e-3)
+        s.set_variant("learned")
+        s.run()
+        le, again = s.get_state(), None
+        s.run()
+        again = s.get_state()
+        st = s.learn_stats()
+        s.learn_set_network(False)
+        s.run()
+        ip = s.get_state()
+    act = p.mask == 0
+    assert st["inferred"] > 0.5 * np.count_nonzero(act)
+    for a, b in zip(le, again):
+        assert np.array_equal(a, b)   # whichever Gram form the first run measured, the second repeats it
+    pert = [x[0][act] - x[1][act][:, :, None] for x in (ex, le, ip)]
+    assert rel(pert[1], pert[0]) < rel(pert[2], pert[0])
