@@ -92,6 +92,7 @@ static void chunk_bounds(int ncol, int n, int c, int *c0, int *c1) {
   }
 }
 constexpr int kSegChunks = 256;   // batched Gram: chunks of 16 observations per CTA at most
+constexpr int kMinSegChunks = 24, kSegsPerSM = 3;   // ... and where the chunks are few
 constexpr int kDrainChunks = 64;  // batched Gram: chunks per tensor-core accumulation (drained to a partial block)
 
 struct LearnState;   // learned form (below)
@@ -1023,11 +1024,16 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   ta.diag_lg_obsloc = h->buf[B_DLGL].as<float>();
   ta.status = h->buf[B_STATUS].as<int>();
   // accumulation segments: each tile's stream is split into ranges of at most
-  // kSegChunks chunks, each its own CTA (which drains its tensor-core
+  // seg_chunks chunks, each its own CTA (which drains its tensor-core
   // accumulator into its result rows every 64 chunks: the FP32 accumulation
   // error grows with the MMAs summed into one accumulator); the partial
   // Grams of a tile's segments are summed in order afterwards; the partials
-  // take at most 24 GB (longer segments otherwise)
+  // take at most 24 GB (longer segments otherwise).  A CTA fills an SM, so a
+  // small analysis is split until each SM has kSegsPerSM of them (but no finer
+  // than kMinSegChunks, where a segment's set-up and its partial block cost as
+  // much as its chunks): with 256-chunk segments the longest stream set the
+  // time (144 x 72 columns, k = 40, 130 CTAs: 301 us with 42% of the SMs
+  // in use, now 211)
   ta.units = (long long)h->nact * G;
   ta.nf = packed_size(k);
   ta.Gpart = nullptr;
@@ -1068,7 +1074,10 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   // leaves one accumulator per tile and no blocks
   int longest = 0;
   for (int t = 0; t < ts.ntiles; t++) longest = std::max(longest, h->h_tile_off[t + 1] - h->h_tile_off[t]);
-  int drain = kDrainChunks, seg_chunks = kSegChunks;
+  const long long cta_chunks = (long long)nchunk_total * ta.npass * G;
+  const long long want = (cta_chunks + 152 * kSegsPerSM - 1) / (152 * kSegsPerSM);
+  int drain = kDrainChunks;
+  int seg_chunks = (int)std::min<long long>(kSegChunks, std::max<long long>(kMinSegChunks, want));
   auto pl = plan(seg_chunks, drain);
   while (pl.first.second > 0 && pl.first.second * block_bytes > 24.0 * (1ull << 30)) {
     if (drain < seg_chunks) {
@@ -1095,6 +1104,9 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
     }
   }
   ta.drain = drain;
+  // longest segments first: the last CTAs to start are the short ones
+  std::stable_sort(h->h_tc_work.begin(), h->h_tc_work.end(),
+                   [](const TcWork &x, const TcWork &y) { return x.ce - x.cs > y.ce - y.cs; });
   CK(h->buf[B_TCWORK].ensure(sizeof(TcWork) * std::max<size_t>(1, h->h_tc_work.size())), "alloc segments");
   CK(h->buf[B_TCSEG].ensure(sizeof(TcSegTile) * std::max<size_t>(1, h->h_tc_seg.size())), "alloc segments");
   CK(cudaMemcpyAsync(h->buf[B_TCWORK].p, h->h_tc_work.data(), sizeof(TcWork) * h->h_tc_work.size(),
