@@ -141,7 +141,7 @@ typedef struct lgpu_timings {
   int variant;       /* variant that ran (LGPU_VARIANT_PLAIN / _BATCHED_TC / _LEARNED) */
   float tiles_ms;    /* BATCHED_TC: part of gram_ms spent building the tile candidate streams */
   long long mma_chunks;  /* BATCHED_TC: (tile, group, pass, 16-observation chunk) steps that ran MMAs */
-  int mma_n;         /* BATCHED_TC: features per pass (MMA N); executed TF32 flops =
+  int mma_n;         /* BATCHED_TC: features per pass (MMA N); executed tensor flops =
                         mma_chunks * 3 products * 2 * 128 * mma_n * 16 */
   int precision;     /* eigensolve precision mode of the run (LGPU_PREC_*) */
   int fp64_units;    /* units whose eigensolve ran in FP64 (re-solved, or all under LGPU_PREC_FP64) */
@@ -160,7 +160,7 @@ typedef struct lgpu_timings {
 /* Gram variants.  PLAIN: one CTA per (column, group), FP32 on the CUDA
  * cores.  BATCHED_TC: tiles of 128 neighbouring columns share their
  * observations; the Gram of a tile is one GEMM on the tensor cores (tcgen05,
- * TF32 with a three-term hi/lo split, FP32 accumulation).  AUTO (default)
+ * FP16 or TF32 operands in a three-term hi/lo split, FP32 accumulation).  AUTO (default)
  * runs both forms, timed, on the first analysis after lgpu_set_grid,
  * lgpu_loc_init or a change of ensemble size, and keeps the faster one
  * (PLAIN below k = 8); the first analysis therefore takes longer.  Both

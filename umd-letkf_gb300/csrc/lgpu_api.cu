@@ -62,7 +62,7 @@ enum {
   B_LAT, B_LON, B_MASK, B_COL2ACT, B_ACTIVE,
   B_BKG, B_MEANB, B_SPRDB, B_ANA, B_MEANA, B_SPRDA, B_SLABVAR, B_SLABLEV, B_VARINC, B_VARLB, B_VARUB,
   B_OLAT, B_OLON, B_OZ, B_OTIME, B_OVAL, B_OERR, B_OOBSID, B_OPLATID, B_HX, B_HXM, B_SATOBS, B_SATPLATS,
-  B_GEOM, B_CELL, B_COUNT, B_SLOT, B_POSTMP, B_ATMP, B_BTMP, B_SA, B_SB, B_SHX, B_SIDX, B_CSTART,
+  B_GEOM, B_CELL, B_COUNT, B_SLOT, B_POSTMP, B_ATMP, B_BTMP, B_SA, B_SB, B_SHX, B_SIDX, B_SMAG, B_CSTART,
   B_CP, B_G, B_T, B_NKEPT, B_DMAXHZ, B_DOBSC, B_DLGC, B_DLGL, B_STATUS, B_LEVDEPTH,
   B_LIST_IDX, B_LIST_R, B_LIST_CNT, B_FLUSH, B_TILECOLS, B_TILEPAR, B_TILEN, B_TILEOFF, B_TILELIST, B_TILEREC, B_EIGSCR,
   B_RAW0, B_RAW1, B_RAW2, B_RAW3, B_RAW4, B_RAW5, B_RAW6, B_RAW7, B_RAWQC, B_RAWHX, B_RAWHXM, B_FLAG, B_POS,
@@ -469,7 +469,7 @@ int lgpu_set_grid(lgpu_handle *h, int nij, const float *lat, const float *lon, c
   CK(h->buf[B_TILECOLS].ensure(sizeof(int) * std::max<size_t>(1, tiles.size())), "alloc tiles");
   CK(h->buf[B_TILEPAR].ensure(sizeof(TilePar) * std::max<size_t>(1, tiles.size() / 128)), "alloc tiles");
   CK(h->buf[B_TILEN].ensure(sizeof(int) * std::max<size_t>(1, tile_count_ints((int)(tiles.size() / 128)))), "alloc tiles");
-  CK(h->buf[B_TILEOFF].ensure(sizeof(int) * (tiles.size() / 128 + 1)), "alloc tiles");
+  CK(h->buf[B_TILEOFF].ensure(sizeof(int) * (tiles.size() / 128 + 2)), "alloc tiles");
   if (!tiles.empty())
     CK(cudaMemcpyAsync(h->buf[B_TILECOLS].p, tiles.data(), sizeof(int) * tiles.size(), cudaMemcpyHostToDevice, h->st),
        "H2D tiles");
@@ -781,6 +781,7 @@ static int prepare_run(lgpu_handle *h, ObsSorted &os, int &launches, const TileS
   CK(h->buf[B_SB].ensure(16 * nobs), "alloc");
   CK(h->buf[B_SHX].ensure(4 * nobs * kp), "alloc sorted hx");
   CK(h->buf[B_SIDX].ensure(4 * nobs), "alloc");
+  CK(h->buf[B_SMAG].ensure(4 * nobs), "alloc");
   CK(h->buf[B_CSTART].ensure(4 * ((size_t)h->ncell + 1)), "alloc");
   CK(h->buf[B_CP].ensure(sizeof(ColPar) * (size_t)h->ncol), "alloc");
   CK(h->buf[B_G].ensure(4 * std::max<size_t>(1, (size_t)units) * packed_size(k)), "alloc Gram");
@@ -795,6 +796,7 @@ static int prepare_run(lgpu_handle *h, ObsSorted &os, int &launches, const TileS
   os.B = h->buf[B_SB].as<float4>();
   os.hx = h->buf[B_SHX].as<float>();
   os.idx = h->buf[B_SIDX].as<int>();
+  os.mag = h->buf[B_SMAG].as<float>();
   os.cell_start = h->buf[B_CSTART].as<int>();
   cudaStream_t st = h->st;
   const bool bound = h->bound_state != nullptr;
@@ -950,8 +952,8 @@ static UpdateArgs update_args(lgpu_handle *h) {
 }
 
 // The batched tensor-core Gram over a tile set (tiles of 128 columns; the
-// records and the weight cache are the handle's scratch): G, nkept and the
-// diagnostics of the tiles' units.  Events ev[6] after the tile streams.
+// lists and records are the handle's scratch): G, nkept and the diagnostics
+// of the tiles' units.  Events ev[6] after the tile streams.
 static int upload_members(lgpu_handle *h, cudaEvent_t after);
 
 // Where a tile set's Gram goes: the row of each column (-1: none), the arrays
@@ -970,19 +972,20 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   cudaStream_t st = h->st;
   const int k = h->k, kp = h->kp, G = h->loc.groups;
   // tile candidate streams: count, size the record buffer, fill
+  uint32_t *tile_mag = (*ts.n).as<uint32_t>() + tile_count_ints(ts.ntiles) - 2 * (size_t)ts.ntiles;
   CK(launch_tile_count(st, ts.ntiles, (*ts.par).as<TilePar>(), h->buf[B_GEOM].as<IndexGeom>(), os,
-                       (*ts.n).as<int>(), (*ts.n).as<int>() + ts.ntiles, (*ts.off).as<int>(), &launches),
+                       (*ts.n).as<int>(), (*ts.n).as<int>() + ts.ntiles, tile_mag, (*ts.off).as<int>(), &launches),
      "tile count");
   // the stream offsets size the record buffer and split each tile's stream
   // into accumulation segments
-  if (h->pin_off_n < (size_t)ts.ntiles + 1) {
+  if (h->pin_off_n < (size_t)ts.ntiles + 2) {
     if (h->pin_off) cudaFreeHost(h->pin_off);
     h->pin_off = nullptr;
     h->pin_off_n = 0;
-    CK(cudaMallocHost(&h->pin_off, sizeof(int) * ((size_t)ts.ntiles + 1)), "alloc stream offsets");
-    h->pin_off_n = (size_t)ts.ntiles + 1;
+    CK(cudaMallocHost(&h->pin_off, sizeof(int) * ((size_t)ts.ntiles + 2)), "alloc stream offsets");
+    h->pin_off_n = (size_t)ts.ntiles + 2;
   }
-  CK(cudaMemcpyAsync(h->pin_off, (*ts.off).as<int>(), sizeof(int) * ((size_t)ts.ntiles + 1), cudaMemcpyDeviceToHost,
+  CK(cudaMemcpyAsync(h->pin_off, (*ts.off).as<int>(), sizeof(int) * ((size_t)ts.ntiles + 2), cudaMemcpyDeviceToHost,
                      st),
      "D2H stream offsets");
   CK(cudaStreamSynchronize(st), "stream size sync");
@@ -1001,6 +1004,8 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
     if (rc != LGPU_OK) return rc;
   }
   TcArgs ta;
+  ta.tile_mag = tile_mag;
+  ta.f16 = h->pin_off[ts.ntiles + 1] == 0;
   ta.ntiles = ts.ntiles;
   ta.groups = G;
   ta.k = k;
@@ -1077,7 +1082,7 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   const long long cta_chunks = (long long)nchunk_total * ta.npass * G;
   const long long want = (cta_chunks + 152 * kSegsPerSM - 1) / (152 * kSegsPerSM);
   int drain = kDrainChunks;
-  int seg_chunks = (int)std::min<long long>(kSegChunks, std::max<long long>(kMinSegChunks, want));
+  int seg_chunks = (int)std::min<long long>(kSegChunks, std::max<long long>(kMinSegChunks, (want + 1) & ~1LL));
   auto pl = plan(seg_chunks, drain);
   while (pl.first.second > 0 && pl.first.second * block_bytes > 24.0 * (1ull << 30)) {
     if (drain < seg_chunks) {
@@ -1889,7 +1894,7 @@ int lgpu_learn_init(lgpu_handle *h, const lgpu_learn_config *cfg) {
     CK(L->tcols.ensure(512 * nt), "alloc tiles");
     CK(L->tpar.ensure(sizeof(TilePar) * nt), "alloc tiles");
     CK(L->tn.ensure(4 * tile_count_ints((int)nt)), "alloc tiles");
-    CK(L->toff.ensure(4 * (nt + 1)), "alloc tiles");
+    CK(L->toff.ensure(4 * (nt + 2)), "alloc tiles");
     if (!tiles.empty()) CK(cudaMemcpy(L->tcols.p, tiles.data(), 4 * tiles.size(), cudaMemcpyHostToDevice), "H2D tiles");
   }
   for (auto &e : L->ev) CK(cudaEventCreate(&e), "event");

@@ -21,31 +21,42 @@
 // surf[16] and member-major y: (k+1 rounded to 4) rows x 16 -- one contiguous
 // block per chunk, read once per (group, pass) CTA with one bulk async copy.
 //
-// GEMM CTA roles (17 warps):
-//   warps 0-15  producers; thread t owns column t % 128 for observations
-//               [4 (t / 128), +4) of each chunk and feature t:
-//               weights: the distance (fast float path without branches;
-//               the exact metric and the per-column localizer where the
-//               fast value lies near the search radius or the keep
-//               threshold: bit-identical keep decisions to the per-column
-//               path), W = rloc / err;
-//               features: y_i * y_j, y_i * dep over the chunk;
-//               both operands are split into tf32 hi + lo parts and stored
-//               in the no-swizzle K-major core-matrix layout of an operand
-//               stage;
-//   warp 16     one thread keeps the record ring filled (cp.async.bulk, one
-//               per chunk, mbarrier transaction counts; a slot is refilled
-//               once every producer has finished the chunk in it), issues
-//               tcgen05.mma kind::tf32 for hi*hi + hi*lo + lo*hi (FP32
-//               accumulation in TMEM, relative error ~2^-21 per product) and
-//               frees the stage with tcgen05.commit; chunks in which no
+// GEMM CTA roles (16 + ceil(N / 32) + 1 warps):
+//   warps 0-15  weights; thread t owns column t % 128 for observations
+//               [4 (t / 128), +4) of each chunk: the distance (fast float path
+//               without branches; the exact metric and the per-column
+//               localizer where the fast value lies near the search radius or
+//               the keep threshold: bit-identical keep decisions to the
+//               per-column path), W = rho;
+//   then        features, a thread each: P = y_i * y_j / err, y_i * dep / err.
+//               Both split their operand into FP16 hi + lo parts (TF32 where
+//               the observations' magnitudes need its exponents, then with
+//               1 / err on the weights), stored in the no-swizzle K-major
+//               core-matrix layout of an operand stage;
+//   last warp   one thread keeps the record ring filled (cp.async.bulk, one
+//               per round of chunks, mbarrier transaction counts; a slot is
+//               refilled once every producer has finished the round in it),
+//               issues tcgen05.mma for hi*hi + hi*lo + lo*hi (FP32
+//               accumulation in TMEM, relative error ~2^-22 per product) and
+//               frees the stages with tcgen05.commit; chunks in which no
 //               column keeps an observation issue no MMA.
+// What bounds it (720 x 360 columns, k = 40, 2.07 M chunks over both passes,
+// 17 ms): with TF32 operands, 16 warps doing weights and features in turn, the
+// shared-memory traffic of operand stores and MMA reads (230 KB a chunk), the
+// producers' instructions and the MMAs (1,300 cycles) took about the same time
+// each, and removing any one alone gained 10 to 20%.  FP16 parts halve the
+// traffic and the MMAs, own warps let features and weights overlap: Gram 21.8
+// -> 18.7 ms, then two chunks per barrier round 17.9, the segment sum's 1.65
+// included; the producers bound it now (without weights 14.9, without features
+// 16.5, without MMAs 18.3).  Sharing the weights between the CTAs of two passes
+// through distributed shared memory was slower in three forms (23.3 ms and
+// more): its cluster-scope fences cost more than the weights.
 // The epilogue reads TMEM lane c = column c and writes the packed Gram block
 // of each unit.  Every wait is bounded; a wait that runs out sets status bit
 // 16, the MMA thread waits (bounded) for its copies in flight and TMEM is
 // freed.
 //
-// Long tile streams are split into up to 4 accumulation segments, each its
+// Long tile streams are split into accumulation segments, each its
 // own CTA, summed in order by k_gram_segsum.  The producers come in two forms
 // with bit-identical output (with and without a warp-level cull of records
 // out of every column's reach); the first analysis of a configuration times
@@ -58,21 +69,46 @@ namespace lgpu {
 namespace {
 
 constexpr int TM = 128;        // columns per tile = MMA M = TMEM lanes
-constexpr int KC = 16;         // observations per chunk (two K=8 MMA steps)
-constexpr int NPW = 16;        // producer warps: 0-7 weights, 8-15 features
-constexpr int MMA_WARP = NPW;
-constexpr int NT = 32 * (NPW + 1);
+constexpr int KC = 16;         // observations per chunk (one FP16 or two TF32 MMA steps)
 constexpr int NPMAX = 432;     // features per pass
-constexpr int NSMAX = 2, NRMAX = 6;
+constexpr int NW = 16;         // weight warps; then the feature warps (one per 32 features), then the MMA warp
+__host__ __device__ constexpr int feature_warps(int np) { return (np + 31) / 32; }
+__host__ __device__ constexpr int gram_threads(int np) { return 32 * (NW + feature_warps(np) + 1); }
+constexpr int NSMAX = 4, NRMAX = 6;
 constexpr uint32_t CMB = 128;                 // bytes per core matrix (8 rows x 16 B)
-constexpr uint32_t SBO = (KC / 4) * CMB;      // bytes per 8-row group (all K of the chunk)
-constexpr uint32_t WB = (TM / 8) * SBO;       // bytes per W operand copy
+// bytes of an operand's element, of an 8-row group (all K of the chunk), of a W operand copy
+__host__ __device__ constexpr uint32_t el_bytes(bool f16) { return f16 ? 2 : 4; }
+__host__ __device__ constexpr uint32_t sbo_of(bool f16) { return KC * el_bytes(f16) / 16 * CMB; }
+__host__ __device__ constexpr uint32_t wb_of(bool f16) { return (TM / 8) * sbo_of(f16); }
+__host__ __device__ constexpr int stages_of(bool f16) { return f16 ? 4 : 2; }
+// chunks per round of the barriers.  A round's waits, fence and arrival cost
+// each producer warp a good part of a chunk's time: with FP16 operands two
+// chunks share them (Gram of 720 x 360 columns, k = 40: 18.7 ms, now 17.9; the
+// TF32 stages have room for two chunks in all).
+__host__ __device__ constexpr int round_of(bool f16) { return f16 ? 2 : 1; }
 constexpr size_t kSmemBudget = 227 * 1024 - 4096;   // dynamic shared memory (static part below 4 KB)
 constexpr int WT = 256;        // threads of the stream kernels
 constexpr int YS = 20;         // floats per member row of a chunk record (16 observations + 4: conflict-free rows)
+template <bool F16>
 __device__ __forceinline__ uint32_t kmaj(int row, int kk) {
-  return (uint32_t)(row >> 3) * SBO + (uint32_t)(kk >> 2) * CMB + (uint32_t)(row & 7) * 16u + (uint32_t)(kk & 3) * 4u;
+  constexpr int PC = F16 ? 8 : 4;   // elements of a core matrix row
+  return (uint32_t)(row >> 3) * sbo_of(F16) + (uint32_t)(kk / PC) * CMB + (uint32_t)(row & 7) * 16u +
+         (uint32_t)(kk % PC) * el_bytes(F16);
 }
+
+// FP16 operands.  W = 2^12 rho lies in (0.4, 4096] for every weight above the
+// keep threshold, and the features y_i y_j / err are scaled by a power of two
+// per tile that puts the largest of its candidates' into [2^14, 2^15): hi = f16
+// (11 bits) and lo = f16 (x - hi) then hold 22 bits of every x down to 2^-3
+// (lo's spacing there is FP16's smallest), 2^-18 of the tile's largest feature.
+// Where a tile's candidates differ by more than that in their largest features,
+// or the largest is not finite or beyond 2^+-60 (the factors of a feature stay
+// normal FP32 numbers), the run takes the TF32 operands, whose exponents are
+// FP32's.
+constexpr float kWScale = 4096.0f;
+constexpr int kPTop = 14, kPRange = 18, kPExp = 60;
+__host__ __device__ inline int f32_exp(uint32_t bits) { return (int)(bits >> 23) - 127; }
+__device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
 
 __device__ __forceinline__ bool in_cap(const TilePar &t, float4 A) {
   const float dx = __fsub_rn(t.cx, A.x), dy = __fsub_rn(t.cy, A.y), dz = __fsub_rn(t.cz, A.z);
@@ -175,41 +211,64 @@ __device__ __forceinline__ void warp_range(const Window &W, int w, int &j0, int 
 // candidates per tile: observations of the window inside the tile's cap, per
 // warp range (tile_wn) and in all
 __global__ void __launch_bounds__(WT) k_tile_count(int ntiles, const TilePar *tps, const IndexGeom *geom,
-                                                   const float4 *obsA, const int *cell_start, int *tile_n,
-                                                   int *tile_wn) {
+                                                   const float4 *obsA, const float *mag, const int *cell_start,
+                                                   int *tile_n, int *tile_wn, uint32_t *tile_mag) {
   __shared__ Window W;
   __shared__ int red[WT / 32];
+  __shared__ uint32_t smax[WT / 32], smin[WT / 32];
   const int tile = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const TilePar tp = tps[tile];
   build_window(W, tp, geom, cell_start);
   int cnt = 0, j0, j1;
   warp_range(W, wid, j0, j1);
+  uint32_t mx = 0, mn = 0x7f800000u;   // largest, smallest positive magnitude (their bits)
 #pragma unroll 4
-  for (int j = j0 + lane; j < j1; j += 32) cnt += in_cap(tp, __ldg(obsA + window_pos(W, j)));
+  for (int j = j0 + lane; j < j1; j += 32) {
+    const int p = window_pos(W, j);
+    const bool in = in_cap(tp, __ldg(obsA + p));
+    const uint32_t m = in ? __float_as_uint(__ldg(mag + p)) : 0u;
+    cnt += in;
+    mx = max(mx, m);
+    mn = m != 0u ? min(mn, m) : mn;
+  }
   cnt = __reduce_add_sync(0xffffffffu, cnt);
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  mn = __reduce_min_sync(0xffffffffu, mn);
   if (lane == 0) {
     red[wid] = cnt;
+    smax[wid] = mx;
+    smin[wid] = mn;
     tile_wn[(size_t)tile * (WT / 32) + wid] = cnt;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     int t = 0;
-    for (int w = 0; w < WT / 32; w++) t += red[w];
+    for (int w = 0; w < WT / 32; w++) {
+      t += red[w];
+      mx = max(mx, smax[w]);
+      mn = min(mn, smin[w]);
+    }
     tile_n[tile] = t;
+    tile_mag[2 * tile] = mx;
+    tile_mag[2 * tile + 1] = mn;
   }
 }
 
 // chunk offsets of the tile streams: tile_off[t] = sum over earlier tiles of
 // ceil(n / 16); tile_off[ntiles] = total chunks.  One block.
-__global__ void k_tile_scan(int ntiles, const int *tile_n, int *tile_off) {
+// tile_off[ntiles + 1]: some tile's magnitudes are out of the FP16 operands' range.
+__global__ void k_tile_scan(int ntiles, const int *tile_n, const uint32_t *tile_mag, int *tile_off) {
   __shared__ int wsum[32];
   __shared__ int carry;
   if (threadIdx.x == 0) carry = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  int wide = 0;
   for (int base = 0; base < ntiles; base += blockDim.x) {
     const int i = base + threadIdx.x;
     const int v = i < ntiles ? (tile_n[i] + KC - 1) / KC : 0;
+    const uint32_t mx = i < ntiles ? tile_mag[2 * i] : 0u, mn = i < ntiles ? tile_mag[2 * i + 1] : 0u;
+    if (mx != 0u) wide |= abs(f32_exp(mx)) > kPExp || f32_exp(mx) - f32_exp(mn) > kPRange;
     int x = v;
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, x, o);
@@ -232,7 +291,11 @@ __global__ void k_tile_scan(int ntiles, const int *tile_n, int *tile_off) {
     if (threadIdx.x == blockDim.x - 1) carry = excl + v;
     __syncthreads();
   }
-  if (threadIdx.x == 0) tile_off[ntiles] = carry;
+  wide = __syncthreads_or(wide);
+  if (threadIdx.x == 0) {
+    tile_off[ntiles] = carry;
+    tile_off[ntiles + 1] = wide;
+  }
 }
 
 // The tile streams, in two steps: the positions of the cap's members in window
@@ -330,6 +393,21 @@ __device__ __forceinline__ void split2(F2 v, F2 &hi, F2 &lo) {
   lo = f2_fma(hi, F2(kFC.minus_one), v);   // exact
 }
 
+// two values -> FP16 hi and lo pairs (the first in the low half)
+__device__ __forceinline__ uint32_t pack_f16(float x, float y) {
+  uint32_t r;
+  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y), "f"(x));
+  return r;
+}
+__device__ __forceinline__ void split_f16(F2 v, uint32_t &hi, uint32_t &lo) {
+  hi = pack_f16(v.x(), v.y());
+  float a, b;
+  asm("{\n\t.reg .f16 l, h;\n\tmov.b32 {l, h}, %2;\n\tcvt.f32.f16 %0, l;\n\tcvt.f32.f16 %1, h;\n\t}"
+      : "=f"(a), "=f"(b) : "r"(hi));
+  const F2 d = f2_fma(F2(a, b), F2(kFC.minus_one), v);   // exact
+  lo = pack_f16(d.x(), d.y());
+}
+
 struct TcSmem {
   unsigned long long full[NSMAX], empty[NSMAX], rfull[NRMAX], done;
   unsigned long long accf;   // drain: the accumulation so far is complete in TMEM (commit + MMA thread)
@@ -388,12 +466,15 @@ __device__ __forceinline__ void bar_arrive(unsigned long long *b) {
 // search chords skips the distance and localizer evaluation (their weights are
 // zero either way; results are bit-identical); pays where search radii are
 // small next to the tile caps, costs registers where they are not
-template <int LOC, int NS, int NR, bool CULL>
-__global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
+template <int LOC, int NR, bool CULL, bool F16>
+__global__ void __launch_bounds__(gram_threads(NPMAX), 1) k_gram_tc(TcArgs a) {
+  constexpr int NS = stages_of(F16), CPR = round_of(F16), NSR = NS / CPR, NRR = NR / CPR;   // NSR, NRR: in rounds
+  constexpr uint32_t SBO = sbo_of(F16), WB = wb_of(F16);
   static_assert(NS <= NSMAX && NR <= NRMAX, "operand stages / record slots beyond the barrier arrays");
   extern __shared__ __align__(1024) unsigned char dsm[];
   __shared__ __align__(16) TcSmem S;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int mma_warp = (int)(blockDim.x >> 5) - 1;   // = the number of producer warps
   // block = (work item, group, pass), pass fastest: the passes of a work item
   // run side by side and share its records in L2
   const int pass = blockIdx.x % a.npass;
@@ -410,7 +491,7 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
   const int t0 = a.tile_off[tile], tn = a.tile_off[tile + 1] - t0;
   const int cs = min(tn, wk.cs), ce = min(tn, wk.ce);
   const int c0 = t0 + cs;
-  const int nchunks = ce - cs;
+  const int nchunks = ce - cs, nrounds = (nchunks + CPR - 1) / CPR;
   const uint32_t tmem_cols = a.tmem_cols;
   if (nchunks <= 0 && wk.blk0 < 0) {
     // no observation within the tile's cap: nothing is kept, and the G of a
@@ -428,21 +509,21 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
   // ---- setup: TMEM, barriers, feature table
   if (wid == 0) tc::tmem_alloc(&S.tmem, tmem_cols);
   if (tid == 0) {
-    for (int s = 0; s < NS; s++) {
-      tc::mbar_init(reinterpret_cast<uint64_t *>(&S.full[s]), NPW);
+    for (int s = 0; s < NS; s++) S.anyk[s] = 0;
+    for (int s = 0; s < NSR; s++) {
+      tc::mbar_init(reinterpret_cast<uint64_t *>(&S.full[s]), (uint32_t)mma_warp);
       tc::mbar_init(reinterpret_cast<uint64_t *>(&S.empty[s]), 1);
-      S.anyk[s] = 0;
     }
-    for (int r = 0; r < NR; r++) tc::mbar_init(reinterpret_cast<uint64_t *>(&S.rfull[r]), 1);
+    for (int r = 0; r < NRR; r++) tc::mbar_init(reinterpret_cast<uint64_t *>(&S.rfull[r]), 1);
     tc::mbar_init(reinterpret_cast<uint64_t *>(&S.done), 1);
     tc::mbar_init(reinterpret_cast<uint64_t *>(&S.accf), 2);
-    tc::mbar_init(reinterpret_cast<uint64_t *>(&S.acce), NPW);
+    tc::mbar_init(reinterpret_cast<uint64_t *>(&S.acce), NW);
     S.issued = 0;
     S.sub_issued = 0;
     S.fault = 0;
     tc::mbar_fence_init();
   }
-  for (int f = tid; f < NP; f += NT) {
+  for (int f = tid; f < NP; f += (int)blockDim.x) {
     const int fg = pass * NP + f;
     int i = 255, j = 255;
     if (fg < nf) packed_ij(fg, k, i, j);
@@ -454,18 +535,23 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
   tc::fence_after();
   const uint32_t tmem = S.tmem;
 
-  // producer thread: column wc, observations [4 wq, 4 wq + 4) of each chunk,
-  // and feature f = tid
-  const int wc = tid & (TM - 1), wq = (tid >> 7) & 3;
+  // weight thread: column wc, observations [e0, e0 + 4) of each chunk
+  const int wc = tid & (TM - 1), wq = (tid >> 7) & 3, e0 = 4 * wq;
   int ncand = 0, nkeep = 0;
   float rsum = 0.0f;
 
-  // The CTA's results: TMEM lane = column wc.  A tile whose stream is one
+  // the tile's power-of-two scale of the features, and what takes it and the
+  // weights' out of the accumulator
+  const uint32_t mmax = F16 ? a.tile_mag[2 * tile] : 0u;
+  const int pe = F16 && mmax != 0u ? kPTop - f32_exp(mmax) : 0;
+  const float pscale = F16 ? pow2(pe) : 1.0f, oscale = F16 ? pow2(-pe) * (1.0f / kWScale) : 1.0f;
+  // The CTA's results: TMEM lane = column wc of a weight thread.  A tile whose stream is one
   // drain interval writes the column's G row (thread tid < TM, warps 0-3);
   // otherwise every drain interval goes to its own partial block,
   // feature-major, so that a warp's stores of one feature are 32 consecutive
-  // floats (the 16 producer warps drain, each warp a quarter of the features
-  // of its lane quarter).
+  // floats (the weight warps drain: warp w its lane quarter w % 4, the
+  // features of quarter w / 4).
+
   const int G = a.groups;
   const int D = a.drain;
   const int nvalid = nf - pass * NP < NP ? nf - pass * NP : NP;
@@ -484,10 +570,10 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
       }
 #pragma unroll
       for (int q = 0; q < 16; q++)
-        if (f0 + q < nvalid) base[(size_t)(f0 + q) * TM] = v[q];
+        if (f0 + q < nvalid) base[(size_t)(f0 + q) * TM] = F16 ? v[q] * oscale : v[q];
     }
   };
-  // drain j (all 16 producer warps, warp w the features of quarter w / 4):
+  // drain j (all weight warps):
   // wait until the MMAs before boundary (j + 1) D have completed, move the
   // accumulator to its block, hand TMEM back to the MMA thread
   const int nflush = nchunks > 0 ? (nchunks - 1) / D : 0;
@@ -501,7 +587,7 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
     if (lane == 0) bar_arrive(&S.acce);
   };
 
-  if (wid < NPW) {
+  if (wid < NW) {
     const int col = a.tile_cols[(size_t)tile * TM + wc];
     const bool colv = col >= 0;
     ColFast cf;
@@ -533,142 +619,209 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
     lk.tsat = a.loc.tloc_sat;
     lk.ictp = (LOC == LOC_OCEAN && lk.tprof > 0.0f) ? inv_c_of(lk.tprof) : 1.0f;
     lk.icts = (LOC == LOC_OCEAN && lk.tsat > 0.0f) ? inv_c_of(lk.tsat) : 1.0f;
-    const int f = tid;
+    for (int rd = 0; rd < nrounds; rd++) {
+      const int sr = rd % NSR, rr = rd % NRR;
+      // the producers drain TMEM at boundary b = (j + 1) D (D a multiple of
+      // CPR) once the stages of chunks b .. b + NS - 1 are produced: the MMA
+      // of chunk b + NS needs the stage chunk b frees, which waits for the drain
+      if (nflushed < nflush && rd * CPR == (nflushed + 1) * D + NS) flush(nflushed++);
+      if (!tc::mbar_wait(reinterpret_cast<uint64_t *>(&S.rfull[rr]), (rd / NRR) & 1)) { S.fault = 1; break; }
+      if (rd >= NSR && !tc::mbar_wait(reinterpret_cast<uint64_t *>(&S.empty[sr]), ((rd / NSR) - 1) & 1)) {
+        S.fault = 1;
+        break;
+      }
+#pragma unroll 1
+      for (int ch = rd * CPR; ch < min(nchunks, (rd + 1) * CPR); ch++) {
+        const int s = ch % NS, r = ch % NR;
+        const unsigned char *rec = ring + (size_t)r * slotb;
+        const float *R = reinterpret_cast<const float *>(rec);
+        unsigned char *Whi = stage_ptr(s), *Wlo = Whi + WB;
+        bool anyk = false;
+        // ---- weights: four observations, fast path without branches
+        float w[4];
+        unsigned inr = 0;
+        F2 ox[2], oy[2], oz[2], c2[2];
+        f2_load2(R + e0, ox[0], ox[1]);
+        f2_load2(R + 16 + e0, oy[0], oy[1]);
+        f2_load2(R + 32 + e0, oz[0], oz[1]);
+        float cmin = 3.0e38f, cmax = 0.0f;
+#pragma unroll
+        for (int u = 0; u < 4; u++) w[u] = 0.0f;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          c2[h] = chord2_fast(cf.nx, cf.ny, cf.nz, ox[h], oy[h], oz[h]);
+          cmin = fminf(cmin, fminf(c2[h].x(), c2[h].y()));
+        }
+        bool go = true;
+        if constexpr (CULL) go = __any_sync(0xffffffffu, cmin <= cf.c2max);
+        if (go) {
+          float near = 1.0f;   // the smallest distance of a decision from its threshold, in units of kGuardFast's scale
+          float c[4], rl[4];
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const F2 r2 = loc_fast<LOC>(lk, cf, g, dist_fast(c2[h], short_asin), R, e0 + 2 * h);
+            c[2 * h] = c2[h].x();
+            c[2 * h + 1] = c2[h].y();
+            rl[2 * h] = r2.x();
+            rl[2 * h + 1] = r2.y();
+          }
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            const bool in = c[u] <= cf.c2in;
+            near = fminf(near, fminf(fabsf(c[u] - cf.c2in) * cf.cscale, fabsf(rl[u] - kKeep)));
+            w[u] = in && rl[u] > kKeep ? rl[u] : 0.0f;
+            inr += in;
+            cmax = fmaxf(cmax, c[u]);
+          }
+          // beyond a chord of 1 the fast distance does not hold
+          if (far) near = cmax > 1.0f ? 0.0f : near;
+          // ---- rare: exact metric and the per-column localizer
+          if (__any_sync(0xffffffffu, near <= kGuardFast) && near <= kGuardFast) {
+            inr = 0;
+#pragma unroll 1
+            for (int u = 0; u < 4; u++) {
+              float cu = c[0], wu = w[0], ru = rl[0];
+#pragma unroll
+              for (int v = 1; v < 4; v++) {
+                cu = u == v ? c[v] : cu;
+                wu = u == v ? w[v] : wu;
+                ru = u == v ? rl[v] : ru;
+              }
+              bool in = cu <= cf.c2in;
+              const bool unsure = cu <= cf.c2max && (cu > 1.0f || fabsf(cu - cf.c2in) * cf.cscale <= kGuardFast ||
+                                                     (in && fabsf(ru - kKeep) <= kGuardFast));
+              if (unsure) {
+                const int e = e0 + u;
+                // the column's parameters from global memory (keeps them out of
+                // the producers' registers)
+                const ColPar &cp = a.cp[col];
+                const float de = dist_from_chord2(chord2_exact(cp.ux, cp.uy, cp.uz, R[e], R[16 + e], R[32 + e]));
+                in = de <= cp.rmax;
+                const float re = in ? localize_cls<LOC>(a.loc, cp, g, de, R[80 + e], R[96 + e], R[112 + e]) : 0.0f;
+                wu = re > kKeep ? re : 0.0f;
+              }
+              inr += in;
+#pragma unroll
+              for (int v = 0; v < 4; v++) w[v] = u == v ? wu : w[v];
+            }
+          }
+        }
+        {
+          ncand += inr;
+          float wmax = 0.0f;
+#pragma unroll
+          for (int u = 0; u < 4; u++) {
+            nkeep += w[u] > 0.0f;
+            rsum += w[u];
+            wmax = fmaxf(wmax, w[u]);
+          }
+          anyk = wmax > 0.0f;
+          const uint32_t off = kmaj<F16>(wc, e0);
+          if constexpr (F16) {
+            uint32_t hi[2], lo[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+              split_f16(f2_mul(F2(w[2 * h], w[2 * h + 1]), f2_all(kWScale)), hi[h], lo[h]);
+            *reinterpret_cast<uint2 *>(Whi + off) = make_uint2(hi[0], hi[1]);
+            *reinterpret_cast<uint2 *>(Wlo + off) = make_uint2(lo[0], lo[1]);
+          } else {
+            F2 ri[2], hi[2], lo[2];
+            f2_load2(R + 48 + e0, ri[0], ri[1]);   // 1/err
+#pragma unroll
+            for (int h = 0; h < 2; h++) split2(f2_mul(F2(w[2 * h], w[2 * h + 1]), ri[h]), hi[h], lo[h]);
+            f2_store2(reinterpret_cast<float *>(Whi + off), hi[0], hi[1]);
+            f2_store2(reinterpret_cast<float *>(Wlo + off), lo[0], lo[1]);
+          }
+        }
+        if (__any_sync(0xffffffffu, anyk) && lane == 0) S.anyk[s] = ch + 1;
+      }
+      tc::fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) bar_arrive(&S.full[sr]);
+    }
+    while (nflushed < nflush) flush(nflushed++);
+  } else if (wid < mma_warp) {
+    // ================================================= feature products: feature f over a chunk's 16 observations
+    const int f = tid - 32 * NW;
     const bool fin = f < NP;
     const int fi = fin ? S.fi[f] : 255, fj = fin ? S.fj[f] : 255;
     // a feature past the last one multiplies row 0; its accumulator is not read
     const int rowi = (fi != 255 ? fi : 0) * YS, rowj = (fi != 255 ? fj : 0) * YS;
-
-    for (int ch = 0; ch < nchunks; ch++) {
-      const int s = ch % NS, r = ch % NR;
-      // the producers drain TMEM at boundary b = (j + 1) D once the stages
-      // of chunks b .. b + NS - 1 are produced: the MMA of chunk b + NS needs
-      // the stage chunk b frees, which waits for the drain
-      if (nflushed < nflush && ch == (nflushed + 1) * D + NS) flush(nflushed++);
-      if (!tc::mbar_wait(reinterpret_cast<uint64_t *>(&S.rfull[r]), (ch / NR) & 1)) { S.fault = 1; break; }
-      if (ch >= NS && !tc::mbar_wait(reinterpret_cast<uint64_t *>(&S.empty[s]), ((ch / NS) - 1) & 1)) {
+    for (int rd = 0; rd < nrounds; rd++) {
+      const int sr = rd % NSR, rr = rd % NRR;
+      if (!tc::mbar_wait(reinterpret_cast<uint64_t *>(&S.rfull[rr]), (rd / NRR) & 1)) { S.fault = 1; break; }
+      if (rd >= NSR && !tc::mbar_wait(reinterpret_cast<uint64_t *>(&S.empty[sr]), ((rd / NSR) - 1) & 1)) {
         S.fault = 1;
         break;
       }
-      const unsigned char *rec = ring + (size_t)r * slotb;
-      const float *R = reinterpret_cast<const float *>(rec);
-      unsigned char *Whi = stage_ptr(s), *Wlo = Whi + WB, *Phi = Whi + 2 * WB, *Plo = Phi + PB;
-      const int e0 = wq * 4;
-      bool anyk = false;
-      // ---- weights: four observations, fast path without branches
-      float w[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      unsigned inr = 0;
-      F2 ox[2], oy[2], oz[2], c2[2];
-      f2_load2(R + e0, ox[0], ox[1]);
-      f2_load2(R + 16 + e0, oy[0], oy[1]);
-      f2_load2(R + 32 + e0, oz[0], oz[1]);
-#pragma unroll
-      for (int h = 0; h < 2; h++) c2[h] = chord2_fast(cf.nx, cf.ny, cf.nz, ox[h], oy[h], oz[h]);
-      bool go = true;
-      if constexpr (CULL)
-        go = __any_sync(0xffffffffu, fminf(fminf(c2[0].x(), c2[0].y()), fminf(c2[1].x(), c2[1].y())) <= cf.c2max);
-      if (go) {
-        float near = 1.0f;   // the smallest distance of a decision from its threshold, in units of kGuardFast's scale
-        float c[4] = {c2[0].x(), c2[0].y(), c2[1].x(), c2[1].y()}, rl[4];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const F2 r2 = loc_fast<LOC>(lk, cf, g, dist_fast(c2[h], short_asin), R, e0 + 2 * h);
-          rl[2 * h] = r2.x();
-          rl[2 * h + 1] = r2.y();
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const bool in = c[u] <= cf.c2in;
-          near = fminf(near, fminf(fabsf(c[u] - cf.c2in) * cf.cscale, fabsf(rl[u] - kKeep)));
-          w[u] = in && rl[u] > kKeep ? rl[u] : 0.0f;
-          inr += in;
-        }
-        // beyond a chord of 1 the fast distance does not hold
-        if (far) near = fmaxf(fmaxf(c[0], c[1]), fmaxf(c[2], c[3])) > 1.0f ? 0.0f : near;
-        // ---- rare: exact metric and the per-column localizer
-        if (__any_sync(0xffffffffu, near <= kGuardFast) && near <= kGuardFast) {
-          inr = 0;
 #pragma unroll 1
-          for (int u = 0; u < 4; u++) {
-            const float cu = u == 0 ? c[0] : u == 1 ? c[1] : u == 2 ? c[2] : c[3];
-            float wu = u == 0 ? w[0] : u == 1 ? w[1] : u == 2 ? w[2] : w[3];
-            const float ru = u == 0 ? rl[0] : u == 1 ? rl[1] : u == 2 ? rl[2] : rl[3];
-            bool in = cu <= cf.c2in;
-            const bool unsure = cu <= cf.c2max && (cu > 1.0f || fabsf(cu - cf.c2in) * cf.cscale <= kGuardFast ||
-                                                   (in && fabsf(ru - kKeep) <= kGuardFast));
-            if (unsure) {
-              const int e = e0 + u;
-              // the column's parameters from global memory (keeps them out of
-              // the producers' registers)
-              const ColPar &cp = a.cp[col];
-              const float de = dist_from_chord2(chord2_exact(cp.ux, cp.uy, cp.uz, R[e], R[16 + e], R[32 + e]));
-              in = de <= cp.rmax;
-              const float re = in ? localize_cls<LOC>(a.loc, cp, g, de, R[80 + e], R[96 + e], R[112 + e]) : 0.0f;
-              wu = re > kKeep ? re : 0.0f;
+      for (int ch = rd * CPR; fin && ch < min(nchunks, (rd + 1) * CPR); ch++) {
+        const int s = ch % NS, r = ch % NR;
+        unsigned char *Phi = stage_ptr(s) + 2 * WB, *Plo = Phi + PB;
+        const float *R = reinterpret_cast<const float *>(ring + (size_t)r * slotb);
+        const float *yi = R + 128 + rowi, *yj = R + 128 + rowj;
+        if constexpr (F16) {
+#pragma unroll
+          for (int grp = 0; grp < 2; grp++) {
+            uint32_t hi[4], lo[4];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+              const int e = 8 * grp + 4 * q;
+              F2 ai[2], bj[2], ri[2];
+              f2_load2(yi + e, ai[0], ai[1]);
+              f2_load2(yj + e, bj[0], bj[1]);
+              f2_load2(R + 48 + e, ri[0], ri[1]);   // 1/err
+#pragma unroll
+              for (int h = 0; h < 2; h++)
+                split_f16(f2_mul(f2_mul(f2_mul(ai[h], ri[h]), f2_all(pscale)), bj[h]), hi[2 * q + h], lo[2 * q + h]);
             }
-            inr += in;
-            w[0] = u == 0 ? wu : w[0];
-            w[1] = u == 1 ? wu : w[1];
-            w[2] = u == 2 ? wu : w[2];
-            w[3] = u == 3 ? wu : w[3];
+            const uint32_t off = kmaj<F16>(f, 8 * grp);
+            *reinterpret_cast<uint4 *>(Phi + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4 *>(Plo + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          }
+        } else {
+#pragma unroll
+          for (int grp = 0; grp < 4; grp++) {
+            F2 ai[2], bj[2], hi[2], lo[2];
+            f2_load2(yi + 4 * grp, ai[0], ai[1]);
+            f2_load2(yj + 4 * grp, bj[0], bj[1]);
+#pragma unroll
+            for (int h = 0; h < 2; h++) split2(f2_mul(ai[h], bj[h]), hi[h], lo[h]);
+            const uint32_t off = kmaj<F16>(f, grp * 4);
+            f2_store2(reinterpret_cast<float *>(Phi + off), hi[0], hi[1]);
+            f2_store2(reinterpret_cast<float *>(Plo + off), lo[0], lo[1]);
           }
         }
       }
-      {
-        ncand += inr;
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          nkeep += w[u] > 0.0f;
-          rsum += w[u];
-        }
-        anyk = fmaxf(fmaxf(w[0], w[1]), fmaxf(w[2], w[3])) > 0.0f;
-        F2 ri[2], hi[2], lo[2];
-        f2_load2(R + 48 + e0, ri[0], ri[1]);   // 1/err
-#pragma unroll
-        for (int h = 0; h < 2; h++) split2(f2_mul(F2(w[2 * h], w[2 * h + 1]), ri[h]), hi[h], lo[h]);
-        const uint32_t off = kmaj(wc, e0);
-        f2_store2(reinterpret_cast<float *>(Whi + off), hi[0], hi[1]);
-        f2_store2(reinterpret_cast<float *>(Wlo + off), lo[0], lo[1]);
-      }
-      // ---- feature products: feature f over the 16 observations
-      if (fin) {
-        const float *yi = R + 128 + rowi, *yj = R + 128 + rowj;
-#pragma unroll
-        for (int grp = 0; grp < 4; grp++) {
-          F2 ai[2], bj[2], hi[2], lo[2];
-          f2_load2(yi + 4 * grp, ai[0], ai[1]);
-          f2_load2(yj + 4 * grp, bj[0], bj[1]);
-#pragma unroll
-          for (int h = 0; h < 2; h++) split2(f2_mul(ai[h], bj[h]), hi[h], lo[h]);
-          const uint32_t off = kmaj(f, grp * 4);
-          f2_store2(reinterpret_cast<float *>(Phi + off), hi[0], hi[1]);
-          f2_store2(reinterpret_cast<float *>(Plo + off), lo[0], lo[1]);
-        }
-      }
-      if (__any_sync(0xffffffffu, anyk) && lane == 0) S.anyk[s] = ch + 1;
       tc::fence_proxy_async();
       __syncwarp();
-      if (lane == 0) bar_arrive(&S.full[s]);
+      if (lane == 0) bar_arrive(&S.full[sr]);
     }
-    while (nflushed < nflush) flush(nflushed++);
-  } else if (wid == MMA_WARP) {
+  } else {
     // ================================================= MMA issue + record loads (one thread)
     if (lane == 0) {
       const unsigned char *src = a.rec + (size_t)c0 * cb;
-      auto load = [&](int ch) {
-        unsigned char *dst = ring + (size_t)(ch % NR) * slotb;
-        uint64_t *bar = reinterpret_cast<uint64_t *>(&S.rfull[ch % NR]);
-        tc::bulk_load(dst, src + (size_t)ch * cb, (uint32_t)cb, bar);
+      // the records of a round, one copy
+      auto load = [&](int rd) {
+        unsigned char *dst = ring + (size_t)(rd % NRR) * CPR * slotb;
+        uint64_t *bar = reinterpret_cast<uint64_t *>(&S.rfull[rd % NRR]);
+        tc::bulk_load(dst, src + (size_t)rd * CPR * cb, (uint32_t)(min(CPR, nchunks - rd * CPR) * cb), bar);
       };
-      int n_loaded = nchunks < NR ? nchunks : NR;
-      for (int ch = 0; ch < n_loaded; ch++) load(ch);
+      int n_loaded = nrounds < NRR ? nrounds : NRR;
+      for (int rd = 0; rd < n_loaded; rd++) load(rd);
       const int nb0 = NP < 256 ? NP : 256, nb1 = NP - nb0;
-      const uint32_t id0 = tc::idesc_tf32(TM, nb0), id1 = nb1 > 0 ? tc::idesc_tf32(TM, nb1) : 0u;
+      auto idesc = [](int n) { return F16 ? tc::idesc_f16(TM, n) : tc::idesc_tf32(TM, n); };
+      const uint32_t id0 = idesc(nb0), id1 = nb1 > 0 ? idesc(nb1) : 0u;
+      auto mma = [](uint32_t d, uint64_t ad, uint64_t bd, uint32_t id, uint32_t acc) {
+        if constexpr (F16) tc::mma_f16(d, ad, bd, id, acc);
+        else tc::mma_tf32(d, ad, bd, id, acc);
+      };
+      constexpr int KS = F16 ? 1 : KC / 8;   // MMA steps of a chunk
       bool issued = false;   // since the last drain
       int nmma = 0, fj = 0;
-      for (int ch = 0; ch < nchunks; ch++) {
-        const int s = ch % NS;
-        if (ch > 0 && ch % a.drain == 0) {
+      for (int rd = 0; rd < nrounds; rd++) {
+        const int sr = rd % NSR;
+        if (rd > 0 && rd * CPR % D == 0) {
           // boundary: hand the accumulation to the producer warps and wait
           // until they have read TMEM; the next MMA starts a fresh accumulation
           S.sub_issued = issued ? 1 : 0;
@@ -679,32 +832,35 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
           fj++;
           issued = false;
         }
-        if (!tc::mbar_wait(reinterpret_cast<uint64_t *>(&S.full[s]), (ch / NS) & 1)) { S.fault = 1; break; }
-        // every producer is done with the records of chunk ch: refill the slot
-        if (n_loaded < nchunks) load(n_loaded++);
-        if (S.anyk[s] == ch + 1) {
-          tc::fence_after();
-          const uint32_t whi = tc::smem_u32(stage_ptr(s)), wlo = whi + WB, phi = whi + 2 * WB, plo = phi + PB;
+        if (!tc::mbar_wait(reinterpret_cast<uint64_t *>(&S.full[sr]), (rd / NSR) & 1)) { S.fault = 1; break; }
+        // every producer is done with the records of the round: refill the slot
+        if (n_loaded < nrounds) load(n_loaded++);
+        bool any = false;
+        for (int ch = rd * CPR; ch < min(nchunks, (rd + 1) * CPR); ch++) {
+          const int s = ch % NS;
+          if (S.anyk[s] == ch + 1) {
+            tc::fence_after();
+            const uint32_t whi = tc::smem_u32(stage_ptr(s)), wlo = whi + WB, phi = whi + 2 * WB, plo = phi + PB;
 #pragma unroll
-          for (int t = 0; t < 3; t++)
+            for (int t = 0; t < 3; t++)
 #pragma unroll
-            for (int ks = 0; ks < KC / 8; ks++) {
-              const uint32_t acc = (issued || t > 0 || ks > 0) ? 1u : 0u;
-              const uint32_t aw = t == 2 ? wlo : whi, bp = t == 1 ? plo : phi;
-              const uint64_t ad = tc::smem_desc(aw + ks * 2 * CMB, CMB, SBO);
-              const uint64_t bd0 = tc::smem_desc(bp + ks * 2 * CMB, CMB, SBO);
-              tc::mma_tf32(tmem, ad, bd0, id0, acc);
-              if (nb1 > 0) {
-                const uint64_t bd1 = tc::smem_desc(bp + (uint32_t)(nb0 / 8) * SBO + ks * 2 * CMB, CMB, SBO);
-                tc::mma_tf32(tmem + (uint32_t)nb0, ad, bd1, id1, acc);
+              for (int ks = 0; ks < KS; ks++) {
+                const uint32_t acc = (issued || t > 0 || ks > 0) ? 1u : 0u;
+                const uint32_t aw = t == 2 ? wlo : whi, bp = t == 1 ? plo : phi;
+                const uint64_t ad = tc::smem_desc(aw + ks * 2 * CMB, CMB, SBO);
+                const uint64_t bd0 = tc::smem_desc(bp + ks * 2 * CMB, CMB, SBO);
+                mma(tmem, ad, bd0, id0, acc);
+                if (nb1 > 0) {
+                  const uint64_t bd1 = tc::smem_desc(bp + (uint32_t)(nb0 / 8) * SBO + ks * 2 * CMB, CMB, SBO);
+                  mma(tmem + (uint32_t)nb0, ad, bd1, id1, acc);
+                }
               }
-            }
-          tc::commit(reinterpret_cast<uint64_t *>(&S.empty[s]));
-          issued = true;
-          nmma++;
-        } else {
-          bar_arrive(&S.empty[s]);
+            issued = any = true;
+            nmma++;
+          }
         }
+        if (any) tc::commit(reinterpret_cast<uint64_t *>(&S.empty[sr]));
+        else bar_arrive(&S.empty[sr]);
       }
       // every MMA issued by this thread has completed once `done` flips
       tc::commit(reinterpret_cast<uint64_t *>(&S.done));
@@ -712,8 +868,8 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
       S.issued = issued ? 1 : 0;
       if (nmma) atomicAdd(a.status + 2, nmma);   // chunks whose MMAs ran (executed-work counter)
       // no record copy may still be in flight when the CTA exits
-      for (int ch = n_loaded > NR ? n_loaded - NR : 0; ch < n_loaded; ch++)
-        if (!tc::mbar_wait(reinterpret_cast<uint64_t *>(&S.rfull[ch % NR]), (ch / NR) & 1)) S.fault = 1;
+      for (int rd = n_loaded > NRR ? n_loaded - NRR : 0; rd < n_loaded; rd++)
+        if (!tc::mbar_wait(reinterpret_cast<uint64_t *>(&S.rfull[rd % NRR]), (rd / NRR) & 1)) S.fault = 1;
     }
   }
   tc::fence_before();
@@ -721,27 +877,31 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
   tc::fence_after();
   const bool fault = S.fault != 0;
   const bool issued = S.issued != 0;
-  // per-column partial counts of observation quarters 1-3, in the (now idle)
+  // per-column partial counts of the observation groups, in the (now idle)
   // operand stage memory
-  int *dcand = reinterpret_cast<int *>(dsm), *dkept = dcand + 3 * TM;
-  float *drsum = reinterpret_cast<float *>(dkept + 3 * TM);
-  if (wid < NPW && wq > 0) {
-    dcand[(wq - 1) * TM + wc] = ncand;
-    dkept[(wq - 1) * TM + wc] = nkeep;
-    drsum[(wq - 1) * TM + wc] = rsum;
+  constexpr int NG = KC / 4;
+  int *dcand = reinterpret_cast<int *>(dsm), *dkept = dcand + NG * TM;
+  float *drsum = reinterpret_cast<float *>(dkept + NG * TM);
+  if (wid < NW) {
+    dcand[wq * TM + wc] = ncand;
+    dkept[wq * TM + wc] = nkeep;
+    drsum[wq * TM + wc] = rsum;
   }
   __syncthreads();
 
   // ---- per-column diagnostics and kept counts
-  int *ckept = reinterpret_cast<int *>(drsum + 3 * TM);   // kept by the column
+  int *ckept = reinterpret_cast<int *>(drsum + NG * TM);   // kept by the column
   if (tid < TM) {
-    for (int q = 0; q < 3; q++) {
-      ncand += dcand[q * TM + wc];
-      nkeep += dkept[q * TM + wc];
-      rsum += drsum[q * TM + wc];
+    ncand = dcand[tid];
+    nkeep = dkept[tid];
+    rsum = drsum[tid];
+    for (int q = 1; q < NG; q++) {
+      ncand += dcand[q * TM + tid];
+      nkeep += dkept[q * TM + tid];
+      rsum += drsum[q * TM + tid];
     }
-    ckept[wc] = nkeep;
-    const int col = a.tile_cols[(size_t)tile * TM + wc];
+    ckept[tid] = nkeep;
+    const int col = a.tile_cols[(size_t)tile * TM + tid];
     if (col >= 0 && pass == 0) {
       const size_t unit = (size_t)a.col2act[col] * G + g;
       if (wk.cblk < 0) {
@@ -750,7 +910,7 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
         if (a.diag_lg_obsloc) a.diag_lg_obsloc[(size_t)g * a.ncol + col] = rsum;
         if (g == 0 && a.diag_obscount) a.diag_obscount[col] = (float)ncand;
       } else {
-        float *cc = a.cnt + (((size_t)wk.cblk * G + g) * TM + wc) * 3;
+        float *cc = a.cnt + (((size_t)wk.cblk * G + g) * TM + tid) * 3;
         cc[0] = (float)nkeep;
         cc[1] = (float)ncand;
         cc[2] = rsum;
@@ -758,11 +918,11 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
     }
   }
   __syncthreads();
-  // ---- epilogue: warp w of the 16 reads TMEM lane quarter w % 4 and stores
-  // the features of quarter w / 4.  (On four warps alone it left the CTA's
+  // ---- epilogue: weight warp w reads TMEM lane quarter w % 4 and stores the
+  // features of quarter w / 4.  (On four warps alone it left the CTA's
   // other warps waiting: simple3d, k = 50, with the rows of columns that keep
   // nothing: 121 us for the whole kernel, now 21.)
-  if (wid < NPW) {
+  if (wid < NW) {
     if (wk.blk0 >= 0) {
       // the last drain interval of the segment
       store_block(wk.blk0 + nflush, issued && !fault, wid >> 2, 4);
@@ -779,6 +939,10 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
         } else {
 #pragma unroll
           for (int q = 0; q < 16; q++) v[q] = 0.0f;
+        }
+        if constexpr (F16) {
+#pragma unroll
+          for (int q = 0; q < 16; q++) v[q] *= oscale;
         }
         if (Gp) {
           if (f0 + 16 <= nvalid && (nf & 3) == 0) {
@@ -800,23 +964,18 @@ __global__ void __launch_bounds__(NT, 1) k_gram_tc(TcArgs a) {
   if (wid == 0) tc::tmem_dealloc(tmem, tmem_cols);
 }
 
-// Stage / ring depths: two operand stages and six record slots (k <= 128:
-// 2 x 70 KB + 6 x 10.8 KB).  At k = 40 they made the Gram 1.8 ms faster than
-// three stages with three slots (the producers waited on the record copies);
-// twelve slots gained nothing more.
-void gram_tc_config(int k, int np, int *ns, int *nr, size_t *smem) {
-  const size_t PB = (size_t)(np / 8) * SBO;
-  const size_t stage = 2 * WB + 2 * PB;
-  const size_t cb = record_bytes(k);
-
-  *ns = 2;
-  *nr = 6;
-  *smem = (size_t)*ns * stage + (size_t)*nr * cb;
+// Stage / ring depths: four FP16 or two TF32 operand stages (k <= 128: 4 x 36 KB
+// or 2 x 70 KB) and six record slots (10.8 KB).  With TF32 operands at k = 40
+// six slots made the Gram 1.8 ms faster than three stages with three slots (the
+// producers waited on the record copies); twelve slots gained nothing more.
+size_t gram_tc_smem(int k, int np, bool f16) {
+  const size_t PB = (size_t)(np / 8) * sbo_of(f16);
+  return stages_of(f16) * (2 * wb_of(f16) + 2 * PB) + NRMAX * record_bytes(k);
 }
 
 }  // namespace
 
-size_t tile_count_ints(int ntiles) { return (size_t)ntiles * (1 + WT / 32); }
+size_t tile_count_ints(int ntiles) { return (size_t)ntiles * (1 + WT / 32 + 2); }
 
 size_t record_bytes(int k) { return 512 + (size_t)(((k + 4) & ~3) * YS) * sizeof(float); }
 
@@ -831,10 +990,11 @@ void gram_tc_passes(int k, int *npass, int *np) {
 }
 
 cudaError_t launch_tile_count(cudaStream_t st, int ntiles, const TilePar *tp, const IndexGeom *geom,
-                              const ObsSorted &obs, int *tile_n, int *tile_wn, int *tile_off, int *launches) {
-  if (ntiles <= 0) return cudaMemsetAsync(tile_off, 0, sizeof(int), st);
-  k_tile_count<<<ntiles, WT, 0, st>>>(ntiles, tp, geom, obs.A, obs.cell_start, tile_n, tile_wn);
-  k_tile_scan<<<1, 1024, 0, st>>>(ntiles, tile_n, tile_off);
+                              const ObsSorted &obs, int *tile_n, int *tile_wn, uint32_t *tile_mag, int *tile_off,
+                              int *launches) {
+  if (ntiles <= 0) return cudaMemsetAsync(tile_off, 0, 2 * sizeof(int), st);
+  k_tile_count<<<ntiles, WT, 0, st>>>(ntiles, tp, geom, obs.A, obs.mag, obs.cell_start, tile_n, tile_wn, tile_mag);
+  k_tile_scan<<<1, 1024, 0, st>>>(ntiles, tile_n, tile_mag, tile_off);
   (*launches) += 2;
   return cudaGetLastError();
 }
@@ -850,27 +1010,27 @@ cudaError_t launch_tile_fill(cudaStream_t st, int ntiles, int nchunks, const Til
   return cudaGetLastError();
 }
 
-template <int LOC, bool CULL>
-static cudaError_t launch_gram_tc_c(cudaStream_t st, const TcArgs &a, size_t smem, long long grid) {
-  cudaError_t e = cudaFuncSetAttribute(k_gram_tc<LOC, 2, 6, CULL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)smem);
+template <int LOC, bool CULL, bool F16>
+static cudaError_t launch_gram_tc_loc(cudaStream_t st, const TcArgs &a, int *launches) {
+  const size_t smem = gram_tc_smem(a.k, a.np, F16);
+  if (smem > kSmemBudget) return cudaErrorInvalidValue;   // k <= 128 fits
+  const long long grid = (long long)a.nwork * a.groups * a.npass;
+  if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
+  auto kern = k_gram_tc<LOC, NRMAX, CULL, F16>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k_gram_tc<LOC, 2, 6, CULL><<<(int)grid, NT, smem, st>>>(a);
+  kern<<<(int)grid, gram_threads(a.np), smem, st>>>(a);
+  (*launches)++;
   return cudaGetLastError();
 }
 
 template <int LOC>
-static cudaError_t launch_gram_tc_loc(cudaStream_t st, const TcArgs &a, int *launches) {
-  int ns, nr;
-  size_t smem;
-  gram_tc_config(a.k, a.np, &ns, &nr, &smem);   // two stages, six record slots
-  (void)ns;
-  (void)nr;
-  if (smem > kSmemBudget) return cudaErrorInvalidValue;   // k <= 128 fits
-  const long long grid = (long long)a.nwork * a.groups * a.npass;
-  if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;
-  (*launches)++;
-  return a.cull ? launch_gram_tc_c<LOC, true>(st, a, smem, grid) : launch_gram_tc_c<LOC, false>(st, a, smem, grid);
+static cudaError_t launch_gram_tc_form(cudaStream_t st, const TcArgs &a, int *launches) {
+  if (a.f16)
+    return a.cull ? launch_gram_tc_loc<LOC, true, true>(st, a, launches)
+                  : launch_gram_tc_loc<LOC, false, true>(st, a, launches);
+  return a.cull ? launch_gram_tc_loc<LOC, true, false>(st, a, launches)
+                : launch_gram_tc_loc<LOC, false, false>(st, a, launches);
 }
 
 cudaError_t launch_gram_tc(cudaStream_t st, const TcArgs &a_in, int *launches) {
@@ -881,9 +1041,9 @@ cudaError_t launch_gram_tc(cudaStream_t st, const TcArgs &a_in, int *launches) {
   while ((int)tc < a.np) tc <<= 1;
   a.tmem_cols = tc;
   switch (a.loc.cls) {
-  case LOC_OCEAN: return launch_gram_tc_loc<LOC_OCEAN>(st, a, launches);
-  case LOC_VTGC: return launch_gram_tc_loc<LOC_VTGC>(st, a, launches);
-  default: return launch_gram_tc_loc<LOC_NOVRT>(st, a, launches);
+  case LOC_OCEAN: return launch_gram_tc_form<LOC_OCEAN>(st, a, launches);
+  case LOC_VTGC: return launch_gram_tc_form<LOC_VTGC>(st, a, launches);
+  default: return launch_gram_tc_form<LOC_NOVRT>(st, a, launches);
   }
 }
 
@@ -979,8 +1139,10 @@ static cudaError_t preload_gram_tc_loc() {
   cudaFuncAttributes fa;
   cudaError_t e = cudaSuccess;
   auto get = [&](const void *f) { if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, f); };
-  get((const void *)k_gram_tc<LOC, 2, 6, false>);
-  get((const void *)k_gram_tc<LOC, 2, 6, true>);
+  get((const void *)k_gram_tc<LOC, NRMAX, false, false>);
+  get((const void *)k_gram_tc<LOC, NRMAX, true, false>);
+  get((const void *)k_gram_tc<LOC, NRMAX, false, true>);
+  get((const void *)k_gram_tc<LOC, NRMAX, true, true>);
   get((const void *)k_tile_count);
   get((const void *)k_tile_scan);
   get((const void *)k_tile_list);

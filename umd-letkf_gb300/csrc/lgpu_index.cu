@@ -312,10 +312,19 @@ __global__ void __launch_bounds__(32 * GW) k_place(int nobs, int k, int kp, cons
   r = __reduce_add_sync(0xffffffffu, r);
   const size_t q = (size_t)(b + r);
   const float *src = hx + (size_t)i * k;
-  for (int m = lane; m < kp; m += 32) o.hx[q * kp + m] = m < k ? src[m] : 0.0f;
-  if (lane == 0) o.A[q] = Atmp[i];
-  if (lane == 1) o.B[q] = Btmp[i];
+  unsigned ymax = 0;   // bits of the largest |y| (NaN above all)
+  for (int m = lane; m < kp; m += 32) {
+    const float y = m < k ? src[m] : 0.0f;
+    ymax = max(ymax, __float_as_uint(fabsf(y)));
+    o.hx[q * kp + m] = y;
+  }
+  ymax = __reduce_max_sync(0xffffffffu, ymax);
+  const float4 A = Atmp[i], B = Btmp[i];
+  if (lane == 0) o.A[q] = A;
+  if (lane == 1) o.B[q] = B;
   if (lane == 2) o.idx[q] = i;
+  // the largest feature of the observation over its error
+  if (lane == 3) o.mag[q] = __uint_as_float(ymax) / A.w * __uint_as_float(max(ymax, __float_as_uint(fabsf(B.x))));
 }
 
 }  // namespace

@@ -377,6 +377,7 @@ struct ObsSorted {
   float *hx;       // [nobs][KP] perturbations, zero padded
   int *idx;        // original observation index
   int *cell_start; // [ncell + 1]
+  float *mag = nullptr;   // largest feature |y_i| max(|y_j|, |dep|) over the error (batched Gram's scale)
 };
 
 // The local-observation search of one (column, group), the threads of a
@@ -513,6 +514,8 @@ struct TcArgs {
   const unsigned char *rec;  // tile candidate streams (chunk records)
   const int *tile_off;       // [ntiles + 1] first chunk of each tile's stream
   const int *tile_n;         // [ntiles] candidates of each tile
+  const uint32_t *tile_mag;  // [ntiles][2] bits of the largest and smallest positive magnitude of a tile's candidates
+  bool f16;                  // FP16 operands (every tile's magnitudes within range)
   int cb;                    // bytes per chunk record (set by the launcher)
   uint32_t tmem_cols;        // TMEM columns per CTA (set by the launcher)
   // accumulation segments and drains: each tile's chunk stream is split into
@@ -544,9 +547,11 @@ cudaError_t launch_tile_prep(cudaStream_t st, int ntiles, const int *tile_cols, 
 // streams' observations (16 per chunk) and the records (record_bytes(k) per
 // chunk of 16)
 size_t record_bytes(int k);
-size_t tile_count_ints(int ntiles);   // tile_n and, behind its ntiles ints, tile_wn
+size_t tile_count_ints(int ntiles);   // tile_n and, behind its ntiles ints, tile_wn, then tile_mag
+// tile_off[ntiles + 1]: whether a tile's magnitudes need the TF32 operands
 cudaError_t launch_tile_count(cudaStream_t st, int ntiles, const TilePar *tp, const IndexGeom *geom,
-                              const ObsSorted &obs, int *tile_n, int *tile_wn, int *tile_off, int *launches);
+                              const ObsSorted &obs, int *tile_n, int *tile_wn, uint32_t *tile_mag, int *tile_off,
+                              int *launches);
 cudaError_t launch_tile_fill(cudaStream_t st, int ntiles, int nchunks, const TilePar *tp, const IndexGeom *geom,
                              const ObsSorted &obs, int k, int kp, const int *tile_n, const int *tile_wn,
                              const int *tile_off, int *list, unsigned char *rec, int *status, int *launches);
