@@ -22,7 +22,7 @@ def _analysis(prob, variant):
 
 # half of the globe's observations with their perturbations and departures times
 # `scale` and their errors times `err` (largest feature over error: scale^2 / err)
-@pytest.mark.parametrize("k", [20, 37, 40])   # one and several feature passes, ragged rows
+@pytest.mark.parametrize("k", [20, 29, 37, 40, 60])   # one to four feature passes, ragged rows
 @pytest.mark.parametrize("scale,err", [
     (1.0, 1.0),
     (2.0 ** -6, 1.0),              # 2^-12: within FP16's range

@@ -11,7 +11,7 @@
 //                                                = y_i(o) * dep(o)   f = (i, rhs)
 //
 // M = 128 columns, N = the k(k+3)/2 packed features (split into passes of at
-// most 432 so the accumulator fits TMEM), K = candidate observations in
+// most 480 so the accumulator fits TMEM), K = candidate observations in
 // chunks of 16.
 //
 // Candidate streams.  Before the GEMM, four small kernels turn each tile's
@@ -70,7 +70,10 @@ namespace {
 
 constexpr int TM = 128;        // columns per tile = MMA M = TMEM lanes
 constexpr int KC = 16;         // observations per chunk (one FP16 or two TF32 MMA steps)
-constexpr int NPMAX = 432;     // features per pass
+// Features per pass: 15 feature warps, 1,024 threads.  At 432 (14 warps) k = 28,
+// 29, 52, 60 or 100 took a pass more, with its weights: Gram of 240 x 120
+// clustered columns, k = 29 0.244 ms, now 0.189; k = 60 0.756, now 0.684.
+constexpr int NPMAX = 480;
 constexpr int NW = 16;         // weight warps; then the feature warps (one per 32 features), then the MMA warp
 __host__ __device__ constexpr int feature_warps(int np) { return (np + 31) / 32; }
 __host__ __device__ constexpr int gram_threads(int np) { return 32 * (NW + feature_warps(np) + 1); }
