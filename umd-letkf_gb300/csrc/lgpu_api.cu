@@ -1868,7 +1868,7 @@ int lgpu_learn_init(lgpu_handle *h, const lgpu_learn_config *cfg) {
       {&L->Pg, 4 * L->nparam}, {&L->Wt, mlp_tiled_weight_bytes(S)},
       {&L->mu_in, 4 * (size_t)S.din}, {&L->sd_in, 4 * (size_t)S.din}, {&L->mu_out, 4 * (size_t)S.dout},
       {&L->sd_out, 4 * (size_t)S.dout},
-      {&L->feat, 64 * (size_t)nf}, {&L->nkf, 4 * (size_t)nf}, {&L->X, 4 * (size_t)nf * S.din},
+      {&L->feat, 64 * (size_t)nf}, {&L->nkf, 4 * (size_t)nf},
       {&L->Xt, rows_pad * (size_t)S.k1 * 2}, {&L->H1, mlp_act_bytes(S, nf)}, {&L->H2, mlp_act_bytes(S, nf)},
       {&L->Yn, 4 * (size_t)nf * S.dout}, {&L->flag, 4 * (size_t)nf}, {&L->gate, 4 * (size_t)nf}, {&L->gate_n, 16},
       {&L->jacc, 16},

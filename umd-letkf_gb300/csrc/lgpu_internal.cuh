@@ -661,7 +661,7 @@ struct LrnInterpArgs {
   const int *src_of_col;      // [ncol] row of the coarse solution or -1
   const float *feat;          // [nfine][16] (0..9 from k_lrn_obsfeat)
   const float *lat;
-  const float *mu, *sd;       // input standardisation [din], or null (raw rows)
+  const float *mu, *sd;       // lrn_input: input standardisation [din]
   float *X;                   // [nfine][din] network input rows (row f at X + f * ldx)
   long long ldx;
   int *flag;                  // [nfine] 1 = a coarse neighbour has no solution

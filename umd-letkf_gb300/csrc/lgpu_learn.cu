@@ -13,9 +13,11 @@
 //                  nearest distance, innovation moments) from per-cell
 //                  aggregates of the observation index and the same
 //                  localizer as the exact path
-//   k_lrn_interp   per column: the bilinear (W, w-bar) of the four coarse
-//                  neighbours, the network input row and, while collecting
-//                  training data, the residual target exact - interpolated
+//   k_lrn_interp   per column, while collecting training data: the bilinear
+//                  (W, w-bar) of the four coarse neighbours as a raw input
+//                  row, and the residual target exact - interpolated
+//   k_lrn_input    per column: the same inputs standardised, as BF16 in the
+//                  network's tiled order
 //   k_lrn_apply    per column: interpolation + de-standardised correction ->
 //                  T = W + w-bar 1^T, the gate score, the fallback list
 //   k_lrn_judge, k_lrn_scatter  judge errors; exact transforms into place
@@ -219,7 +221,7 @@ __device__ __forceinline__ float geometry_feature(const LrnInterpArgs &a, int f,
   return sqrtf(spread) / (float)a.k;
 }
 
-// raw rows for the training store (and, with mu, standardised FP32 rows)
+// raw rows for the training store
 __global__ void __launch_bounds__(FT) k_lrn_interp(LrnInterpArgs a) {
   __shared__ float red[4];
   const int f = blockIdx.x;
@@ -241,7 +243,7 @@ __global__ void __launch_bounds__(FT) k_lrn_interp(LrnInterpArgs a) {
         spread += nb.w[q] * d * d;
       }
     }
-    x[e] = a.mu ? (v - a.mu[e]) / a.sd[e] : v;
+    x[e] = v;
     if (a.Yt) {
       const int act = a.col2act[col];
       const float ex = a.wex[(size_t)act * k + i];
@@ -254,7 +256,7 @@ __global__ void __launch_bounds__(FT) k_lrn_interp(LrnInterpArgs a) {
     const int q = threadIdx.x;
     const float v = geometry_feature(a, f, col, nb, spread, q);
     const int e = kk + k + q;
-    x[e] = a.mu ? (v - a.mu[e]) / a.sd[e] : v;
+    x[e] = v;
   }
   if (threadIdx.x == 0) a.flag[f] = nb.missing;
 }
