@@ -298,7 +298,13 @@ int lgpu_get_obslist_noalloc(lgpu_handle *h, int ij, int group, int *idx, float 
  * moments, position in the coarse cell, neighbour spread) to a correction
  * of (W, w-bar): layers din -> hidden -> hidden -> dout, GELU, BF16 weights
  * and activations with FP32 accumulation; inference on the tensor cores
- * (tcgen05 kind::f16), training on the CUDA cores (Adam). */
+ * (tcgen05 kind::f16), training on the CUDA cores (Adam).
+ *
+ * What lgpu_learn_init makes holds for its ensemble size, its active columns
+ * and loc_novrt: a learned analysis or lgpu_learn_collect under another
+ * localizer class is LGPU_ERR_UNSUPPORTED, after a change of the ensemble size
+ * or of the active columns LGPU_ERR_ORDER (new radii or coordinates are
+ * taken as they come). */
 typedef struct lgpu_learn_config {
   int nx, ny;            /* lattice */
   int stride;            /* coarse lattice stride (>= 2) */

@@ -156,6 +156,8 @@ struct lgpu_handle {
 };
 
 static void learn_free(lgpu_handle *h);
+static void learn_retune(lgpu_handle *h);
+static int learn_new_grid(lgpu_handle *h, const float *lat, const float *lon);
 
 namespace {
 
@@ -413,6 +415,8 @@ int lgpu_loc_init(lgpu_handle *h, const lgpu_loc_config *c) {
     return fail(h, LGPU_ERR_UNSUPPORTED_LOCALIZER, "localizer class " + cls + " not found.");
   }
   if (L.groups <= 0) return fail(h, LGPU_ERR_CONFIG, "localizer class needs to properly define 'maxgroups'");
+  // (the learned form runs on loc_novrt alone, whose only parameters are the table's)
+  if (L.cls != h->loc.cls || std::memcmp(&L.hz, &h->loc.hz, sizeof(L.hz)) != 0) learn_retune(h);
   h->loc = L;
   h->loc_ok = true;
   h->auto_choice = 0;
@@ -483,7 +487,7 @@ int lgpu_set_grid(lgpu_handle *h, int nij, const float *lat, const float *lon, c
   h->h_col2act = c2a;
   h->grid_ok = true;
   h->ran = false;
-  return LGPU_OK;
+  return learn_new_grid(h, lat, lon);
 }
 
 namespace {
@@ -1764,6 +1768,11 @@ struct LearnState {
   // for them (0 = not yet measured) and its producers
   DevBuf tcols, tpar, tn, toff;
   int ntiles = 0, gram_choice = 0, cull = -1;
+  // what the buffers, the network and the lattice were made for
+  int k = 0;
+  std::vector<int> col2act;
+  std::vector<float> lat, lon;   // the grid of the lattice's tiles
+  bool grid_same = true;         // the handle's active columns are these
   long long nstore = 0;
   long long hold0 = 0;     // first row of the last collected analysis (held out from training when ncollect >= 2)
   int ncollect = 0;
@@ -1788,6 +1797,54 @@ static void learn_free(lgpu_handle *h) {
   for (auto &e : L->ev) if (e) cudaEventDestroy(e);
   delete L;
   h->learn = nullptr;
+}
+
+// the Gram form measured for the lattice holds for one localizer and grid
+static void learn_retune(lgpu_handle *h) {
+  if (!h->learn) return;
+  h->learn->gram_choice = 0;
+  h->learn->cull = -1;
+}
+
+// the lattice's columns in tiles (of the coordinates in L->lat, L->lon)
+static int learn_tiles(lgpu_handle *h) {
+  LearnState *L = h->learn;
+  const std::vector<int> tiles = build_tiles(L->coarse, L->lat.data(), L->lon.data());
+  L->ntiles = (int)(tiles.size() / 128);
+  const size_t nt = std::max(1, L->ntiles);
+  CK(L->tcols.ensure(512 * nt), "alloc tiles");
+  CK(L->tpar.ensure(sizeof(TilePar) * nt), "alloc tiles");
+  CK(L->tn.ensure(4 * tile_count_ints((int)nt)), "alloc tiles");
+  CK(L->toff.ensure(4 * (nt + 2)), "alloc tiles");
+  if (!tiles.empty()) CK(cudaMemcpy(L->tcols.p, tiles.data(), 4 * tiles.size(), cudaMemcpyHostToDevice), "H2D tiles");
+  return LGPU_OK;
+}
+
+// After lgpu_set_grid.  The columns' roles, and the rows of every buffer,
+// follow the active columns: with others the learned form is refused until
+// the next lgpu_learn_init (learn_check).  Moved columns keep their roles.
+static int learn_new_grid(lgpu_handle *h, const float *lat, const float *lon) {
+  LearnState *L = h->learn;
+  if (!L) return LGPU_OK;
+  L->grid_same = h->h_col2act == L->col2act;
+  if (!L->grid_same ||
+      (std::equal(L->lat.begin(), L->lat.end(), lat) && std::equal(L->lon.begin(), L->lon.end(), lon)))
+    return LGPU_OK;
+  L->lat.assign(lat, lat + h->ncol);
+  L->lon.assign(lon, lon + h->ncol);
+  learn_retune(h);
+  return learn_tiles(h);
+}
+
+// The learned form runs on what lgpu_learn_init was given: its buffers hold one
+// row per active column for that ensemble size, and one group.
+static int learn_check(lgpu_handle *h) {
+  const LearnState *L = h->learn;
+  if (h->loc.cls != LOC_NOVRT || h->loc.groups != 1)
+    return fail(h, LGPU_ERR_UNSUPPORTED, "the learned form supports loc_novrt (one group per column) only");
+  if (h->k != L->k) return fail(h, LGPU_ERR_ORDER, "the ensemble size changed since learn_init");
+  if (!L->grid_same) return fail(h, LGPU_ERR_ORDER, "the grid's active columns changed since learn_init");
+  return LGPU_OK;
 }
 
 namespace {
@@ -1825,7 +1882,14 @@ int lgpu_learn_init(lgpu_handle *h, const lgpu_learn_config *cfg) {
   learn_free(h);
   LearnState *L = new LearnState();
   h->learn = L;
+  // a failure below leaves no half-made state behind
+  struct Undo {
+    lgpu_handle *h;
+    ~Undo() { if (h) learn_free(h); }
+  } undo{h};
   L->cfg = *cfg;
+  L->k = h->k;
+  L->col2act = h->h_col2act;
   const int k = h->k, nx = cfg->nx, ny = cfg->ny, s = cfg->stride;
   L->shape.din = k * k + k + 16;
   L->shape.k1 = (L->shape.din + 15) & ~15;
@@ -1884,19 +1948,12 @@ int lgpu_learn_init(lgpu_handle *h, const lgpu_learn_config *cfg) {
     for (int i = 0; i < k; i++) w[(size_t)k * k + i] = (float)k;
     CK(cudaMemcpy(L->wout.p, w.data(), 4 * w.size(), cudaMemcpyHostToDevice), "H2D loss weights");
   }
-  {
-    std::vector<float> lat(h->ncol), lon(h->ncol);
-    CK(cudaMemcpy(lat.data(), h->buf[B_LAT].p, 4 * (size_t)h->ncol, cudaMemcpyDeviceToHost), "D2H lat");
-    CK(cudaMemcpy(lon.data(), h->buf[B_LON].p, 4 * (size_t)h->ncol, cudaMemcpyDeviceToHost), "D2H lon");
-    const std::vector<int> tiles = build_tiles(L->coarse, lat.data(), lon.data());
-    L->ntiles = (int)(tiles.size() / 128);
-    const size_t nt = std::max(1, L->ntiles);
-    CK(L->tcols.ensure(512 * nt), "alloc tiles");
-    CK(L->tpar.ensure(sizeof(TilePar) * nt), "alloc tiles");
-    CK(L->tn.ensure(4 * tile_count_ints((int)nt)), "alloc tiles");
-    CK(L->toff.ensure(4 * (nt + 2)), "alloc tiles");
-    if (!tiles.empty()) CK(cudaMemcpy(L->tcols.p, tiles.data(), 4 * tiles.size(), cudaMemcpyHostToDevice), "H2D tiles");
-  }
+  L->lat.resize(h->ncol);
+  L->lon.resize(h->ncol);
+  CK(cudaMemcpy(L->lat.data(), h->buf[B_LAT].p, 4 * (size_t)h->ncol, cudaMemcpyDeviceToHost), "D2H lat");
+  CK(cudaMemcpy(L->lon.data(), h->buf[B_LON].p, 4 * (size_t)h->ncol, cudaMemcpyDeviceToHost), "D2H lon");
+  int rc = learn_tiles(h);
+  if (rc != LGPU_OK) return rc;
   for (auto &e : L->ev) CK(cudaEventCreate(&e), "event");
   CK(cudaMemcpyAsync(L->d_fine.p, L->fine_ok.data(), 4 * L->fine_ok.size(), cudaMemcpyHostToDevice, h->st), "H2D");
   CK(cudaMemcpyAsync(L->d_rank.p, L->rank.data(), 4 * (size_t)h->ncol, cudaMemcpyHostToDevice, h->st), "H2D");
@@ -1924,6 +1981,7 @@ int lgpu_learn_init(lgpu_handle *h, const lgpu_learn_config *cfg) {
   L->st.coarse = (int)L->coarse.size();
   L->st.fallback = (int)L->fine_miss.size();
   L->st.tau = L->tau;
+  undo.h = nullptr;
   return LGPU_OK;
 }
 
@@ -1973,6 +2031,8 @@ int lgpu_learn_collect(lgpu_handle *h, long long *rows) {
   if (!h->learn) return fail(h, LGPU_ERR_ORDER, "learn_collect before learn_init");
   LearnState *L = h->learn;
   if (h->bound_state) return fail(h, LGPU_ERR_UNSUPPORTED, "learn_collect with a bound state");
+  int rc = learn_check(h);
+  if (rc != LGPU_OK) return rc;
   const int k = h->k;
   const MlpShape &S = L->shape;
   // the exact analysis, with the mean weights of every unit
@@ -1980,7 +2040,7 @@ int lgpu_learn_collect(lgpu_handle *h, long long *rows) {
   if (variant == LGPU_VARIANT_LEARNED) h->variant = LGPU_VARIANT_AUTO;
   CK(h->learn->wbar_all.ensure(4 * (size_t)std::max(1, h->nact) * k), "alloc");
   h->learn_wbar = L->wbar_all.as<float>();
-  int rc = lgpu_solver_run(h);
+  rc = lgpu_solver_run(h);
   h->learn_wbar = nullptr;
   h->variant = variant;
   if (rc != LGPU_OK) return rc;
@@ -2247,10 +2307,12 @@ static int learned_run(lgpu_handle *h) {
   if (!L) return fail(h, LGPU_ERR_ORDER, "LEARNED variant before learn_init");
   if (!L->trained) return fail(h, LGPU_ERR_ORDER, "LEARNED variant before learn_train");
   if (h->bound_state) return fail(h, LGPU_ERR_UNSUPPORTED, "the LEARNED variant with a bound state");
+  int rc = learn_check(h);
+  if (rc != LGPU_OK) return rc;
   ObsSorted os;
   int launches = 0;
   const TileSet lat_tiles{L->ntiles, &L->tcols, &L->tpar, &L->tn, &L->toff};
-  int rc = prepare_run(h, os, launches, L->gram_choice == LGPU_VARIANT_PLAIN ? nullptr : &lat_tiles);
+  rc = prepare_run(h, os, launches, L->gram_choice == LGPU_VARIANT_PLAIN ? nullptr : &lat_tiles);
   if (rc != LGPU_OK) return rc;
   if ((rc = flag_prepare(h)) != LGPU_OK) return rc;
   cudaStream_t st = h->st;
