@@ -205,6 +205,10 @@ int lgpu_set_variant(lgpu_handle *h, int variant);   /* no reference counterpart
 #define LGPU_PREC_FP64 2
 int lgpu_set_precision(lgpu_handle *h, int mode, float gap_threshold);
 
+/* A run needs a state of the grid's size and observations of the state's
+ * ensemble size: after lgpu_set_grid with another number of columns the state
+ * has to be set again, after a change of the ensemble size the observations
+ * (LGPU_ERR_ORDER). */
 int lgpu_set_grid(lgpu_handle *h, int nij, const float *lat, const float *lon, const int *mask);
 int lgpu_set_state(lgpu_handle *h, int k, int ns, const float *state, const float *mean,
                    const float *sprd, int nvars, const lgpu_statevar *vars);

@@ -127,6 +127,7 @@ struct lgpu_handle {
   int k = 0, ns = 0, kp = 0;
   std::vector<lgpu_statevar> vars;
   int nobs = 0;
+  int state_ncol = 0, obs_k = 0;   // columns of the state, members of the observations as they were given
   IndexGeom geom{};
   int ncell = 0;
   int nunits = 0;
@@ -545,6 +546,7 @@ int prepare_state(lgpu_handle *h, int k, int ns, const float *state, const float
   h->k = k;
   h->ns = ns;
   h->kp = (k + 3) & ~3;
+  h->state_ncol = h->ncol;
   h->vars.assign(vars, vars + nvars);
   return LGPU_OK;
 }
@@ -613,6 +615,7 @@ int lgpu_set_obs(lgpu_handle *h, int nobs, const lgpu_obs *o, const float *hx, c
     return fail(h, LGPU_ERR_ARG, "set_obs: bad arguments");
   for (int i = 0; i < nobs; i++)
     if (!(o->err[i] > 0.0f)) return fail(h, LGPU_ERR_ARG, "set_obs: observation error must be > 0 at obs " + std::to_string(i));
+  h->obs_ok = false;
   CK(cudaSetDevice(h->device), "cudaSetDevice");
   const auto t_host = std::chrono::steady_clock::now();
   const size_t n = std::max(nobs, 1), k = h->k;
@@ -635,6 +638,7 @@ int lgpu_set_obs(lgpu_handle *h, int nobs, const lgpu_obs *o, const float *hx, c
   CK(cudaEventElapsedTime(&h->obs_h2d_ms, h->ev_obs[0], h->ev_obs[1]), "timing");
   h->obs_host_ms = std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t_host).count();
   h->nobs = nobs;
+  h->obs_k = h->k;
   h->obs_ok = true;
   h->ran = false;
   return LGPU_OK;
@@ -651,6 +655,7 @@ int lgpu_set_obs_raw(lgpu_handle *h, int nobs, const lgpu_obs *o, const int *qc,
   for (int i = 0; i < nobs; i++)
     if ((!qc || qc[i] <= 0) && !(o->err[i] > 0.0f))
       return fail(h, LGPU_ERR_ARG, "set_obs_raw: observation error must be > 0 at obs " + std::to_string(i));
+  h->obs_ok = false;
   CK(cudaSetDevice(h->device), "cudaSetDevice");
   const size_t n = std::max(nobs, 1), k = h->k;
   const int raw[8] = {B_RAW0, B_RAW1, B_RAW2, B_RAW3, B_RAW4, B_RAW5, B_RAW6, B_RAW7};
@@ -693,6 +698,7 @@ int lgpu_set_obs_raw(lgpu_handle *h, int nobs, const lgpu_obs *o, const int *qc,
   CK(cudaStreamSynchronize(h->st), "set_obs_raw");
   h->nobs = kept;
   if (nobs_kept) *nobs_kept = kept;
+  h->obs_k = h->k;
   h->obs_ok = true;
   h->ran = false;
   return LGPU_OK;
@@ -709,6 +715,7 @@ int lgpu_set_state_members(lgpu_handle *h, int k, int ns, const float *members, 
 int lgpu_get_background(lgpu_handle *h, float *state, float *mean, float *sprd) {
   if (!h) return LGPU_ERR_ARG;
   if (!h->state_ok) return fail(h, LGPU_ERR_ORDER, "get_background before set_state");
+  if (h->state_ncol != h->ncol) return fail(h, LGPU_ERR_ORDER, "the state was set for a grid of another size");
   CK(cudaSetDevice(h->device), "cudaSetDevice");
   const size_t nx = (size_t)h->ncol * h->ns * h->k, nm = (size_t)h->ncol * h->ns;
   if (state) CK(cudaMemcpyAsync(state, h->buf[B_BKG].p, nx * 4, cudaMemcpyDeviceToHost, h->st), "D2H");
@@ -721,6 +728,7 @@ int lgpu_get_background(lgpu_handle *h, float *state, float *mean, float *sprd) 
 int lgpu_get_obs_prepared(lgpu_handle *h, float *hx, float *hx_mean, float *lat, float *lon, float *val, float *err) {
   if (!h) return LGPU_ERR_ARG;
   if (!h->obs_ok) return fail(h, LGPU_ERR_ORDER, "get_obs_prepared before set_obs");
+  if (hx && h->nobs > 0 && h->obs_k != h->k) return fail(h, LGPU_ERR_ORDER, "the observations were set for another ensemble size");
   CK(cudaSetDevice(h->device), "cudaSetDevice");
   const size_t n = h->nobs, k = h->k;
   if (n > 0) {
@@ -748,6 +756,9 @@ static int prepare_run(lgpu_handle *h, ObsSorted &os, int &launches, const TileS
   if (!h->solver_ok) return fail(h, LGPU_ERR_ORDER, "solver_run before solver_init");
   if (!h->loc_ok) return fail(h, LGPU_ERR_ORDER, "solver_run before loc_init");
   if (!h->grid_ok || !h->state_ok || !h->obs_ok) return fail(h, LGPU_ERR_ORDER, "solver_run before grid/state/obs were set");
+  // the buffers have the sizes their calls found
+  if (h->state_ncol != h->ncol) return fail(h, LGPU_ERR_ORDER, "the state was set for a grid of another size");
+  if (h->nobs > 0 && h->obs_k != h->k) return fail(h, LGPU_ERR_ORDER, "the observations were set for another ensemble size");
   CK(cudaSetDevice(h->device), "cudaSetDevice");
   const int k = h->k, kp = h->kp, ns = h->ns, G = h->loc.groups;
   if (h->loc.cls == LOC_OCEAN && h->loc.vtloc_surf == 1) {
