@@ -2067,6 +2067,9 @@ int lgpu_learn_collect(lgpu_handle *h, long long *rows) {
   if (n > 0) {
     cudaStream_t st = h->st;
     int launches = 0;
+    CK(lrn_identity(st, h->nunits, k, h->buf[B_NKEPT].as<int>(), h->buf[B_T].as<float>(), L->wbar_all.as<float>(),
+                    &launches),
+       "transforms without observations");
     CK(L->ecols.ensure(4 * (size_t)std::max(n, std::max(1, h->nact))), "alloc");
     CK(cudaMemcpyAsync(L->ecols.p, sample.data(), 4 * (size_t)n, cudaMemcpyHostToDevice, st), "H2D sample");
     CK(L->feat.ensure(64 * (size_t)n), "alloc");
@@ -2304,6 +2307,7 @@ static int learned_exact(lgpu_handle *h, const ObsSorted &os, int n, bool lattic
   EigSplit sp;
   int batch = 0;
   if ((rc = eig_scratch(h, n, ea, sp, batch)) != LGPU_OK) return rc;
+  CK(lrn_identity(st, n, k, ea.nkept, ea.T, ea.wbar, &launches), "transforms without observations");
   if (h->prec == LGPU_PREC_FP64) {
     CK(launch_eig64(st, ea, 0, &launches), "FP64 eigen kernel");
     return LGPU_OK;
