@@ -230,6 +230,8 @@ struct Grid {
   // columns' vectors would start in the same banks
   static constexpr int CP4 = (CN + 3) / 4 * 4;
   static constexpr int CP = LB > 1 && CP4 % (64 / LB) == 0 ? CP4 + 4 : CP4;
+  static constexpr int NV = (CN + 3) / 4;                   // vectors of a lane's column pairs (CP may hold one more)
+  static_assert(2 * (NV - 1) < CH2, "every vector holds a column pair of the lane");
   static constexpr int VB = LB * CP;                        // one column-ordered vector
   static constexpr int NP = sizeof(R) == 4 ? 16 : 32;
   static constexpr int KM = KR > KC ? KR : KC;
@@ -279,7 +281,7 @@ template <class G, int Q0, class R>
 __device__ __forceinline__ void load_cols(const R *buf, int b, Pair<R> *v) {
   const R *p = buf + b * G::CP;
 #pragma unroll
-  for (int q = Q0 / 2; q < G::CP / 4; q++) {
+  for (int q = Q0 / 2; q < G::NV; q++) {
     Pair<R> t[2];
     ld2(p + 4 * q, t);
 #pragma unroll
@@ -310,7 +312,7 @@ template <class G, int Q0, class R>
 __device__ __forceinline__ void store_cols(R *buf, int b, const Pair<R> *v) {
   R *p = buf + b * G::CP;
 #pragma unroll
-  for (int q = Q0 / 2; q < G::CP / 4; q++)
+  for (int q = Q0 / 2; q < G::NV; q++)
     st2(p + 4 * q, v[2 * q], 2 * q + 1 < G::CH2 ? v[2 * q + 1] : Pair<R>(R(0), R(0)));
 }
 
@@ -419,7 +421,7 @@ __device__ __forceinline__ void two_sided(typename G::Row (&A)[G::RN], typename 
     }
     const R *wp = wb + b * G::CP, *vp = vb + b * G::CP;
 #pragma unroll
-    for (int q = C0 / 2; q < G::CP / 4; q++) {
+    for (int q = C0 / 2; q < G::NV; q++) {
       P2 wc[2], vc[2];
       ld2(wp + 4 * q, wc);
       if (!G::KEEP && q >= Q0 / 2) ld2(vp + 4 * q, vc);
