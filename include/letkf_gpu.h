@@ -464,6 +464,12 @@ int lgpu_debug_weight(lgpu_handle *h, int n, const float *lat1, const float *lon
  * FP64-solved unit count in fp64_units (the other fields are not set). */
 int lgpu_debug_transform(lgpu_handle *h, int nunits, int k, const float *gram, float *trans);
 
+/* Verification of the ways round a full device: the work buffers of this
+ * handle's following runs that have such a way (transform scratch, the batched
+ * Gram's streams and partial blocks) fail to allocate above `bytes`; 0: no
+ * limit. */
+int lgpu_debug_alloc_limit(lgpu_handle *h, size_t bytes);
+
 #ifdef __cplusplus
 }
 #endif

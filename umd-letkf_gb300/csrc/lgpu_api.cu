@@ -151,6 +151,7 @@ struct lgpu_handle {
   int prec = LGPU_PREC_FP32;   // eigensolve precision mode
   float gap_thresh = 1e-6f;    // FP32_RESOLVE: relative eigenvalue gap that sends a unit to FP64
   DevBuf buf[B_COUNT_ALL];
+  size_t alloc_limit = 0;      // work buffers above this many bytes fail to allocate (0: no limit)
   lgpu_timings tim{};
   LearnState *learn = nullptr;      // learned form, after lgpu_learn_init
   float *learn_wbar = nullptr;      // mean weights of every unit while training rows are collected
@@ -181,6 +182,14 @@ int cuda_fail(lgpu_handle *h, cudaError_t e, const char *what) {
     cudaError_t _e = (call);                             \
     if (_e != cudaSuccess) return cuda_fail(h, _e, what); \
   } while (0)
+
+// work buffers whose size follows the run, with a way round where the device
+// has no room for them
+cudaError_t work_alloc(lgpu_handle *h, int b, size_t bytes) {
+  cudaError_t e = h->alloc_limit > 0 && bytes > h->alloc_limit ? cudaErrorMemoryAllocation : h->buf[b].ensure(bytes);
+  if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();
+  return e;
+}
 
 std::string upper(const char *s) {
   std::string r(s ? s : "");
@@ -907,22 +916,25 @@ static void flag_args(lgpu_handle *h, EigArgs &ea) {
   ea.flag_cap = 2 * std::max(1, h->nunits);
 }
 
+constexpr int kFewUnits = 32;   // units in flight that a run needs room for
+
 // scratch of the transforms of `units` units: the reflectors of the units in
-// flight, and with FP32_RESOLVE the gap test (at most 8 GB, units in batches)
+// flight, and with FP32_RESOLVE the gap test (at most 8 GB, units in batches).
+// Where the device has less, fewer units at a time: the same results.
 static int eig_scratch(lgpu_handle *h, int units, EigArgs &ea, EigSplit &sp, int &batch) {
   sp = EigSplit{};
-  batch = std::max(1, units);
   const int k = h->k;
   const bool resolve = h->prec == LGPU_PREC_FP32_RESOLVE;
-  const size_t vb = eig_scratch_bytes(k, std::max(1, units), h->prec != LGPU_PREC_FP64, h->prec != LGPU_PREC_FP32);
-  size_t need = vb + 256;
-  if (resolve) {
-    const size_t per = eig_split_bytes_per_unit(k);
-    const size_t budget = (size_t)8 << 30;
-    batch = (int)std::min<size_t>((size_t)batch, std::max<size_t>(1024, budget / per));
-    need += per * (size_t)batch + 2 * 256;
+  const size_t per = eig_split_bytes_per_unit(k), budget = (size_t)8 << 30;
+  size_t vb = 0;
+  for (int n = std::max(1, units);; n = (n + 1) / 2) {
+    vb = eig_scratch_bytes(k, n, h->prec != LGPU_PREC_FP64, h->prec != LGPU_PREC_FP32);
+    batch = (int)std::min<size_t>((size_t)n, std::max<size_t>(1024, budget / per));
+    ea.slots = n;
+    const cudaError_t e = work_alloc(h, B_EIGSCR, vb + 256 + (resolve ? per * (size_t)batch + 2 * 256 : 0));
+    if (e == cudaSuccess) break;
+    if (e != cudaErrorMemoryAllocation || n <= kFewUnits) return cuda_fail(h, e, "alloc transform scratch");
   }
-  CK(h->buf[B_EIGSCR].ensure(need), "alloc transform scratch");
   unsigned char *base = h->buf[B_EIGSCR].as<unsigned char>();
   size_t off = 0;
   auto take = [&](size_t bytes) { unsigned char *p = base + off; off += (bytes + 255) & ~(size_t)255; return p; };
@@ -1006,8 +1018,8 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   CK(cudaStreamSynchronize(st), "stream size sync");
   h->h_tile_off.assign(h->pin_off, h->pin_off + ts.ntiles + 1);
   const int nchunk_total = h->h_tile_off[ts.ntiles];
-  CK(h->buf[B_TILEREC].ensure(std::max<size_t>(16, (size_t)nchunk_total * record_bytes(k))), "alloc tile streams");
-  CK(h->buf[B_TILELIST].ensure(std::max<size_t>(16, (size_t)nchunk_total * 16 * sizeof(int))), "alloc tile streams");
+  CK(work_alloc(h, B_TILEREC, std::max<size_t>(16, (size_t)nchunk_total * record_bytes(k))), "alloc tile streams");
+  CK(work_alloc(h, B_TILELIST, std::max<size_t>(16, (size_t)nchunk_total * 16 * sizeof(int))), "alloc tile streams");
   CK(launch_tile_fill(st, ts.ntiles, nchunk_total, (*ts.par).as<TilePar>(), h->buf[B_GEOM].as<IndexGeom>(), os, k, kp,
                       (*ts.n).as<int>(), (*ts.n).as<int>() + ts.ntiles, (*ts.off).as<int>(),
                       h->buf[B_TILELIST].as<int>(), h->buf[B_TILEREC].as<unsigned char>(),
@@ -1113,12 +1125,10 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   if (pl.first.second > 0) {
     const size_t gp = (size_t)pl.first.second * (size_t)block_bytes;
     const size_t cn = (size_t)pl.first.first * G * 128 * 3 * 4;
-    if ((h->buf[B_GPART].cap >= gp || h->buf[B_GPART].ensure(gp) == cudaSuccess) &&
-        (h->buf[B_GCNT].cap >= cn || h->buf[B_GCNT].ensure(cn) == cudaSuccess)) {
+    if (work_alloc(h, B_GPART, gp) == cudaSuccess && work_alloc(h, B_GCNT, cn) == cudaSuccess) {
       ta.Gpart = h->buf[B_GPART].as<float>();
       ta.cnt = h->buf[B_GCNT].as<float>();
     } else {
-      cudaGetLastError();   // clear the failed allocation: one accumulator per tile
       drain = 1 << 30;
       pl = plan(1 << 30, drain);
     }
@@ -1300,7 +1310,11 @@ static int solver_run(lgpu_handle *h) {
   EigSplit sp{};
   int batch = 0;
   if (rows) {
-    CK(h->buf[B_EIGSCR].ensure(eig_rows_bytes(k, h->nunits)), "alloc transform scratch");
+    for (batch = eig_rows_batch(k, h->nunits);; batch = (batch + 1) / 2) {
+      const cudaError_t e = work_alloc(h, B_EIGSCR, eig_rows_bytes(k, batch));
+      if (e == cudaSuccess) break;
+      if (e != cudaErrorMemoryAllocation || batch <= kFewUnits) return cuda_fail(h, e, "alloc transform scratch");
+    }
     ea.scratch = h->buf[B_EIGSCR].p;
   } else if ((rc = eig_scratch(h, h->nunits, ea, sp, batch)) != LGPU_OK) {
     return rc;
@@ -1318,7 +1332,7 @@ static int solver_run(lgpu_handle *h) {
     for (int j = c1 - 1; j >= c0 && a1 < 0; j--) if (h->h_col2act[j] >= 0) a1 = h->h_col2act[j] + 1;
     CK(cudaEventRecord(h->ev_chunk[c][0], st), "event");
     if (rows)
-      CK(launch_eig_rows(st, ea, &launches), "eigen kernels");   // never with a bound state: one chunk
+      CK(launch_eig_rows(st, ea, batch, &launches), "eigen kernels");   // never with a bound state: one chunk
     else if (!fp64 && a0 >= 0)
       CK(launch_eig_split(st, ea, sp, batch, a0 * G, (a1 - a0) * G, &launches), "eigen kernels");
     CK(cudaEventRecord(h->ev_chunk[c][3], st), "event");
@@ -1599,6 +1613,12 @@ int lgpu_get_obslist_noalloc(lgpu_handle *h, int ij, int group, int *idx, float 
   }
   *n = cnt[0];
   if (ncand) *ncand = cnt[1];
+  return LGPU_OK;
+}
+
+int lgpu_debug_alloc_limit(lgpu_handle *h, size_t bytes) {
+  if (!h) return LGPU_ERR_ARG;
+  h->alloc_limit = bytes;
   return LGPU_OK;
 }
 
@@ -2236,7 +2256,8 @@ int lgpu_learn_train(lgpu_handle *h, int epochs, int batch, float lr, float *los
 // analysis runs both, timed, as AUTO does: the batched form shares the
 // observations of 128 lattice columns, which lie `stride` grid steps apart, so
 // its gain falls with the stride (12,888 columns at stride 2, k = 32, search
-// radius 1,460 km: plain 1,190 us, batched with its streams 540).
+// radius 1,460 km: plain 1,190 us, batched with its streams 540).  Where the
+// device has no room for the tile streams, the plain form runs.
 static int learned_exact(lgpu_handle *h, const ObsSorted &os, int n, bool lattice, int &launches) {
   LearnState *L = h->learn;
   if (n <= 0) return LGPU_OK;
@@ -2277,7 +2298,8 @@ static int learned_exact(lgpu_handle *h, const ObsSorted &os, int n, bool lattic
     CK(cudaEventRecord(h->ev_tune[0], st), "event");
     if ((rc = plain(0, nlat)) != LGPU_OK) return rc;
     CK(cudaEventRecord(h->ev_tune[1], st), "event");
-    if ((rc = run_batched_tiles(h, os, ts, dst, launches, false)) != LGPU_OK) return rc;
+    rc = run_batched_tiles(h, os, ts, dst, launches, false);
+    if (rc != LGPU_OK && rc != LGPU_ERR_NOMEM) return rc;
     CK(cudaEventRecord(h->ev_tune[2], st), "event");
     CK(cudaEventSynchronize(h->ev_tune[2]), "tune sync");
     float tp = 0.0f, tb = 0.0f;
@@ -2285,10 +2307,12 @@ static int learned_exact(lgpu_handle *h, const ObsSorted &os, int n, bool lattic
     CK(cudaEventElapsedTime(&tb, h->ev_tune[1], h->ev_tune[2]), "timing");
     tb -= h->tc_tune_ms;
     h->tc_tune_ms = 0.0f;
-    L->gram_choice = tb <= tp ? LGPU_VARIANT_BATCHED_TC : LGPU_VARIANT_PLAIN;
+    L->gram_choice = rc == LGPU_OK && tb <= tp ? LGPU_VARIANT_BATCHED_TC : LGPU_VARIANT_PLAIN;
     if (L->gram_choice == LGPU_VARIANT_PLAIN && (rc = plain(0, nlat)) != LGPU_OK) return rc;
   } else if (nlat > 0 && L->gram_choice == LGPU_VARIANT_BATCHED_TC) {
-    if ((rc = run_batched_tiles(h, os, ts, dst, launches, false)) != LGPU_OK) return rc;
+    rc = run_batched_tiles(h, os, ts, dst, launches, false);
+    if (rc == LGPU_ERR_NOMEM) rc = plain(0, nlat);
+    if (rc != LGPU_OK) return rc;
   } else if ((rc = plain(0, nlat)) != LGPU_OK) {
     return rc;
   }

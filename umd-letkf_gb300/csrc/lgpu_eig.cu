@@ -1025,7 +1025,7 @@ cudaError_t launch_g(cudaStream_t st, const EigArgs &a, const EigSplit &sp, int 
   const size_t smem = (size_t)G::UPB * G::UNIT * sizeof(typename G::R);
   cudaError_t e = cudaFuncSetAttribute(k_transform<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const int grid = std::min(resident_blocks<G>(), (nb + G::UPB - 1) / G::UPB);
+  const int grid = std::min(resident_blocks<G>(), (std::min(nb, a.slots) + G::UPB - 1) / G::UPB);
   k_transform<G><<<grid, G::THREADS, smem, st>>>(a, PolesOf<typename G::R>::get(), sp,
                                                  reinterpret_cast<typename G::R *>(a.scratch), u0, nb, range,
                                                  above, upto);
@@ -1202,6 +1202,7 @@ cudaError_t launch_eig_debug(cudaStream_t st, int nunits, int k, const float *G,
   size_t off = 0;
   auto take = [&](size_t bytes) { unsigned char *p = buf + off; off += (bytes + 255) & ~(size_t)255; return p; };
   a.scratch = take(vb);
+  a.slots = (int)n;
   if (prec == LGPU_PREC_FP64) {
     e = launch_eig64(st, a, 0, &l);
     cudaError_t e2 = cudaStreamSynchronize(st);

@@ -917,17 +917,16 @@ static size_t eig_rows_per_unit(int k) {
   return (size_t)k * k * 4 + (size_t)2 * k * 4 + (size_t)eig_log_cap(k) * 8 + 4 + (size_t)k * 4;
 }
 
-// units of one batch: the scratch takes at most 8 GB
-static int eig_rows_batch(int k, int units) {
+int eig_rows_batch(int k, int units) {
   const size_t budget = (size_t)8 << 30;
   return (int)std::min<size_t>((size_t)std::max(1, units), std::max<size_t>(1024, budget / eig_rows_per_unit(k)));
 }
 
-size_t eig_rows_bytes(int k, int units) { return eig_rows_per_unit(k) * (size_t)eig_rows_batch(k, units) + 5 * 256; }
+size_t eig_rows_bytes(int k, int batch) { return eig_rows_per_unit(k) * (size_t)batch + 5 * 256; }
 
-cudaError_t launch_eig_rows(cudaStream_t st, const EigArgs &a, int *launches) {
+cudaError_t launch_eig_rows(cudaStream_t st, const EigArgs &a, int batch, int *launches) {
   if (a.nunits <= 0) return cudaSuccess;
-  const int k = a.k, batch = eig_rows_batch(k, a.nunits);
+  const int k = a.k;
   unsigned char *base = static_cast<unsigned char *>(a.scratch);
   size_t off = 0;
   auto take = [&](size_t bytes) { unsigned char *p = base + off; off += (bytes + 255) & ~(size_t)255; return p; };

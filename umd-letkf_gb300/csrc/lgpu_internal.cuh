@@ -581,12 +581,14 @@ struct EigArgs {
   int flag_cap;
   float gap_thresh;
   void *scratch;          // eig_scratch_bytes: the reflectors of the units in flight
+  int slots;              // units that scratch was sized for
 };
 // the FP32 eigendecomposition form (lgpu_eig_rows.cu) of units 0..nunits, for
-// the solutions stored as training rows; scratch of eig_rows_bytes
-size_t eig_rows_bytes(int k, int units);
-cudaError_t launch_eig_rows(cudaStream_t st, const EigArgs &a, int *launches);
-// scratch of launches over at most `units` units at a time in the precisions named
+// the solutions stored as training rows, in batches; scratch of eig_rows_bytes
+int eig_rows_batch(int k, int units);   // units of a batch that take at most 8 GB
+size_t eig_rows_bytes(int k, int batch);
+cudaError_t launch_eig_rows(cudaStream_t st, const EigArgs &a, int batch, int *launches);
+// scratch of launches in the precisions named, with at most `units` units in flight
 size_t eig_scratch_bytes(int k, int units, bool fp32, bool fp64);
 // FP64 transform (a team of warps per unit): units ulist[0..nunits) or
 // ubase + 0..nunits; T (and w-bar) written in FP32
