@@ -464,6 +464,11 @@ int lgpu_debug_weight(lgpu_handle *h, int n, const float *lat1, const float *lon
  * FP64-solved unit count in fp64_units (the other fields are not set). */
 int lgpu_debug_transform(lgpu_handle *h, int nunits, int k, const float *gram, float *trans);
 
+/* Operand type of the last run's Gram (with LEARNED: of its lattice's): 16
+ * (batched, FP16 parts), 32 (batched, TF32 parts: the observations' magnitudes
+ * need its exponents), 0 (plain FP32), -1 before a run. */
+int lgpu_debug_gram_operands(const lgpu_handle *h);
+
 /* Verification of the ways round a full device: the work buffers of this
  * handle's following runs that have such a way (transform scratch, the batched
  * Gram's streams and partial blocks) fail to allocate above `bytes`; 0: no

@@ -135,6 +135,7 @@ struct lgpu_handle {
   int ntiles = 0;
   bool used_tc = false;
   int mma_n = 0;
+  int gram_bits = 0;     // operands of the last run's Gram: 16 or 32 (batched), 0 (plain)
   int auto_choice = 0;   // AUTO: the Gram variant measured faster (0 = not yet measured)
   int gram_nseg = 1;     // most accumulation segments of a tile in the last batched Gram
   std::vector<int> h_tile_off;       // tile stream offsets of the last batched Gram (read back)
@@ -805,7 +806,7 @@ static int prepare_run(lgpu_handle *h, ObsSorted &os, int &launches, const TileS
   CK(h->buf[B_SB].ensure(16 * nobs), "alloc");
   CK(h->buf[B_SHX].ensure(4 * nobs * kp), "alloc sorted hx");
   CK(h->buf[B_SIDX].ensure(4 * nobs), "alloc");
-  CK(h->buf[B_SMAG].ensure(4 * nobs), "alloc");
+  CK(h->buf[B_SMAG].ensure(8 * nobs), "alloc");
   CK(h->buf[B_CSTART].ensure(4 * ((size_t)h->ncell + 1)), "alloc");
   CK(h->buf[B_CP].ensure(sizeof(ColPar) * (size_t)h->ncol), "alloc");
   CK(h->buf[B_G].ensure(4 * std::max<size_t>(1, (size_t)units) * packed_size(k)), "alloc Gram");
@@ -820,7 +821,7 @@ static int prepare_run(lgpu_handle *h, ObsSorted &os, int &launches, const TileS
   os.B = h->buf[B_SB].as<float4>();
   os.hx = h->buf[B_SHX].as<float>();
   os.idx = h->buf[B_SIDX].as<int>();
-  os.mag = h->buf[B_SMAG].as<float>();
+  os.mag = h->buf[B_SMAG].as<float2>();
   os.cell_start = h->buf[B_CSTART].as<int>();
   cudaStream_t st = h->st;
   const bool bound = h->bound_state != nullptr;
@@ -1033,6 +1034,7 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   TcArgs ta;
   ta.tile_mag = tile_mag;
   ta.f16 = h->pin_off[ts.ntiles + 1] == 0;
+  h->gram_bits = ta.f16 ? 16 : 32;
   ta.ntiles = ts.ntiles;
   ta.groups = G;
   ta.k = k;
@@ -1232,6 +1234,7 @@ static int solver_run(lgpu_handle *h) {
     return run_batched_tiles(h, os, grid_tiles, dst, launches, start_upload && bound);
   };
   auto run_plain = [&]() -> int {
+    h->gram_bits = 0;
     GramArgs ga;
     ga.nunits = h->nunits;
     ga.groups = G;
@@ -1615,6 +1618,8 @@ int lgpu_get_obslist_noalloc(lgpu_handle *h, int ij, int group, int *idx, float 
   if (ncand) *ncand = cnt[1];
   return LGPU_OK;
 }
+
+int lgpu_debug_gram_operands(const lgpu_handle *h) { return h && h->ran ? h->gram_bits : -1; }
 
 int lgpu_debug_alloc_limit(lgpu_handle *h, size_t bytes) {
   if (!h) return LGPU_ERR_ARG;
@@ -2265,6 +2270,7 @@ static int learned_exact(lgpu_handle *h, const ObsSorted &os, int n, bool lattic
   const int k = h->k;
   auto plain = [&](int r0, int r1) -> int {
     if (r1 <= r0) return LGPU_OK;
+    if (lattice && r0 == 0) h->gram_bits = 0;
     GramArgs ga;
     ga.nunits = r1 - r0;
     ga.groups = 1;

@@ -102,14 +102,17 @@ __device__ __forceinline__ uint32_t kmaj(int row, int kk) {
 // FP16 operands.  W = 2^12 rho lies in (0.4, 4096] for every weight above the
 // keep threshold, and the features y_i y_j / err are scaled by a power of two
 // per tile that puts the largest of its candidates' into [2^14, 2^15): hi = f16
-// (11 bits) and lo = f16 (x - hi) then hold 22 bits of every x down to 2^-3
-// (lo's spacing there is FP16's smallest), 2^-18 of the tile's largest feature.
-// Where a tile's candidates differ by more than that in their largest features,
-// or the largest is not finite or beyond 2^+-60 (the factors of a feature stay
-// normal FP32 numbers), the run takes the TF32 operands, whose exponents are
-// FP32's.
+// (11 bits) and lo = f16 (x - hi) leave at most 2^-22 |x|, or 2^-25 where lo's
+// spacing is FP16's smallest (x below 2^-3).  The largest y_i y_j / err of every
+// candidate has to be at least 2^-3, 17 powers of two below the tile's top, so
+// an observation's operands are off by at most 2^-22 of its own largest y_i y_j
+// / err in the features y_i y_j, and of its own largest feature in y_i dep
+// (TF32's hi + lo: 2^-21 of each feature).  Where a tile's candidates differ by
+// more, in their perturbations or in departures far beyond these, or the
+// largest is not finite or beyond 2^+-60 (the factors of a feature stay normal
+// FP32 numbers), the run takes the TF32 operands, whose exponents are FP32's.
 constexpr float kWScale = 4096.0f;
-constexpr int kPTop = 14, kPRange = 18, kPExp = 60;
+constexpr int kPTop = 14, kPRange = 17, kPExp = 60;
 __host__ __device__ inline int f32_exp(uint32_t bits) { return (int)(bits >> 23) - 127; }
 __device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
 
@@ -214,7 +217,7 @@ __device__ __forceinline__ void warp_range(const Window &W, int w, int &j0, int 
 // candidates per tile: observations of the window inside the tile's cap, per
 // warp range (tile_wn) and in all
 __global__ void __launch_bounds__(WT) k_tile_count(int ntiles, const TilePar *tps, const IndexGeom *geom,
-                                                   const float4 *obsA, const float *mag, const int *cell_start,
+                                                   const float4 *obsA, const float2 *mag, const int *cell_start,
                                                    int *tile_n, int *tile_wn, uint32_t *tile_mag) {
   __shared__ Window W;
   __shared__ int red[WT / 32];
@@ -224,15 +227,15 @@ __global__ void __launch_bounds__(WT) k_tile_count(int ntiles, const TilePar *tp
   build_window(W, tp, geom, cell_start);
   int cnt = 0, j0, j1;
   warp_range(W, wid, j0, j1);
-  uint32_t mx = 0, mn = 0x7f800000u;   // largest, smallest positive magnitude (their bits)
+  uint32_t mx = 0, mn = 0x7f800000u;   // largest feature, smallest positive y_i y_j of an observation's largest (bits)
 #pragma unroll 4
   for (int j = j0 + lane; j < j1; j += 32) {
     const int p = window_pos(W, j);
     const bool in = in_cap(tp, __ldg(obsA + p));
-    const uint32_t m = in ? __float_as_uint(__ldg(mag + p)) : 0u;
+    const float2 m = in ? __ldg(mag + p) : make_float2(0.0f, 0.0f);
     cnt += in;
-    mx = max(mx, m);
-    mn = m != 0u ? min(mn, m) : mn;
+    mx = max(mx, __float_as_uint(m.x));
+    mn = m.y != 0.0f ? min(mn, __float_as_uint(m.y)) : mn;
   }
   cnt = __reduce_add_sync(0xffffffffu, cnt);
   mx = __reduce_max_sync(0xffffffffu, mx);
@@ -967,8 +970,8 @@ __global__ void __launch_bounds__(gram_threads(NPMAX), 1) k_gram_tc(TcArgs a) {
   if (wid == 0) tc::tmem_dealloc(tmem, tmem_cols);
 }
 
-// Stage / ring depths: four FP16 or two TF32 operand stages (k <= 128: 4 x 36 KB
-// or 2 x 70 KB) and six record slots (10.8 KB).  With TF32 operands at k = 40
+// Stage / ring depths: four FP16 or two TF32 operand stages (k <= 128: 4 x 38 KB
+// or 2 x 76 KB) and six record slots (10.8 KB).  With TF32 operands at k = 40
 // six slots made the Gram 1.8 ms faster than three stages with three slots (the
 // producers waited on the record copies); twelve slots gained nothing more.
 size_t gram_tc_smem(int k, int np, bool f16) {

@@ -323,8 +323,11 @@ __global__ void __launch_bounds__(32 * GW) k_place(int nobs, int k, int kp, cons
   if (lane == 0) o.A[q] = A;
   if (lane == 1) o.B[q] = B;
   if (lane == 2) o.idx[q] = i;
-  // the largest feature of the observation over its error
-  if (lane == 3) o.mag[q] = __uint_as_float(ymax) / A.w * __uint_as_float(max(ymax, __float_as_uint(fabsf(B.x))));
+  // the observation's largest features over its error: of all, and y_i y_j
+  if (lane == 3) {
+    const float y = __uint_as_float(ymax), s = y / A.w;
+    o.mag[q] = make_float2(s * __uint_as_float(max(ymax, __float_as_uint(fabsf(B.x)))), s * y);
+  }
 }
 
 }  // namespace

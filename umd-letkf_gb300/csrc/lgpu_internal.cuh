@@ -377,7 +377,7 @@ struct ObsSorted {
   float *hx;       // [nobs][KP] perturbations, zero padded
   int *idx;        // original observation index
   int *cell_start; // [ncell + 1]
-  float *mag = nullptr;   // largest feature |y_i| max(|y_j|, |dep|) over the error (batched Gram's scale)
+  float2 *mag = nullptr;  // largest |y_i| max(|y_j|, |dep|) and largest y_i^2 over the error (batched Gram's scale)
 };
 
 // The local-observation search of one (column, group), the threads of a
@@ -514,7 +514,7 @@ struct TcArgs {
   const unsigned char *rec;  // tile candidate streams (chunk records)
   const int *tile_off;       // [ntiles + 1] first chunk of each tile's stream
   const int *tile_n;         // [ntiles] candidates of each tile
-  const uint32_t *tile_mag;  // [ntiles][2] bits of the largest and smallest positive magnitude of a tile's candidates
+  const uint32_t *tile_mag;  // [ntiles][2] bits of a tile's largest mag.x and smallest positive mag.y
   bool f16;                  // FP16 operands (every tile's magnitudes within range)
   int cb;                    // bytes per chunk record (set by the launcher)
   uint32_t tmem_cols;        // TMEM columns per CTA (set by the launcher)

@@ -114,7 +114,8 @@ EXPORTS = ["lgpu_set_variant", "lgpu_create", "lgpu_destroy", "lgpu_last_error",
            "lgpu_get_state", "lgpu_get_diag", "lgpu_get_timings", "lgpu_solver_final", "lgpu_get_obslist",
            "lgpu_debug_metric", "lgpu_debug_gc", "lgpu_host_alloc", "lgpu_host_free", "lgpu_flush_l2",
            "lgpu_get_obslist_noalloc", "lgpu_set_obs_raw", "lgpu_set_state_members", "lgpu_get_background",
-           "lgpu_get_obs_prepared", "lgpu_debug_transform", "lgpu_debug_alloc_limit", "lgpu_bind_state",
+           "lgpu_get_obs_prepared", "lgpu_debug_transform", "lgpu_debug_alloc_limit", "lgpu_debug_gram_operands",
+           "lgpu_bind_state",
            "lgpu_debug_weight", "lgpu_learn_init", "lgpu_learn_collect", "lgpu_learn_train", "lgpu_learn_stats_get",
            "lgpu_learn_param_count", "lgpu_learn_get_params", "lgpu_learn_set_params", "lgpu_mlp_debug",
            "lgpu_learn_set_network", "lgpu_set_precision", "lgpu_write_diag", "lgpu_get_loc_diag",
@@ -166,6 +167,7 @@ def lib(path=None):
     L.lgpu_get_background.argtypes = [H, FP, FP, FP]
     L.lgpu_debug_transform.argtypes = [H, ctypes.c_int, ctypes.c_int, FP, FP]
     L.lgpu_debug_alloc_limit.argtypes = [H, ctypes.c_size_t]
+    L.lgpu_debug_gram_operands.argtypes = [H]
     L.lgpu_get_obs_prepared.argtypes = [H, FP, FP, FP, FP, FP, FP]
     L.lgpu_bind_state.argtypes = [H, ctypes.c_int, ctypes.c_int, FP, FP, FP, ctypes.c_int, ctypes.POINTER(_Var)]
     L.lgpu_learn_init.argtypes = [H, ctypes.POINTER(_LearnCfg)]
@@ -595,6 +597,9 @@ class Solver:
         out = np.zeros(n, np.float32)
         self._ck(self.L.lgpu_debug_metric(self.h, n, *[_fp(x) for x in a], _fp(out)))
         return out
+
+    def debug_gram_operands(self):
+        return self.L.lgpu_debug_gram_operands(self.h)
 
     def debug_alloc_limit(self, nbytes):
         return self._ck(self.L.lgpu_debug_alloc_limit(self.h, int(nbytes)))
