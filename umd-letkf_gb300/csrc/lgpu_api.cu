@@ -93,7 +93,17 @@ static void chunk_bounds(int ncol, int n, int c, int *c0, int *c1) {
 }
 constexpr int kSegChunks = 256;   // batched Gram: chunks of 16 observations per CTA at most
 constexpr int kMinSegChunks = 24, kSegsPerSM = 3;   // ... and where the chunks are few
-constexpr int kDrainChunks = 64;  // batched Gram: chunks per tensor-core accumulation (drained to a partial block)
+// batched Gram: chunks per tensor-core accumulation (drained to a partial
+// block).  Every MMA cuts its sum off at the accumulator's last bit, so a Gram's
+// error grows with the chunks in one accumulation, and a drain costs a block's
+// stores and the segment sum's reads.  The short interval is for the runs that
+// the plain FP32 Gram would take if the batched one were not faster (kFewChunks
+// per SM), and for the learned form's lattice, so that they are no further from
+// 64 bits than that form was: 144 x 72 columns, k = 40, error of the spread
+// 4.1e-7 with 64 chunks, 2.9e-7 with 16 (plain 2.4e-7; 3.2e-7 when the plain
+// form ran with the transform before), Gram 0.29 and 0.33 ms.  Everywhere at 16
+// it costs 13 to 27% of the Gram (0.68 -> 0.81 ms at 360 x 180, k = 32).
+constexpr int kDrainChunks = 64, kShortDrain = 16, kFewChunks = 96;
 
 struct LearnState;   // learned form (below)
 
@@ -991,6 +1001,7 @@ struct GramDest {
   float *G;
   int *nkept;
   int *cull;
+  bool short_drain;   // accumulations of kShortDrain chunks whatever the run's size
 };
 
 // start_upload: a bound state's members start uploading once the tile fill is
@@ -1059,8 +1070,7 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   ta.status = h->buf[B_STATUS].as<int>();
   // accumulation segments: each tile's stream is split into ranges of at most
   // seg_chunks chunks, each its own CTA (which drains its tensor-core
-  // accumulator into its result rows every 64 chunks: the FP32 accumulation
-  // error grows with the MMAs summed into one accumulator); the partial
+  // accumulator into its result rows every `drain` chunks); the partial
   // Grams of a tile's segments are summed in order afterwards; the partials
   // take at most 24 GB (longer segments otherwise).  A CTA fills an SM, so a
   // small analysis is split until each SM has kSegsPerSM of them (but no finer
@@ -1110,7 +1120,7 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   for (int t = 0; t < ts.ntiles; t++) longest = std::max(longest, h->h_tile_off[t + 1] - h->h_tile_off[t]);
   const long long cta_chunks = (long long)nchunk_total * ta.npass * G;
   const long long want = (cta_chunks + 152 * kSegsPerSM - 1) / (152 * kSegsPerSM);
-  int drain = kDrainChunks;
+  int drain = dst.short_drain || cta_chunks <= 152LL * kFewChunks ? kShortDrain : kDrainChunks;
   int seg_chunks = (int)std::min<long long>(kSegChunks, std::max<long long>(kMinSegChunks, (want + 1) & ~1LL));
   auto pl = plan(seg_chunks, drain);
   while (pl.first.second > 0 && pl.first.second * block_bytes > 24.0 * (1ull << 30)) {
@@ -1230,7 +1240,7 @@ static int solver_run(lgpu_handle *h) {
   bool uploading = false;   // a bound state's members are on their way
   auto run_batched = [&](bool start_upload) -> int {
     uploading = start_upload && bound;
-    const GramDest dst{h->buf[B_COL2ACT].as<int>(), h->buf[B_G].as<float>(), h->buf[B_NKEPT].as<int>(), &h->tc_cull};
+    const GramDest dst{h->buf[B_COL2ACT].as<int>(), h->buf[B_G].as<float>(), h->buf[B_NKEPT].as<int>(), &h->tc_cull, false};
     return run_batched_tiles(h, os, grid_tiles, dst, launches, start_upload && bound);
   };
   auto run_plain = [&]() -> int {
@@ -2291,7 +2301,7 @@ static int learned_exact(lgpu_handle *h, const ObsSorted &os, int n, bool lattic
     return LGPU_OK;
   };
   const TileSet ts{L->ntiles, &L->tcols, &L->tpar, &L->tn, &L->toff};
-  const GramDest dst{L->d_rank.as<int>(), L->Gsub.as<float>(), L->nksub.as<int>(), &L->cull};
+  const GramDest dst{L->d_rank.as<int>(), L->Gsub.as<float>(), L->nksub.as<int>(), &L->cull, true};
   const int nlat = lattice ? (int)L->coarse.size() : 0;
   int rc = LGPU_OK;
   if (k < 8) L->gram_choice = LGPU_VARIANT_PLAIN;   // as AUTO
