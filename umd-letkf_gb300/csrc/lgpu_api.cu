@@ -12,6 +12,7 @@
 #include <sys/mman.h>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <string>
 #include <vector>
 #include <cmath>
@@ -113,7 +114,7 @@ struct lgpu_handle {
   cudaStream_t cst = nullptr;      // host<->device copies of a bound state
   cudaEvent_t ev[8] = {};
   cudaEvent_t ev_in[2] = {};       // bound state: mean/spread uploaded; members' upload started
-  cudaEvent_t ev_tune[3] = {};     // AUTO: timing of the two Gram forms
+  cudaEvent_t ev_tune[2] = {};     // AUTO: timing of the two Gram forms
   cudaEvent_t ev_cull[3] = {};     // batched Gram: timing of its two producer forms
   // per column chunk: eigensolve start, update start, update end, FP64 eigensolve start
   cudaEvent_t ev_chunk[kOutChunks][4] = {};
@@ -162,6 +163,7 @@ struct lgpu_handle {
   int prec = LGPU_PREC_FP32;   // eigensolve precision mode
   float gap_thresh = 1e-6f;    // FP32_RESOLVE: relative eigenvalue gap that sends a unit to FP64
   DevBuf buf[B_COUNT_ALL];
+  int work_grown = 0;          // work buffers allocated so far
   size_t alloc_limit = 0;      // work buffers above this many bytes fail to allocate (0: no limit)
   lgpu_timings tim{};
   LearnState *learn = nullptr;      // learned form, after lgpu_learn_init
@@ -197,6 +199,7 @@ int cuda_fail(lgpu_handle *h, cudaError_t e, const char *what) {
 // work buffers whose size follows the run, with a way round where the device
 // has no room for them
 cudaError_t work_alloc(lgpu_handle *h, int b, size_t bytes) {
+  if (h->buf[b].cap < bytes) h->work_grown++;
   cudaError_t e = h->alloc_limit > 0 && bytes > h->alloc_limit ? cudaErrorMemoryAllocation : h->buf[b].ensure(bytes);
   if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();
   return e;
@@ -1187,6 +1190,43 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   return LGPU_OK;
 }
 
+// Runs the plain and the batched Gram, timed; *choice becomes the faster form,
+// whose result stands.  A batched run that had to allocate its work buffers
+// stood still meanwhile, and is timed again (101 x 53 columns, k = 37: 0.35 ms
+// with the allocations, 0.19 without, plain 0.21; 240 x 120, k = 100: 1.74,
+// 1.50, plain 2.2 to 2.4).  Returns the batched form's LGPU_ERR_NOMEM with the plain result.
+static int pick_gram(lgpu_handle *h, const std::function<int()> &plain, const std::function<int()> &batched,
+                     int *choice) {
+  float ms[2] = {0.0f, 0.0f};
+  int rc = LGPU_OK;
+  auto timed = [&](const std::function<int()> &form, float *t) -> int {
+    CK(cudaEventRecord(h->ev_tune[0], h->st), "event");
+    const int r = form();
+    if (r != LGPU_OK) return r;
+    CK(cudaEventRecord(h->ev_tune[1], h->st), "event");
+    CK(cudaEventSynchronize(h->ev_tune[1]), "tune sync");
+    CK(cudaEventElapsedTime(t, h->ev_tune[0], h->ev_tune[1]), "timing");
+    *t -= h->tc_tune_ms;   // the batched form's producer tuning ran its Gram twice
+    h->tc_tune_ms = 0.0f;
+    return LGPU_OK;
+  };
+  h->tc_tune_ms = 0.0f;
+  if ((rc = timed(plain, &ms[0])) != LGPU_OK) return rc;
+  const int grown = h->work_grown;
+  rc = timed(batched, &ms[1]);
+  if (rc == LGPU_OK && h->work_grown != grown) {
+    CK(cudaMemsetAsync(h->buf[B_STATUS].as<int>() + 2, 0, sizeof(int), h->st), "memset");   // the MMA counter
+    rc = timed(batched, &ms[1]);
+  }
+  if (rc != LGPU_OK && rc != LGPU_ERR_NOMEM) return rc;
+  *choice = rc == LGPU_OK && ms[1] <= ms[0] ? LGPU_VARIANT_BATCHED_TC : LGPU_VARIANT_PLAIN;
+  if (*choice == LGPU_VARIANT_PLAIN) {
+    const int again = plain();
+    if (again != LGPU_OK) return again;
+  }
+  return rc;
+}
+
 static int solver_run(lgpu_handle *h);
 
 // A bound state's members, uploaded on the copy stream in the column chunks
@@ -1276,21 +1316,8 @@ static int solver_run(lgpu_handle *h) {
     h->preloaded = true;
   }
   if (choice == 0) {
-    CK(cudaEventRecord(h->ev_tune[0], st), "event");
-    if ((rc = run_plain()) != LGPU_OK) return rc;
-    CK(cudaEventRecord(h->ev_tune[1], st), "event");
-    if ((rc = run_batched(false)) != LGPU_OK) return rc;
-    CK(cudaEventRecord(h->ev_tune[2], st), "event");
-    CK(cudaEventSynchronize(h->ev_tune[2]), "tune sync");
-    float tp = 0.0f, tb = 0.0f;
-    CK(cudaEventElapsedTime(&tp, h->ev_tune[0], h->ev_tune[1]), "timing");
-    CK(cudaEventElapsedTime(&tb, h->ev_tune[1], h->ev_tune[2]), "timing");
-    tb -= h->tc_tune_ms;   // the batched form's producer tuning ran its Gram twice
-    h->tc_tune_ms = 0.0f;
-    h->auto_choice = tb <= tp ? LGPU_VARIANT_BATCHED_TC : LGPU_VARIANT_PLAIN;
-    // the kept result is the chosen form's
-    if (h->auto_choice == LGPU_VARIANT_PLAIN && (rc = run_plain()) != LGPU_OK) return rc;
-    choice = h->auto_choice;
+    if ((rc = pick_gram(h, run_plain, [&] { return run_batched(false); }, &choice)) != LGPU_OK) return rc;
+    h->auto_choice = choice;
   } else if (choice == LGPU_VARIANT_BATCHED_TC) {
     // the whole Gram at once (a bound state's members upload meanwhile)
     if ((rc = run_batched(true)) != LGPU_OK) return rc;
@@ -2311,20 +2338,9 @@ static int learned_exact(lgpu_handle *h, const ObsSorted &os, int n, bool lattic
       CK(preload_gram_tc(h->loc.cls), "kernel load");
       h->preloaded = true;
     }
-    CK(cudaEventRecord(h->ev_tune[0], st), "event");
-    if ((rc = plain(0, nlat)) != LGPU_OK) return rc;
-    CK(cudaEventRecord(h->ev_tune[1], st), "event");
-    rc = run_batched_tiles(h, os, ts, dst, launches, false);
+    rc = pick_gram(h, [&] { return plain(0, nlat); },
+                   [&] { return run_batched_tiles(h, os, ts, dst, launches, false); }, &L->gram_choice);
     if (rc != LGPU_OK && rc != LGPU_ERR_NOMEM) return rc;
-    CK(cudaEventRecord(h->ev_tune[2], st), "event");
-    CK(cudaEventSynchronize(h->ev_tune[2]), "tune sync");
-    float tp = 0.0f, tb = 0.0f;
-    CK(cudaEventElapsedTime(&tp, h->ev_tune[0], h->ev_tune[1]), "timing");
-    CK(cudaEventElapsedTime(&tb, h->ev_tune[1], h->ev_tune[2]), "timing");
-    tb -= h->tc_tune_ms;
-    h->tc_tune_ms = 0.0f;
-    L->gram_choice = rc == LGPU_OK && tb <= tp ? LGPU_VARIANT_BATCHED_TC : LGPU_VARIANT_PLAIN;
-    if (L->gram_choice == LGPU_VARIANT_PLAIN && (rc = plain(0, nlat)) != LGPU_OK) return rc;
   } else if (nlat > 0 && L->gram_choice == LGPU_VARIANT_BATCHED_TC) {
     rc = run_batched_tiles(h, os, ts, dst, launches, false);
     if (rc == LGPU_ERR_NOMEM) rc = plain(0, nlat);
