@@ -1081,11 +1081,9 @@ auto with_grid_f64(int k, F f) {
 // FP64 grids for a list of few flagged units: four warps or more a unit.  A
 // warp issues FP64 to its own quarter of the SM, one multiply-add in two
 // clocks, so one warp a unit runs a lone unit at a quarter of the SM's rate
-// (k = 37, 5 units: 442 us, now 324).  With many units the lists' larger
-// padding and barriers cost more than they gain (k = 37, 4,248 units: 6.5 ms
-// against 3.0), so a list beyond one wave of these blocks takes the other
-// grids.  The list's length stays on the device: both kernels are launched, and
-// the one whose range it is not in returns at once.
+// (k = 37, up to 112 units: 433 us, now 321).  The list's length stays on the
+// device: both kernels are launched, and the one whose range it is not in
+// returns at once.
 template <class F>
 auto with_grid_f64_few(int k, F f) {
 #define LGPU_GRID(...) return f(Grid<double, __VA_ARGS__>())
@@ -1106,6 +1104,20 @@ cudaError_t launch_f64(cudaStream_t st, const EigArgs &a, int u0, int nb, int *l
       a.k, [&](auto g) { return launch_g<decltype(g)>(st, a, EigSplit{}, u0, nb, nullptr, 0, 0, launches); });
 }
 
+// The longest list that takes these grids.  The block scheduler starts to put
+// two blocks on an SM between 112 and 120 of them.  Beyond, where this grid
+// covers more rows than the other one (k = 17 to 24: 32 to 24; 33 to 40: 48 to
+// 40) or both cover 16, the other is the faster one at once (us, this grid and
+// the other, 120 to 304 units: k = 16 104 and 94, k = 24 226 and 175, k = 37
+// 473 and 434).  Where both cover the same this one holds to its full wave of
+// two blocks an SM (304 units: k = 32 270 and 289, k = 48 543 and 653, k = 64
+// 950 and 1,219; 456 units: 524 and 287, 1,072 and 653, 1,877 and 1,228).
+constexpr int kOneAnSM = 112;
+template <class G>
+int few_units(int k) {
+  return k <= 24 || (k > 32 && k <= 40) ? kOneAnSM : resident_blocks<G>();
+}
+
 constexpr int kAll = 0x7fffffff;
 
 // the entries [range[1], range[0]) of the flagged list (as many blocks as
@@ -1115,7 +1127,7 @@ cudaError_t launch_f64_list(cudaStream_t st, const EigArgs &a, const int *range,
   cudaError_t e = with_grid_f64_few(a.k, [&](auto g) {
     using G = decltype(g);
     with_grid_f64(a.k, [&](auto h) {
-      if (!std::is_same<G, decltype(h)>::value) few = resident_blocks<G>();
+      if (!std::is_same<G, decltype(h)>::value) few = few_units<G>(a.k);
     });
     return launch_g<G>(st, a, EigSplit{}, 0, a.nunits, range, 0, few, launches);
   });
