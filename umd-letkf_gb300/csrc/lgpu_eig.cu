@@ -57,41 +57,28 @@ struct Poles {
   R s[kLevels][NP], w[kLevels][NP];
 };
 
-// sn, cn, dn of parameter m = 1 - m1 at u, by descending Landen transformation
-// (Abramowitz & Stegun 16.4: the arithmetic-geometric mean scale)
-void ellip_sncndn(double u, double m1, double &sn, double &cn, double &dn) {
-  double a[32], c[32];
-  double b = std::sqrt(m1);
-  a[0] = 1.0;
-  c[0] = std::sqrt(1.0 - m1);
-  int n = 0;
-  while (std::fabs(c[n]) > 1e-17 && n < 30) {
-    a[n + 1] = 0.5 * (a[n] + b);
-    c[n + 1] = 0.5 * (a[n] - b);
-    b = std::sqrt(a[n] * b);
-    n++;
+// Jacobi's elliptic functions of parameter 1 - m1 by the arithmetic-geometric
+// mean (Abramowitz & Stegun 17.6, 16.4): the quarter period K, and sn / cn at u
+// in (0, K) as the tangent of the amplitude, which is halved down the scale.
+struct Elliptic {
+  double agm = 1.0, ratio[32], K;   // the mean, half differences over means on the way to it
+  int steps = 0;
+  explicit Elliptic(double m1) {
+    double b = std::sqrt(m1);
+    while (agm - b > 1e-16 * agm && steps < 32) {
+      const double mean = 0.5 * (agm + b);
+      ratio[steps++] = 0.5 * (agm - b) / mean;
+      b = std::sqrt(agm * b);
+      agm = mean;
+    }
+    K = 1.5707963267948966 / agm;
   }
-  double phi = std::ldexp(a[n] * u, n), prev = phi;
-  for (; n > 0; n--) {
-    prev = phi;
-    phi = 0.5 * (phi + std::asin(c[n] / a[n] * std::sin(phi)));
+  double sc(double u) const {
+    double phi = std::ldexp(agm * u, steps);
+    for (int i = steps; i-- > 0;) phi = 0.5 * (phi + std::asin(ratio[i] * std::sin(phi)));
+    return std::tan(phi);
   }
-  sn = std::sin(phi);
-  cn = std::cos(phi);
-  const double den = std::cos(prev - phi);
-  dn = std::fabs(den) < 0.1 ? std::sqrt(1.0 - (1.0 - m1) * sn * sn) : cn / den;
-}
-
-// complete elliptic integral K of parameter 1 - m1
-double ellip_k(double m1) {
-  double a = 1.0, b = std::sqrt(m1);
-  for (int i = 0; i < 40 && std::fabs(a - b) > 1e-16 * a; i++) {
-    const double t = 0.5 * (a + b);
-    b = std::sqrt(a * b);
-    a = t;
-  }
-  return 1.5707963267948966 / a;
-}
+};
 
 // Smallest term counts whose error over [1, 4^(level + 1)] is below `tol`
 // (NP at most: the wide levels, whose condition leaves the working precision
@@ -100,14 +87,15 @@ template <class R, int NP>
 Poles<R, NP> make_poles(double tol) {
   Poles<R, NP> P{};
   for (int l = 0; l < kLevels; l++) {
-    const double kappa = std::ldexp(1.0, 2 * (l + 1)), K = ellip_k(1.0 / kappa);
+    const double kappa = std::ldexp(1.0, 2 * (l + 1)), m1 = 1.0 / kappa;
+    const Elliptic E(m1);
     double s[NP], w[NP];
     for (int n = 3; n <= NP; n++) {
       for (int j = 0; j < n; j++) {
-        double sn, cn, dn;
-        ellip_sncndn((j + 0.5) * K / n, 1.0 / kappa, sn, cn, dn);
-        s[j] = sn / cn * (sn / cn);
-        w[j] = 2.0 * K / (3.14159265358979323846 * n) * dn / (cn * cn);
+        // t = sn / cn: 1 / cn^2 = 1 + t^2, dn^2 / cn^2 = 1 + m1 t^2
+        const double t = E.sc((j + 0.5) * E.K / n), t2 = t * t;
+        s[j] = t2;
+        w[j] = 2.0 * E.K / (3.14159265358979323846 * n) * std::sqrt((1.0 + t2) * (1.0 + m1 * t2));
       }
       double err = 0.0;
       for (int t = 0; t <= 400; t++) {
