@@ -179,18 +179,8 @@ __device__ __forceinline__ void st2(double *p, Pair<double> a, Pair<double> b) {
   *reinterpret_cast<double2 *>(p + 2) = make_double2(b.a, b.b);
 }
 
-// sqrt and reciprocal of positive normal values, to an ulp or so: the
-// hardware's approximations and one Newton step, without the rounded forms'
-// range checks
-__device__ __forceinline__ float sqrt_pos(float x) {
-  const float r = rsqrt_approx(x), q = x * r;
-  return fmar(0.5f * r, fmar(-q, q, x), q);
-}
+// sqrt and reciprocal of positive normal values (FP32: within an ulp, lgpu_f32x2.cuh)
 __device__ __forceinline__ double sqrt_pos(double x) { return sqrt(x); }
-__device__ __forceinline__ float rcp_pos(float x) {
-  const float r = rcp_approx(x);
-  return fmar(r, fmar(-x, r, 1.0f), r);
-}
 __device__ __forceinline__ double rcp_pos(double x) { return __drcp_rn(x); }
 
 // 16 bytes global -> shared, asynchronously
