@@ -179,9 +179,14 @@ __device__ __forceinline__ void st2(double *p, Pair<double> a, Pair<double> b) {
   *reinterpret_cast<double2 *>(p + 2) = make_double2(b.a, b.b);
 }
 
-// sqrt and reciprocal of positive normal values (FP32: within an ulp, lgpu_f32x2.cuh)
+// sqrt and reciprocal of positive normal values (FP32: within an ulp,
+// lgpu_f32x2.cuh; the FP64 overloads would hide these without the declarations)
+using lgpu::rcp_pos;
+using lgpu::sqrt_pos;
 __device__ __forceinline__ double sqrt_pos(double x) { return sqrt(x); }
 __device__ __forceinline__ double rcp_pos(double x) { return __drcp_rn(x); }
+static_assert(std::is_same<decltype(sqrt_pos(1.0f)), float>::value && std::is_same<decltype(rcp_pos(1.0f)), float>::value,
+              "FP32 roots stay FP32");
 
 // 16 bytes global -> shared, asynchronously
 __device__ __forceinline__ void copy16_async(void *dst, const void *src) {
