@@ -1052,7 +1052,6 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   ta.ntiles = ts.ntiles;
   ta.groups = G;
   ta.k = k;
-  ta.kp = kp;
   gram_tc_passes(k, &ta.npass, &ta.np);
   h->mma_n = ta.np;
   ta.nf = packed_size(k);
@@ -1064,7 +1063,6 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   ta.tp = (*ts.par).as<TilePar>();
   ta.rec = h->buf[B_TILEREC].as<unsigned char>();
   ta.tile_off = (*ts.off).as<int>();
-  ta.tile_n = (*ts.n).as<int>();
   ta.G = dst.G;
   ta.nkept = dst.nkept;
   ta.diag_obscount = h->buf[B_DOBSC].as<float>();
@@ -1081,8 +1079,6 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
   // much as its chunks): with 256-chunk segments the longest stream set the
   // time (144 x 72 columns, k = 40, 130 CTAs: 301 us with 42% of the SMs
   // in use, now 211)
-  ta.units = (long long)h->nact * G;
-  ta.nf = packed_size(k);
   ta.Gpart = nullptr;
   ta.cnt = nullptr;
   auto plan = [&](int seg_chunks, int drain) {
@@ -1186,7 +1182,7 @@ static int run_batched_tiles(lgpu_handle *h, const ObsSorted &os, const TileSet 
     ta.cull = *dst.cull;
     CK(launch_gram_tc(st, ta, &launches), "tensor-core gram kernel");
   }
-  CK(launch_gram_segsum(st, ta, h->buf[B_ACTIVE].as<int>(), &launches), "gram segment sum");
+  CK(launch_gram_segsum(st, ta, &launches), "gram segment sum");
   return LGPU_OK;
 }
 

@@ -199,11 +199,10 @@ __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group 
 
 // The lane grid of one unit: RN rows and CN columns per lane; LA is a
 // multiple of LB, and LB <= 8 divides a warp, so the lanes of a row lie in one warp.
-template <class R_, int RN_, int CN_, int LA_, int LB_, int MB_, bool KEEP_ = true>
+template <class R_, int RN_, int CN_, int LA_, int LB_, int MB_>
 struct Grid {
   using R = R_;
   static constexpr int RN = RN_, CN = CN_, LA = LA_, LB = LB_;
-  static constexpr bool KEEP = KEEP_;                       // the reflector stays in registers between its two uses
   static constexpr int MB = MB_;                            // blocks per SM the registers are bounded for
   static constexpr int L = LA * LB;
   static constexpr int CH2 = CN / 2;                        // column pairs per lane
@@ -363,13 +362,12 @@ struct Vec {
 };
 
 // The two-sided update M -= v w^T + w v^T with w = p - (t/2)(p.v) v, p = t M v.
-// vb, vcol / vrow: the reflector in shared memory and at the lane's column
-// pairs from Q0 and rows from R0, zero up to j.  FULL (back-transformation): every row and column; else
+// vcol / vrow: the reflector at the lane's column pairs from Q0 and rows from
+// R0, zero up to j.  FULL (back-transformation): every row and column; else
 // (reduction) the trailing block, where w is zero up to j.
 template <class G, int R0, int Q0, bool FULL>
 __device__ __forceinline__ void two_sided(typename G::Row (&A)[G::RN], typename G::R *wb, int j, int a, int b,
-                                          typename G::R t, const typename G::R *vb, const Pair<typename G::R> *vcol,
-                                          const typename G::R *vrow) {
+                                          typename G::R t, const Pair<typename G::R> *vcol, const typename G::R *vrow) {
   using R = typename G::R;
   using P2 = Pair<R>;
   constexpr int W0 = FULL ? 0 : R0, C0 = FULL ? 0 : Q0;
@@ -402,12 +400,11 @@ __device__ __forceinline__ void two_sided(typename G::Row (&A)[G::RN], typename 
       nw[r] = P2(-w[r], -w[r]);
       if (r >= R0) nv[r] = P2(-vrow[r], -vrow[r]);
     }
-    const R *wp = wb + b * G::CP, *vp = vb + b * G::CP;
+    const R *wp = wb + b * G::CP;
 #pragma unroll
     for (int q = C0 / 2; q < G::NV; q++) {
-      P2 wc[2], vc[2];
+      P2 wc[2];
       ld2(wp + 4 * q, wc);
-      if (!G::KEEP && q >= Q0 / 2) ld2(vp + 4 * q, vc);
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const int i = 2 * q + h;
@@ -415,7 +412,7 @@ __device__ __forceinline__ void two_sided(typename G::Row (&A)[G::RN], typename 
 #pragma unroll
         for (int r = W0; r < G::RN; r++) {
           P2 x = A[r][i];
-          if (i >= Q0) x = pfma(nw[r], G::KEEP ? vcol[i] : vc[h], x);
+          if (i >= Q0) x = pfma(nw[r], vcol[i], x);
           if (r >= R0) x = pfma(nv[r], wc[h], x);
           A[r][i] = x;
         }
@@ -557,7 +554,7 @@ __device__ __forceinline__ void reduce_phase(typename G::Row (&A)[G::RN], const 
       load_cols<G, Q0>(vb, b, vcol);
       load_rows<G, R0>(vb, a, vrow);
     }
-    two_sided<G, R0, Q0, false>(A, U.w(j), j, a, b, t, U.v(j), vcol, vrow);
+    two_sided<G, R0, Q0, false>(A, U.w(j), j, a, b, t, vcol, vrow);
     if constexpr (G::L > 32)
       z.template reflect<P * G::LA>(U, k, l, ((j - P * G::LA) * G::LB / 32 + G::L / 64) % (G::L / 32), t, U.v(j));
     tp = t;
@@ -599,7 +596,7 @@ __device__ __forceinline__ void back_phase(typename G::Row (&A)[G::RN], const Un
     load_cols<G, Q0>(vb, b, vcol);
     load_rows<G, R0>(vb, a, vrow);
     if constexpr (G::L <= 32) z.template reflect<P * G::LA>(U, k, l, 0, t, vb);
-    two_sided<G, R0, Q0, true>(A, U.w(j), j, a, b, t, vb, vcol, vrow);
+    two_sided<G, R0, Q0, true>(A, U.w(j), j, a, b, t, vcol, vrow);
     if constexpr (G::L > 32) z.template reflect<P * G::LA>(U, k, l, j % (G::L / 32), t, vb);
   }
 }
@@ -1017,8 +1014,8 @@ cudaError_t launch_g(cudaStream_t st, const EigArgs &a, const EigSplit &sp, int 
 }
 
 // calls f with the lane grid of an ensemble size
-// FP32: one warp holds four units up to k = 24, two up to 40, one up to 64; a
-// team of two warps a unit up to 80, of four above.
+// FP32: one warp holds four units up to k = 24, two up to 40, one up to 72; a
+// team of two warps a unit up to 112, of four above.
 template <class F>
 auto with_grid_f32(int k, F f) {
 #define LGPU_GRID(...) return f(Grid<float, __VA_ARGS__>())

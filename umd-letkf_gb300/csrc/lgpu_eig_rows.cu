@@ -859,7 +859,7 @@ static cudaError_t launch_tri_r(cudaStream_t st, const EigArgs &a, const EigRows
   return cudaGetLastError();
 }
 
-// the register-resident first stage with a two-warp team per unit (48 < k <= 64)
+// the register-resident first stage with a team of NW warps per unit (k above 48)
 template <int K, int NW>
 static cudaError_t launch_tri_t_k(cudaStream_t st, const EigArgs &a, const EigRows &sp, int u0, int nb) {
   const size_t smem = tri_t_smem<K, NW>();

@@ -1130,8 +1130,7 @@ __global__ void __launch_bounds__(SST) k_gram_segsum(TcArgs a) {
 }
 }  // namespace
 
-cudaError_t launch_gram_segsum(cudaStream_t st, const TcArgs &a, const int *active, int *launches) {
-  (void)active;
+cudaError_t launch_gram_segsum(cudaStream_t st, const TcArgs &a, int *launches) {
   if (a.nsegtiles <= 0) return cudaSuccess;
   const long long grid = (long long)a.nsegtiles * a.groups * ((a.nf + 31) / 32);
   if (grid > 0x7fffffffLL) return cudaErrorInvalidValue;

@@ -505,7 +505,7 @@ struct TcSegTile {
 };
 
 struct TcArgs {
-  int ntiles, groups, k, kp, npass, np, nf, ncol;
+  int ntiles, groups, k, npass, np, nf, ncol;
   const int *tile_cols;   // [ntiles][128] column index or -1
   const int *col2act;
   const ColPar *cp;
@@ -513,7 +513,6 @@ struct TcArgs {
   const TilePar *tp;         // per-tile cap parameters
   const unsigned char *rec;  // tile candidate streams (chunk records)
   const int *tile_off;       // [ntiles + 1] first chunk of each tile's stream
-  const int *tile_n;         // [ntiles] candidates of each tile
   const uint32_t *tile_mag;  // [ntiles][2] bits of a tile's largest mag.x and smallest positive mag.y
   bool f16;                  // FP16 operands (every tile's magnitudes within range)
   int cb;                    // bytes per chunk record (set by the launcher)
@@ -527,7 +526,6 @@ struct TcArgs {
   int nwork;
   int drain;              // chunks per drain interval
   int cull;               // 1: a warp skips the distance and localizer of four records none of its columns can reach
-  long long units;
   float *Gpart;              // [partial block][group][nf][128] (feature-major: coalesced drains)
   float *cnt;                // [count block][group][128][3]: kept, candidates, sum rho
   const TcSegTile *segtiles; // [nsegtiles] tiles with more than one segment
@@ -539,7 +537,7 @@ struct TcArgs {
 };
 // G += the partial Grams of segments 1..nseg-1; kept counts and diagnostics
 // from the per-segment counts
-cudaError_t launch_gram_segsum(cudaStream_t st, const TcArgs &a, const int *active, int *launches);
+cudaError_t launch_gram_segsum(cudaStream_t st, const TcArgs &a, int *launches);
 cudaError_t launch_tile_prep(cudaStream_t st, int ntiles, const int *tile_cols, const ColPar *cp, TilePar *tp,
                              int *launches);
 // tile candidate streams: counts (in all, and per warp's part of the window) +

@@ -40,24 +40,6 @@ __device__ __forceinline__ float bsum128(float v, float *red) {
   return red[0] + red[1] + red[2] + red[3];
 }
 
-__device__ __forceinline__ float bmax128(float v, float *red) {
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) red[wid] = v;
-  __syncthreads();
-  return fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
-}
-
-__device__ __forceinline__ float bmin128(float v, float *red) {
-  for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) red[wid] = v;
-  __syncthreads();
-  return fminf(fminf(red[0], red[1]), fminf(red[2], red[3]));
-}
-
 // Per-cell aggregates of the cell-sorted observation table: centroid
 // direction (sum of unit vectors) and count; sums of dep, dep^2, 1/err,
 // dep/err.  One thread per cell.

@@ -238,8 +238,6 @@ struct GemmArgs {
   const float *Zp;     // EPI 2: pre-activation [M][ldc]
 };
 
-// EPI 0: C = acc; 1: C = acc + bias (pre-activation), H = bf16(gelu(C));
-// 2: C = acc * gelu'(Zp); 3: C = acc + bias
 // one operand's slice (GK x W elements, element (kk, x) at dst[kk * pitch + x])
 // of a matrix with strides sx (along the tile) and sk; zero outside X x K.
 // 16 bytes at a time where the tile's direction is contiguous and aligned.
@@ -273,6 +271,8 @@ __device__ __forceinline__ void gemm_fetch(float *dst, const float *src, long lo
 }
 static_assert(GT == 128 && GK == 32, "a slice's k over the warps");
 
+// EPI 0: C = acc; 1: C = acc + bias (pre-activation), H = bf16(gelu(C));
+// 2: C = acc * gelu'(Zp); 3: C = acc + bias
 template <int EPI>
 __global__ void __launch_bounds__(GT) k_mlp_gemm(GemmArgs g) {
   extern __shared__ __align__(16) float gsm[];
