@@ -337,7 +337,9 @@ int lgpu_learn_init(lgpu_handle *h, const lgpu_learn_config *cfg);
 /* Runs an exact analysis (the AUTO / PLAIN / BATCHED_TC form in force; the
  * analysis result is the exact one) and adds training rows: network inputs
  * and residual targets (exact - interpolated) of a sample of the
- * non-lattice columns.  *rows receives the number of rows stored. */
+ * non-lattice columns.  A column without observations enters the rows with
+ * W = 0 and w-bar = 0 (in a learned analysis with W = I).  *rows receives the
+ * number of rows stored. */
 int lgpu_learn_collect(lgpu_handle *h, long long *rows);
 /* Standardises the stored rows (first call), runs `epochs` passes of Adam
  * with mini-batches of `batch` rows, then calibrates the gate threshold.

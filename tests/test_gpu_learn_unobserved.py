@@ -1,7 +1,7 @@
 """GPU: the learned form where lattice columns keep no observation.  Their
-transform is the identity (the update keeps their background), whatever the
-handle or the memory held before: an analysis and a training run have to be
-those of a handle that saw nothing else."""
+transform is the identity in an analysis (the update keeps their background) and
+zero in the training rows, whatever the handle or the memory held before: an
+analysis and a training run have to be those of a handle that saw nothing else."""
 import numpy as np
 import pytest
 

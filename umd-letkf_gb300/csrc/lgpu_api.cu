@@ -2125,8 +2125,10 @@ int lgpu_learn_collect(lgpu_handle *h, long long *rows) {
   if (n > 0) {
     cudaStream_t st = h->st;
     int launches = 0;
-    CK(lrn_identity(st, h->nunits, k, h->buf[B_NKEPT].as<int>(), h->buf[B_T].as<float>(), L->wbar_all.as<float>(),
-                    &launches),
+    // the training rows know a column without observations as W = 0, what a
+    // new handle's memory held: earlier training runs repeat to the bit
+    CK(lrn_unobserved(st, h->nunits, k, h->buf[B_NKEPT].as<int>(), 0.0f, h->buf[B_T].as<float>(),
+                      L->wbar_all.as<float>(), &launches),
        "transforms without observations");
     CK(L->ecols.ensure(4 * (size_t)std::max(n, std::max(1, h->nact))), "alloc");
     CK(cudaMemcpyAsync(L->ecols.p, sample.data(), 4 * (size_t)n, cudaMemcpyHostToDevice, st), "H2D sample");
@@ -2359,7 +2361,7 @@ static int learned_exact(lgpu_handle *h, const ObsSorted &os, int n, bool lattic
   EigSplit sp;
   int batch = 0;
   if ((rc = eig_scratch(h, n, ea, sp, batch)) != LGPU_OK) return rc;
-  CK(lrn_identity(st, n, k, ea.nkept, ea.T, ea.wbar, &launches), "transforms without observations");
+  CK(lrn_unobserved(st, n, k, ea.nkept, 1.0f, ea.T, ea.wbar, &launches), "transforms without observations");
   if (h->prec == LGPU_PREC_FP64) {
     CK(launch_eig64(st, ea, 0, &launches), "FP64 eigen kernel");
     return LGPU_OK;

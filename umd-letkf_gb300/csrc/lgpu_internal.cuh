@@ -696,8 +696,9 @@ cudaError_t lrn_obsfeat(cudaStream_t st, int nfine, const int *cols, const ColPa
                         const int *cell_start, const float4 *c0, const float4 *c1, const IndexGeom *geom,
                         float *feat, int *nkept, int *launches);
 cudaError_t lrn_interp(cudaStream_t st, const LrnInterpArgs &a, int *launches);
-// T = I and w-bar = 0 for the units of 0..n that keep no observation
-cudaError_t lrn_identity(cudaStream_t st, int n, int k, const int *nkept, float *T, float *wbar, int *launches);
+// T = diag I and w-bar = 0 for the units of 0..n that keep no observation
+cudaError_t lrn_unobserved(cudaStream_t st, int n, int k, const int *nkept, float diag, float *T, float *wbar,
+                           int *launches);
 // the same as BF16 rows in the network's tiled order (standardised inputs only)
 cudaError_t lrn_input(cudaStream_t st, const LrnInterpArgs &a, int k1, unsigned char *Xt, int *launches);
 cudaError_t lrn_apply(cudaStream_t st, const LrnApplyArgs &a, int *launches);

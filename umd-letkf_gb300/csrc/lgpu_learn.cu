@@ -421,12 +421,14 @@ __global__ void __launch_bounds__(FT) k_lrn_judge(int nj, const int *jcols, cons
 // A unit that keeps no observation has no transform (the update keeps its
 // background), and the transform kernels leave its rows as they were.  The
 // learned form interpolates between units, judges and trains on them: here
-// such a unit's transform is the identity, its mean weights zero.
-__global__ void __launch_bounds__(FT) k_lrn_identity(int n, int k, const int *nkept, float *T, float *wbar) {
+// such a unit's transform becomes `diag` times the identity, its mean weights
+// zero.
+__global__ void __launch_bounds__(FT) k_lrn_unobserved(int n, int k, const int *nkept, float diag, float *T,
+                                                       float *wbar) {
   const int kk = k * k;
   for (int u = blockIdx.x; u < n; u += gridDim.x) {
     if (nkept[u] > 0) continue;
-    for (int e = threadIdx.x; e < kk; e += FT) T[(size_t)u * kk + e] = e % (k + 1) == 0 ? 1.0f : 0.0f;
+    for (int e = threadIdx.x; e < kk; e += FT) T[(size_t)u * kk + e] = e % (k + 1) == 0 ? diag : 0.0f;
     for (int e = threadIdx.x; e < k; e += FT) wbar[(size_t)u * k + e] = 0.0f;
   }
 }
@@ -552,9 +554,10 @@ cudaError_t lrn_input(cudaStream_t st, const LrnInterpArgs &a, int k1, unsigned 
   return cudaGetLastError();
 }
 
-cudaError_t lrn_identity(cudaStream_t st, int n, int k, const int *nkept, float *T, float *wbar, int *launches) {
+cudaError_t lrn_unobserved(cudaStream_t st, int n, int k, const int *nkept, float diag, float *T, float *wbar,
+                           int *launches) {
   if (n <= 0) return cudaSuccess;
-  k_lrn_identity<<<std::min(n, 152 * 16), FT, 0, st>>>(n, k, nkept, T, wbar);
+  k_lrn_unobserved<<<std::min(n, 152 * 16), FT, 0, st>>>(n, k, nkept, diag, T, wbar);
   (*launches)++;
   return cudaGetLastError();
 }
