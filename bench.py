@@ -272,6 +272,7 @@ def gpu_arm(args, dist):
     stage = {k: statistics.mean(t[k] for t in tims)
              for k in ("index_ms", "prep_ms", "gram_ms", "tiles_ms", "eig_ms", "update_ms")}
     launches = tims[-1]["launches"]
+    operands = "TF32" if s.debug_gram_operands() == 32 else "FP16"   # of the batched Gram
     diag = s.get_diag()
     kept = float(np.sum(diag["lg_obscount"], dtype=np.float64))
     cand = float(np.sum(diag["obscount"], dtype=np.float64))
@@ -286,7 +287,7 @@ def gpu_arm(args, dist):
     eig_flop = 13.0 * k ** 3 * units
     upd_bytes = 2.0 * ncol * ns * k * 4 + 4.0 * ncol * ns * 4
     gram_kernel_ms = stage["gram_ms"] - stage["tiles_ms"]
-    # executed tensor work of the batched Gram: 3 FP16 products x 2 flop x
+    # executed tensor work of the batched Gram: 3 products x 2 flop x
     # M=128 x N=features per pass x K=16 per chunk that ran MMAs
     mma_flop = float(tims[-1]["mma_chunks"]) * 3 * 2 * 128 * tims[-1]["mma_n"] * 16
     stages = {
@@ -299,7 +300,7 @@ def gpu_arm(args, dist):
         "kept_pairs": kept, "candidate_pairs": cand}
     times = {"gram": gram_kernel_ms, "eig": stage["eig_ms"], "update": stage["update_ms"]}
     dom = max(times, key=times.get)
-    kname = {"gram": "k_gram_tc" if tims[-1]["variant"] == 2 else "k_gram", "eig": "k_eig", "update": "k_update"}[dom]
+    kname = {"gram": "k_gram_tc" if tims[-1]["variant"] == 2 else "k_gram", "eig": "k_transform", "update": "k_update"}[dom]
     traffic = read_traffic(kname) if args.workload == "c2" else None   # the committed captures are of C2
     if dom == "update":
         ach = upd_bytes / (stage["update_ms"] * 1e-3) / 1e9
@@ -312,16 +313,17 @@ def gpu_arm(args, dist):
         roof = {"kernel": kname, "bound": "tensor", "achieved": ach, "peak": bf16, "unit": "TFLOP/s",
                 "frac": ach / bf16, "traffic": traffic,
                 "peak_source": peak_kind + " bf16_tflops (burst)",
-                "note": ("FP16 three-term split on tcgen05 (TF32 where the magnitudes need it): the split triples the "
-                         "MMAs, so bf16/3 bounds this kernel's algorithmic rate" if dom == "gram" else
+                "note": ("%s three-term split on tcgen05: the split triples the MMAs, so bf16/%d bounds this kernel's "
+                         "algorithmic rate" % (operands, 3 if operands == "FP16" else 6) if dom == "gram" else
                          "FP32 on the CUDA cores (no tensor work); nominal FP32 SIMT peak %.1f TFLOP/s, "
                          "frac of it %.4f" % (simt, ach / simt))}
     if dom == "gram" and mma_flop > 0:
         ex = mma_flop / (gram_kernel_ms * 1e-3) / 1e12
-        roof["tensor_executed"] = {"tflops": ex, "peak_f16_tflops": bf16, "frac": ex / bf16,
-                                   "note": "MMA work issued (3 FP16 products per FP32 product, zero weights "
-                                           "and padding included) over the Gram kernels' time; FP16 dense "
-                                           "peak taken as the measured bf16 peak"}
+        peak = bf16 if operands == "FP16" else bf16 / 2
+        roof["tensor_executed"] = {"tflops": ex, "operands": operands, "peak_tflops": peak, "frac": ex / peak,
+                                   "note": "MMA work issued (3 products per FP32 product, zero weights and padding "
+                                           "included) over the Gram kernels' time; dense peak taken as the measured "
+                                           "bf16 peak (half of it with TF32)"}
     variant = {1: "plain", 2: "batched_tc"}.get(tims[-1]["variant"], "?")
     plain = None
     if variant != "plain" and not args.no_plain:

@@ -130,8 +130,8 @@ typedef struct lgpu_obs {
  * library's stream. */
 typedef struct lgpu_timings {
   float total_ms;    /* whole run */
-  float index_ms;    /* observation preparation + spatial index */
-  float prep_ms;     /* per-column localisation parameters */
+  float index_ms;    /* observation preparation, spatial index, per-column localisation parameters, tile caps */
+  float prep_ms;     /* wait for a bound state's mean and spread, then loc_ocean's column parameters that need it; else about 0 */
   float gram_ms;     /* search + localisation + Gram/RHS */
   float eig_ms;      /* eigensolve + transform */
   float update_ms;   /* X_b * T + relaxation/inflation/bounds epilogue */
@@ -169,11 +169,12 @@ typedef struct lgpu_timings {
 #define LGPU_VARIANT_PLAIN 1
 #define LGPU_VARIANT_BATCHED_TC 2
 /* LEARNED (after lgpu_learn_init and lgpu_learn_train; loc_novrt only): exact
- * solves (PLAIN Gram) on the columns of a coarse lattice, a random judge
- * sample and the columns the confidence gate sends back; every other column
- * gets the bilinear interpolation of the coarse (W, w-bar) corrected by the
- * learned network.  The update and its epilogue are those of the exact
- * forms.  No counterpart in the reference, which solves every column
+ * solves on the columns of a coarse lattice (PLAIN or BATCHED_TC Gram, whichever
+ * the first analysis measures faster), a random judge sample and the columns
+ * the confidence gate sends back (PLAIN Gram); every other column gets the
+ * bilinear interpolation of the coarse (W, w-bar) corrected by the learned
+ * network.  The update and its epilogue are those of the exact forms.  No
+ * counterpart in the reference, which solves every column
  * (src/letkf_solver.F90:203-384). */
 #define LGPU_VARIANT_LEARNED 3
 
