@@ -93,7 +93,12 @@ static void chunk_bounds(int ncol, int n, int c, int *c0, int *c1) {
   }
 }
 constexpr int kSegChunks = 256;   // batched Gram: chunks of 16 observations per CTA at most
-constexpr int kMinSegChunks = 24, kSegsPerSM = 3;   // ... and where the chunks are few
+// ... and where the chunks are few.  Both lie on a plateau (Gram us at 1, 2, 3,
+// 4, 6 segments an SM: vtgc 90 x 45 x 10, k = 20 284, 273, 270, 282, 294; ocean
+// 144 x 72, k = 40 442, 450, 442, 470, 496; 360 x 180, k = 32 672, 673, 682,
+// 686, 714; at 12, 16, 24, 32, 48 chunks at least: 144 x 72, k = 40 330, 329,
+// 331, 322, 326; runs of one setting differ by 6).
+constexpr int kMinSegChunks = 24, kSegsPerSM = 3;
 // batched Gram: chunks per tensor-core accumulation (drained to a partial
 // block).  Every MMA cuts its sum off at the accumulator's last bit, so a Gram's
 // error grows with the chunks in one accumulation, and a drain costs a block's
